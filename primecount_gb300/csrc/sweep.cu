@@ -297,20 +297,25 @@ __global__ void k_factor_zero_small(T* __restrict__ out, int64_t size, int64_t l
 }
 
 // ================================================================ the sweep
+// A level of the batch: its leaf records ...
 struct LevelP {
   union {
     int64_t lo;       // leaf range (lo, hi] while the levels are set up ...
     uint64_t xlo;     // ... then the low word of x / p (flag 16: the high word is not 0)
   };
   int64_t hi;         // factor indices (family 1) or prime indices (family 2)
-  uint64_t jlo;       // first 30-coprime rank of the cross-off co-factors
-  uint32_t jn;        // number of cross-off co-factors
-  uint32_t prime;
   uint32_t thr;       // factor-table threshold (family 1)
-  uint32_t flags;     // 1: leaves, 2: family 2, 4: small prime (pattern cross-off), 8: formula count, 16: x / p >= 2^64
-  int32_t level;      // b
-  uint32_t fcount;    // flag 8: numbers of the segment removed at this level (PiTable formula)
+  uint32_t flags;     // 1: leaves, 2: family 2, 4: small prime (pattern cross-off), 16: x / p >= 2^64,
+                      // 32: x / p < 2^64 and every divisor m < 2^31
 };
+// ... and its multiples in the segment
+struct __align__(16) LevelM {
+  uint32_t first;     // offset of the first multiple of p (NO_FIRST: none); flag 4: pattern phase of the first word
+  uint32_t jn8;       // 8 * (# multiples) + wheel index of the first co-factor
+  uint32_t prime;
+  uint32_t pinv;      // floor((2^32 - 1) / p)
+};
+#define NO_FIRST 0x7FFFFFFFu
 
 // One problem of a sweep: D (gourdon = 1), S2_hard (0) or the special leaves
 // of phi(x, a) (2).  A sweep runs the segments of one or of many problems
@@ -332,7 +337,6 @@ struct SweepArgs {
   const SweepQ* qs;      // the problems, by item0 ascending
   int32_t nq;
   int32_t words;         // bitmap words per CTA (max segment = words * 240 numbers)
-  int32_t rec_cap;       // leaf records per chunk
   int32_t wave_len;
   int64_t wave_first;    // first work item of the wave
   const int64_t* rowoff; // [wave_len]: first cell of the item's row in cnt / smu
@@ -388,42 +392,57 @@ __device__ __forceinline__ uint64_t div_xp(uint64_t xlo, uint64_t xhi, uint64_t 
   return (uint64_t) (xp / m);
 }
 
-// exclusive prefix of the chunk counts by the first SW warps (nch / SW chunks
-// per warp, a multiple of 64; ccount and pref 16-byte aligned); the other
-// warps only meet the two barriers
+// Exclusive prefix of the chunk counts, one value per 4 chunks (32 words), n4
+// of them, by the first SCAN_WARPS warps (ccount 16-byte aligned).  scan_part
+// leaves each warp's part relative to its start and the parts' sums in wtmp;
+// scan_chunks, called by the whole block, the whole prefix.
 #define SCAN_WARPS 4
-__device__ __forceinline__ void scan_chunks(const uint32_t* __restrict__ ccount, uint32_t* __restrict__ pref, int nch,
-                                            uint32_t* wtmp)
+// values per warp
+__device__ __forceinline__ int scan_per(int n4) { return 32 * ((n4 + 32 * SCAN_WARPS - 1) / (32 * SCAN_WARPS)); }
+
+__device__ __forceinline__ void scan_part(const uint32_t* __restrict__ ccount, uint32_t* __restrict__ pref, int n4,
+                                          uint32_t* wtmp)
 {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int cpl = nch / (32 * SCAN_WARPS);             // chunks per lane, a multiple of 2
-  const int my = (warp * 32 + lane) * cpl;
-  uint32_t sum = 0, incl = 0;
-  if (warp < SCAN_WARPS) {
-    for (int i = 0; i < cpl; i += 2) {
-      const uint2 v = *(const uint2*) (ccount + my + i);
-      sum += v.x + v.y;
-    }
-    incl = sum;
-    for (int d = 1; d < 32; d <<= 1) {
-      const uint32_t t = __shfl_up_sync(0xffffffffu, incl, d);
-      if (lane >= d) incl += t;
-    }
-    if (lane == 31) wtmp[warp] = incl;
+  const int ql = scan_per(n4) / 32;                    // values per lane
+  const int i0 = min(n4, (warp * 32 + lane) * ql), i1 = min(n4, i0 + ql);
+  uint32_t sum = 0;
+  for (int i = i0; i < i1; i++) {
+    const uint4 v = ((const uint4*) ccount)[i];
+    pref[i] = sum;
+    sum += v.x + v.y + v.z + v.w;
+  }
+  uint32_t incl = sum;
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += t;
+  }
+  if (lane == 31) wtmp[warp] = incl;
+  for (int i = i0; i < i1; i++) pref[i] += incl - sum;
+}
+
+__device__ __forceinline__ void scan_chunks(const uint32_t* __restrict__ ccount, uint32_t* __restrict__ pref, int n4,
+                                            uint32_t* wtmp)
+{
+  const int warp = threadIdx.x >> 5;
+  if (warp < SCAN_WARPS) scan_part(ccount, pref, n4, wtmp);
+  __syncthreads();
+  if (warp < SCAN_WARPS && warp > 0) {
+    const int per = scan_per(n4);
+    uint32_t base = 0;
+    for (int w = 0; w < warp; w++) base += wtmp[w];
+    for (int i = warp * per + (threadIdx.x & 31); i < min(n4, (warp + 1) * per); i += 32) pref[i] += base;
   }
   __syncthreads();
-  if (warp < SCAN_WARPS) {
-    uint32_t run = incl - sum;
-    for (int w = 0; w < warp; w++) run += wtmp[w];
-    for (int i = 0; i < cpl; i += 2) {
-      const uint2 v = *(const uint2*) (ccount + my + i);
-      uint2 o;
-      o.x = run; run += v.x;
-      o.y = run; run += v.y;
-      *(uint2*) (pref + my + i) = o;
-    }
-  }
-  __syncthreads();
+}
+
+// the count before chunk c: the prefix of its 4 chunks and the chunks before it
+__device__ __forceinline__ uint32_t before_chunk(const uint32_t* __restrict__ ccount, const uint32_t* __restrict__ pref,
+                                                 uint32_t c)
+{
+  const uint4 v = ((const uint4*) ccount)[c >> 2];
+  const uint32_t k = c & 3;
+  return pref[c >> 2] + (k > 0 ? v.x : 0u) + (k > 1 ? v.y : 0u) + (k > 2 ? v.z : 0u);
 }
 
 // mask_le(r) from a shared table of the counts of wheel residues <= r
@@ -439,8 +458,8 @@ static __device__ __forceinline__ int64_t dpi_t(const uint64_t* __restrict__ pt,
 
 // # unsieved numbers in [low, low + off]: the chunk prefix plus the popcounts
 // of the chunk's words up to the word of off, its 8 words read at once
-__device__ __forceinline__ uint32_t query(const uint64_t* __restrict__ bits, const uint32_t* __restrict__ pref,
-                                          const uint8_t* nbt, uint32_t off)
+__device__ __forceinline__ uint32_t query(const uint64_t* __restrict__ bits, const uint32_t* __restrict__ ccount,
+                                          const uint32_t* __restrict__ pref, const uint8_t* nbt, uint32_t off)
 {
   const uint32_t w = off / 240;
   const uint32_t r = off - w * 240;
@@ -452,7 +471,7 @@ __device__ __forceinline__ uint32_t query(const uint64_t* __restrict__ bits, con
   auto part = [&](uint32_t i, uint64_t v) -> uint32_t {
     return (uint32_t) __popcll(i < k ? v : (i == k ? (v & mk) : 0ull));
   };
-  return pref[c] + part(0, w01.x) + part(1, w01.y) + part(2, w23.x) + part(3, w23.y) + part(4, w45.x) +
+  return before_chunk(ccount, pref, c) + part(0, w01.x) + part(1, w01.y) + part(2, w23.x) + part(3, w23.y) + part(4, w45.x) +
          part(5, w45.y) + part(6, w67.x) + part(7, w67.y);
 }
 
@@ -478,148 +497,218 @@ __device__ __forceinline__ uint32_t chunk_sum_below(const uint32_t* __restrict__
   return part;
 }
 
-// Cross off the number at offset w * 240 + rr of the segment: a 32-bit atomic
-// on the half of the 64-bit word that holds its bit (bits 0-31 of a word are
-// the lower half), true when the number was still unsieved
-__device__ __forceinline__ bool cross_off(uint64_t* bits, const uint8_t* bt, uint32_t w, uint32_t rr)
+// Shared-memory atomics under a predicate, without a branch: several stay in
+// flight together.  and_if: clears bit m of the word at a, returns the bit as
+// it was (m when on is false).
+static __device__ __forceinline__ uint32_t and_if(bool on, uint32_t* a, uint32_t m)
 {
-  const uint32_t bi = bt[rr];
-  const uint32_t m = 1u << (bi & 31);
-  return (atomicAnd((uint32_t*) bits + 2 * w + (bi >> 5), ~m) & m) != 0;
+  uint32_t old = m;
+  asm volatile("{ .reg .pred p; setp.ne.u32 p, %1, 0; @p atom.shared.and.b32 %0, [%2], %3; }"
+               : "+r"(old)
+               : "r"((uint32_t) on), "r"((uint32_t) __cvta_generic_to_shared(a)), "r"(~m)
+               : "memory");
+  return old & m;
 }
 
-// Cross off the multiples of the levels [l0, l1) at once (their co-factor
-// counts prefixed in hoff): with few multiples per level a warp takes each
-// level and its lanes the level's multiples; otherwise the multiples are
-// spread flat over the threads, each finding its level by a binary search.
-// Different levels can share a half-word, so the clears are atomic.
-template <int NT>
-__device__ __forceinline__ void cross_off_levels(uint64_t* bits, uint32_t* ccount, const LevelP* lp,
-                                                 const int64_t* hoff, int l0, int l1, uint64_t low,
-                                                 const uint8_t* bt)
+static __device__ __forceinline__ void dec_if(bool on, uint32_t* a)
 {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t h0 = hoff[l0], h1 = hoff[l1];
-  if (h1 - h0 <= 64 * (int64_t) (l1 - l0)) {
-    for (int lv = l0 + warp; lv < l1; lv += NT / 32) {
-      const uint64_t prime = lp[lv].prime, jlo = lp[lv].jlo;
-      const uint32_t jn = (uint32_t) (hoff[lv + 1] - hoff[lv]);
-      for (uint32_t j = lane; j < jn; j += 32) {
-        const uint64_t jj = jlo + j;
-        const uint64_t q = 30 * (jj >> 3) + woff((uint32_t) (jj & 7));
-        const uint32_t off = (uint32_t) (prime * q - low);
-        const uint32_t w = off / 240, rr = off - w * 240;
-        if (cross_off(bits, bt, w, rr)) atomicSub(&ccount[w >> 3], 1u);
-      }
-    }
-    return;
-  }
-  for (int64_t h = h0 + tid; h < h1; h += NT) {
-    int lo = l0, hi = l1 - 1;       // last level with hoff <= h
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (hoff[mid] <= h) lo = mid; else hi = mid - 1;
-    }
-    const LevelP& Q = lp[lo];
-    const uint64_t jj = Q.jlo + (uint64_t) (h - hoff[lo]);
-    const uint64_t q = 30 * (jj >> 3) + woff((uint32_t) (jj & 7));
-    const uint32_t off = (uint32_t) ((uint64_t) Q.prime * q - low);
-    const uint32_t w = off / 240, rr = off - w * 240;
-    if (cross_off(bits, bt, w, rr)) atomicSub(&ccount[w >> 3], 1u);
-  }
+  asm volatile("{ .reg .pred p; setp.ne.u32 p, %0, 0; @p red.shared.add.u32 [%1], %2; }"
+               :
+               : "r"((uint32_t) on), "r"((uint32_t) __cvta_generic_to_shared(a)), "r"(0xFFFFFFFFu)
+               : "memory");
 }
 
-// Record of one table entry: the offset of the leaf in the segment, bit 30 =
-// negative sign, or REC_NONE when the factor-table filter rejects the entry.
+// Record of one table entry: the offset of the leaf in the segment (low OB
+// bits), the level's index in its batch, bit 31 = negative sign; REC_NONE when
+// the factor-table filter rejects the entry.
 #define REC_NONE 0xFFFFFFFFu
 // table entries per thread and round of the record phase
 #define PA_UNROLL 8
-// levels (and groups of levels) with at most this many record slots in a
-// window are answered without a chunk prefix scan
-#ifndef SMALL_QUERIES
+// a level answered alone with at most this many record slots in a window
+// goes without a chunk prefix scan
 #define SMALL_QUERIES 32
-#endif
-// consecutive levels with p^3 >= high answered together (see k_sweep)
-#define GROUP_MAX 64
+// factor-table indices below this one are numbers below 2^31
+#define NARROW_INDEX 446000000ll
+// a level answered alone with more records than this uses prefix counts per
+// word where they fit (see k_sweep)
+#define WORD_RECORDS 1024
+// levels answered together at most (see k_sweep)
+#define GROUP_MAX 256
+// a level with more records than this is answered alone
+#define SOLO_RECORDS 512
+// a group holds at most this many records, and levels times records; with
+// more than LANE_RECORDS in at most LANE_LEVELS levels, a thread per record
+#define GROUP_RECORDS 1024
+#define GROUP_WORK 32768
+#define LANE_RECORDS 256
+#define LANE_LEVELS 64
 
-// exclusive block scan of three int64 values per thread into out[NT + 1] arrays
-template <int NT>
-__device__ __forceinline__ void block_scan3(long long v0, long long v1, long long v2, int64_t* o0, int64_t* o1,
-                                            int64_t* o2, long long (*wt)[3])
+// exclusive block scan of two values of the first LB threads into out[LB + 1] arrays
+template <int LB>
+__device__ __forceinline__ void block_scan2(long long v0, uint32_t v1, int64_t* o0, uint32_t* o1, long long (*wt)[2])
 {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  long long i0 = v0, i1 = v1, i2 = v2;
+  long long i0 = v0;
+  uint32_t i1 = v1;
   for (int d = 1; d < 32; d <<= 1) {
-    long long t0 = __shfl_up_sync(0xffffffffu, i0, d);
-    long long t1 = __shfl_up_sync(0xffffffffu, i1, d);
-    long long t2 = __shfl_up_sync(0xffffffffu, i2, d);
-    if (lane >= d) { i0 += t0; i1 += t1; i2 += t2; }
+    const long long t0 = __shfl_up_sync(0xffffffffu, i0, d);
+    const uint32_t t1 = __shfl_up_sync(0xffffffffu, i1, d);
+    if (lane >= d) { i0 += t0; i1 += t1; }
   }
-  if (lane == 31) { wt[warp][0] = i0; wt[warp][1] = i1; wt[warp][2] = i2; }
+  if (lane == 31) { wt[warp][0] = i0; wt[warp][1] = i1; }
   __syncthreads();
-  long long e0 = i0 - v0, e1 = i1 - v1, e2 = i2 - v2;
-  for (int w = 0; w < warp; w++) { e0 += wt[w][0]; e1 += wt[w][1]; e2 += wt[w][2]; }
-  o0[tid] = e0; o1[tid] = e1; o2[tid] = e2;
-  if (tid == NT - 1) { o0[NT] = e0 + v0; o1[NT] = e1 + v1; o2[NT] = e2 + v2; }
+  long long e0 = i0 - v0;
+  uint32_t e1 = i1 - v1;
+  for (int w = 0; w < warp; w++) { e0 += wt[w][0]; e1 += (uint32_t) wt[w][1]; }
+  if (tid < LB) { o0[tid] = e0; o1[tid] = e1; }
+  if (tid == LB - 1) { o0[LB] = e0 + v0; o1[LB] = e1 + v1; }
 }
 
-// the level j in [l0, l1) of flat record pos: loff[j] <= pos < loff[j + 1]
-// (loff[l0] <= pos < loff[l1]), by binary search
-static __device__ __forceinline__ int level_of(const int64_t* loff, int l0, int l1, int64_t pos)
+// floor(t / p) for t < 2^31 from v = floor((2^32 - 1) / p)
+static __device__ __forceinline__ uint32_t div_small(uint32_t t, uint32_t p, uint32_t v)
 {
-  int j = l0;
-  for (int n = l1 - l0; n > 1;) {
-    const int half = n >> 1;
-    if (loff[j + half] <= pos) j += half;
-    n -= half;
-  }
-  return j;
+  uint32_t e = __umulhi(t, v);
+  if (t - e * p >= p) e++;
+  return e;
 }
+
+// Number of a level's multiples at offsets <= the first multiple + t, with
+// e = floor(t / p): the co-factors from the first one (wheel index jl) up to
+// e further, nb[r] = # wheel residues <= r.
+static __device__ __forceinline__ uint32_t wheel_rank(uint32_t e, uint32_t jl, const uint8_t* nb)
+{
+  const uint32_t s = woff(jl) + e;
+  const uint32_t t = s / 30;
+  return 8 * t + nb[s - 30 * t] - jl;
+}
+
+// Removed numbers of a group's level at offsets <= off: the rank of off among
+// the level's multiples, then the prefix of the removal masks (mp = the
+// level's first mask word; pre = prefix counts of all mask words).
+static __device__ __forceinline__ uint32_t removed_le(const LevelM& Q, uint32_t off, uint32_t mp, const uint32_t* mk,
+                                                      const uint16_t* pre, const uint8_t* nb)
+{
+  const int32_t t = (int32_t) (off - Q.first);
+  if (t < 0) return 0;
+  const uint32_t d = wheel_rank(div_small((uint32_t) t, Q.prime, Q.pinv), Q.jn8 & 7, nb);
+  const uint32_t w = mp + (d >> 5);
+  return (uint32_t) pre[w] - pre[mp] + (uint32_t) __popc(mk[w] & ((1u << (d & 31)) - 1u));
+}
+
+// k_sweep: one CTA per segment at a time, the levels in order.
+//
+// A level with p >= 64 and at most SOLO_RECORDS records is answered in a
+// group of up to GROUP_MAX consecutive levels, all records against one bitmap
+// state:
+//   1. every level's multiples still unsieved before the group, as 32-bit
+//      masks (lane l of a warp reads the multiples l, l + 32, ...; those are
+//      4 wheel turns = p half-words apart with the same bit); the bitmap is
+//      only read, the mask words are spread evenly over the warps;
+//   2. the masks' numbers are cleared.  A number in the masks of two levels
+//      (a multiple of both primes) is cleared by one of them; the other finds
+//      it gone and takes it out of all masks but the lowest level's;
+//   3. a prefix of the mask popcounts and of the chunk counts;
+//   4. a record n of level l: the numbers <= n left after the group plus
+//      those that the group's levels from l on removed at or below n.
+// Three barriers per group instead of two to four per level: what bounds the
+// sparse segments is the latency of the chain of levels (2 CTAs of 8 warps
+// per SM, issue active 44 %), so levels are taken together as long as the
+// work that grows with the group stays small.  The collisions of step 2 grow
+// with (levels / p)^2 times the segment's length and the corrections of step 4
+// with levels times records: GROUP_WORK and the p / 32 levels of a full
+// segment are where longer groups stop gaining (p / 24 and p / 48: 0.5-1 %
+// slower).  A level with more than SOLO_RECORDS records fills the block by
+// itself and needs no corrections (256: the same, 1024: 2-8 % slower).
+// Measured on a GB300: D(1e20) 1323 -> 947 ms, D(1e18) 89.2 -> 58.4 ms,
+// D(1e15) 3.38 -> 2.89 ms, S2_hard(1e17) 42.0 -> 27.9 ms.
+// levels per batch (a thread each)
+constexpr int sweep_batch(int nt) { return nt < 256 ? nt : 256; }
+
+// leaf records per window; removal mask words of a group (at least the
+// 2 words / 67 + 1 of the longest level, p = 67, up to 21 000 words);
+// collisions of a group kept for the end of its clears
+#define REC_CAP 3584
+#define MASK_WORDS 640
+#define COLLISIONS 512
+
+// dynamic shared memory of k_sweep: byte offsets; then the chunk counts
+// (4 bytes per 8 words) and their prefix (4 bytes per 32 words)
+struct SweepLayout { int pat, loff, lp, lm, wofs, rec, masks, mpre, clist, cop, bits; };
+constexpr SweepLayout sweep_layout(int nt)
+{
+  const int lb = sweep_batch(nt);
+  SweepLayout y{};
+  y.pat = 0;
+  y.lm = (y.pat + PAT_WORDS * 8 + 15) / 16 * 16;
+  y.loff = y.lm + lb * (int) sizeof(LevelM);
+  y.lp = y.loff + (lb + 1) * 8;
+  y.wofs = y.lp + lb * (int) sizeof(LevelP);
+  y.rec = y.wofs + (lb + 1) * 4;
+  y.masks = y.rec + REC_CAP * 4;
+  y.clist = y.masks + 2 * (MASK_WORDS + 1) * 4;
+  y.mpre = y.clist + COLLISIONS * 4;
+  y.cop = y.mpre + (MASK_WORDS + 2) * 2;
+  y.bits = (y.cop + 480 * 2 + 15) / 16 * 16;
+  return y;
+}
+static size_t sweep_smem(int words, int nt) { return (size_t) sweep_layout(nt).bits + (size_t) words * 8 + (size_t) (words / 8) * 5; }
 
 template <typename FT, int NT>
 __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k_sweep(const SweepArgs A)
 {
+  constexpr int NW = NT / 32;
+  constexpr int LB = sweep_batch(NT);                  // levels per batch
+  constexpr int OB = 23;                               // offset bits of a record
+  constexpr uint32_t OM = (1u << OB) - 1u;
+  // the arrays of fixed size first, at constant offsets
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int nch = A.words >> 3;
-  uint64_t* bits = (uint64_t*) smem_raw;
-  uint64_t* pat = bits + A.words;                      // wheel patterns of the primes 7..61
-  int64_t* loff = (int64_t*) (pat + PAT_WORDS);        // record offsets of the batch levels
-  int64_t* hoff = loff + (NT + 1);                     // cross-off co-factor offsets
-  int64_t* rpre = hoff + (NT + 1);                     // prefix of the formula counts
-  uint32_t* ccount = (uint32_t*) (((uintptr_t) (rpre + (NT + 1)) + 15) & ~(uintptr_t) 15);  // 16-byte aligned
-  uint32_t* pref = ccount + nch;
-  LevelP* lp = (LevelP*) (pref + nch);
-  uint32_t* rec = (uint32_t*) (lp + NT);
-  uint16_t* runend = (uint16_t*) (rec + A.rec_cap);    // end of the run of leafless levels from i
-  uint16_t* cop = runend + NT;
-  uint32_t* s_pc = (uint32_t*) (((uintptr_t) (cop + 480) + 3) & ~(uintptr_t) 3);   // pi(q_lo - 1) of flag-8 levels
+  constexpr SweepLayout Y = sweep_layout(NT);
+  uint64_t* const pat = (uint64_t*) (smem_raw + Y.pat);        // wheel patterns of the primes 7..61
+  int64_t* const loff = (int64_t*) (smem_raw + Y.loff);        // record offsets of the batch levels
+  LevelP* const lp = (LevelP*) (smem_raw + Y.lp);
+  LevelM* const lm = (LevelM*) (smem_raw + Y.lm);
+  uint32_t* const wofs = (uint32_t*) (smem_raw + Y.wofs);      // mask word offsets of the batch levels
+  uint32_t* const rec = (uint32_t*) (smem_raw + Y.rec);        // leaf records of a window
+  uint32_t* const masks = (uint32_t*) (smem_raw + Y.masks);    // removal masks of a group, two buffers
+  uint16_t* const mpre = (uint16_t*) (smem_raw + Y.mpre);      // their prefix counts
+  uint32_t* const clist = (uint32_t*) (smem_raw + Y.clist);    // numbers that two levels of a group share
+  uint16_t* const cop = (uint16_t*) (smem_raw + Y.cop);
+  uint64_t* const bits = (uint64_t*) (smem_raw + Y.bits);
+  uint32_t* const hw = (uint32_t*) bits;                       // half-words: 120 numbers each
+  const int nch_all = A.words >> 3;
+  uint32_t* const ccount = (uint32_t*) (bits + A.words);       // numbers left per 8-word chunk
+  uint32_t* const pref = ccount + nch_all;                     // their prefix, per 4 chunks
 
   __shared__ int s_ws;
   __shared__ uint32_t wtmp[32];
-  __shared__ int s_gsmu[GROUP_MAX];                    // signed leaf counts of a level group
-  __shared__ uint64_t s_gmag[GROUP_MAX];               // reciprocals of the group's primes
+  __shared__ int s_gsmu[2][LB];                        // signed leaf counts of a group's levels, by group parity
   __shared__ int s_smu;
+  __shared__ int s_ncoll;
   __shared__ int s_ncomp[2];                           // accepted records of a compacted window, by window parity
   __shared__ int s_stop;
   __shared__ uint32_t s_rem[3];
   __shared__ uint32_t s_total;
   __shared__ uint64_t s_mlow, s_mhigh;                 // floor((2^64 - 1) / d) of low1 and high
-  __shared__ long long wt3[32][3];
-  __shared__ int s_brk[32];
-  __shared__ long long s_red[NT / 32];
+  __shared__ long long wt2[32][2];
+  __shared__ uint8_t s_gend[LB];                       // [l]: levels of a group that starts at level l, less 1
+  __shared__ uint32_t s_solo[LB / 32];                      // levels of the batch answered alone
+  __shared__ long long s_red[NW];
   __shared__ unsigned long long s_ctr[5];
 
   __shared__ SweepQ s_q;                               // the problem of the current segment
   __shared__ uint8_t s_nb[240];                        // # wheel residues <= r, r in [0, 240)
-  __shared__ uint8_t s_bitt[240];                      // bit of residue r in its 64-bit word (r coprime to 30)
+  __shared__ uint8_t s_bit[120];                       // bit of residue r in its half-word (r coprime to 30)
+  __shared__ uint8_t s_delta[256];                     // [jl][lane]: co-factor jl + lane less co-factor jl
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int cap = A.rec_cap;
   const FT* __restrict__ factor = (const FT*) A.factor;
   for (int i = tid; i < 480; i += NT) cop[i] = A.coprime[i];
-  for (int i = tid; i < 240; i += NT) {
-    s_nb[i] = (uint8_t) ((i / 30) * 8 + cnt8((uint32_t) (i % 30)));
-    s_bitt[i] = (uint8_t) bit_of((uint32_t) i);
+  for (int i = tid; i < 240; i += NT) s_nb[i] = (uint8_t) ((i / 30) * 8 + cnt8((uint32_t) (i % 30)));
+  for (int i = tid; i < 120; i += NT) s_bit[i] = (uint8_t) bit_of((uint32_t) i);
+  for (int i = tid; i < 256; i += NT) {
+    const uint32_t jl = (uint32_t) i >> 5, j = jl + ((uint32_t) i & 31);
+    s_delta[i] = (uint8_t) (30 * (j >> 3) + woff(j & 7) - woff(jl));
   }
+  for (int i = tid; i < 2 * LB; i += NT) s_gsmu[i / LB][i % LB] = 0;
   // wheel patterns: word r of prime p keeps the numbers 240 r + {1,7,..,29}
   // (mod 240 p) that p does not divide
   for (int i = tid; i < PAT_WORDS; i += NT) {
@@ -635,6 +724,7 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
     pat[i] = w;
   }
   if (tid < 5) s_ctr[tid] = 0;
+  int gpar = 0;                                        // group parity
 
   for (;;) {
     __syncthreads();
@@ -684,8 +774,11 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
 
     // fill the segment: every number coprime to 30 in [low, high)
     const uint32_t span = (uint32_t) (high - low);
+    const float gscale = 44.0f * rsqrtf((float) span);   // levels of a group per p: p / 32 in a segment of 2e6 numbers
     const int wused = (int) ((span + 239) / 240);
-    for (int w = tid; w < A.words; w += NT) {
+    // the chunks that the segment uses, in whole groups of 4
+    const int n4 = (wused + 31) >> 5, nch = 4 * n4;
+    for (int w = tid; w < 8 * nch; w += NT) {
       uint64_t v = w < wused ? ~0ull : 0ull;
       if (w == wused - 1) v &= mask_le((span - 1) % 240);
       bits[w] = v;
@@ -695,6 +788,7 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
       s_mlow = UINT64_MAX / (uint64_t) low1;
       s_mhigh = UINT64_MAX / (uint64_t) high;
       s_ncomp[0] = s_ncomp[1] = 0;
+      s_ncoll = 0;
     }
     __syncthreads();
     {
@@ -711,54 +805,51 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
     __syncthreads();
     uint32_t total = s_total;
     bool dirty = true;
+    // prefix counts per word of the segment, in the bitmap's unused tail: a
+    // query then takes one word instead of the 8 of its chunk
+    const int nchu = (wused + 7) >> 3;
+    uint32_t* const wpre = (uint32_t*) (bits + 8 * nchu);
+    const bool wp_fits = 12 * nchu <= nch_all * 8;
+    bool wp_ok = false;
     long long lsum = 0;
     unsigned long long nleaves = 0, ntwo = 0, nentries = 0;
+    unsigned alone_n = 0;  // levels answered alone so far (rotates s_rem)
     unsigned win = 0;      // windows of the segment so far (parity selects the compaction counter)
 
-    for (int b0 = 1; b0 <= Bs; b0 += NT) {
-      // ---- per-level parameters of levels b0 .. b0+NT-1, one thread each
+    for (int b0 = 1; b0 <= Bs; b0 += LB) {
+      // ---- per-level parameters of levels b0 .. b0+LB-1, one thread each
       int64_t E = 0;
-      uint32_t fcnt = 0;
+      uint32_t mwords = 0;
       {
         const int b = b0 + tid;
         LevelP P;
-        P.lo = P.hi = 0; P.jlo = 0; P.jn = 0; P.prime = 0; P.thr = 0; P.flags = 0; P.level = b; P.fcount = 0;
-        uint32_t pcv = 0;
+        LevelM M;
+        P.lo = P.hi = 0; P.thr = 0; P.flags = 0;
+        M.first = NO_FIRST; M.jn8 = 0; M.prime = 2; M.pinv = 0x7FFFFFFFu;
         uint32_t ncross = 0;   // multiples of p_b in the segment (work counter)
-        if (b <= Bs) {
+        if (tid < LB && b <= Bs) {
           const uint64_t p = A.primes[b];
           const uint64_t pm = A.pmagic[b];     // floor((2^64 - 1) / p): the divisions by p below
-          P.prime = (uint32_t) p;
-          if (p >= 64) {
+          M.prime = (uint32_t) p;
+          M.pinv = 0xFFFFFFFFu / (uint32_t) p;
+          if (p >= 7) {
             uint64_t qlo = div_magic((uint64_t) low + p - 1, p, pm);
             if (qlo < 1) qlo = 1;
-            uint64_t qhi = div_magic((uint64_t) high - 1, p, pm);
+            const uint64_t qhi = div_magic((uint64_t) high - 1, p, pm);
+            uint64_t jlo = 0;
             if (qlo <= qhi) {
-              P.jlo = cnt_le(qlo - 1);
-              P.jn = (uint32_t) (cnt_le(qhi) - P.jlo);
+              jlo = cnt_le(qlo - 1);
+              ncross = (uint32_t) (cnt_le(qhi) - jlo);
             }
-            // p^3 >= high: the numbers of the segment whose least prime factor
-            // is p are p itself and p*q for primes q >= p, so the count of
-            // level b follows from the PiTable
-            if ((u128) p * p * p >= (u128) high && (int64_t) qhi <= A.pi_max) {
-              uint32_t f = ((uint64_t) low <= p && p < (uint64_t) high) ? 1u : 0u;
-              const uint64_t qa = qlo > p ? qlo : p;
-              const int64_t pc = dpi(A.pitab, qa - 1);
-              if (qhi >= qa) f += (uint32_t) (dpi(A.pitab, qhi) - pc);
-              P.fcount = f;
-              P.flags |= 8;
-              pcv = (uint32_t) pc;
+            if (p < 64) {
+              M.first = (uint32_t) ((uint64_t) (low / 240) % p);   // pattern phase of the first word
+              P.flags |= 4;
+            } else if (ncross) {
+              M.jn8 = 8 * ncross + (uint32_t) (jlo & 7);
+              M.first = (uint32_t) (p * (30 * (jlo >> 3) + woff((uint32_t) (jlo & 7))) - (uint64_t) low);
+              mwords = (ncross + 31) >> 5;
             }
-          } else if (p >= 7) {
-            P.jlo = (uint64_t) ((low / 240) % p);   // pattern phase of the first word
-            P.flags |= 4;
-            // its multiples in the segment, for the work counter only
-            uint64_t qlo = ((uint64_t) low + p - 1) / p;
-            if (qlo < 1) qlo = 1;
-            const uint64_t qhi = ((uint64_t) high - 1) / p;
-            if (qlo <= qhi) ncross = (uint32_t) (cnt_le(qhi) - cnt_le(qlo - 1));
           }
-          if (p >= 64) ncross = P.jn;
           if (b >= bmin_leaf && b <= bmax_leaf) {
             const uint64_t* xt = PQ.xp_tab + 3 * b;
             const u128 xp = ((u128) xt[1] << 64) | xt[0];
@@ -817,70 +908,92 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
               E = P.hi - P.lo;
               P.xlo = xt[0];
               if (xt[1]) P.flags |= 16;
+              else if ((P.flags & 2) ? A.pi_max < (1ll << 31) : P.hi < NARROW_INDEX) P.flags |= 32;
             }
           }
         }
-        fcnt = P.fcount;
-        lp[tid] = P;
-        s_pc[tid] = pcv;
+        if (tid < LB) { lp[tid] = P; lm[tid] = M; }
         ncross = __reduce_add_sync(0xffffffffu, ncross);
         if (lane == 0 && ncross) atomicAdd(&s_ctr[4], (unsigned long long) ncross);
       }
       __syncthreads();
-      const int nb = (int) dmin(NT, (int64_t) (Bs - b0 + 1));
+      const int nb = (int) dmin(LB, (int64_t) (Bs - b0 + 1));
       {
         // goto next_segment (D.cpp:131-132): no leaves from s_stop on
-        const bool has_leaves = (b0 + tid < s_stop) && E > 0;
-        if (!has_leaves) E = 0;
-        const uint32_t jn = lp[tid].jn;
-        // flat offsets of records, run cross-off co-factors and formula counts
-        block_scan3<NT>(E, (lp[tid].flags & 8) ? (long long) jn : 0, (long long) fcnt, loff, hoff, rpre, wt3);
-        // runs: levels without leaves whose count follows from the formula
-        const bool breaker = (tid >= nb) || has_leaves || !(lp[tid].flags & 8);
-        const unsigned bal = __ballot_sync(0xffffffffu, breaker);
-        if (lane == 0) s_brk[warp] = bal ? warp * 32 + __ffs((int) bal) - 1 : NT;
+        if (b0 + tid >= s_stop) E = 0;
+        const bool alone = tid < nb && ((lp[tid].flags & 4) || E > SOLO_RECORDS);
+        const unsigned bal = __ballot_sync(0xffffffffu, alone);
+        if (lane == 0 && warp < LB / 32) s_solo[warp] = bal;
+        // flat offsets of records and of mask words
+        block_scan2<LB>(E, mwords, loff, wofs, wt2);
         __syncthreads();
-        const unsigned mine = bal & (0xffffffffu << lane);
-        int re;
-        if (mine) re = warp * 32 + __ffs((int) mine) - 1;
-        else {
-          re = NT;
-          for (int w2 = warp + 1; w2 < NT / 32; w2++)
-            if (s_brk[w2] < NT) { re = s_brk[w2]; break; }
+        // the end of a group starting at this level: the next level alone, or
+        // the first that one of the group's limits keeps out
+        if (tid < nb) {
+          int hi = nb;
+          for (int w = tid >> 5; w < LB / 32; w++) {
+            uint32_t m = s_solo[w];
+            if (w == (tid >> 5)) m &= 0xfffffffeu << lane;
+            if (m) { hi = 32 * w + __ffs((int) m) - 1; break; }
+          }
+          hi = min(hi, tid + min(max(1, A.group_max), max(2, (int) ((float) lm[tid].prime * gscale))));
+          int lo = tid + 1;
+          while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            const int64_t n = loff[mid] - loff[tid];
+            if (wofs[mid] - wofs[tid] <= (uint32_t) MASK_WORDS && n <= GROUP_RECORDS && n * (mid - tid) <= GROUP_WORK) lo = mid;
+            else hi = mid - 1;
+          }
+          s_gend[tid] = (uint8_t) (lo - tid - 1);
         }
-        runend[tid] = (uint16_t) dmin(re, nb);
         __syncthreads();
       }
-      const int64_t total_e = loff[nb];
-      // FactorTable entries read: every record of the batch's levels is
-      // read once by the windows below (two-prime levels read primes instead)
+      // FactorTable entries read: every record of the batch's levels counts
+      // once (two-prime levels read primes instead)
       if (tid < nb && !(lp[tid].flags & 2)) nentries += (unsigned long long) (loff[tid + 1] - loff[tid]);
 
       int li = 0;          // next batch level to finish
       int64_t w0 = 0;      // first flat record of the window
       while (li < nb) {
-        const int64_t wend = w0 + cap;
+        // the next level answered alone, from li on
+        int ns = nb;
+        for (int w = li >> 5; w < LB / 32; w++) {
+          uint32_t m = s_solo[w];
+          if (w == (li >> 5)) m &= 0xffffffffu << (li & 31);
+          if (m) { ns = 32 * w + __ffs((int) m) - 1; break; }
+        }
+        const bool solo = ns == li;
+        // the window: of a level alone, its next records; else the records of
+        // the levels li .. ns - 1 from level li on, as many as fit
+        const int64_t la = loff[li], lz = loff[li + 1];
+        if (w0 < la) w0 = la;
+        const int nrec = (int) dmin(REC_CAP, (solo ? lz : loff[ns]) - w0);
+        const int64_t wend = w0 + nrec;
+        // the levels before lfull lie wholly in the window
+        int lfull = ns;
+        if (!solo && loff[ns] > wend) {
+          int lo = li;
+          while (lo < lfull) {
+            const int mid = (lo + lfull + 1) >> 1;
+            if (loff[mid] <= wend) lo = mid; else lfull = mid - 1;
+          }
+        }
         win++;
-        // ---- phase A: the window's leaf records, flat over levels, PA_UNROLL
-        // entries per thread in three stages so that their table loads, then
-        // their reciprocal loads, are in flight together
-        const int nrec = (int) dmax(0, dmin(wend, total_e) - w0);
-        // a window inside one level (the dense case): that level's constants
-        // held in registers, no level lookup per entry
-        const bool one_level = nrec > 0 && loff[li] <= w0 && loff[li + 1] >= w0 + nrec;
-        // a window of one level of FactorTable entries whose records are all
-        // answered by the per-level path: the accepted records are compacted
-        // to the front (their order is free, all are answered against one
-        // bitmap state), the rejected ones are dropped
-        const bool compact = one_level && !(lp[li].flags & 2) && (loff[li] < w0 || !(lp[li].flags & 8));
-        const int clev = compact ? li : -1;                // the level whose records are compacted
         if (tid == 0) s_ncomp[(win + 1) & 1] = 0;
-        if (one_level) {
+        // ---- phase A: the window's leaf records, PA_UNROLL entries per thread
+        // in three stages so that their table loads, then their reciprocal
+        // loads, are in flight together
+        if (solo && nrec > 0) {
+          // one level: its constants held in registers, no level lookup per
+          // entry.  Accepted FactorTable entries are compacted to the front
+          // (their order is free, all are answered against one bitmap state),
+          // the rejected ones are dropped.
           const LevelP& Q = lp[li];
-          const int64_t hi0 = Q.hi - (w0 - loff[li]);        // table index of entry f is hi0 - f
+          const int64_t hi0 = Q.hi - (w0 - la);              // table index of entry f is hi0 - f
           const bool two = (Q.flags & 2) != 0;
+          const bool compact = !two, narrow = (Q.flags & 32) != 0;
           const uint32_t thr = Q.thr;
-          const uint64_t* xt = PQ.xp_tab + 3 * (int64_t) Q.level;
+          const uint64_t* xt = PQ.xp_tab + 3 * (int64_t) (b0 + li);
           const uint64_t xlo = xt[0], xhi = xt[1];
           unsigned nl = 0;
           if (compact && hi0 < 0x7FFFFFFFll) {
@@ -914,6 +1027,28 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
                 pos += __popc(bal[u]);
               }
               __syncwarp();
+              if (narrow) {
+                // m < 2^31: the remainder less the true quotient's is below
+                // 2 m < 2^32, so its low word decides the correction
+                for (int j0 = 0; j0 < tot; j0 += 32 * 4) {
+                  uint32_t e[4];
+                  uint64_t mv[4];
+#pragma unroll
+                  for (int d = 0; d < 4; d++) {
+                    const int j = j0 + 32 * d + lane;
+                    e[d] = j < tot ? rec[base + j] : 0u;
+                    mv[d] = j < tot ? __ldg(&A.finv[e[d] & 0x7FFFFFFFu]) : 0ull;
+                  }
+#pragma unroll
+                  for (int d = 0; d < 4; d++) {
+                    const int j = j0 + 32 * d + lane;
+                    const uint32_t mi = e[d] & 0x7FFFFFFFu, m32 = 2310u * (mi / 480u) + cop[mi % 480u];
+                    const uint32_t t = (uint32_t) __umul64hi(xlo, mv[d]);
+                    const uint32_t r = t - (uint32_t) low + ((uint32_t) xlo - t * m32 >= m32 ? 1u : 0u);
+                    if (j < tot) rec[base + j] = r | (e[d] & 0x80000000u);
+                  }
+                }
+              } else
               for (int j0 = 0; j0 < tot; j0 += 32 * 4) {
                 uint32_t e[4];
                 uint64_t mv[4];
@@ -930,9 +1065,7 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
                     const uint32_t mi = e[d] & 0x7FFFFFFFu;
                     const uint64_t m = 2310ull * (mi / 480u) + cop[mi % 480u];
                     const uint64_t nn = xhi == 0 ? div_magic(xlo, m, mv[d]) : div_xp(xlo, xhi, m);
-                    uint32_t r = (uint32_t) (nn - (uint64_t) low);
-                    if (e[d] & 0x80000000u) r |= 1u << 30;
-                    rec[base + j] = r;
+                    rec[base + j] = (uint32_t) (nn - (uint64_t) low) | (e[d] & 0x80000000u);
                   }
                 }
               }
@@ -968,18 +1101,11 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
                 const int64_t idx = hi0 - f;
                 uint64_t m = 0;
                 if (two) m = fv[u];
-                else if (fv[u] > thr) {
-                  if ((uint64_t) idx <= 0xFFFFFFFFull) {
-                    const uint32_t mi = (uint32_t) idx;
-                    m = 2310ull * (mi / 480u) + cop[mi % 480u];
-                  } else {
-                    m = 2310ull * ((uint64_t) idx / 480) + cop[(uint64_t) idx % 480];
-                  }
-                }
+                else if (fv[u] > thr) m = 2310ull * ((uint64_t) idx / 480) + cop[(uint64_t) idx % 480];
                 if (m) {
                   const uint64_t nn = xhi == 0 ? div_magic(xlo, m, minv[u]) : div_xp(xlo, xhi, m);
                   uint32_t r = (uint32_t) (nn - (uint64_t) low);
-                  if (!two && !(fv[u] & 1)) r |= 1u << 30;
+                  if (!two && !(fv[u] & 1)) r |= 0x80000000u;
                   rv[u] = r;
                   nl++;
                 }
@@ -1009,17 +1135,12 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
           nleaves += nl;
           if (two) ntwo += nl;
         }
-        if (nrec > 0 && !one_level) {
-          // the window's records belong to levels li .. lw
-          int lw = li;
-          {
-            const int64_t last = w0 + nrec - 1;
-            int hi = nb - 1;
-            while (lw < hi) {
-              const int mid = (lw + hi + 1) >> 1;
-              if (loff[mid] <= last) lw = mid; else hi = mid - 1;
-            }
-          }
+        if (!solo && nrec > 0) {
+          // the window's records belong to levels li .. lw; those of a level
+          // that ends beyond the window are made again with the next one and
+          // not counted here
+          const int lw = min(lfull, ns - 1);
+          const int nfull = (int) (loff[lfull] - w0);
           for (int f0 = tid; f0 < nrec; f0 += PA_UNROLL * NT) {
             int jl[PA_UNROLL];
             int el[PA_UNROLL];
@@ -1084,8 +1205,8 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
                 }
               }
             }
-            // n = (x / p) / m, the record: offset in the segment, bit 30 for
-            // the negative sign of -mu(m) (an even factor-table entry)
+            // n = (x / p) / m, the record: offset in the segment, level, bit 31
+            // for the negative sign of -mu(m) (an even factor-table entry)
 #pragma unroll
             for (int u = 0; u < PA_UNROLL; u++) {
               const int f = f0 + u * NT;
@@ -1093,12 +1214,21 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
                 const LevelP& Q = lp[jl[u]];
                 uint32_t r = REC_NONE;
                 if (mdiv[u]) {
-                  const uint64_t nn = (Q.flags & 16) ? div_xp(Q.xlo, PQ.xp_tab[3 * (int64_t) Q.level + 1], mdiv[u])
-                                                     : div_magic(Q.xlo, mdiv[u], minv[u]);
-                  r = (uint32_t) (nn - (uint64_t) low);
-                  if (!(Q.flags & 2) && !(fv[u] & 1)) r |= 1u << 30;
-                  nleaves++;
-                  if (Q.flags & 2) ntwo++;
+                  uint32_t nn;
+                  if (Q.flags & 32) {
+                    const uint32_t m32 = (uint32_t) mdiv[u];
+                    nn = (uint32_t) __umul64hi(Q.xlo, minv[u]);
+                    nn += (uint32_t) Q.xlo - nn * m32 >= m32 ? 1u : 0u;
+                  } else {
+                    nn = (uint32_t) ((Q.flags & 16) ? div_xp(Q.xlo, PQ.xp_tab[3 * (int64_t) (b0 + jl[u]) + 1], mdiv[u])
+                                                    : div_magic(Q.xlo, mdiv[u], minv[u]));
+                  }
+                  r = (nn - (uint32_t) low) | ((uint32_t) jl[u] << OB);
+                  if (!(Q.flags & 2) && !(fv[u] & 1)) r |= 0x80000000u;
+                  if (f < nfull) {
+                    nleaves++;
+                    if (Q.flags & 2) ntwo++;
+                  }
                 }
                 rec[f] = r;
               }
@@ -1106,293 +1236,498 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
           }
         }
         if (nrec > 0) __syncthreads();
-        // ---- phase B: levels in order
-        while (li < nb) {
-          // the level's shared-memory fields, loaded together
-          const int re = runend[li];
-          const uint32_t lflags = lp[li].flags;
-          const int64_t la = loff[li], lz = loff[li + 1];
-          if (re > li) {
-            // a run of leafless levels li .. re-1 with formula counts: their
-            // counts from the prefix, all their multiples crossed off at once
-            const int64_t r0 = rpre[li];
-            for (int t = tid; t < re - li; t += NT)
-              A.cnt[rowbase + b0 + li + t] = total - (uint32_t) (rpre[li + t] - r0);
-            const int64_t h0 = hoff[li], h1 = hoff[re];
-            cross_off_levels<NT>(bits, ccount, lp, hoff, li, re, (uint64_t) low, s_bitt);
-            const uint32_t removed = (uint32_t) (rpre[re] - r0);
-            total -= removed;
-            if (h1 > h0) dirty = true;
-            li = re;
-            __syncthreads();
-            continue;
-          }
-          // ---- levels li .. lj-1 with p^3 >= high whose records all lie in this
-          // window: the numbers such a level removes are p and the p q with
-          // prime q >= p, so the count at level l of a record's n is the count
-          // at level li minus sum_{li <= b < l} ([low <= p_b <= n] +
-          // pi(n / p_b) - pi(q_lo_b - 1)).  All their records are answered
-          // against one bitmap state, then all their multiples crossed off at
-          // once: one barrier pass instead of one per level.
-          if ((lflags & 8) && la >= w0) {
-            // lj: the first level from li on that cannot join the group, found
-            // by each warp's lanes checking 32 levels at once
-            int lj;
-            {
-              const int gm = A.group_max;
-              int j = li + lane;
-              bool no = !(j < nb && j - li < gm && (lp[j].flags & 8) && loff[j + 1] <= wend);
-              unsigned bal = __ballot_sync(0xffffffffu, no);
-              if (bal) lj = li + __ffs((int) bal) - 1;
-              else {
-                j += 32;
-                no = !(j < nb && j - li < gm && (lp[j].flags & 8) && loff[j + 1] <= wend);
-                bal = __ballot_sync(0xffffffffu, no);
-                lj = bal ? li + 32 + __ffs((int) bal) - 1 : li + 64;
-              }
-            }
-            if (lj - li >= 2) {
-              const int ra = (int) (loff[li] - w0), rb = (int) (loff[lj] - w0);
-              if (tid < lj - li) {
-                s_gsmu[tid] = 0;
-                s_gmag[tid] = A.pmagic[b0 + li + tid];
-              }
-              // a few records: a warp per record, its lanes summing the chunk
-              // counts below the record's chunk and the removals of one group
-              // level each (no prefix scan)
-              const bool few = dirty && rb > ra && rb - ra <= SMALL_QUERIES;
-              if (rb > ra && dirty && !few) { scan_chunks(ccount, pref, nch, wtmp); dirty = false; }
-              else __syncthreads();
-              if (few) {
-                for (int k2 = ra + warp; k2 < rb; k2 += NT / 32) {
-                  const uint32_t r = rec[k2];
-                  if (r == REC_NONE) continue;
-                  // the record's level: the levels li + t whose records end at or
-                  // before it, counted by the lanes (a group has at most 64 levels)
-                  const int64_t pos = w0 + k2;
-                  int lv = li + __popc(__ballot_sync(0xffffffffu, li + lane < lj && loff[li + lane + 1] <= pos));
-                  if (lj - li > 32)
-                    lv += __popc(__ballot_sync(0xffffffffu, li + 32 + lane < lj && loff[li + 33 + lane] <= pos));
-                  const uint32_t off = r & 0x3FFFFFFFu;
-                  const uint64_t n = (uint64_t) low + off;
-                  const uint32_t wd = off / 240, ch = wd >> 3, kw = wd & 7;
-                  uint32_t part = chunk_sum_below(ccount, ch, lane);
-                  if (lane < 8) {
-                    const uint64_t v = bits[8 * ch + lane];
-                    const uint32_t j = (uint32_t) lane;
-                    part += (uint32_t) __popcll(j < kw ? v : (j == kw ? (v & mask_le_t(s_nb, off - wd * 240)) : 0ull));
+
+        if (!solo) {
+          // ---- phase B, groups of levels whose records lie in the window
+          int pl = li, plen = 0;                        // the previous group, its signs not written yet
+          while (li < lfull) {
+            const uint32_t wb0 = wofs[li];
+            const int lj = min(lfull, li + 1 + s_gend[li]);
+            const int G = lj - li;
+            const int W = (int) (wofs[lj] - wb0);
+            const int ra = (int) (loff[li] - w0), rb = (int) (loff[lj] - w0);
+            uint32_t* mk = masks + gpar * (MASK_WORDS + 1);
+            // short levels (at most 8 mask words on average): a warp takes
+            // levels, four at a time; else it takes the words [wa, wz) of
+            // consecutive levels from lf on, four words at a time
+            const bool shortl = W <= 8 * G;
+            const int wa = W * warp / NW, wz = W * (warp + 1) / NW;
+            int lf = li;
+            if (!shortl)
+              for (int t = 0; t < G; t += 32)
+                lf += __popc(__ballot_sync(0xffffffffu, li + t + 1 + lane < lj && (int) (wofs[li + t + 1 + lane] - wb0) <= wa));
+            // 1. the masks
+            if (shortl) {
+              for (int l = li + warp; l < lj; l += 4 * NW) {
+                uint32_t h[4], m[4], jn[4], p[4], w[4];
+                uint32_t most = 0;
+#pragma unroll
+                for (int d = 0; d < 4; d++) {
+                  const int k = min(l + d * NW, lj - 1);
+                  const LevelM Q = lm[k];
+                  p[d] = Q.prime;
+                  jn[d] = l + d * NW < lj ? Q.jn8 >> 3 : 0u;
+                  w[d] = wofs[k] - wb0;
+                  const uint32_t off = Q.first + Q.prime * s_delta[(Q.jn8 & 7) * 32 + lane];
+                  h[d] = off / 120;
+                  m[d] = 1u << s_bit[off - 120 * h[d]];
+                  most = max(most, jn[d]);
+                }
+                for (uint32_t j = 0; j < most; j += 32) {
+                  uint32_t v[4];
+#pragma unroll
+                  for (int d = 0; d < 4; d++) {
+                    const bool on = j + lane < jn[d];
+                    v[d] = hw[on ? h[d] : 0u] & (on ? m[d] : 0u);
+                    h[d] += p[d];
                   }
-                  // the numbers <= n removed by the levels li .. lv-1, one per lane
-                  for (int b = li + lane; b < lv; b += 32) {
-                    const uint64_t pb = lp[b].prime;
-                    if (pb <= n && pb >= (uint64_t) low) part--;
-                    const int64_t d = dpi_t(A.pitab, s_nb, div_magic(n, pb, s_gmag[b - li])) - (int64_t) s_pc[b];
-                    if (d > 0) part -= (uint32_t) d;
-                  }
-                  // the count is below 2^32: the sum modulo 2^32 is exact
-                  const uint32_t c = __reduce_add_sync(0xffffffffu, part);
-                  if (lane == 0) {
-                    if (r & (1u << 30)) { lsum -= c; atomicAdd(&s_gsmu[lv - li], -1); }
-                    else { lsum += c; atomicAdd(&s_gsmu[lv - li], 1); }
+#pragma unroll
+                  for (int d = 0; d < 4; d++) {
+                    const uint32_t bal = __ballot_sync(0xffffffffu, v[d] != 0);
+                    if (lane == d && j < jn[d]) mk[w[d] + (j >> 5)] = bal;
                   }
                 }
-              } else if (rb > ra) {
-                for (int k2 = ra + tid; k2 < rb; k2 += NT) {
-                  const int lv = level_of(loff, li, lj, w0 + k2);
-                  const uint32_t r = rec[k2];
-                  int sg = 0;
+              }
+            } else
+            for (int wi = wa, l = lf; wi < wz; l++) {
+              const int wl = (int) (wofs[l] - wb0), e = min(wz, (int) (wofs[l + 1] - wb0));
+              if (wi >= e) continue;
+              const LevelM Q = lm[l];
+              const uint32_t p = Q.prime, jn = Q.jn8 >> 3;
+              const uint32_t off = Q.first + p * s_delta[(Q.jn8 & 7) * 32 + lane];
+              uint32_t h = off / 120;
+              const uint32_t m = 1u << s_bit[off - 120 * h];
+              uint32_t idx = 32 * (uint32_t) (wi - wl) + lane;
+              h += p * (uint32_t) (wi - wl);
+              while (wi < e) {
+                const int n = min(32, e - wi);
+                uint32_t mine = 0;
+                for (int u = 0; u < n; u += 4) {
+                  uint32_t v[4];
+#pragma unroll
+                  for (int d = 0; d < 4; d++) {
+                    const bool on = u + d < n && idx + 32 * d < jn;
+                    v[d] = hw[on ? h + d * p : 0u] & (on ? m : 0u);
+                  }
+#pragma unroll
+                  for (int d = 0; d < 4; d++) {
+                    const uint32_t bal = __ballot_sync(0xffffffffu, v[d] != 0);
+                    if (lane == u + d) mine = bal;
+                  }
+                  idx += 128;
+                  h += 4 * p;
+                }
+                if (lane < n) mk[wi + lane] = mine;
+                wi += n;
+              }
+            }
+            __syncthreads();
+            // the signed leaf counts of the previous group
+            for (int t = tid; t < plen; t += NT) {
+              const int v = s_gsmu[gpar ^ 1][t];
+              if (v) { A.smu[rowbase + b0 + pl + t] = v; s_gsmu[gpar ^ 1][t] = 0; }
+            }
+            // 2. the clears.  Up to four collisions o[0 .. n - 1], numbers
+            // that another level of the group cleared: the lanes test the
+            // group's levels, all but the lowest that divides a number drop
+            // it from their masks.
+            auto resolve = [&](const uint32_t* o, int n) {
+              int lowest[4] = {-1, -1, -1, -1};
+              for (int t0 = 0; t0 < G; t0 += 32) {
+                const int t = t0 + lane;
+                const LevelM R = lm[li + min(t, G - 1)];
+                uint32_t e[4];
+                bool div[4];
+#pragma unroll
+                for (int d = 0; d < 4; d++) {
+                  const int32_t dt = (int32_t) (o[min(d, n - 1)] - R.first);
+                  e[d] = div_small((uint32_t) dt, R.prime, R.pinv);
+                  div[d] = dt >= 0 && t < G && d < n && e[d] * R.prime == (uint32_t) dt;
+                }
+#pragma unroll
+                for (int d = 0; d < 4; d++) {
+                  const unsigned bal = __ballot_sync(0xffffffffu, div[d]);
+                  if (bal) {
+                    if (lowest[d] < 0) lowest[d] = t0 + __ffs((int) bal) - 1;
+                    if (div[d] && t != lowest[d]) {
+                      const uint32_t dd = wheel_rank(e[d], R.jn8 & 7, s_nb) - 1;
+                      atomicAnd(&mk[wofs[li + t] - wb0 + (dd >> 5)], ~(1u << (dd & 31)));
+                    }
+                  }
+                }
+              }
+            };
+            // a collision at offset o, listed for the end of the clears;
+            // beyond the list's end this lane does the same by itself
+            auto collide = [&](uint32_t o) {
+              const int at = atomicAdd(&s_ncoll, 1);
+              if (at < COLLISIONS) { clist[at] = o; return; }
+              bool first = true;
+              for (int t = 0; t < G; t++) {
+                const LevelM R = lm[li + t];
+                const int32_t dt = (int32_t) (o - R.first);
+                if (dt < 0) continue;
+                const uint32_t e = div_small((uint32_t) dt, R.prime, R.pinv);
+                if (e * R.prime != (uint32_t) dt) continue;
+                if (!first) {
+                  const uint32_t dd = wheel_rank(e, R.jn8 & 7, s_nb) - 1;
+                  atomicAnd(&mk[wofs[li + t] - wb0 + (dd >> 5)], ~(1u << (dd & 31)));
+                }
+                first = false;
+              }
+            };
+            if (shortl) {
+              for (int l = li + warp; l < lj; l += 4 * NW) {
+                uint32_t h[4], m[4], nw[4], p[4], w[4];
+                uint32_t most = 0;
+#pragma unroll
+                for (int d = 0; d < 4; d++) {
+                  const int k = min(l + d * NW, lj - 1);
+                  const LevelM Q = lm[k];
+                  p[d] = Q.prime;
+                  nw[d] = l + d * NW < lj ? ((Q.jn8 >> 3) + 31) >> 5 : 0u;
+                  w[d] = wofs[k] - wb0;
+                  const uint32_t off = Q.first + Q.prime * s_delta[(Q.jn8 & 7) * 32 + lane];
+                  h[d] = off / 120;
+                  m[d] = 1u << s_bit[off - 120 * h[d]];
+                  most = max(most, nw[d]);
+                }
+                for (uint32_t j = 0; j < most; j++) {
+                  uint32_t old[4];
+                  bool on[4];
+                  unsigned lost = 0;
+#pragma unroll
+                  for (int d = 0; d < 4; d++) on[d] = ((j < nw[d] ? mk[w[d] + j] : 0u) >> lane) & 1u;
+#pragma unroll
+                  for (int d = 0; d < 4; d++) old[d] = and_if(on[d], hw + h[d], m[d]);
+#pragma unroll
+                  for (int d = 0; d < 4; d++) {
+                    dec_if(on[d] && old[d], ccount + (h[d] >> 4));
+                    if (!old[d]) lost |= 1u << d;
+                    h[d] += p[d];
+                  }
+                  while (lost) {
+                    const LevelM Q = lm[l + (__ffs((int) lost) - 1) * NW];
+                    lost &= lost - 1;
+                    collide(Q.first + Q.prime * (s_delta[(Q.jn8 & 7) * 32 + lane] + 120 * j));
+                  }
+                }
+              }
+            } else
+            for (int wi = wa, l = lf; wi < wz; l++) {
+              const int wl = (int) (wofs[l] - wb0), e = min(wz, (int) (wofs[l + 1] - wb0));
+              if (wi >= e) continue;
+              const LevelM Q = lm[l];
+              const uint32_t p = Q.prime;
+              const uint32_t off = Q.first + p * s_delta[(Q.jn8 & 7) * 32 + lane];
+              uint32_t h = off / 120;
+              const uint32_t res = off - 120 * h;
+              const uint32_t m = 1u << s_bit[res];
+              h += p * (uint32_t) (wi - wl);
+              for (; wi < e; wi += 4, h += 4 * p) {
+                uint32_t old[4];
+                bool on[4];
+                unsigned lost = 0;
+#pragma unroll
+                for (int d = 0; d < 4; d++) on[d] = ((wi + d < e ? mk[wi + d] : 0u) >> lane) & 1u;
+#pragma unroll
+                for (int d = 0; d < 4; d++) old[d] = and_if(on[d], hw + (h + d * p), m);
+#pragma unroll
+                for (int d = 0; d < 4; d++) {
+                  dec_if(on[d] && old[d], ccount + ((h + d * p) >> 4));
+                  if (!old[d]) lost |= 1u << d;
+                }
+                while (lost) {
+                  const uint32_t d = (uint32_t) __ffs((int) lost) - 1;
+                  lost &= lost - 1;
+                  collide(120 * (h + d * p) + res);
+                }
+              }
+              wi = e;
+            }
+            __syncthreads();
+            if (s_ncoll) {
+              const int nc = min(s_ncoll, COLLISIONS);
+              for (int i = 4 * warp; i < nc; i += 4 * NW) resolve(clist + i, min(4, nc - i));
+              __syncthreads();
+              if (tid == 0) s_ncoll = 0;                 // next used after two more barriers
+            }
+            // 3. the prefix of the masks' counts (the last warp) and of the
+            // chunk counts (the first SCAN_WARPS warps, each its part)
+            if (warp == NW - 1) {
+              const int per = ((W + 31) / 32) | 1;      // odd: no bank conflicts
+              const int i0 = min(W, lane * per), i1 = min(W, i0 + per);
+              uint32_t sum = 0;
+              for (int i = i0; i < i1; i++) sum += __popc(mk[i]);
+              uint32_t incl = sum;
+              for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t t = __shfl_up_sync(0xffffffffu, incl, d);
+                if (lane >= d) incl += t;
+              }
+              uint32_t run = incl - sum;
+              for (int i = i0; i < i1; i++) {
+                mpre[i] = (uint16_t) run;
+                run += __popc(mk[i]);
+              }
+              if (lane == 31) { mpre[W] = (uint16_t) run; mk[W] = 0; }
+            }
+            if (rb > ra && warp < SCAN_WARPS) scan_part(ccount, pref, n4, wtmp);
+            __syncthreads();
+            // the levels' counts C(s, b)
+            for (int t = tid; t < G; t += NT)
+              A.cnt[rowbase + b0 + li + t] = total - mpre[wofs[li + t] - wb0];
+            total -= mpre[W];
+            // 4. the records
+            if (rb > ra) {
+              const uint32_t t0 = wtmp[0], t1 = t0 + wtmp[1], t2 = t1 + wtmp[2];
+              const uint32_t per = 4 * (uint32_t) scan_per(n4);   // chunks per scan warp
+              auto part_base = [&](uint32_t ch) { return ch < per ? 0u : (ch < 2 * per ? t0 : (ch < 3 * per ? t1 : t2)); };
+              if (rb - ra <= LANE_RECORDS || G > LANE_LEVELS) {
+                // A warp takes a run of records, drops the rejected ones and
+                // answers four at a time: eight lanes each for the words of the
+                // record's chunk, then all lanes over the group's levels, each
+                // level's parameters loaded once for the four.
+                const int run = rb - ra <= 8 * NW ? 8 : (rb - ra <= 16 * NW ? 16 : 32);
+                const int sub = lane & 7, own = lane >> 3;
+                for (int k0 = ra + run * warp; k0 < rb; k0 += run * NW) {
+                  const uint32_t rv = lane < run && k0 + lane < rb ? rec[k0 + lane] : REC_NONE;
+                  const unsigned acc = __ballot_sync(0xffffffffu, rv != REC_NONE);
+                  const int na = __popc(acc);
+                  if (rv != REC_NONE) rec[k0 + __popc(acc & ((1u << lane) - 1u))] = rv;
+                  __syncwarp();
+                  for (int i = 0; i < na; i += 4) {
+                    uint32_t off[4];
+                    int lv[4];
+                    uint32_t part[4];
+#pragma unroll
+                    for (int d = 0; d < 4; d++) {
+                      const uint32_t r = rec[k0 + min(i + d, na - 1)];
+                      off[d] = r & OM;
+                      lv[d] = (int) ((r & 0x7FFFFFFFu) >> OB);
+                      part[d] = 0;
+                    }
+                    const uint32_t rown = rec[k0 + min(i + own, na - 1)], oo = rown & OM;
+                    const uint32_t wd = oo / 240, ch = wd >> 3, kw = wd & 7;
+                    const uint64_t v = bits[8 * ch + sub];
+                    const uint64_t vm = (uint32_t) sub == kw ? mask_le_t(s_nb, oo - wd * 240) : 0ull;
+                    uint32_t base = (uint32_t) __popcll(v & ((uint32_t) sub < kw ? ~0ull : vm));
+                    if (sub == 0) base += before_chunk(ccount, pref, ch) + part_base(ch);
+                    // the run's records are in level order: lv[0] is the lowest
+                    for (int b = lv[0] + lane; b - lane < lj; b += 32) {
+                      const int k = min(b, lj - 1);
+                      const LevelM Q = lm[k];
+                      const uint32_t mp = wofs[k] - wb0;
+                      const uint32_t jl = Q.jn8 & 7, r0 = woff(jl), p0 = mpre[mp];
+#pragma unroll
+                      for (int d = 0; d < 4; d++) {
+                        const int32_t t = (int32_t) (off[d] - Q.first);
+                        const bool on = t >= 0 && b >= lv[d] && b < lj;
+                        const uint32_t s2 = r0 + div_small(on ? (uint32_t) t : 0u, Q.prime, Q.pinv);
+                        const uint32_t q2 = s2 / 30;
+                        const uint32_t dd = 8 * q2 + s_nb[s2 - 30 * q2] - jl;
+                        const uint32_t w = mp + (on ? dd >> 5 : 0u);
+                        const uint32_t c = (uint32_t) mpre[w] - p0 + (uint32_t) __popc(mk[w] & ((1u << (dd & 31)) - 1u));
+                        part[d] += on ? c : 0u;
+                      }
+                    }
+                    base += __shfl_xor_sync(0xffffffffu, base, 4);
+                    base += __shfl_xor_sync(0xffffffffu, base, 2);
+                    base += __shfl_xor_sync(0xffffffffu, base, 1);
+#pragma unroll
+                    for (int d = 0; d < 4; d++) {
+                      const uint32_t c = __reduce_add_sync(0xffffffffu, part[d]);
+                      if (own == d) base += c;
+                    }
+                    if (sub == 0 && i + own < na) {
+                      const int l = (int) ((rown & 0x7FFFFFFFu) >> OB) - li;
+                      if (rown >> 31) { lsum -= base; atomicAdd(&s_gsmu[gpar][l], -1); }
+                      else { lsum += base; atomicAdd(&s_gsmu[gpar][l], 1); }
+                    }
+                  }
+                }
+              } else {
+                for (int k2 = ra + tid; k2 - lane < rb; k2 += NT) {
+                  const uint32_t r = k2 < rb ? rec[k2] : REC_NONE;
+                  int sg = 0, lv = li;
                   if (r != REC_NONE) {
-                    const uint32_t off = r & 0x3FFFFFFFu;
-                    uint32_t c = query(bits, pref, s_nb, off);
-                    const uint64_t n = (uint64_t) low + off;
-                    // four levels at a time: their PiTable words are loaded together
-                    int b = li;
-                    for (; b + 4 <= lv; b += 4) {
-                      uint64_t t[4];
-#pragma unroll
-                      for (int u = 0; u < 4; u++) {
-                        const uint64_t pb = lp[b + u].prime;
-                        if (pb <= n && pb >= (uint64_t) low) c--;
-                        t[u] = div_magic(n, pb, s_gmag[b + u - li]);
-                      }
-                      ulonglong2 e[4];
-#pragma unroll
-                      for (int u = 0; u < 4; u++) e[u] = ((const ulonglong2*) A.pitab)[t[u] / 240];
-#pragma unroll
-                      for (int u = 0; u < 4; u++) {
-                        // for t < 6 this reads 3 + a few bits, still below s_pc[b] >= pi(63): dropped by d > 0
-                        const int64_t pt = (int64_t) (e[u].x + __popcll(e[u].y & mask_le_t(s_nb, (uint32_t) (t[u] % 240))));
-                        const int64_t d = pt - (int64_t) s_pc[b + u];
-                        if (d > 0) c -= (uint32_t) d;
-                      }
-                    }
-                    for (; b < lv; b++) {
-                      const uint64_t pb = lp[b].prime;
-                      if (pb <= n && pb >= (uint64_t) low) c--;
-                      const int64_t d = dpi_t(A.pitab, s_nb, div_magic(n, pb, s_gmag[b - li])) - (int64_t) s_pc[b];
-                      if (d > 0) c -= (uint32_t) d;
-                    }
-                    if (r & (1u << 30)) { lsum -= c; sg = -1; }
+                    const uint32_t off = r & OM;
+                    lv = (int) ((r & 0x7FFFFFFFu) >> OB);
+                    uint32_t c = query(bits, ccount, pref, s_nb, off) + part_base(off / 1920);
+                    for (int b = lv; b < lj; b++)
+                      c += removed_le(lm[b], off, wofs[b] - wb0, mk, mpre, s_nb);
+                    if (r >> 31) { lsum -= c; sg = -1; }
                     else { lsum += c; sg = 1; }
                   }
                   // signed counts per level, aggregated over the lanes of one level
-                  const unsigned act = __activemask();
-                  const unsigned same = __match_any_sync(act, lv);
+                  const unsigned same = __match_any_sync(0xffffffffu, lv);
                   const int tot = __reduce_add_sync(same, sg);
-                  if (tot && lane == __ffs((int) same) - 1) atomicAdd(&s_gsmu[lv - li], tot);
+                  if (tot && lane == __ffs((int) same) - 1) atomicAdd(&s_gsmu[gpar][lv - li], tot);
                 }
-              }
-              __syncthreads();
-              // the levels' counts C(s, b) and signed leaf counts M(s, b)
-              const int64_t r0 = rpre[li];
-              for (int t = tid; t < lj - li; t += NT) {
-                const int64_t cell = rowbase + b0 + li + t;
-                A.cnt[cell] = total - (uint32_t) (rpre[li + t] - r0);
-                if (s_gsmu[t]) A.smu[cell] = s_gsmu[t];
-              }
-              // all their multiples crossed off at once
-              const int64_t h0 = hoff[li], h1 = hoff[lj];
-              cross_off_levels<NT>(bits, ccount, lp, hoff, li, lj, (uint64_t) low, s_bitt);
-              total -= (uint32_t) (rpre[lj] - r0);
-              if (h1 > h0) dirty = true;
-              li = lj;
-              __syncthreads();
-              continue;
-            }
-          }
-          if (lz > la && la >= wend) break;               // records start in a later window
-          const int l = b0 + li;
-          if (la >= w0 && tid == NT - 1) A.cnt[rowbase + l] = total;   // the last thread: rarely a multiple to cross off
-          const int ra = (int) (dmax(la, w0) - w0);
-          const int rz = (int) (dmin(lz, wend) - w0);           // end of the level's window records
-          const int rb = li == clev ? s_ncomp[win & 1] : rz;   // end of those still to answer
-          if (rb > ra) {
-            if (dirty && rb - ra <= SMALL_QUERIES) {
-              // a few records: a warp per record sums the chunk counts below
-              // the record's chunk itself, instead of a block-wide prefix
-              // scan (the prefix array stays out of date)
-              int smu_w = 0;
-              for (int k2 = ra + warp; k2 < rb; k2 += NT / 32) {
-                const uint32_t r = rec[k2];
-                if (r == REC_NONE) continue;
-                const uint32_t off = r & 0x3FFFFFFFu;
-                const uint32_t wd = off / 240, ch = wd >> 3, kw = wd & 7;
-                uint32_t part = chunk_sum_below(ccount, ch, lane);
-                if (lane < 8) {
-                  const uint64_t v = bits[8 * ch + lane];
-                  const uint32_t j = (uint32_t) lane;
-                  part += (uint32_t) __popcll(j < kw ? v : (j == kw ? (v & mask_le_t(s_nb, off - wd * 240)) : 0ull));
-                }
-                const uint32_t c = __reduce_add_sync(0xffffffffu, part);
-                if (r & (1u << 30)) { if (lane == 0) lsum -= c; smu_w--; }
-                else { if (lane == 0) lsum += c; smu_w++; }
-              }
-              if (lane == 0 && smu_w) atomicAdd(&s_smu, smu_w);
-            } else {
-              if (dirty) { scan_chunks(ccount, pref, nch, wtmp); dirty = false; }
-              if (ra + 32 * warp < rb) {
-                int smu_t = 0;
-                for (int k2 = ra + tid; k2 < rb; k2 += NT) {
-                  const uint32_t r = rec[k2];
-                  if (r != REC_NONE) {
-                    const uint32_t c = query(bits, pref, s_nb, r & 0x3FFFFFFFu);
-                    if (r & (1u << 30)) { lsum -= c; smu_t--; }
-                    else { lsum += c; smu_t++; }
-                  }
-                }
-                smu_t = __reduce_add_sync(0xffffffffu, smu_t);
-                if (lane == 0 && smu_t) atomicAdd(&s_smu, smu_t);
               }
             }
-            __syncthreads();
+            pl = li;
+            plen = rb > ra ? G : 0;
+            gpar ^= 1;
+            li = lj;
           }
-          if (rz > ra && lz <= wend && tid == NT - 1) { A.smu[rowbase + l] = s_smu; s_smu = 0; }
-          if (lz > wend) break;                            // the level continues in the next window
-          // ---- cross off p_l and its multiples, count the numbers removed first
-          const LevelP& P = lp[li];
-          const uint32_t pjn = P.jn, pprime = P.prime;
-          const uint64_t pjlo = P.jlo;
-          uint32_t rem = 0;
-          if (lflags & 4) {
-            // small prime: AND with its wheel pattern, one owner thread per word
-            const uint32_t p = P.prime;
-            int po = 0;
-            for (int k = 0; c_small_p[k] != p; k++) po += c_small_p[k];
-            // four consecutive words per thread and round (two 16-byte accesses)
-            uint32_t r = (uint32_t) ((P.jlo + 4 * tid) % p);
-            const uint32_t step = (4 * NT) % p;
-            for (int w = 4 * tid; w < A.words; w += 4 * NT) {
-              uint32_t d = 0;
-              if (w < wused) {
-                const ulonglong2 o0 = *(const ulonglong2*) (bits + w);
-                const ulonglong2 o1 = *(const ulonglong2*) (bits + w + 2);
-                const uint32_t r1 = r + 1 == p ? 0u : r + 1;
-                const uint32_t r2 = r1 + 1 == p ? 0u : r1 + 1;
-                const uint32_t r3 = r2 + 1 == p ? 0u : r2 + 1;
-                ulonglong2 n0, n1;
-                n0.x = o0.x & pat[po + r];
-                n0.y = (w + 1 < wused) ? (o0.y & pat[po + r1]) : o0.y;
-                n1.x = (w + 2 < wused) ? (o1.x & pat[po + r2]) : o1.x;
-                n1.y = (w + 3 < wused) ? (o1.y & pat[po + r3]) : o1.y;
-                if (n0.x != o0.x || n0.y != o0.y) {
-                  *(ulonglong2*) (bits + w) = n0;
-                  d = __popcll(o0.x ^ n0.x) + __popcll(o0.y ^ n0.y);
-                }
-                if (n1.x != o1.x || n1.y != o1.y) {
-                  *(ulonglong2*) (bits + w + 2) = n1;
-                  d += __popcll(o1.x ^ n1.x) + __popcll(o1.y ^ n1.y);
-                }
-              }
-              rem += d;
-              // 2 consecutive lanes own the 8 words of one chunk
-              d += __shfl_down_sync(0xffffffffu, d, 1, 2);
-              if ((lane & 1) == 0 && d) ccount[w >> 3] -= d;
-              r += step;
-              if (r >= p) r -= p;
-            }
-          } else if (pjn) {
-            if ((uint32_t) tid < pjn) {
-              // co-factors tid, tid + NT, ...: NT / 8 wheel turns apart, so
-              // the multiples are NT p / 64 words apart with the same bit
-              const uint64_t p = pprime;
-              const uint64_t jj = pjlo + (uint64_t) tid;
-              const uint64_t q = 30 * (jj >> 3) + woff((uint32_t) (jj & 7));
-              const uint32_t off = (uint32_t) (p * q - (uint64_t) low);
-              const uint32_t w = off / 240;
-              const uint32_t bi = s_bitt[off - w * 240];
-              const uint32_t m = 1u << (bi & 31);
-              // the number's 32-bit half-word, and the half-word stride
-              uint32_t h = 2 * w + (bi >> 5);
-              const uint32_t hstep = (uint32_t) p * (NT / 32);
-              uint32_t* const hw = (uint32_t*) bits;
-              for (uint32_t j = tid; j < pjn; j += NT, h += hstep) {
-                const uint32_t old = hw[h];
-                if (old & m) { hw[h] = old & ~m; rem++; atomicSub(&ccount[h >> 4], 1u); }
-              }
-            }
+          __syncthreads();
+          for (int t = tid; t < plen; t += NT) {
+            const int v = s_gsmu[gpar ^ 1][t];
+            if (v) { A.smu[rowbase + b0 + pl + t] = v; s_gsmu[gpar ^ 1][t] = 0; }
           }
-          if (lflags & 8) {
-            __syncthreads();
-            total -= P.fcount;
-            if (pjn) dirty = true;
-          } else if (!(lflags & 4) && pjn <= (uint32_t) NT) {
-            // at most one multiple per thread: the barrier counts the removals
-            const uint32_t rr = (uint32_t) __syncthreads_count(rem != 0);
-            total -= rr;
-            if (rr) dirty = true;
-            if (tid == NT - 1) s_rem[(l + 2) % 3] = 0;
-          } else {
-            rem = __reduce_add_sync(0xffffffffu, rem);
-            if (lane == 0 && rem) atomicAdd(&s_rem[l % 3], rem);
-            __syncthreads();
-            const uint32_t rr = s_rem[l % 3];
-            total -= rr;
-            if (rr) dirty = true;
-            if (tid == NT - 1) s_rem[(l + 2) % 3] = 0;
-          }
-          li++;
+          dirty = true;
+          continue;
         }
-        w0 = wend;
+
+        // ---- phase B of a level alone
+        const uint32_t lflags = lp[li].flags;
+        const int l = b0 + li;
+        if (w0 == la && tid == NT - 1) A.cnt[rowbase + l] = total;   // the last thread: rarely a multiple to cross off
+        const int rb = (lflags & 2) ? nrec : s_ncomp[win & 1];       // records still to answer
+        if (nrec > 0 && rb > 0) {
+          if (dirty && rb <= SMALL_QUERIES) {
+            // a few records: a warp per record sums the chunk counts below
+            // the record's chunk itself, instead of a block-wide prefix
+            // scan (the prefix array stays out of date)
+            int smu_w = 0;
+            for (int k2 = warp; k2 < rb; k2 += NW) {
+              const uint32_t r = rec[k2];
+              const uint32_t off = r & 0x7FFFFFFFu;
+              const uint32_t wd = off / 240, ch = wd >> 3, kw = wd & 7;
+              uint32_t part = chunk_sum_below(ccount, ch, lane);
+              if (lane < 8) {
+                const uint64_t v = bits[8 * ch + lane];
+                const uint32_t j = (uint32_t) lane;
+                part += (uint32_t) __popcll(j < kw ? v : (j == kw ? (v & mask_le_t(s_nb, off - wd * 240)) : 0ull));
+              }
+              const uint32_t c = __reduce_add_sync(0xffffffffu, part);
+              if (r >> 31) { if (lane == 0) lsum -= c; smu_w--; }
+              else { if (lane == 0) lsum += c; smu_w++; }
+            }
+            if (lane == 0 && smu_w) atomicAdd(&s_smu, smu_w);
+          } else {
+            if (dirty) { scan_chunks(ccount, pref, n4, wtmp); dirty = false; wp_ok = false; }
+            const bool by_word = wp_fits && lz - la > WORD_RECORDS;
+            if (by_word && !wp_ok) {
+              for (int c = tid; c < nchu; c += NT) {
+                const ulonglong2* q = (const ulonglong2*) (bits + 8 * c);
+                uint32_t run = before_chunk(ccount, pref, (uint32_t) c);
+                uint4 o[2];
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                  const ulonglong2 a = q[2 * i], b = q[2 * i + 1];
+                  o[i].x = run; run += __popcll(a.x);
+                  o[i].y = run; run += __popcll(a.y);
+                  o[i].z = run; run += __popcll(b.x);
+                  o[i].w = run; run += __popcll(b.y);
+                }
+                ((uint4*) (wpre + 8 * c))[0] = o[0];
+                ((uint4*) (wpre + 8 * c))[1] = o[1];
+              }
+              wp_ok = true;
+              __syncthreads();
+            }
+            if (32 * warp < rb) {
+              // a thread's counts fit 32 bits: at most 3584 / 128 records of 2^21 numbers
+              int smu_t = 0, sum_t = 0;
+              if (by_word) {
+#pragma unroll 2
+                for (int k2 = tid; k2 < rb; k2 += NT) {
+                  const uint32_t r = rec[k2], off = r & 0x7FFFFFFFu;
+                  const uint32_t w = off / 240;
+                  const int c = (int) (wpre[w] + (uint32_t) __popcll(bits[w] & mask_le_t(s_nb, off - 240 * w)));
+                  sum_t += r >> 31 ? -c : c;
+                  smu_t += r >> 31 ? -1 : 1;
+                }
+              } else {
+                for (int k2 = tid; k2 < rb; k2 += NT) {
+                  const uint32_t r = rec[k2];
+                  const int c = (int) query(bits, ccount, pref, s_nb, r & 0x7FFFFFFFu);
+                  sum_t += r >> 31 ? -c : c;
+                  smu_t += r >> 31 ? -1 : 1;
+                }
+              }
+              lsum += sum_t;
+              smu_t = __reduce_add_sync(0xffffffffu, smu_t);
+              if (lane == 0 && smu_t) atomicAdd(&s_smu, smu_t);
+            }
+          }
+          __syncthreads();
+        }
+        if (wend < lz) { w0 = wend; continue; }          // the level continues in the next window
+        if (lz > la && tid == NT - 1) { A.smu[rowbase + l] = s_smu; s_smu = 0; }
+        // ---- cross off p_l and its multiples, count the numbers removed first
+        const LevelM P = lm[li];
+        const uint32_t pjn = P.jn8 >> 3;
+        uint32_t rem = 0;
+        if (lflags & 4) {
+          // small prime: AND with its wheel pattern, one owner thread per word
+          const uint32_t p = P.prime;
+          int po = 0;
+          for (int k = 0; c_small_p[k] != p; k++) po += c_small_p[k];
+          // four consecutive words per thread and round (two 16-byte accesses)
+          uint32_t r = (uint32_t) ((P.first + 4 * tid) % p);
+          const uint32_t step = (4 * NT) % p;
+          for (int w = 4 * tid; w - 4 * lane < 8 * nch; w += 4 * NT) {
+            uint32_t d = 0;
+            if (w < wused) {
+              const ulonglong2 o0 = *(const ulonglong2*) (bits + w);
+              const ulonglong2 o1 = *(const ulonglong2*) (bits + w + 2);
+              const uint32_t r1 = r + 1 == p ? 0u : r + 1;
+              const uint32_t r2 = r1 + 1 == p ? 0u : r1 + 1;
+              const uint32_t r3 = r2 + 1 == p ? 0u : r2 + 1;
+              ulonglong2 n0, n1;
+              n0.x = o0.x & pat[po + r];
+              n0.y = (w + 1 < wused) ? (o0.y & pat[po + r1]) : o0.y;
+              n1.x = (w + 2 < wused) ? (o1.x & pat[po + r2]) : o1.x;
+              n1.y = (w + 3 < wused) ? (o1.y & pat[po + r3]) : o1.y;
+              if (n0.x != o0.x || n0.y != o0.y) {
+                *(ulonglong2*) (bits + w) = n0;
+                d = __popcll(o0.x ^ n0.x) + __popcll(o0.y ^ n0.y);
+              }
+              if (n1.x != o1.x || n1.y != o1.y) {
+                *(ulonglong2*) (bits + w + 2) = n1;
+                d += __popcll(o1.x ^ n1.x) + __popcll(o1.y ^ n1.y);
+              }
+            }
+            rem += d;
+            // 2 consecutive lanes own the 8 words of one chunk
+            d += __shfl_down_sync(0xffffffffu, d, 1, 2);
+            if ((lane & 1) == 0 && d) ccount[w >> 3] -= d;
+            r += step;
+            if (r >= p) r -= p;
+          }
+        } else if ((uint32_t) tid < pjn) {
+          // co-factors tid, tid + NT, ...: NT / 8 wheel turns apart, so the
+          // multiples are NT p / 32 half-words apart with the same bit; no two
+          // multiples of one p >= 64 share a half-word: plain updates
+          const uint32_t p = P.prime;
+          const uint32_t off = P.first + p * (s_delta[(P.jn8 & 7) * 32 + lane] + 120u * warp);
+          uint32_t h = off / 120;
+          const uint32_t m = 1u << s_bit[off - 120 * h];
+          const uint32_t hstep = p * NW;
+          for (uint32_t j = tid; j < pjn; j += NT, h += hstep) {
+            const uint32_t old = hw[h];
+            if (old & m) { hw[h] = old & ~m; rem++; atomicSub(&ccount[h >> 4], 1u); }
+          }
+        }
+        if (!(lflags & 4) && pjn <= (uint32_t) NT) {
+          // at most one multiple per thread: the barrier counts the removals
+          const uint32_t rr = (uint32_t) __syncthreads_count(rem != 0);
+          total -= rr;
+          if (rr) dirty = true;
+          if (tid == NT - 1) s_rem[(alone_n + 2) % 3] = 0;
+        } else {
+          rem = __reduce_add_sync(0xffffffffu, rem);
+          if (lane == 0 && rem) atomicAdd(&s_rem[alone_n % 3], rem);
+          __syncthreads();
+          const uint32_t rr = s_rem[alone_n % 3];
+          total -= rr;
+          if (rr) dirty = true;
+          if (tid == NT - 1) s_rem[(alone_n + 2) % 3] = 0;
+        }
+        alone_n++;
+        li++;
       }
     }
     // segment result
@@ -1412,7 +1747,7 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
     __syncthreads();
     if (tid == 0) {
       long long t = 0;
-      for (int i = 0; i < NT / 32; i++) t += s_red[i];
+      for (int i = 0; i < NW; i++) t += s_red[i];
       A.segsum[ws] = t;
     }
   }
@@ -1919,12 +2254,12 @@ static std::vector<int64_t> plan_segments(const SweepProblem& pb, const Tables& 
   return seg;
 }
 
-// levels with p^3 >= high answered in one pass (PCG_SWEEP_GROUP overrides)
+// levels answered together at most (PCG_SWEEP_GROUP overrides; 0: each by itself)
 static int sweep_group_max()
 {
   static const int g = [] {
     const char* e = getenv("PCG_SWEEP_GROUP");
-    const int v = e ? atoi(e) : 32;
+    const int v = e ? atoi(e) : GROUP_MAX;
     return v < 0 ? 0 : (v > GROUP_MAX ? GROUP_MAX : v);
   }();
   return g;
@@ -2069,9 +2404,7 @@ SweepResult run_sweep(Ctx& c, const SweepProblem& pb, const Tuning& tune_in, cud
   const int wq = std::max(8 * NT, 2048);   // whole chunks per thread and per scan lane pair
   words = std::max(words, wq);
   words = (words + wq - 1) / wq * wq;
-  const int cap = 3584;
-  size_t smem = (size_t) words * 8 + PAT_WORDS * 8 + (size_t) (NT + 1) * 8 * 3 + (size_t) (words / 8) * 8 +
-                sizeof(LevelP) * NT + (size_t) cap * 4 + (size_t) NT * 2 + 480 * 2 + (size_t) NT * 4 + 32;
+  const size_t smem = sweep_smem(words, NT);
   if (smem > c.smem_optin) fail(PCG_EINVAL, "segment too large for shared memory");
   int fbytes = pb.gourdon ? c.tab.fd_bytes : c.tab.fr_bytes;
   auto occupancy = [&](int* occ) {
@@ -2163,7 +2496,6 @@ SweepResult run_sweep(Ctx& c, const SweepProblem& pb, const Tuning& tune_in, cud
   a.nq = 1;
   a.rowoff = rowbuf.as<int64_t>();
   a.words = words;
-  a.rec_cap = cap;
   a.primes = c.tab.primes.as<uint32_t>();
   a.nprimes = c.tab.nprimes;
   a.pitab = c.tab.pitab.as<uint64_t>();
@@ -2405,9 +2737,7 @@ void run_sweep_batch(Ctx& c, const std::vector<SweepProblem>& pbs, const Tuning&
   const int wq = std::max(8 * NT, 2048);
   words = std::max(words, wq);
   words = (words + wq - 1) / wq * wq;
-  const int cap = 3584;
-  const size_t smem = (size_t) words * 8 + PAT_WORDS * 8 + (size_t) (NT + 1) * 8 * 3 + (size_t) (words / 8) * 8 +
-                      sizeof(LevelP) * NT + (size_t) cap * 4 + (size_t) NT * 2 + 480 * 2 + (size_t) NT * 4 + 32;
+  const size_t smem = sweep_smem(words, NT);
   if (smem > c.smem_optin) fail(PCG_EINVAL, "segment too large for shared memory");
   const int fbytes = T.fd_bytes;
   int occ = 0;
@@ -2596,7 +2926,6 @@ void run_sweep_batch(Ctx& c, const std::vector<SweepProblem>& pbs, const Tuning&
   a.qs = qbuf.as<SweepQ>();
   a.nq = (int) qs.size();
   a.words = words;
-  a.rec_cap = cap;
   a.primes = T.primes.as<uint32_t>();
   a.nprimes = T.nprimes;
   a.pitab = T.pitab.as<uint64_t>();
@@ -2783,9 +3112,7 @@ SweepResult run_sweep_noalloc(Ctx& c, const SweepProblem& pb, cudaStream_t s)
 
   const int NT = 256;
   const int words = 8192;
-  const int cap = 3584;
-  size_t smem = (size_t) words * 8 + PAT_WORDS * 8 + (size_t) (NT + 1) * 8 * 3 + (size_t) (words / 8) * 8 +
-                sizeof(LevelP) * NT + (size_t) cap * 4 + (size_t) NT * 2 + 480 * 2 + (size_t) NT * 4 + 32;
+  const size_t smem = sweep_smem(words, NT);
   const int fbytes = T.fd_bytes;
   int occ = 0;
   if (fbytes == 2) occupancy_sweep<uint16_t, 256>(&occ, smem);
@@ -2881,7 +3208,6 @@ SweepResult run_sweep_noalloc(Ctx& c, const SweepProblem& pb, cudaStream_t s)
   a.nq = 1;
   a.rowoff = d_row;
   a.words = words;
-  a.rec_cap = cap;
   a.primes = T.primes.as<uint32_t>();
   a.nprimes = T.nprimes;
   a.pitab = T.pitab.as<uint64_t>();
