@@ -651,7 +651,7 @@ static uint64_t table_bytes_beyond(const Ctx& c, int64_t y, int64_t z, int64_t s
 {
   uint64_t b = 0;
   if (y > c.tab.prime_limit) b += (uint64_t) (y / 240 + 1) * (16 + 20) + (uint64_t) pi_estimate(c, y) * 12;
-  if (z > c.tab.fd_z) b += (uint64_t) (wheel2310().to_index((uint64_t) z) + 1) * (2 + 8);
+  if (z > c.tab.fd_z) b += (uint64_t) (wheel2310().to_index((uint64_t) z) + 1) * 2;
   if (sqrtx + 240 > c.tab.pibig_limit) b += (uint64_t) (sqrtx / 240 + 2) * (16 + 20);
   return b;
 }
@@ -694,7 +694,7 @@ static uint64_t phi_query_bytes(const Ctx& c, int64_t x, int64_t a)
            (uint64_t) pi_estimate(c, iroot((u128) x, 3)) * 64;
   const int64_t y = std::max<int64_t>(pa, std::min<int64_t>(sq - 1, 8 * iroot((u128) x, 3)));
   uint64_t b = sweep_device_bytes(c.num_sms, x / y, a + 1, 8192);
-  b += (uint64_t) (wheel2310().to_index((uint64_t) y) + 1) * (2 + 8) + (uint64_t) (y / 240 + 1) * 36;
+  b += (uint64_t) (wheel2310().to_index((uint64_t) y) + 1) * 2 + (uint64_t) (y / 240 + 1) * 36;
   b += (uint64_t) c.num_sms * 8 * 16;                         // the ordinary leaves' partial sums
   return b + 65536;
 }

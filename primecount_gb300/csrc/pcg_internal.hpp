@@ -89,10 +89,6 @@ struct Tables {
   int64_t fr_y = -1;
   int fr_bytes = 2;
   DevBuf factor_dr;
-  // floor((2^64 - 1) / m) for the numbers m coprime to 2310, by factor-table
-  // index, for the indices [0, finv_n)
-  int64_t finv_n = 0;
-  DevBuf finv;
   // PiTable up to sqrt(x) for the A, B, C formulas of pi(x) (no primes array)
   int64_t pibig_limit = -1;
   DevBuf pibig;

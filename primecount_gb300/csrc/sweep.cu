@@ -306,7 +306,7 @@ struct LevelP {
   int64_t hi;         // factor indices (family 1) or prime indices (family 2)
   uint32_t thr;       // factor-table threshold (family 1)
   uint32_t flags;     // 1: leaves, 2: family 2, 4: small prime (pattern cross-off), 16: x / p >= 2^64,
-                      // 32: x / p < 2^64 and every divisor m < 2^31
+                      // 32: every divisor m < 2^30 in a segment of at most LEAF_SPAN numbers, 64: every m < 2^32
 };
 // ... and its multiples in the segment
 struct __align__(16) LevelM {
@@ -347,7 +347,6 @@ struct SweepArgs {
   const void* factor;
   const uint16_t* coprime;
   const int16_t* cindex;
-  const uint64_t* finv;      // floor((2^64 - 1) / m) by factor-table index
   const uint64_t* pmagic;    // floor((2^64 - 1) / p) by prime index
   uint32_t* cnt;            // rows of the wave's items: [rowoff[i], rowoff[i] + bglob + 1)
   int32_t* smu;             // same cells
@@ -448,14 +447,6 @@ __device__ __forceinline__ uint32_t before_chunk(const uint32_t* __restrict__ cc
 // mask_le(r) from a shared table of the counts of wheel residues <= r
 static __device__ __forceinline__ uint64_t mask_le_t(const uint8_t* nbt, uint32_t r) { return low_bits(nbt[r]); }
 
-// dpi with the shared residue-count table
-static __device__ __forceinline__ int64_t dpi_t(const uint64_t* __restrict__ pt, const uint8_t* nbt, uint64_t x)
-{
-  if (x < 6) return (0x322100u >> (4 * x)) & 15u;
-  const uint64_t i = x / 240;
-  return (int64_t) (pt[2 * i] + __popcll(pt[2 * i + 1] & mask_le_t(nbt, (uint32_t) (x - 240 * i))));
-}
-
 // # unsieved numbers in [low, low + off]: the chunk prefix plus the popcounts
 // of the chunk's words up to the word of off, its 8 words read at once
 __device__ __forceinline__ uint32_t query(const uint64_t* __restrict__ bits, const uint32_t* __restrict__ ccount,
@@ -475,47 +466,59 @@ __device__ __forceinline__ uint32_t query(const uint64_t* __restrict__ bits, con
          part(5, w45.y) + part(6, w67.x) + part(7, w67.y);
 }
 
-// This lane's part of the sum of the chunk counts [0, ch): the lane takes the
-// 4-chunk groups lane, lane + 32, ... (16-byte loads, ch <= the number of
-// chunks, a multiple of 4), four groups' loads in flight together
-__device__ __forceinline__ uint32_t chunk_sum_below(const uint32_t* __restrict__ ccount, uint32_t ch, int lane)
+// Offset of the leaf n = floor(xp / m) in the segment [low, ...), xp = x / p
+// given by its low word: r = xp - low m lies in [0, span m), so xp's high
+// word is not needed, and n - low = floor(r / m) < span comes from a
+// single-precision quotient.  Relative error: 2^-24 for m, 2^-23 for its
+// approximate reciprocal, 2^-23 for r, 2^-24 for the product, below 0.75 for
+// span <= 2^21 (LEAF_SPAN), so the quotient is off by at most one and the
+// remainder corrects it.  No reciprocal table: the gather of 8 bytes per leaf
+// was the longest wait of the dense segments.
+#define LEAF_SPAN (1u << 21)
+static __device__ __forceinline__ uint32_t leaf_quotient(uint64_t r, uint32_t m)
 {
-  uint32_t part = 0;
-  for (uint32_t i0 = 0; i0 < ch; i0 += 512) {
-    uint4 v[4];
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-      const uint32_t i = i0 + 128 * u + 4 * lane;
-      v[u] = i < ch ? *(const uint4*) (ccount + i) : make_uint4(0u, 0u, 0u, 0u);
-    }
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-      const uint32_t i = i0 + 128 * u + 4 * lane;
-      part += v[u].x + (i + 1 < ch ? v[u].y : 0u) + (i + 2 < ch ? v[u].z : 0u) + (i + 3 < ch ? v[u].w : 0u);
-    }
-  }
-  return part;
+  float inv;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(__uint2float_rn(m)));
+  const float rf = __fmaf_rn(__uint2float_rn((uint32_t) (r >> 32)), 4294967296.0f, __uint2float_rn((uint32_t) r));
+  return __float2uint_rz(rf * inv);
 }
 
-// Shared-memory atomics under a predicate, without a branch: several stay in
-// flight together.  and_if: clears bit m of the word at a, returns the bit as
-// it was (m when on is false).
-static __device__ __forceinline__ uint32_t and_if(bool on, uint32_t* a, uint32_t m)
+// m < 2^30: the remainder fits 32 signed bits
+static __device__ __forceinline__ uint32_t leaf_narrow(uint64_t xlo, uint64_t low, uint32_t m)
 {
-  uint32_t old = m;
-  asm volatile("{ .reg .pred p; setp.ne.u32 p, %1, 0; @p atom.shared.and.b32 %0, [%2], %3; }"
-               : "+r"(old)
-               : "r"((uint32_t) on), "r"((uint32_t) __cvta_generic_to_shared(a)), "r"(~m)
-               : "memory");
-  return old & m;
+  const uint64_t r = xlo - low * m;
+  uint32_t d = leaf_quotient(r, m);
+  const int32_t t = (int32_t) ((uint32_t) r - d * m);
+  if (t < 0) d--;
+  if (t >= (int32_t) m) d++;
+  return d;
 }
 
-static __device__ __forceinline__ void dec_if(bool on, uint32_t* a)
+// m < 2^32, any segment (below 2^23 numbers: the quotient is off by at most 3)
+static __device__ __forceinline__ uint32_t leaf_wide(uint64_t xlo, uint64_t low, uint32_t m)
 {
-  asm volatile("{ .reg .pred p; setp.ne.u32 p, %0, 0; @p red.shared.add.u32 [%1], %2; }"
-               :
-               : "r"((uint32_t) on), "r"((uint32_t) __cvta_generic_to_shared(a)), "r"(0xFFFFFFFFu)
-               : "memory");
+  const uint64_t r = xlo - low * m;
+  uint32_t d = leaf_quotient(r, m);
+  int64_t t = (int64_t) (r - (uint64_t) d * m);
+  while (t < 0) { t += m; d--; }
+  while (t >= (int64_t) m) { t -= m; d++; }
+  return d;
+}
+
+// Shared-memory atomics of the lanes with on, without a branch: the others
+// update word lane of the array by nothing.  (A predicated atomic is compiled
+// to a branch around it: 55 cycles a warp each, one after another; these
+// overlap, 2 cycles each per SM.)  and_if: clears bit m of a[i], returns the
+// bit as it was (m when on is false).
+static __device__ __forceinline__ uint32_t and_if(bool on, uint32_t* a, uint32_t i, uint32_t m)
+{
+  const uint32_t old = atomicAnd(&a[on ? i : threadIdx.x & 31], on ? ~m : 0xFFFFFFFFu);
+  return on ? old & m : m;
+}
+
+static __device__ __forceinline__ void dec_if(bool on, uint32_t* a, uint32_t i)
+{
+  atomicSub(&a[on ? i : threadIdx.x & 31], on ? 1u : 0u);
 }
 
 // Record of one table entry: the offset of the leaf in the segment (low OB
@@ -524,18 +527,18 @@ static __device__ __forceinline__ void dec_if(bool on, uint32_t* a)
 #define REC_NONE 0xFFFFFFFFu
 // table entries per thread and round of the record phase
 #define PA_UNROLL 8
-// a level answered alone with at most this many record slots in a window
-// goes without a chunk prefix scan
-#define SMALL_QUERIES 32
-// factor-table indices below this one are numbers below 2^31
-#define NARROW_INDEX 446000000ll
+// table entries per lane and round of a level answered alone
+#define SOLO_UNROLL 14
+// factor-table indices below these are numbers below 2^30 and 2^32
+#define NARROW_INDEX 223000000ll
+#define WIDE_INDEX 892000000ll
 // a level answered alone with more records than this uses prefix counts per
 // word where they fit (see k_sweep)
 #define WORD_RECORDS 1024
 // levels answered together at most (see k_sweep)
 #define GROUP_MAX 256
 // a level with more records than this is answered alone
-#define SOLO_RECORDS 512
+#define SOLO_RECORDS 256
 // a group holds at most this many records, and levels times records; with
 // more than LANE_RECORDS in at most LANE_LEVELS levels, a thread per record
 #define GROUP_RECORDS 1024
@@ -618,9 +621,12 @@ static __device__ __forceinline__ uint32_t removed_le(const LevelM& Q, uint32_t 
 // with levels times records: GROUP_WORK and the p / 32 levels of a full
 // segment are where longer groups stop gaining (p / 24 and p / 48: 0.5-1 %
 // slower).  A level with more than SOLO_RECORDS records fills the block by
-// itself and needs no corrections (256: the same, 1024: 2-8 % slower).
-// Measured on a GB300: D(1e20) 1323 -> 947 ms, D(1e18) 89.2 -> 58.4 ms,
-// D(1e15) 3.38 -> 2.89 ms, S2_hard(1e17) 42.0 -> 27.9 ms.
+// itself and needs no corrections (128 and 384: up to 4 % slower).
+// Measured on a GB300, levels one at a time -> groups: D(1e20) 1323 -> 947 ms,
+// D(1e18) 89.2 -> 58.4 ms, D(1e15) 3.38 -> 2.89 ms, S2_hard(1e17) 42.0 -> 27.9 ms;
+// then leaf offsets without the reciprocal table and a level alone streamed
+// by independent warps: 797, 50.1, 2.70, 25.8 ms; then branch-free shared
+// atomics: 775, 48.4, 2.65, 25.2 ms.
 // levels per batch (a thread each)
 constexpr int sweep_batch(int nt) { return nt < 256 ? nt : 256; }
 
@@ -684,7 +690,6 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
   __shared__ int s_gsmu[2][LB];                        // signed leaf counts of a group's levels, by group parity
   __shared__ int s_smu;
   __shared__ int s_ncoll;
-  __shared__ int s_ncomp[2];                           // accepted records of a compacted window, by window parity
   __shared__ int s_stop;
   __shared__ uint32_t s_rem[3];
   __shared__ uint32_t s_total;
@@ -787,7 +792,6 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
       s_total = 0; s_rem[0] = s_rem[1] = s_rem[2] = 0; s_smu = 0; s_stop = 0x7FFFFFFF;
       s_mlow = UINT64_MAX / (uint64_t) low1;
       s_mhigh = UINT64_MAX / (uint64_t) high;
-      s_ncomp[0] = s_ncomp[1] = 0;
       s_ncoll = 0;
     }
     __syncthreads();
@@ -814,7 +818,6 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
     long long lsum = 0;
     unsigned long long nleaves = 0, ntwo = 0, nentries = 0;
     unsigned alone_n = 0;  // levels answered alone so far (rotates s_rem)
-    unsigned win = 0;      // windows of the segment so far (parity selects the compaction counter)
 
     for (int b0 = 1; b0 <= Bs; b0 += LB) {
       // ---- per-level parameters of levels b0 .. b0+LB-1, one thread each
@@ -908,7 +911,8 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
               E = P.hi - P.lo;
               P.xlo = xt[0];
               if (xt[1]) P.flags |= 16;
-              else if ((P.flags & 2) ? A.pi_max < (1ll << 31) : P.hi < NARROW_INDEX) P.flags |= 32;
+              if (span <= LEAF_SPAN && ((P.flags & 2) ? A.pi_max < (1ll << 30) : P.hi < NARROW_INDEX)) P.flags |= 32;
+              else if ((P.flags & 2) || P.hi < WIDE_INDEX) P.flags |= 64;
             }
           }
         }
@@ -953,7 +957,6 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
       if (tid < nb && !(lp[tid].flags & 2)) nentries += (unsigned long long) (loff[tid + 1] - loff[tid]);
 
       int li = 0;          // next batch level to finish
-      int64_t w0 = 0;      // first flat record of the window
       while (li < nb) {
         // the next level answered alone, from li on
         int ns = nb;
@@ -962,183 +965,26 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
           if (w == (li >> 5)) m &= 0xffffffffu << (li & 31);
           if (m) { ns = 32 * w + __ffs((int) m) - 1; break; }
         }
-        const bool solo = ns == li;
-        // the window: of a level alone, its next records; else the records of
-        // the levels li .. ns - 1 from level li on, as many as fit
-        const int64_t la = loff[li], lz = loff[li + 1];
-        if (w0 < la) w0 = la;
-        const int nrec = (int) dmin(REC_CAP, (solo ? lz : loff[ns]) - w0);
-        const int64_t wend = w0 + nrec;
-        // the levels before lfull lie wholly in the window
-        int lfull = ns;
-        if (!solo && loff[ns] > wend) {
-          int lo = li;
-          while (lo < lfull) {
-            const int mid = (lo + lfull + 1) >> 1;
-            if (loff[mid] <= wend) lo = mid; else lfull = mid - 1;
-          }
-        }
-        win++;
-        if (tid == 0) s_ncomp[(win + 1) & 1] = 0;
-        // ---- phase A: the window's leaf records, PA_UNROLL entries per thread
-        // in three stages so that their table loads, then their reciprocal
-        // loads, are in flight together
-        if (solo && nrec > 0) {
-          // one level: its constants held in registers, no level lookup per
-          // entry.  Accepted FactorTable entries are compacted to the front
-          // (their order is free, all are answered against one bitmap state),
-          // the rejected ones are dropped.
-          const LevelP& Q = lp[li];
-          const int64_t hi0 = Q.hi - (w0 - la);              // table index of entry f is hi0 - f
-          const bool two = (Q.flags & 2) != 0;
-          const bool compact = !two, narrow = (Q.flags & 32) != 0;
-          const uint32_t thr = Q.thr;
-          const uint64_t* xt = PQ.xp_tab + 3 * (int64_t) (b0 + li);
-          const uint64_t xlo = xt[0], xhi = xt[1];
-          unsigned nl = 0;
-          if (compact && hi0 < 0x7FFFFFFFll) {
-            // filter first: the accepted entries' indices (bit 31: negative
-            // sign) are compacted, then their reciprocals loaded and their
-            // divisions done on full warps (about 1/3 of the entries pass)
-            for (int f0 = tid; f0 - lane < nrec; f0 += PA_UNROLL * NT) {
-              uint32_t fv[PA_UNROLL];
-#pragma unroll
-              for (int u = 0; u < PA_UNROLL; u++) {
-                const int f = f0 + u * NT;
-                fv[u] = f < nrec ? (uint32_t) __ldg(&factor[hi0 - f]) : 0u;
-              }
-              unsigned bal[PA_UNROLL];
-              int tot = 0;
-#pragma unroll
-              for (int u = 0; u < PA_UNROLL; u++) {
-                bal[u] = __ballot_sync(0xffffffffu, f0 + u * NT < nrec && fv[u] > thr);
-                tot += __popc(bal[u]);
-              }
-              int base = 0;
-              if (lane == 0 && tot) base = atomicAdd(&s_ncomp[win & 1], tot);
-              base = __shfl_sync(0xffffffffu, base, 0);
-              const unsigned lt = (1u << lane) - 1u;
-              int pos = base;
-#pragma unroll
-              for (int u = 0; u < PA_UNROLL; u++) {
-                if ((bal[u] >> lane) & 1u)
-                  rec[pos + __popc(bal[u] & lt)] =
-                      (uint32_t) (hi0 - (f0 + u * NT)) | ((fv[u] & 1u) ? 0u : 0x80000000u);
-                pos += __popc(bal[u]);
-              }
-              __syncwarp();
-              if (narrow) {
-                // m < 2^31: the remainder less the true quotient's is below
-                // 2 m < 2^32, so its low word decides the correction
-                for (int j0 = 0; j0 < tot; j0 += 32 * 4) {
-                  uint32_t e[4];
-                  uint64_t mv[4];
-#pragma unroll
-                  for (int d = 0; d < 4; d++) {
-                    const int j = j0 + 32 * d + lane;
-                    e[d] = j < tot ? rec[base + j] : 0u;
-                    mv[d] = j < tot ? __ldg(&A.finv[e[d] & 0x7FFFFFFFu]) : 0ull;
-                  }
-#pragma unroll
-                  for (int d = 0; d < 4; d++) {
-                    const int j = j0 + 32 * d + lane;
-                    const uint32_t mi = e[d] & 0x7FFFFFFFu, m32 = 2310u * (mi / 480u) + cop[mi % 480u];
-                    const uint32_t t = (uint32_t) __umul64hi(xlo, mv[d]);
-                    const uint32_t r = t - (uint32_t) low + ((uint32_t) xlo - t * m32 >= m32 ? 1u : 0u);
-                    if (j < tot) rec[base + j] = r | (e[d] & 0x80000000u);
-                  }
-                }
-              } else
-              for (int j0 = 0; j0 < tot; j0 += 32 * 4) {
-                uint32_t e[4];
-                uint64_t mv[4];
-#pragma unroll
-                for (int d = 0; d < 4; d++) {
-                  const int j = j0 + 32 * d + lane;
-                  e[d] = j < tot ? rec[base + j] : 0u;
-                  mv[d] = (j < tot && xhi == 0) ? __ldg(&A.finv[e[d] & 0x7FFFFFFFu]) : 0ull;
-                }
-#pragma unroll
-                for (int d = 0; d < 4; d++) {
-                  const int j = j0 + 32 * d + lane;
-                  if (j < tot) {
-                    const uint32_t mi = e[d] & 0x7FFFFFFFu;
-                    const uint64_t m = 2310ull * (mi / 480u) + cop[mi % 480u];
-                    const uint64_t nn = xhi == 0 ? div_magic(xlo, m, mv[d]) : div_xp(xlo, xhi, m);
-                    rec[base + j] = (uint32_t) (nn - (uint64_t) low) | (e[d] & 0x80000000u);
-                  }
-                }
-              }
-              if (lane == 0) nl += (unsigned) tot;
-            }
-          } else
-          // f0 - lane is the same for the lanes of a warp: the loop is warp-uniform
-          for (int f0 = tid; f0 - lane < nrec; f0 += PA_UNROLL * NT) {
-            uint32_t fv[PA_UNROLL];
-            uint64_t minv[PA_UNROLL];
-#pragma unroll
-            for (int u = 0; u < PA_UNROLL; u++) {
-              const int f = f0 + u * NT;
-              fv[u] = 0;
-              minv[u] = 0;
-              if (f < nrec) {
-                const int64_t idx = hi0 - f;
-                if (two) {
-                  fv[u] = __ldg(&A.primes[idx]);
-                  minv[u] = __ldg(&A.pmagic[idx]);
-                } else {
-                  fv[u] = (uint32_t) __ldg(&factor[idx]);
-                  minv[u] = __ldg(&A.finv[idx]);
-                }
-              }
-            }
-            uint32_t rv[PA_UNROLL];
-#pragma unroll
-            for (int u = 0; u < PA_UNROLL; u++) {
-              const int f = f0 + u * NT;
-              rv[u] = REC_NONE;
-              if (f < nrec) {
-                const int64_t idx = hi0 - f;
-                uint64_t m = 0;
-                if (two) m = fv[u];
-                else if (fv[u] > thr) m = 2310ull * ((uint64_t) idx / 480) + cop[(uint64_t) idx % 480];
-                if (m) {
-                  const uint64_t nn = xhi == 0 ? div_magic(xlo, m, minv[u]) : div_xp(xlo, xhi, m);
-                  uint32_t r = (uint32_t) (nn - (uint64_t) low);
-                  if (!two && !(fv[u] & 1)) r |= 0x80000000u;
-                  rv[u] = r;
-                  nl++;
-                }
-                if (!compact) rec[f] = rv[u];
-              }
-            }
-            if (compact) {
-              // one shared counter update per warp for its PA_UNROLL x 32 entries
-              unsigned bal[PA_UNROLL];
-              int tot = 0;
-#pragma unroll
-              for (int u = 0; u < PA_UNROLL; u++) {
-                bal[u] = __ballot_sync(0xffffffffu, rv[u] != REC_NONE);
-                tot += __popc(bal[u]);
-              }
-              int base = 0;
-              if (lane == 0 && tot) base = atomicAdd(&s_ncomp[win & 1], tot);
-              base = __shfl_sync(0xffffffffu, base, 0);
-              const unsigned lt = (1u << lane) - 1u;
-#pragma unroll
-              for (int u = 0; u < PA_UNROLL; u++) {
-                if (rv[u] != REC_NONE) rec[base + __popc(bal[u] & lt)] = rv[u];
-                base += __popc(bal[u]);
-              }
+        if (ns > li) {
+          // ---- levels li .. ns - 1 in groups.  The window: their records
+          // from level li on, as many as fit; the levels before lfull lie
+          // wholly in it
+          const int64_t w0 = loff[li];
+          const int nrec = (int) dmin(REC_CAP, loff[ns] - w0);
+          const int64_t wend = w0 + nrec;
+          int lfull = ns;
+          if (loff[ns] > wend) {
+            int lo = li;
+            while (lo < lfull) {
+              const int mid = (lo + lfull + 1) >> 1;
+              if (loff[mid] <= wend) lo = mid; else lfull = mid - 1;
             }
           }
-          nleaves += nl;
-          if (two) ntwo += nl;
-        }
-        if (!solo && nrec > 0) {
-          // the window's records belong to levels li .. lw; those of a level
-          // that ends beyond the window are made again with the next one and
-          // not counted here
+          if (nrec > 0) {
+          // the records, PA_UNROLL entries per thread so that their table
+          // loads are in flight together; they belong to levels li .. lw,
+          // those of a level that ends beyond the window are made again with
+          // the next one and not counted here
           const int lw = min(lfull, ns - 1);
           const int nfull = (int) (loff[lfull] - w0);
           for (int f0 = tid; f0 < nrec; f0 += PA_UNROLL * NT) {
@@ -1167,22 +1013,13 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
               fv[u] = 0;
               if (f >= nrec) jl[u] = -1;
             }
-            // table entries and the reciprocals of their divisors, loaded
-            // together (the reciprocal of a rejected entry goes unused)
-            uint64_t mdiv[PA_UNROLL], minv[PA_UNROLL];
+            uint64_t mdiv[PA_UNROLL];
 #pragma unroll
             for (int u = 0; u < PA_UNROLL; u++) {
-              minv[u] = 0;
               if (jl[u] >= 0) {
                 const LevelP& Q = lp[jl[u]];
                 const int64_t idx = Q.hi - el[u];
-                if (Q.flags & 2) {
-                  fv[u] = __ldg(&A.primes[idx]);
-                  minv[u] = __ldg(&A.pmagic[idx]);
-                } else {
-                  fv[u] = (uint32_t) __ldg(&factor[idx]);
-                  minv[u] = __ldg(&A.finv[idx]);
-                }
+                fv[u] = (Q.flags & 2) ? __ldg(&A.primes[idx]) : (uint32_t) __ldg(&factor[idx]);
               }
             }
             // the divisor m of each accepted entry (0: rejected by the
@@ -1214,16 +1051,10 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
                 const LevelP& Q = lp[jl[u]];
                 uint32_t r = REC_NONE;
                 if (mdiv[u]) {
-                  uint32_t nn;
-                  if (Q.flags & 32) {
-                    const uint32_t m32 = (uint32_t) mdiv[u];
-                    nn = (uint32_t) __umul64hi(Q.xlo, minv[u]);
-                    nn += (uint32_t) Q.xlo - nn * m32 >= m32 ? 1u : 0u;
-                  } else {
-                    nn = (uint32_t) ((Q.flags & 16) ? div_xp(Q.xlo, PQ.xp_tab[3 * (int64_t) (b0 + jl[u]) + 1], mdiv[u])
-                                                    : div_magic(Q.xlo, mdiv[u], minv[u]));
-                  }
-                  r = (nn - (uint32_t) low) | ((uint32_t) jl[u] << OB);
+                  if (Q.flags & 32) r = leaf_narrow(Q.xlo, (uint64_t) low, (uint32_t) mdiv[u]);
+                  else if (Q.flags & 64) r = leaf_wide(Q.xlo, (uint64_t) low, (uint32_t) mdiv[u]);
+                  else r = (uint32_t) (div_xp(Q.xlo, PQ.xp_tab[3 * (int64_t) (b0 + jl[u]) + 1], mdiv[u]) - (uint64_t) low);
+                  r |= (uint32_t) jl[u] << OB;
                   if (!(Q.flags & 2) && !(fv[u] & 1)) r |= 0x80000000u;
                   if (f < nfull) {
                     nleaves++;
@@ -1235,10 +1066,8 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
             }
           }
         }
-        if (nrec > 0) __syncthreads();
+          if (nrec > 0) __syncthreads();
 
-        if (!solo) {
-          // ---- phase B, groups of levels whose records lie in the window
           int pl = li, plen = 0;                        // the previous group, its signs not written yet
           while (li < lfull) {
             const uint32_t wb0 = wofs[li];
@@ -1399,10 +1228,10 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
 #pragma unroll
                   for (int d = 0; d < 4; d++) on[d] = ((j < nw[d] ? mk[w[d] + j] : 0u) >> lane) & 1u;
 #pragma unroll
-                  for (int d = 0; d < 4; d++) old[d] = and_if(on[d], hw + h[d], m[d]);
+                  for (int d = 0; d < 4; d++) old[d] = and_if(on[d], hw, h[d], m[d]);
 #pragma unroll
                   for (int d = 0; d < 4; d++) {
-                    dec_if(on[d] && old[d], ccount + (h[d] >> 4));
+                    dec_if(on[d] && old[d], ccount, h[d] >> 4);
                     if (!old[d]) lost |= 1u << d;
                     h[d] += p[d];
                   }
@@ -1431,10 +1260,10 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
 #pragma unroll
                 for (int d = 0; d < 4; d++) on[d] = ((wi + d < e ? mk[wi + d] : 0u) >> lane) & 1u;
 #pragma unroll
-                for (int d = 0; d < 4; d++) old[d] = and_if(on[d], hw + (h + d * p), m);
+                for (int d = 0; d < 4; d++) old[d] = and_if(on[d], hw, h + d * p, m);
 #pragma unroll
                 for (int d = 0; d < 4; d++) {
-                  dec_if(on[d] && old[d], ccount + ((h + d * p) >> 4));
+                  dec_if(on[d] && old[d], ccount, (h + d * p) >> 4);
                   if (!old[d]) lost |= 1u << d;
                 }
                 while (lost) {
@@ -1579,83 +1408,128 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
           continue;
         }
 
-        // ---- phase B of a level alone
+        // ---- a level answered alone: against one bitmap state, so the warps
+        // stream the level's entries independently, chunks of up to 448 in
+        // turn: the accepted ones' positions are compacted into the warp's
+        // part of rec (about 1/3 pass), the next chunk's entries loaded, then
+        // the leaves divided and counted on full warps.  One barrier at the
+        // end of the level instead of two per window of records.
         const uint32_t lflags = lp[li].flags;
         const int l = b0 + li;
-        if (w0 == la && tid == NT - 1) A.cnt[rowbase + l] = total;   // the last thread: rarely a multiple to cross off
-        const int rb = (lflags & 2) ? nrec : s_ncomp[win & 1];       // records still to answer
-        if (nrec > 0 && rb > 0) {
-          if (dirty && rb <= SMALL_QUERIES) {
-            // a few records: a warp per record sums the chunk counts below
-            // the record's chunk itself, instead of a block-wide prefix
-            // scan (the prefix array stays out of date)
-            int smu_w = 0;
-            for (int k2 = warp; k2 < rb; k2 += NW) {
-              const uint32_t r = rec[k2];
-              const uint32_t off = r & 0x7FFFFFFFu;
-              const uint32_t wd = off / 240, ch = wd >> 3, kw = wd & 7;
-              uint32_t part = chunk_sum_below(ccount, ch, lane);
-              if (lane < 8) {
-                const uint64_t v = bits[8 * ch + lane];
-                const uint32_t j = (uint32_t) lane;
-                part += (uint32_t) __popcll(j < kw ? v : (j == kw ? (v & mask_le_t(s_nb, off - wd * 240)) : 0ull));
-              }
-              const uint32_t c = __reduce_add_sync(0xffffffffu, part);
-              if (r >> 31) { if (lane == 0) lsum -= c; smu_w--; }
-              else { if (lane == 0) lsum += c; smu_w++; }
-            }
-            if (lane == 0 && smu_w) atomicAdd(&s_smu, smu_w);
-          } else {
-            if (dirty) { scan_chunks(ccount, pref, n4, wtmp); dirty = false; wp_ok = false; }
-            const bool by_word = wp_fits && lz - la > WORD_RECORDS;
-            if (by_word && !wp_ok) {
-              for (int c = tid; c < nchu; c += NT) {
-                const ulonglong2* q = (const ulonglong2*) (bits + 8 * c);
-                uint32_t run = before_chunk(ccount, pref, (uint32_t) c);
-                uint4 o[2];
+        if (tid == NT - 1) A.cnt[rowbase + l] = total;   // the last thread: rarely a multiple to cross off
+        const int64_t E2 = loff[li + 1] - loff[li];
+        if (E2 > 0) {
+          if (dirty) { scan_chunks(ccount, pref, n4, wtmp); dirty = false; wp_ok = false; }
+          const bool by_word = wp_fits && E2 > WORD_RECORDS;
+          if (by_word && !wp_ok) {
+            for (int c = tid; c < nchu; c += NT) {
+              const ulonglong2* q = (const ulonglong2*) (bits + 8 * c);
+              uint32_t run = before_chunk(ccount, pref, (uint32_t) c);
+              uint4 o[2];
 #pragma unroll
-                for (int i = 0; i < 2; i++) {
-                  const ulonglong2 a = q[2 * i], b = q[2 * i + 1];
-                  o[i].x = run; run += __popcll(a.x);
-                  o[i].y = run; run += __popcll(a.y);
-                  o[i].z = run; run += __popcll(b.x);
-                  o[i].w = run; run += __popcll(b.y);
-                }
-                ((uint4*) (wpre + 8 * c))[0] = o[0];
-                ((uint4*) (wpre + 8 * c))[1] = o[1];
+              for (int i = 0; i < 2; i++) {
+                const ulonglong2 a = q[2 * i], b = q[2 * i + 1];
+                o[i].x = run; run += __popcll(a.x);
+                o[i].y = run; run += __popcll(a.y);
+                o[i].z = run; run += __popcll(b.x);
+                o[i].w = run; run += __popcll(b.y);
               }
-              wp_ok = true;
-              __syncthreads();
+              ((uint4*) (wpre + 8 * c))[0] = o[0];
+              ((uint4*) (wpre + 8 * c))[1] = o[1];
             }
-            if (32 * warp < rb) {
-              // a thread's counts fit 32 bits: at most 3584 / 128 records of 2^21 numbers
-              int smu_t = 0, sum_t = 0;
-              if (by_word) {
-#pragma unroll 2
-                for (int k2 = tid; k2 < rb; k2 += NT) {
-                  const uint32_t r = rec[k2], off = r & 0x7FFFFFFFu;
-                  const uint32_t w = off / 240;
-                  const int c = (int) (wpre[w] + (uint32_t) __popcll(bits[w] & mask_le_t(s_nb, off - 240 * w)));
-                  sum_t += r >> 31 ? -c : c;
-                  smu_t += r >> 31 ? -1 : 1;
+            wp_ok = true;
+            __syncthreads();
+          }
+          const uint64_t xlo = lp[li].xlo;
+          const int64_t hi0 = lp[li].hi;                   // entry f has the table index hi0 - f
+          int smu_t = 0;
+          // the numbers of [low, low + off] left
+          auto count = [&](uint32_t off) -> int {
+            if (!by_word) return (int) query(bits, ccount, pref, s_nb, off);
+            const uint32_t w = off / 240;
+            return (int) (wpre[w] + (uint32_t) __popcll(bits[w] & mask_le_t(s_nb, off - 240 * w)));
+          };
+          if (lflags & 2) {
+            // two-prime leaves: every entry is one, all signs positive
+            for (int64_t f = tid; f < E2; f += NT) {
+              const uint32_t q = __ldg(&A.primes[hi0 - f]);
+              lsum += count((lflags & 32) ? leaf_narrow(xlo, (uint64_t) low, q) : leaf_wide(xlo, (uint64_t) low, q));
+              smu_t++;
+            }
+            nleaves += (unsigned) smu_t;
+            ntwo += (unsigned) smu_t;
+          } else {
+            const uint32_t thr = lp[li].thr;
+            const int ch = (int) dmin(32 * SOLO_UNROLL, 32 * ((E2 + 32 * NW - 1) / (32 * NW)));
+            uint16_t* const wl = (uint16_t*) rec + warp * 32 * SOLO_UNROLL;
+            uint32_t fv[SOLO_UNROLL];
+            auto load = [&](int64_t f0) {
+              const int n = (int) dmin(ch, E2 - f0);
+              const FT* const t = factor + (hi0 - f0) - lane;
+#pragma unroll
+              for (int u = 0; u < SOLO_UNROLL; u++) fv[u] = 32 * u + lane < n ? (uint32_t) __ldg(t - 32 * u) : 0u;
+            };
+            int64_t f0 = (int64_t) warp * ch;
+            if (f0 < E2) load(f0);
+            for (; f0 < E2; f0 += NW * ch) {
+              int tot = 0;
+              const unsigned lt = (1u << lane) - 1u;
+#pragma unroll
+              for (int u = 0; u < SOLO_UNROLL; u++) {
+                const bool acc = fv[u] > thr;              // 0 beyond the chunk: no entry passes thr >= 1
+                const unsigned bal = __ballot_sync(0xffffffffu, acc);
+                if (acc) wl[tot + __popc(bal & lt)] = (uint16_t) ((32 * u + lane) | ((fv[u] & 1u) ? 0u : 0x8000u));
+                tot += __popc(bal);
+              }
+              if (f0 + NW * ch < E2) load(f0 + NW * ch);
+              __syncwarp();
+              int sum_t = 0;                               // at most 14 counts below 2^23
+              if ((lflags & 32) && by_word) {
+                const uint32_t c0 = (uint32_t) (hi0 - f0);
+                for (int j0 = 0; j0 < tot; j0 += 32 * 4) {
+                  uint32_t e[4], off[4];
+#pragma unroll
+                  for (int d = 0; d < 4; d++) e[d] = wl[min(j0 + 32 * d + lane, tot - 1)];
+#pragma unroll
+                  for (int d = 0; d < 4; d++) {
+                    const uint32_t mi = c0 - (e[d] & 0x7FFFu);
+                    off[d] = leaf_narrow(xlo, (uint64_t) low, 2310u * (mi / 480u) + cop[mi % 480u]);
+                  }
+#pragma unroll
+                  for (int d = 0; d < 4; d++) {
+                    const int c = count(off[d]);
+                    const bool on = j0 + 32 * d + lane < tot;
+                    sum_t += on ? (e[d] & 0x8000u ? -c : c) : 0;
+                    smu_t += on ? (e[d] & 0x8000u ? -1 : 1) : 0;
+                  }
                 }
               } else {
-                for (int k2 = tid; k2 < rb; k2 += NT) {
-                  const uint32_t r = rec[k2];
-                  const int c = (int) query(bits, ccount, pref, s_nb, r & 0x7FFFFFFFu);
-                  sum_t += r >> 31 ? -c : c;
-                  smu_t += r >> 31 ? -1 : 1;
+                const uint64_t xhi = (lflags & 16) ? PQ.xp_tab[3 * (int64_t) l + 1] : 0ull;
+                for (int j = lane; j < tot; j += 32) {
+                  const uint32_t e = wl[j];
+                  const uint64_t idx = (uint64_t) (hi0 - f0) - (e & 0x7FFFu);
+                  uint32_t off;
+                  if (lflags & (32 | 64)) {
+                    const uint32_t mi = (uint32_t) idx, m = 2310u * (mi / 480u) + cop[mi % 480u];
+                    off = (lflags & 32) ? leaf_narrow(xlo, (uint64_t) low, m) : leaf_wide(xlo, (uint64_t) low, m);
+                  } else {
+                    off = (uint32_t) (div_xp(xlo, xhi, 2310ull * (idx / 480) + cop[idx % 480]) - (uint64_t) low);
+                  }
+                  const int c = count(off);
+                  sum_t += e & 0x8000u ? -c : c;
+                  smu_t += e & 0x8000u ? -1 : 1;
                 }
               }
               lsum += sum_t;
-              smu_t = __reduce_add_sync(0xffffffffu, smu_t);
-              if (lane == 0 && smu_t) atomicAdd(&s_smu, smu_t);
+              if (lane == 0) nleaves += (unsigned) tot;
+              __syncwarp();
             }
           }
+          smu_t = __reduce_add_sync(0xffffffffu, smu_t);
+          if (lane == 0 && smu_t) atomicAdd(&s_smu, smu_t);
           __syncthreads();
+          if (tid == NT - 1) { A.smu[rowbase + l] = s_smu; s_smu = 0; }
         }
-        if (wend < lz) { w0 = wend; continue; }          // the level continues in the next window
-        if (lz > la && tid == NT - 1) { A.smu[rowbase + l] = s_smu; s_smu = 0; }
         // ---- cross off p_l and its multiples, count the numbers removed first
         const LevelM P = lm[li];
         const uint32_t pjn = P.jn8 >> 3;
@@ -1918,16 +1792,6 @@ __global__ void k_prime_magic(const uint32_t* __restrict__ primes, int64_t n, ui
   magic[i] = UINT64_MAX / primes[i];
 }
 
-// floor((2^64 - 1) / m) for the numbers m coprime to 2310 with factor-table
-// index in [0, n)
-__global__ void k_factor_inv(const uint16_t* __restrict__ cop, int64_t n, uint64_t* __restrict__ inv)
-{
-  const int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint64_t m = 2310 * (uint64_t) (i / 480) + cop[i % 480];
-  inv[i] = UINT64_MAX / m;
-}
-
 void ensure_prime_tables(Ctx& c, int64_t limit, cudaStream_t s)
 {
   Tables& t = c.tab;
@@ -2061,17 +1925,6 @@ static void build_factor(Ctx& c, DevBuf& out, int64_t limit, int64_t y, int gour
   }
 }
 
-// reciprocals of the factor-table numbers for the indices [0, n)
-static void ensure_finv(Ctx& c, int64_t n, cudaStream_t s)
-{
-  Tables& t = c.tab;
-  if (t.finv_n >= n) return;
-  t.finv.alloc((size_t) n * 8);
-  k_factor_inv<<<(unsigned) ((n + 255) / 256), 256, 0, s>>>(t.coprime.as<uint16_t>(), n, t.finv.as<uint64_t>());
-  PCG_CUDA(cudaGetLastError());
-  t.finv_n = n;
-}
-
 void ensure_factor_d(Ctx& c, int64_t y, int64_t z, cudaStream_t s)
 {
   Tables& t = c.tab;
@@ -2087,7 +1940,6 @@ void ensure_factor_d(Ctx& c, int64_t y, int64_t z, cudaStream_t s)
   t.fd_bytes = (z <= 386083ll * 386083 - 1 && !force32) ? 2 : 4;
   if (t.fd_bytes == 2) build_factor<uint16_t>(c, t.factor_d, z, y, 1, s);
   else build_factor<uint32_t>(c, t.factor_d, z, y, 1, s);
-  ensure_finv(c, wheel2310().to_index((uint64_t) std::max<int64_t>(z, 1)) + 1, s);
   PCG_CUDA(cudaStreamSynchronize(s));
   t.fd_y = y;
   t.fd_z = z;
@@ -2103,7 +1955,6 @@ void ensure_factor_dr(Ctx& c, int64_t y, cudaStream_t s)
   t.fr_bytes = (y <= 65534ll * 65534 - 1) ? 2 : 4;
   if (t.fr_bytes == 2) build_factor<uint16_t>(c, t.factor_dr, y, y, 0, s);
   else build_factor<uint32_t>(c, t.factor_dr, y, y, 0, s);
-  ensure_finv(c, wheel2310().to_index((uint64_t) std::max<int64_t>(y, 1)) + 1, s);
   PCG_CUDA(cudaStreamSynchronize(s));
   t.fr_y = y;
   t.build_ms += now_ms() - t0;
@@ -2504,7 +2355,6 @@ SweepResult run_sweep(Ctx& c, const SweepProblem& pb, const Tuning& tune_in, cud
   a.coprime = c.tab.coprime.as<uint16_t>();
   a.group_max = tune.group >= 0 ? std::min(tune.group, GROUP_MAX) : sweep_group_max();
   a.cindex = c.tab.cindex.as<int16_t>();
-  a.finv = c.tab.finv.as<uint64_t>();
   a.pmagic = c.tab.pmagic.as<uint64_t>();
   a.cnt = c.cnt.as<uint32_t>();
   a.smu = c.smu.as<int32_t>();
@@ -2934,7 +2784,6 @@ void run_sweep_batch(Ctx& c, const std::vector<SweepProblem>& pbs, const Tuning&
   a.coprime = T.coprime.as<uint16_t>();
   a.group_max = tune.group >= 0 ? std::min(tune.group, GROUP_MAX) : sweep_group_max();
   a.cindex = T.cindex.as<int16_t>();
-  a.finv = T.finv.as<uint64_t>();
   a.pmagic = T.pmagic.as<uint64_t>();
   a.cnt = c.cnt.as<uint32_t>();
   a.smu = c.smu.as<int32_t>();
@@ -3216,7 +3065,6 @@ SweepResult run_sweep_noalloc(Ctx& c, const SweepProblem& pb, cudaStream_t s)
   a.coprime = T.coprime.as<uint16_t>();
   a.group_max = sweep_group_max();
   a.cindex = T.cindex.as<int16_t>();
-  a.finv = T.finv.as<uint64_t>();
   a.pmagic = T.pmagic.as<uint64_t>();
   a.cnt = d_cnt;
   a.smu = d_smu;
