@@ -2041,7 +2041,8 @@ static bool plan_segments_core(const SweepProblem& pb, const Tables& t, int64_t 
                             : std::min(std::sqrt(z), std::sqrt(x / std::max(a, 1.0)));
     return (double) host_pi(t, (uint64_t) std::min(lim, (double) t.prime_limit));
   };
-  const double c_level = 30.0;
+  // a level of a segment costs about as much as this many leaves
+  const double c_level = 100.0;
   auto cell = [&](unsigned k, unsigned step) {
     for (int i = (int) k; i < G; i += (int) step) {
       const double len = g[i + 1] - g[i];
@@ -2057,7 +2058,15 @@ static bool plan_segments_core(const SweepProblem& pb, const Tables& t, int64_t 
   cum[0] = 0;
   for (int i = 0; i < G; i++) cum[i + 1] = cum[i] + cost[i];
   const double total = cum[G];
-  const double target = std::max(total / (grid * 6.0), 1.0);
+  // One segment per CTA while that keeps a segment below 10^7 leaves, else as
+  // many per CTA as it takes, equally many for all: every cut repeats the
+  // chain of levels, which is most of the work of a small x.  Six per CTA
+  // instead: D(1e13) 0.84 -> 0.38 ms, D(1e15) 2.65 -> 1.15 ms, D(1e17) 15.1 ->
+  // 11.2 ms; at 1e18 (45.7 ms by two per CTA) one is 48.4 ms, six 48.4 ms; at
+  // 1e20 segments of 6e6, 1.2e7, 2.4e7: 780, 771, 775 ms.  Below 1000 leaves
+  // a segment is all overhead (D(1e11) 0.19 -> 0.15 ms).
+  const double per_cta = std::max(1.0, std::ceil(total / (grid * 1e7)));
+  const double target = std::max(total / (grid * per_cta), 1000.0);
   // cumulative cost at n (linear inside a grid cell)
   auto C = [&](double n) {
     const int i = (int) (std::upper_bound(g, g + G + 1, n) - g);
@@ -2508,12 +2517,13 @@ SweepResult run_sweep(Ctx& c, const SweepProblem& pb, const Tuning& tune_in, cud
 // Device working memory of one sweep over [0, L) with cols columns, at the
 // default launch shape (words per segment, 2 CTAs per SM): the count and sign
 // rows of a wave, the segment, x / p, row and job tables and the sums.  The
-// segment planner cuts at most about L / (words * 240) + 6 grid segments.
+// segment planner cuts at most L / (words * 240) full segments and, where
+// leaves are dense, a segment per 10^7 leaves or CTA: below as many again.
 uint64_t sweep_device_bytes(int num_sms, int64_t L, int64_t cols, int words)
 {
   if (L <= 0 || cols <= 1) return 0;
   const int64_t grid = (int64_t) num_sms * 2;
-  const int64_t nseg = L / ((int64_t) words * 240) + 6 * grid + 2;
+  const int64_t nseg = 2 * (L / ((int64_t) words * 240)) + 6 * grid + 2;
   const int64_t max_rows = std::max<int64_t>(1, (int64_t) (1ull << 30) / (cols * 8));
   const int64_t wave = std::max<int64_t>(1, std::min<int64_t>({nseg, grid * 8, max_rows}));
   return (uint64_t) (wave * cols * 8 + wave * 16 + (nseg + 1) * 8 + cols * 56 +
@@ -2606,6 +2616,8 @@ void run_sweep_batch(Ctx& c, const std::vector<SweepProblem>& pbs, const Tuning&
     int64_t cols = 0;
   };
   std::vector<Plan> plans(nq);
+  double work_all = 0;
+  for (const SweepProblem& p : pbs) work_all += std::pow((double) p.x, 0.6);
   {
     std::vector<double> dens((size_t) host_pi(T, (uint64_t) std::min<int64_t>(ymax, T.prime_limit)) + 2, 0.0);
     for (size_t b = 1; b < dens.size() && (int64_t) b <= T.nprimes; b++)
@@ -2636,9 +2648,13 @@ void run_sweep_batch(Ctx& c, const std::vector<SweepProblem>& pbs, const Tuning&
             P.xp[3 * b + 1] = (uint64_t) (q >> 64);
             P.xp[3 * b + 2] = q3 > (u128) INT64_MAX ? (uint64_t) INT64_MAX : (uint64_t) q3;
           }
+          // this problem's share of the CTAs (twice: several items per CTA
+          // even out), its work taken as x^0.6
+          const int spread = nq == 1 ? grid
+              : (int) std::max(1.0, std::min((double) grid, std::ceil(2.0 * grid * std::pow((double) x, 0.6) / work_all)));
           // small problems: one cost cell per segment is plenty
           const int G = (int) std::min<int64_t>(PLAN_GRID, std::max<int64_t>(16, 4 * (L / smax + 1)));
-          plan_segments_core(pb, T, L, x_star, pi_sqrt, bglob, smax, grid, dens.data(), 1,
+          plan_segments_core(pb, T, L, x_star, pi_sqrt, bglob, smax, spread, dens.data(), 1,
                              [&](int64_t v) { P.seg.push_back(v); return true; }, G);
           P.q.x_lo = (uint64_t) x;
           P.q.x_hi = (uint64_t) (x >> 64);
