@@ -660,8 +660,8 @@ static uint64_t table_bytes_beyond(const Ctx& c, int64_t y, int64_t z, int64_t s
 static uint64_t psieve_bytes(int64_t lo, int64_t hi)
 {
   if (hi <= lo) return 0;
-  const int64_t seg = 12288ll * 240;
-  return (uint64_t) ((hi - lo) / seg + 2) * 24 + (uint64_t) (isqrt((u128) hi) / 8 + 64) * 12;
+  const int64_t seg = 12288ll * 240;                          // shorter ranges: up to 4 segments per SM
+  return (uint64_t) ((hi - lo) / seg + 1024) * 24 + (uint64_t) (isqrt((u128) hi) / 8 + 64) * 12;
 }
 
 static uint64_t pi_query_bytes(const Ctx& c, u128 x)

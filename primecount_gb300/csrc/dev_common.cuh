@@ -83,6 +83,30 @@ static __device__ __forceinline__ u128 div128(u128 a, uint64_t d)
 }
 
 
+// Wheel patterns of the primes 7..61 (their multiples repeat every p words):
+// the p words of prime p one after another, word r keeping the numbers
+// 240 r + {1, 7, .., 29} (mod 240 p) that p does not divide.  Made at compile
+// time: 64 remainders per word cost a block several microseconds.
+#define PAT_PRIMES 15
+#define PAT_WORDS 491   // 7 + 11 + ... + 61
+struct WheelPatterns { uint64_t w[PAT_WORDS]; };
+constexpr WheelPatterns wheel_patterns()
+{
+  constexpr uint32_t sp[PAT_PRIMES] = {7, 11, 13, 17, 19, 23, 29, 31, 37, 41, 43, 47, 53, 59, 61};
+  constexpr uint32_t off[8] = {1, 7, 11, 13, 17, 19, 23, 29};
+  WheelPatterns t{};
+  int at = 0;
+  for (int i = 0; i < PAT_PRIMES; i++)
+    for (uint32_t r = 0; r < sp[i]; r++) {
+      uint64_t v = 0;
+      for (int j = 0; j < 64; j++)
+        if ((240 * r + 30 * (uint32_t) (j / 8) + off[j % 8]) % sp[i]) v |= 1ull << j;
+      t.w[at++] = v;
+    }
+  return t;
+}
+static __device__ const WheelPatterns g_patterns = wheel_patterns();
+
 // floor(n / q) from m = floor((2^64 - 1) / q), q >= 1: the high product is
 // floor(n / q) or one less
 static __device__ __forceinline__ uint64_t div_magic(uint64_t n, uint64_t q, uint64_t m)

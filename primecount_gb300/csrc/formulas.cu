@@ -572,31 +572,32 @@ __global__ void k_outer_S2e(uint64_t x_lo, uint64_t x_hi, int64_t y, int64_t z, 
 //  * 67 <= p < mid_limit: a warp per prime, lane l owning the multiples p q
 //    with q = c_l (mod 120), c_l the l-th residue coprime to 30.  Those
 //    multiples are 120 p apart, i.e. exactly p 32-bit words (120 numbers) with
-//    the same bit, so the inner loop is one shared atomicAnd and one add;
+//    the same bit, so the inner loop is one shared atomicAnd and one add.  The
+//    first multiples of 32 primes are found at once, a lane each;
 //  * larger p: a lane per prime stepping q along the 30-wheel.
 // ceil(lo / p) comes from a precomputed reciprocal floor((2^64 - 1) / p) and
-// one correction step.
+// one correction step.  Bound by integer issue (the primes' starts and the
+// multiples).  Measured on a GB300: the starts of 32 primes at once and medium
+// primes up to segment / 128 instead of a warp per start and segment / 256:
+// pi(5e9) 1.34 -> 1.20 ms, B of pi(2e19) beside D 84 -> 70 ms.
 #define PS_NT 512
-#define PS_SMALL 15
-#define PS_PAT 491                // 7 + 11 + ... + 61 pattern words
+#define PS_SMALL PAT_PRIMES
 #define PS_GAPS 0x26424246u       // gaps between consecutive wheel offsets, a nibble each
 struct PsArgs {
   uint64_t x_lo, x_hi;
   int64_t lo0;           // first segment start (multiple of 240)
   int64_t end;           // sieve [lo0, end)
-  int64_t seg;           // numbers per segment = words * 240
+  int64_t len;           // numbers per segment = words * 240
   int64_t nseg;
   int64_t qlo, qhi;      // B queries: primes p in (qlo, qhi]
   int32_t mode;          // 0 count, 1 B
-  int32_t words;         // 64-bit words per segment (a multiple of 4096, at most 16384)
+  int32_t words;         // 64-bit words per segment (a multiple of 64, at most 16384)
   int32_t nbase;         // primes >= 67 up to sqrt(end)
   int32_t nmid;          // base[0, nmid) crossed off a warp per prime
   const uint32_t* base;
   const uint64_t* magic; // floor((2^64 - 1) / base[k])
   const uint64_t* pibig; // PiTable bits for the B queries
-  int64_t* seg_c;
-  int64_t* seg_m;
-  int64_t* seg_l;
+  int64_t* seg;          // [nseg][3]: primes of the segment, its B queries, the sum of their counts
   int* queue;
 };
 
@@ -606,8 +607,6 @@ static __device__ __forceinline__ uint64_t ceil_div_magic(uint64_t n, uint32_t p
   if (n - q * p >= p) q++;
   return q + (q * p != n);
 }
-
-__constant__ uint32_t c_ps_small[PS_SMALL] = {7, 11, 13, 17, 19, 23, 29, 31, 37, 41, 43, 47, 53, 59, 61};
 
 __global__ void __launch_bounds__(PS_NT, 2) k_psieve(const PsArgs A)
 {
@@ -626,17 +625,7 @@ __global__ void __launch_bounds__(PS_NT, 2) k_psieve(const PsArgs A)
   const int nch = words / 8;
   const u128 x = ((u128) A.x_hi << 64) | A.x_lo;
   for (int i = tid; i < 120; i += PS_NT) s_bit[i] = (uint8_t) bit_of((uint32_t) i);
-  for (int i = tid; i < PS_PAT; i += PS_NT) {
-    int k = 0, b0 = 0;
-    while (i >= b0 + (int) c_ps_small[k]) { b0 += c_ps_small[k]; k++; }
-    const uint32_t p = c_ps_small[k], r = (uint32_t) (i - b0);
-    uint64_t v = 0;
-    for (int b = 0; b < 64; b++) {
-      const uint32_t n = 240u * r + 30u * (b >> 3) + woff(b & 7);
-      if (n % p) v |= 1ull << b;
-    }
-    pat[i] = v;
-  }
+  for (int i = tid; i < PAT_WORDS; i += PS_NT) pat[i] = g_patterns.w[i];
   uint64_t small_mask = 0;                               // 7..61 in word 0
 #pragma unroll
   for (int i = 0; i < PS_SMALL; i++) small_mask |= 1ull << bit_of(SP[i]);
@@ -647,8 +636,8 @@ __global__ void __launch_bounds__(PS_NT, 2) k_psieve(const PsArgs A)
     __syncthreads();
     const int64_t s = s_s;
     if (s >= A.nseg) break;
-    const uint64_t lo = (uint64_t) (A.lo0 + s * A.seg);
-    const uint64_t hi = (uint64_t) dmin((int64_t) lo + A.seg, A.end);
+    const uint64_t lo = (uint64_t) (A.lo0 + s * A.len);
+    const uint64_t hi = (uint64_t) dmin((int64_t) lo + A.len, A.end);
     const uint32_t span = (uint32_t) (hi - lo);
     const int wused = (int) ((span + 239) / 240);
     const uint32_t nw32 = (span + 119) / 120;
@@ -680,20 +669,33 @@ __global__ void __launch_bounds__(PS_NT, 2) k_psieve(const PsArgs A)
       }
     }
     __syncthreads();
-    // medium primes: a warp per prime, a residue class of q mod 120 per lane
-    for (int k = warp; k < A.nmid; k += PS_NT / 32) {
-      const uint32_t p = A.base[k];
-      if ((uint64_t) p * p >= hi) break;
-      uint64_t qmin = ceil_div_magic(lo, p, A.magic[k]);
-      if (qmin < p) qmin = p;
-      const uint32_t qm = (uint32_t) (qmin % 120);
-      const uint64_t q = qmin + (lane_res >= qm ? lane_res - qm : lane_res + 120 - qm);
-      const uint64_t pq = (uint64_t) p * q;
-      if (pq < hi) {
-        const uint32_t off = (uint32_t) (pq - lo);
+    // medium primes: a warp per prime (primes warp, warp + 16, ...: the small
+    // ones have the most multiples), a residue class of q mod 120 per lane;
+    // lane l first finds the first co-factor >= max(p, lo / p) of the l-th
+    for (int k0 = warp; k0 < A.nmid; k0 += PS_NT) {
+      const int k = k0 + lane * (PS_NT / 32);
+      const int n = min(32, (A.nmid - k0 + PS_NT / 32 - 1) / (PS_NT / 32));
+      uint32_t p = 0, qm = 0;
+      uint32_t o = 0xFFFFFFFFu;                          // offset of p qmin, or nothing to do
+      if (lane < n) {
+        p = A.base[k];
+        if ((uint64_t) p * p < hi) {
+          uint64_t qmin = ceil_div_magic(lo, p, A.magic[k]);
+          if (qmin < p) qmin = p;
+          qm = (uint32_t) (qmin % 120);
+          const uint64_t pq = (uint64_t) p * qmin;
+          if (pq < hi) o = (uint32_t) (pq - lo);
+        }
+      }
+      for (int t = 0; t < n; t++) {
+        const uint32_t ot = __shfl_sync(0xffffffffu, o, t);
+        if (ot == 0xFFFFFFFFu) continue;
+        const uint32_t pt = __shfl_sync(0xffffffffu, p, t), qt = __shfl_sync(0xffffffffu, qm, t);
+        const uint32_t off = ot + pt * (lane_res >= qt ? lane_res - qt : lane_res + 120 - qt);
         uint32_t w = off / 120;
         const uint32_t msk = ~(1u << s_bit[off - 120 * w]);
-        for (; w < nw32; w += p) atomicAnd(&bits32[w], msk);
+        if (off >= span) w = nw32;
+        for (; w < nw32; w += pt) atomicAnd(&bits32[w], msk);
       }
     }
     // large primes: a lane per prime along the 30-wheel
@@ -716,16 +718,16 @@ __global__ void __launch_bounds__(PS_NT, 2) k_psieve(const PsArgs A)
       }
     }
     __syncthreads();
-    // chunk prefix (8 words per chunk; nch / PS_NT chunks per thread)
+    // chunk prefix (8 words per chunk; up to 4 chunks per thread)
     {
-      const int cpt = nch / PS_NT;
+      const int cpt = (nch + PS_NT - 1) / PS_NT;
       const int base = tid * cpt;
       uint32_t loc[4];
       uint32_t sum = 0;
 #pragma unroll
       for (int c = 0; c < 4; c++) {
         uint32_t t = 0;
-        if (c < cpt)
+        if (c < cpt && base + c < nch)
           for (int i = 0; i < 8; i++) t += __popcll(bits[8 * (base + c) + i]);
         loc[c] = t;
         sum += t;
@@ -741,8 +743,8 @@ __global__ void __launch_bounds__(PS_NT, 2) k_psieve(const PsArgs A)
       for (int w = 0; w < warp; w++) run += wt[w];
 #pragma unroll
       for (int c = 0; c < 4; c++)
-        if (c < cpt) { pref[base + c] = run; run += loc[c]; }
-      if (tid == PS_NT - 1 && A.seg_c) A.seg_c[s] = run;
+        if (c < cpt && base + c < nch) { pref[base + c] = run; run += loc[c]; }
+      if (tid == PS_NT - 1) A.seg[3 * s] = run;
       __syncthreads();
     }
     if (A.mode == 1) {
@@ -779,8 +781,8 @@ __global__ void __launch_bounds__(PS_NT, 2) k_psieve(const PsArgs A)
       if (tid == 0) {
         long long a = 0, b = 0;
         for (int i = 0; i < PS_NT / 32; i++) { a += red[0][i]; b += red[1][i]; }
-        A.seg_l[s] = a;
-        A.seg_m[s] = b;
+        A.seg[3 * s + 1] = b;
+        A.seg[3 * s + 2] = a;
       }
     }
   }
@@ -805,101 +807,111 @@ struct PsOut {
 };
 
 // segment words and the warp/lane split of the prime sieve (PCG_PS_WORDS,
-// PCG_PS_MID override them; words must be 4096, 8192, 12288 or 16384)
-static int ps_words()
+// PCG_PS_MID override them; words must be 4096, 8192, 12288 or 16384).
+// Segments of 12288 words are the fastest while they fill the chip; a shorter
+// range is cut into two segments per SM of at least 256 words (61 440 numbers:
+// the primes' starts cost more below).  With 12288 words always, pi(1e6) ran on
+// one SM: 75 -> 32 us; pi(1e13) (B over 5 segments) 0.97 -> 0.61 ms.
+static int ps_words(int64_t numbers, int num_sms)
 {
   static const int w = [] {
     const char* e = getenv("PCG_PS_WORDS");
-    const int v = e ? atoi(e) : 12288;
-    return (v >= 4096 && v <= 16384 && v % 4096 == 0) ? v : 12288;
+    const int v = e ? atoi(e) : 0;
+    return (v >= 4096 && v <= 16384 && v % 4096 == 0) ? v : 0;
   }();
-  return w;
+  if (w) return w;
+  const int64_t per = (numbers / 240 + 1 + 2 * num_sms - 1) / (2 * num_sms);
+  return (int) std::max<int64_t>(256, std::min<int64_t>(12288, (per + 63) / 64 * 64));
 }
 
 static int64_t ps_mid_div()
 {
   static const int64_t d = [] {
     const char* e = getenv("PCG_PS_MID");
-    const int64_t v = e ? atoll(e) : 256;
-    return v > 0 ? v : 256;
+    const int64_t v = e ? atoll(e) : 128;
+    return v > 0 ? v : 128;
   }();
   return d;
 }
 
-// sieve [lo0, end) in segments; B queries for primes in (qlo, qhi] when b_mode
+// sieve [lo0, end) in segments; B queries for primes in (qlo, qhi]
 static PsOut run_psieve(Ctx& c, u128 x, int64_t lo0, int64_t end, bool b_mode, int64_t qlo, int64_t qhi,
                         cudaStream_t s, uint64_t* launches)
 {
   PsOut o;
   lo0 -= lo0 % 240;
   o.lo0 = lo0;
-  const int words = ps_words();
-  const int64_t seg = (int64_t) words * 240;
-  o.nseg = (end - lo0 + seg - 1) / seg;
-  if (o.nseg <= 0) return o;
-  std::vector<uint32_t> base = base_primes67(isqrt((u128) end) + 1);
-  std::vector<uint64_t> magic(base.size());
+  if (end <= lo0) return o;
+  const int words = ps_words(end - lo0, c.num_sms);
+  const int64_t len = (int64_t) words * 240;
+  o.nseg = (end - lo0 + len - 1) / len;
+  // sieving primes >= 67 and their reciprocals: the context's tables where
+  // they reach, else made here.  primes[1..18] = 2, ..., 61.
+  const int64_t limit = isqrt((u128) end) + 1;
+  const bool resident = c.tab.prime_limit >= limit;
+  std::vector<uint64_t> made;                              // reciprocals, then the primes
+  int64_t nbase;
+  const int64_t mid_limit = len / ps_mid_div();
   int nmid = 0;
-  const int64_t mid_limit = seg / ps_mid_div();
-  for (size_t i = 0; i < base.size(); i++) {
-    magic[i] = UINT64_MAX / base[i];
-    if ((int64_t) base[i] < mid_limit) nmid = (int) i + 1;
-  }
   DevBuf& d_base = c.tmp[T_PS_BASE];
-  DevBuf& d_magic = c.tmp[T_PS_MAGIC];
-  DevBuf& d_c = c.tmp[T_PS_C];
-  DevBuf& d_m = c.tmp[T_PS_M];
-  DevBuf& d_l = c.tmp[T_PS_L];
-  DevBuf& d_q = c.tmp[T_PS_Q];
-  d_base.alloc(std::max<size_t>(base.size(), 1) * 4);
-  d_magic.alloc(std::max<size_t>(base.size(), 1) * 8);
-  d_c.alloc((size_t) o.nseg * 8);
-  d_m.alloc((size_t) o.nseg * 8);
-  d_l.alloc((size_t) o.nseg * 8);
-  d_q.alloc(64);
-  if (!base.empty()) {
-    PCG_CUDA(cudaMemcpyAsync(d_base.p, base.data(), base.size() * 4, cudaMemcpyHostToDevice, s));
-    PCG_CUDA(cudaMemcpyAsync(d_magic.p, magic.data(), magic.size() * 8, cudaMemcpyHostToDevice, s));
+  DevBuf& d_seg = c.tmp[T_PS_C];
+  if (resident) {
+    nbase = std::max<int64_t>(0, host_pi(c.tab, (uint64_t) limit) - 18);
+    nmid = (int) std::max<int64_t>(0, std::min<int64_t>(nbase, host_pi(c.tab, (uint64_t) std::min(limit, std::max<int64_t>(mid_limit, 1)) - 1) - 18));
+  } else {
+    const std::vector<uint32_t> base = base_primes67(limit);
+    nbase = (int64_t) base.size();
+    made.resize((size_t) (nbase + (nbase + 1) / 2));
+    for (int64_t i = 0; i < nbase; i++) {
+      made[(size_t) i] = UINT64_MAX / base[(size_t) i];
+      if ((int64_t) base[(size_t) i] < mid_limit) nmid = (int) i + 1;
+    }
+    if (nbase) memcpy(&made[(size_t) nbase], base.data(), (size_t) nbase * 4);
+    d_base.alloc(std::max<size_t>(made.size(), 1) * 8);
+    if (nbase) PCG_CUDA(cudaMemcpyAsync(d_base.p, made.data(), made.size() * 8, cudaMemcpyHostToDevice, s));
   }
-  PCG_CUDA(cudaMemsetAsync(d_q.p, 0, 64, s));
-  PCG_CUDA(cudaMemsetAsync(d_m.p, 0, (size_t) o.nseg * 8, s));
-  PCG_CUDA(cudaMemsetAsync(d_l.p, 0, (size_t) o.nseg * 8, s));
+  d_seg.alloc((size_t) (3 * o.nseg + 1) * 8);              // results, then the work queue
+  PCG_CUDA(cudaMemsetAsync(d_seg.p, 0, (size_t) (3 * o.nseg + 1) * 8, s));
   PsArgs a;
   memset(&a, 0, sizeof(a));
   a.x_lo = (uint64_t) x;
   a.x_hi = (uint64_t) (x >> 64);
   a.lo0 = lo0;
   a.end = end;
-  a.seg = seg;
+  a.len = len;
   a.nseg = o.nseg;
   a.qlo = qlo;
   a.qhi = qhi;
   a.mode = b_mode ? 1 : 0;
   a.words = words;
-  a.nbase = (int) base.size();
+  a.nbase = (int) nbase;
   a.nmid = nmid;
-  a.base = d_base.as<uint32_t>();
-  a.magic = d_magic.as<uint64_t>();
+  a.base = resident ? c.tab.primes.as<uint32_t>() + 19 : (const uint32_t*) (d_base.as<uint64_t>() + nbase);
+  a.magic = resident ? c.tab.pmagic.as<uint64_t>() + 19 : d_base.as<uint64_t>();
   a.pibig = c.tab.pibig.as<uint64_t>();
-  a.seg_c = d_c.as<int64_t>();
-  a.seg_m = d_m.as<int64_t>();
-  a.seg_l = d_l.as<int64_t>();
-  a.queue = d_q.as<int>();
-  const size_t smem = (size_t) words * 8 + (size_t) (words / 8) * 4 + PS_PAT * 8;
-  PCG_CUDA(cudaFuncSetAttribute(k_psieve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
+  a.seg = d_seg.as<int64_t>();
+  a.queue = (int*) (d_seg.as<int64_t>() + 3 * o.nseg);
+  const size_t smem = (size_t) words * 8 + (size_t) (words / 8) * 4 + PAT_WORDS * 8;
+  // the largest size whatever this call's: threads with other sizes set it too
+  PCG_CUDA(cudaFuncSetAttribute(k_psieve, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                16384 * 8 + 16384 / 8 * 4 + PAT_WORDS * 8));
   int occ = 0;
   PCG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_psieve, PS_NT, smem));
   const int grid = (int) std::min<int64_t>((int64_t) c.num_sms * std::max(occ, 1), o.nseg);
   k_psieve<<<grid, PS_NT, smem, s>>>(a);
   PCG_CUDA(cudaGetLastError());
   if (launches) *launches += 1;
+  std::vector<int64_t> r((size_t) (3 * o.nseg));
+  PCG_CUDA(cudaMemcpyAsync(r.data(), d_seg.p, r.size() * 8, cudaMemcpyDeviceToHost, s));
+  PCG_CUDA(cudaStreamSynchronize(s));
   o.c.resize((size_t) o.nseg);
   o.m.resize((size_t) o.nseg);
   o.l.resize((size_t) o.nseg);
-  PCG_CUDA(cudaMemcpyAsync(o.c.data(), d_c.p, (size_t) o.nseg * 8, cudaMemcpyDeviceToHost, s));
-  PCG_CUDA(cudaMemcpyAsync(o.m.data(), d_m.p, (size_t) o.nseg * 8, cudaMemcpyDeviceToHost, s));
-  PCG_CUDA(cudaMemcpyAsync(o.l.data(), d_l.p, (size_t) o.nseg * 8, cudaMemcpyDeviceToHost, s));
-  PCG_CUDA(cudaStreamSynchronize(s));
+  for (int64_t i = 0; i < o.nseg; i++) {
+    o.c[(size_t) i] = r[(size_t) (3 * i)];
+    o.m[(size_t) i] = r[(size_t) (3 * i + 1)];
+    o.l[(size_t) i] = r[(size_t) (3 * i + 2)];
+  }
   return o;
 }
 

@@ -115,7 +115,7 @@ void exclusive_scan_u32(const uint32_t* in, int64_t n, uint64_t* out, cudaStream
 
 // slots of Ctx::tmp
 enum TmpSlot {
-  T_PS_BASE, T_PS_MAGIC, T_PS_C, T_PS_M, T_PS_L, T_PS_Q,      // prime sieve (B, small pi)
+  T_PS_BASE, T_PS_C,                                          // prime sieve (B, small pi)
   T_LK_V, T_LK_R,                                             // PiTable lookups
   T_AC_QLO, T_AC_QCNT, T_AC_QOFF, T_AC_OUTS,                  // A + C outers
   T_PR_PIECES, T_PR_FIRST, T_PR_SPLIT, T_PR_PART, T_PR_SUMS,  // pair sums

@@ -358,9 +358,7 @@ struct SweepArgs {
 };
 
 // primes 7..61 sieved with wheel patterns (their multiples repeat every p words)
-#define NSMALL 15
-#define PAT_WORDS 491   // 7+11+13+17+19+23+29+31+37+41+43+47+53+59+61
-__constant__ uint32_t c_small_p[NSMALL + 1] = {7, 11, 13, 17, 19, 23, 29, 31, 37, 41, 43, 47, 53, 59, 61, 0};
+__constant__ uint32_t c_small_p[PAT_PRIMES + 1] = {7, 11, 13, 17, 19, 23, 29, 31, 37, 41, 43, 47, 53, 59, 61, 0};
 
 // min(floor(a / d), cap) for d >= 1, cap >= 0, with md = floor((2^64 - 1) / d):
 // one high product when a < 2^64
@@ -657,6 +655,8 @@ constexpr SweepLayout sweep_layout(int nt)
   y.bits = (y.cop + 480 * 2 + 15) / 16 * 16;
   return y;
 }
+// the most of it: 227 KB a block less the static arrays of k_sweep
+#define SWEEP_SMEM_MAX ((227 - 4) * 1024)
 static size_t sweep_smem(int words, int nt) { return (size_t) sweep_layout(nt).bits + (size_t) words * 8 + (size_t) (words / 8) * 5; }
 
 template <typename FT, int NT>
@@ -714,20 +714,7 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
     s_delta[i] = (uint8_t) (30 * (j >> 3) + woff(j & 7) - woff(jl));
   }
   for (int i = tid; i < 2 * LB; i += NT) s_gsmu[i / LB][i % LB] = 0;
-  // wheel patterns: word r of prime p keeps the numbers 240 r + {1,7,..,29}
-  // (mod 240 p) that p does not divide
-  for (int i = tid; i < PAT_WORDS; i += NT) {
-    int k = 0, base = 0;
-    while (k < NSMALL - 1 && i >= base + c_small_p[k]) { base += c_small_p[k]; k++; }
-    const uint32_t p = c_small_p[k];
-    const uint32_t r = (uint32_t) (i - base);
-    uint64_t w = ~0ull;
-    for (int j = 0; j < 64; j++) {
-      const uint32_t v = 240 * r + 30 * (j >> 3) + woff(j & 7);
-      if (v % p == 0) w &= ~(1ull << j);
-    }
-    pat[i] = w;
-  }
+  for (int i = tid; i < PAT_WORDS; i += NT) pat[i] = g_patterns.w[i];
   if (tid < 5) s_ctr[tid] = 0;
   int gpar = 0;                                        // group parity
 
@@ -1970,24 +1957,25 @@ static void add_combine_jobs(std::vector<CombineJob>& jobs, int64_t colbase, int
 }
 
 template <typename FT, int NT>
-static void set_sweep_attr(size_t smem)
+static void set_sweep_attr()
 {
   // per device and cheap: set on every call (worker threads and several
-  // devices share the function)
-  PCG_CUDA(cudaFuncSetAttribute(k_sweep<FT, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
+  // devices share the function), to the most that any call may ask for, since
+  // calls of other sizes run at the same time
+  PCG_CUDA(cudaFuncSetAttribute(k_sweep<FT, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SWEEP_SMEM_MAX));
 }
 
 template <typename FT, int NT>
 static void occupancy_sweep(int* occ, size_t smem)
 {
-  set_sweep_attr<FT, NT>(smem);
+  set_sweep_attr<FT, NT>();
   PCG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, k_sweep<FT, NT>, NT, smem));
 }
 
 template <typename FT, int NT>
 static void launch_sweep(const SweepArgs& a, int grid, size_t smem, cudaStream_t s)
 {
-  set_sweep_attr<FT, NT>(smem);
+  set_sweep_attr<FT, NT>();
   k_sweep<FT, NT><<<grid, NT, smem, s>>>(a);
 }
 
@@ -2265,7 +2253,7 @@ SweepResult run_sweep(Ctx& c, const SweepProblem& pb, const Tuning& tune_in, cud
   words = std::max(words, wq);
   words = (words + wq - 1) / wq * wq;
   const size_t smem = sweep_smem(words, NT);
-  if (smem > c.smem_optin) fail(PCG_EINVAL, "segment too large for shared memory");
+  if (smem > std::min<size_t>(c.smem_optin, SWEEP_SMEM_MAX)) fail(PCG_EINVAL, "segment too large for shared memory");
   int fbytes = pb.gourdon ? c.tab.fd_bytes : c.tab.fr_bytes;
   auto occupancy = [&](int* occ) {
     if (NT == 512) { if (fbytes == 2) occupancy_sweep<uint16_t, 512>(occ, smem); else occupancy_sweep<uint32_t, 512>(occ, smem); }
@@ -2598,7 +2586,7 @@ void run_sweep_batch(Ctx& c, const std::vector<SweepProblem>& pbs, const Tuning&
   words = std::max(words, wq);
   words = (words + wq - 1) / wq * wq;
   const size_t smem = sweep_smem(words, NT);
-  if (smem > c.smem_optin) fail(PCG_EINVAL, "segment too large for shared memory");
+  if (smem > std::min<size_t>(c.smem_optin, SWEEP_SMEM_MAX)) fail(PCG_EINVAL, "segment too large for shared memory");
   const int fbytes = T.fd_bytes;
   int occ = 0;
   if (NT == 512) { if (fbytes == 2) occupancy_sweep<uint16_t, 512>(&occ, smem); else occupancy_sweep<uint32_t, 512>(&occ, smem); }
@@ -2782,9 +2770,9 @@ void run_sweep_batch(Ctx& c, const std::vector<SweepProblem>& pbs, const Tuning&
   unsigned long long* d_counters = (unsigned long long*) c.misc.p;
   int* d_queue = (int*) ((char*) c.misc.p + 256);
   // the launch attributes are set before the capture
-  if (NT == 512) { if (fbytes == 2) set_sweep_attr<uint16_t, 512>(smem); else set_sweep_attr<uint32_t, 512>(smem); }
-  else if (NT == 256) { if (fbytes == 2) set_sweep_attr<uint16_t, 256>(smem); else set_sweep_attr<uint32_t, 256>(smem); }
-  else { if (fbytes == 2) set_sweep_attr<uint16_t, 128>(smem); else set_sweep_attr<uint32_t, 128>(smem); }
+  if (NT == 512) { if (fbytes == 2) set_sweep_attr<uint16_t, 512>(); else set_sweep_attr<uint32_t, 512>(); }
+  else if (NT == 256) { if (fbytes == 2) set_sweep_attr<uint16_t, 256>(); else set_sweep_attr<uint32_t, 256>(); }
+  else { if (fbytes == 2) set_sweep_attr<uint16_t, 128>(); else set_sweep_attr<uint32_t, 128>(); }
   PCG_CUDA(cudaStreamSynchronize(s));
 
   SweepArgs a;
