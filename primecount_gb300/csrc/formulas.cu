@@ -40,15 +40,18 @@ static double fnow_ms()
 template <int NT>
 __device__ __forceinline__ void block_sum_i128(i128 v, i128* out)
 {
-  __shared__ long long lo_s[NT], hi_s[NT];
-  // split into 2^62-bounded halves so that a block of partial sums cannot overflow
-  lo_s[threadIdx.x] = (long long) (v & (i128) 0x3FFFFFFFFFFFFFFFll);
-  hi_s[threadIdx.x] = (long long) (v >> 62);
+  __shared__ i128 w[NT / 32];
+  for (int d = 16; d > 0; d >>= 1) {
+    const uint64_t lo = __shfl_down_sync(0xffffffffu, (uint64_t) v, d);
+    const uint64_t hi = __shfl_down_sync(0xffffffffu, (uint64_t) (v >> 64), d);
+    v += (i128) (((u128) hi << 64) | lo);
+  }
+  if ((threadIdx.x & 31) == 0) w[threadIdx.x >> 5] = v;
   __syncthreads();
   if (threadIdx.x == 0) {
-    i128 lo = 0, hi = 0;
-    for (int i = 0; i < NT; i++) { lo += lo_s[i]; hi += hi_s[i]; }
-    *out += lo + hi * ((i128) 1 << 62);
+    i128 t = 0;
+    for (int i = 0; i < NT / 32; i++) t += w[i];
+    *out = t;
   }
   __syncthreads();
 }
@@ -336,41 +339,55 @@ __global__ void __launch_bounds__(256) k_pairs(const PairOuter* __restrict__ out
   block_sum_i128<256>(acc, &partial[blockIdx.x]);
 }
 
-// sum of the terms of nout outers: big outers cut into pieces, then one
-// block per piece
-static i128 run_pairs(Ctx& c, const PairOuter* outs, int64_t nout, cudaStream_t s, uint64_t* launches)
+// Launches the sum of the terms of nout outers, its blocks' partial sums in
+// T_PR_PART; returns their number.  Outers are cut into pieces of PAIR_SPLIT
+// terms, one block per piece, when the prime table is long enough for an
+// outer to hold several (at most DIRECT_TERMS terms each: as they are, without
+// the scan and the wait for the number of pieces: 60 us of a small pi(x)).
+#define DIRECT_TERMS 65536
+static int launch_pairs(Ctx& c, const PairOuter* outs, int64_t nout, cudaStream_t s, uint64_t* launches)
 {
   if (nout <= 0) return 0;
-  DevBuf& pieces = c.tmp[T_PR_PIECES];
-  DevBuf& first = c.tmp[T_PR_FIRST];
-  pieces.alloc((size_t) (nout + 1) * 4);
-  first.alloc((size_t) (nout + 1) * 8);
-  k_pair_pieces<<<(unsigned) ((nout + 256) / 256), 256, 0, s>>>(outs, nout, pieces.as<uint32_t>());
-  PCG_CUDA(cudaGetLastError());
-  exclusive_scan_u32(pieces.as<uint32_t>(), nout + 1, first.as<uint64_t>(), s, &c.tmp[T_PR_SUMS]);
-  uint64_t np = 0;
-  PCG_CUDA(cudaMemcpyAsync(&np, first.as<uint64_t>() + nout, 8, cudaMemcpyDeviceToHost, s));
-  PCG_CUDA(cudaStreamSynchronize(s));
-  if (np == 0) return 0;
-  DevBuf& split = c.tmp[T_PR_SPLIT];
-  split.alloc((size_t) np * sizeof(PairOuter));
-  k_pair_split<<<(unsigned) ((nout + 127) / 128), 128, 0, s>>>(outs, nout, first.as<uint64_t>(),
-                                                               split.as<PairOuter>());
-  PCG_CUDA(cudaGetLastError());
+  uint64_t np = (uint64_t) nout;
+  if (c.tab.nprimes > DIRECT_TERMS) {
+    DevBuf& pieces = c.tmp[T_PR_PIECES];
+    DevBuf& first = c.tmp[T_PR_FIRST];
+    pieces.alloc((size_t) (nout + 1) * 4);
+    first.alloc((size_t) (nout + 1) * 8);
+    k_pair_pieces<<<(unsigned) ((nout + 256) / 256), 256, 0, s>>>(outs, nout, pieces.as<uint32_t>());
+    PCG_CUDA(cudaGetLastError());
+    exclusive_scan_u32(pieces.as<uint32_t>(), nout + 1, first.as<uint64_t>(), s, &c.tmp[T_PR_SUMS]);
+    PCG_CUDA(cudaMemcpyAsync(&np, first.as<uint64_t>() + nout, 8, cudaMemcpyDeviceToHost, s));
+    PCG_CUDA(cudaStreamSynchronize(s));
+    if (np == 0) return 0;
+    DevBuf& split = c.tmp[T_PR_SPLIT];
+    split.alloc((size_t) np * sizeof(PairOuter));
+    k_pair_split<<<(unsigned) ((nout + 127) / 128), 128, 0, s>>>(outs, nout, first.as<uint64_t>(),
+                                                                 split.as<PairOuter>());
+    PCG_CUDA(cudaGetLastError());
+    outs = split.as<PairOuter>();
+    if (launches) *launches += 5;
+  }
   const int grid = (int) std::min<uint64_t>(np, (uint64_t) c.num_sms * 8);
   DevBuf& part = c.tmp[T_PR_PART];
   part.alloc((size_t) grid * 16);
-  PCG_CUDA(cudaMemsetAsync(part.p, 0, (size_t) grid * 16, s));
   const bool small = c.tab.prime_limit < (1ll << 31) && c.tab.pibig_limit + 240 < (1ll << 36);
   if (small)
-    k_pairs<true><<<grid, 256, 0, s>>>(split.as<PairOuter>(), (int64_t) np, c.tab.primes.as<uint32_t>(),
-                                       c.tab.pmagic.as<uint64_t>(), c.tab.pibig.as<uint64_t>(), part.as<i128>());
+    k_pairs<true><<<grid, 256, 0, s>>>(outs, (int64_t) np, c.tab.primes.as<uint32_t>(), c.tab.pmagic.as<uint64_t>(),
+                                       c.tab.pibig.as<uint64_t>(), part.as<i128>());
   else
-    k_pairs<false><<<grid, 256, 0, s>>>(split.as<PairOuter>(), (int64_t) np, c.tab.primes.as<uint32_t>(),
-                                        c.tab.pmagic.as<uint64_t>(), c.tab.pibig.as<uint64_t>(), part.as<i128>());
+    k_pairs<false><<<grid, 256, 0, s>>>(outs, (int64_t) np, c.tab.primes.as<uint32_t>(), c.tab.pmagic.as<uint64_t>(),
+                                        c.tab.pibig.as<uint64_t>(), part.as<i128>());
   PCG_CUDA(cudaGetLastError());
-  if (launches) *launches += 6;
-  return sum_partials(part, grid, s);
+  if (launches) *launches += 1;
+  return grid;
+}
+
+// the sum itself
+static i128 run_pairs(Ctx& c, const PairOuter* outs, int64_t nout, cudaStream_t s, uint64_t* launches)
+{
+  const int grid = launch_pairs(c, outs, nout, s, launches);
+  return grid ? sum_partials(c.tmp[T_PR_PART], grid, s) : 0;
 }
 
 struct AcParams {
@@ -444,58 +461,57 @@ __global__ void k_outer_C1(AcParams P, PairOuter* __restrict__ outs)
   outs[j] = O;
 }
 
-// C1 products m = q r: number of q per b, then one outer per (b, q)
-__global__ void k_c1_qcount(AcParams P, int64_t* __restrict__ qlo, int64_t* __restrict__ qcnt)
+// C1 products m = q r: the primes q of each b, (qlo[j], qlo[j] + count], and
+// one outer per (b, q); off[j] = outers before b's
+__global__ void k_c1_expand(AcParams P, const int64_t* __restrict__ qlo, const int64_t* __restrict__ off, int64_t nb,
+                            int64_t n, PairOuter* __restrict__ outs)
 {
-  const int64_t j = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t t = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  int64_t j = 0, hi = nb - 1;                            // the last j with off[j] <= t
+  while (j < hi) {
+    const int64_t mid = (j + hi + 1) >> 1;
+    if (off[mid] <= t) j = mid; else hi = mid - 1;
+  }
   const int64_t b = P.bC10 + 1 + j;
-  if (b > P.bC11) return;
   u128 xp;
   int64_t min_m, max_m;
   c1_range(P, b, xp, min_m, max_m);
-  const int64_t p = P.primes[b];
-  int64_t lo = 0, cnt = 0;
-  if (min_m < max_m) {
-    const int64_t max_q = dmin(P.y, disqrt((u128) max_m));
-    const int64_t min_q = dmax(p, min_m / P.y);
-    if (min_q < max_q) {
-      lo = dpi(P.pismall, (uint64_t) min_q);
-      cnt = dpi(P.pismall, (uint64_t) max_q) - lo;
-    }
+  const int64_t qi = qlo[j] + 1 + (t - off[j]);
+  const uint64_t q = P.primes[qi];
+  const int64_t min_r = dmax((int64_t) q, min_m / (int64_t) q);
+  const int64_t max_r = dmin(P.y, max_m / (int64_t) q);
+  PairOuter O;
+  const u128 xpq = div128(xp, q);
+  O.xp_lo = (uint64_t) xpq;
+  O.xp_hi = (uint64_t) (xpq >> 64);
+  O.cap = 0;
+  O.b = (int32_t) b;
+  O.mode = 2;
+  O.i_lo = O.i_hi = 0;
+  if (min_r < max_r) {
+    O.i_lo = dpi(P.pismall, (uint64_t) min_r);
+    O.i_hi = dpi(P.pismall, (uint64_t) max_r);
+    if (O.i_hi > O.i_lo && xpq / P.primes[O.i_hi] < 6) O.mode = 6;
   }
-  qlo[j] = lo;
-  qcnt[j] = cnt;
+  outs[t] = O;
 }
 
-__global__ void k_c1_expand(AcParams P, const int64_t* __restrict__ qlo, const int64_t* __restrict__ qcnt,
-                            const int64_t* __restrict__ qoff, PairOuter* __restrict__ outs)
+// qlo[j] and the number of q of b = bC10 + 1 + j, from the host tables
+static int64_t c1_q_range(const Tables& T, const AcParams& P, int64_t b, int64_t* lo)
 {
-  const int64_t j = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t b = P.bC10 + 1 + j;
-  if (b > P.bC11) return;
-  u128 xp;
-  int64_t min_m, max_m;
-  c1_range(P, b, xp, min_m, max_m);
-  for (int64_t t = 0; t < qcnt[j]; t++) {
-    const int64_t qi = qlo[j] + 1 + t;
-    const uint64_t q = P.primes[qi];
-    const int64_t min_r = dmax((int64_t) q, min_m / (int64_t) q);
-    const int64_t max_r = dmin(P.y, max_m / (int64_t) q);
-    PairOuter O;
-    const u128 xpq = div128(xp, q);
-    O.xp_lo = (uint64_t) xpq;
-    O.xp_hi = (uint64_t) (xpq >> 64);
-    O.cap = 0;
-    O.b = (int32_t) b;
-    O.mode = 2;
-    O.i_lo = O.i_hi = 0;
-    if (min_r < max_r) {
-      O.i_lo = dpi(P.pismall, (uint64_t) min_r);
-      O.i_hi = dpi(P.pismall, (uint64_t) max_r);
-      if (O.i_hi > O.i_lo && xpq / P.primes[O.i_hi] < 6) O.mode = 6;
-    }
-    outs[qoff[j] + t] = O;
-  }
+  const u128 x = ((u128) P.x_hi << 64) | P.x_lo;
+  const int64_t p = T.h_primes[(size_t) b];
+  const u128 xp = x / (u128) p, xpp = xp / ((u128) p * p);
+  const int64_t max_m = xp < (u128) P.z ? (int64_t) xp : P.z;
+  const int64_t min_m = std::max(xpp > (u128) INT64_MAX ? INT64_MAX : (int64_t) xpp, P.z / p);
+  *lo = 0;
+  if (min_m >= max_m) return 0;
+  const int64_t max_q = std::min(P.y, isqrt((u128) max_m));
+  const int64_t min_q = std::max(p, min_m / P.y);
+  if (min_q >= max_q) return 0;
+  *lo = host_pi(T, (uint64_t) min_q);
+  return host_pi(T, (uint64_t) max_q) - *lo;
 }
 
 // C2 outers: primes q in (max(x / p^3, p, xp / sqrt(x)), min(x / p^2, y)]
@@ -801,8 +817,10 @@ static std::vector<uint32_t> base_primes67(int64_t limit)
   return p;
 }
 
+// per segment s: r[3 s] primes counted, r[3 s + 1] B queries, r[3 s + 2] the
+// sum of their counts
 struct PsOut {
-  std::vector<int64_t> c, m, l;
+  std::vector<int64_t> r;
   int64_t lo0 = 0, nseg = 0;
 };
 
@@ -834,8 +852,9 @@ static int64_t ps_mid_div()
   return d;
 }
 
-// sieve [lo0, end) in segments; B queries for primes in (qlo, qhi]
-static PsOut run_psieve(Ctx& c, u128 x, int64_t lo0, int64_t end, bool b_mode, int64_t qlo, int64_t qhi,
+// launches the sieve of [lo0, end) in segments, results in T_PS_C; B queries
+// for primes in (qlo, qhi]
+static PsOut launch_psieve(Ctx& c, u128 x, int64_t lo0, int64_t end, bool b_mode, int64_t qlo, int64_t qhi,
                         cudaStream_t s, uint64_t* launches)
 {
   PsOut o;
@@ -901,18 +920,30 @@ static PsOut run_psieve(Ctx& c, u128 x, int64_t lo0, int64_t end, bool b_mode, i
   k_psieve<<<grid, PS_NT, smem, s>>>(a);
   PCG_CUDA(cudaGetLastError());
   if (launches) *launches += 1;
-  std::vector<int64_t> r((size_t) (3 * o.nseg));
-  PCG_CUDA(cudaMemcpyAsync(r.data(), d_seg.p, r.size() * 8, cudaMemcpyDeviceToHost, s));
-  PCG_CUDA(cudaStreamSynchronize(s));
-  o.c.resize((size_t) o.nseg);
-  o.m.resize((size_t) o.nseg);
-  o.l.resize((size_t) o.nseg);
-  for (int64_t i = 0; i < o.nseg; i++) {
-    o.c[(size_t) i] = r[(size_t) (3 * i)];
-    o.m[(size_t) i] = r[(size_t) (3 * i + 1)];
-    o.l[(size_t) i] = r[(size_t) (3 * i + 2)];
+  return o;
+}
+
+static PsOut run_psieve(Ctx& c, u128 x, int64_t lo0, int64_t end, bool b_mode, int64_t qlo, int64_t qhi,
+                        cudaStream_t s, uint64_t* launches)
+{
+  PsOut o = launch_psieve(c, x, lo0, end, b_mode, qlo, qhi, s, launches);
+  o.r.resize((size_t) (3 * o.nseg));
+  if (o.nseg > 0) {
+    PCG_CUDA(cudaMemcpyAsync(o.r.data(), c.tmp[T_PS_C].p, o.r.size() * 8, cudaMemcpyDeviceToHost, s));
+    PCG_CUDA(cudaStreamSynchronize(s));
   }
   return o;
+}
+
+// sum over the B queries of the numbers of primes <= x / p, run = pi(lo0 - 1)
+static i128 b_sum(const int64_t* r, int64_t nseg, i128 run)
+{
+  i128 B = 0;
+  for (int64_t i = 0; i < nseg; i++) {
+    B += (i128) r[3 * i + 2] + (i128) r[3 * i + 1] * run;
+    run += r[3 * i];
+  }
+  return B;
 }
 
 // pi(x) for small x: a direct sieve count (2, 3, 5 are not in the bitmap)
@@ -922,7 +953,7 @@ static i128 pi_sieve_count(Ctx& c, int64_t x, cudaStream_t s, uint64_t* launches
   if (x < 7) return x >= 5 ? 3 : (x >= 3 ? 2 : 1);
   PsOut o = run_psieve(c, (u128) x, 0, x + 1, false, 0, 0, s, launches);
   i128 t = 3;
-  for (int64_t i = 0; i < o.nseg; i++) t += o.c[(size_t) i];
+  for (int64_t i = 0; i < o.nseg; i++) t += o.r[(size_t) (3 * i)];
   return t;
 }
 
@@ -1000,12 +1031,40 @@ static i128 sum_pi_x_over_p(Ctx& c, u128 x, int64_t y, int64_t sqrtx, cudaStream
     // pi(lo0 - 1) from the PiTable up to sqrt(x) (lo0 >= sqrt(x) > 1e5 here)
     i128 run = 0;
     if (o.lo0 >= 7) run = pi_lookup(c, std::vector<uint64_t>{(uint64_t) (o.lo0 - 1)}, s)[0];
-    for (int64_t i = 0; i < o.nseg; i++) {
-      B += (i128) o.l[(size_t) i] + (i128) o.m[(size_t) i] * run;
-      run += o.c[(size_t) i];
-    }
+    B = b_sum(o.r.data(), o.nseg, run);
   }
   return B;
+}
+
+// Sigma4..6 (Sigma.cpp:25-140): over the primes p = primes[i], i in (i0, i1]
+// = (pi(x*), pi(x^(1/3))], the sums of pi(x / (p y)) for p <= sqrt(x / y), of
+// pi(x / p^2) for the others and of pi(sqrt(x / p))^2, a block's three partial
+// sums each; and pi of the nlook values look[].  (On the host with the
+// lookups alone on the device: 0.1 ms of pi(1e13), 6 ms of pi(1e18).)
+#define SIGMA_BLOCKS 128
+struct SigmaArgs {
+  uint64_t x_lo, x_hi;
+  int64_t y, sqrt_xy, i0, i1;
+  uint64_t look[3];
+  int nlook;
+};
+__global__ void __launch_bounds__(256) k_sigma(const SigmaArgs A, const uint32_t* __restrict__ primes,
+                                               const uint64_t* __restrict__ pibig, i128* __restrict__ part,
+                                               int64_t* __restrict__ found)
+{
+  const u128 x = ((u128) A.x_hi << 64) | A.x_lo;
+  i128 s4 = 0, s5 = 0, s6 = 0;
+  for (int64_t i = A.i0 + 1 + (int64_t) blockIdx.x * 256 + threadIdx.x; i <= A.i1; i += 256ll * gridDim.x) {
+    const uint64_t p = primes[i];
+    if ((int64_t) p <= A.sqrt_xy) s4 += dpi(pibig, (uint64_t) (div128(x, p) / (uint64_t) A.y));
+    else s5 += dpi(pibig, (uint64_t) (div128(x, p) / p));
+    const i128 r = dpi(pibig, (uint64_t) disqrt(div128(x, p)));
+    s6 += r * r;
+  }
+  block_sum_i128<256>(s4, &part[3 * blockIdx.x]);
+  block_sum_i128<256>(s5, &part[3 * blockIdx.x + 1]);
+  block_sum_i128<256>(s6, &part[3 * blockIdx.x + 2]);
+  if (blockIdx.x == 0 && (int) threadIdx.x < A.nlook) found[threadIdx.x] = dpi(pibig, A.look[threadIdx.x]);
 }
 
 // with_d = false leaves D out (R.d = 0, R.pi without it): the batch form
@@ -1043,138 +1102,156 @@ static PiParts pi_gourdon(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, bo
     R.launches += r.stats.kernel_launches;
     R.ms_d = fnow_ms() - t1;
   };
+  // All of them are launched before the one wait for their results.
   auto other_terms = [&](cudaStream_t s, uint64_t* nl) {
-    // ---- A + C
-    {
-      double t1 = fnow_ms();
-      const u128 xy = x / (u128) y, xz = x / (u128) z;
-      AcParams P;
-      memset(&P, 0, sizeof(P));
-      P.x_lo = (uint64_t) x;
-      P.x_hi = (uint64_t) (x >> 64);
-      P.y = y;
-      P.z = z;
-      P.k = k;
-      P.x_star = x_star;
-      P.x13 = x13;
-      P.sqrtx = sqrtx;
-      P.primes = T.primes.as<uint32_t>();
-      P.pismall = T.pitab.as<uint64_t>();
-      P.pibig = T.pibig.as<uint64_t>();
-      const int64_t pi_sqrtz = host_pi(T, (uint64_t) isqrt((u128) z));
-      P.bA0 = host_pi(T, (uint64_t) x_star);
-      P.bA1 = host_pi(T, (uint64_t) x13);
-      P.bC10 = std::max<int64_t>(k, host_pi(T, (uint64_t) iroot(xz, 3)));
-      P.bC11 = pi_sqrtz;
-      P.bC20 = std::max<int64_t>({k, host_pi(T, (uint64_t) iroot(xy, 3)), pi_sqrtz});
-      P.bC21 = host_pi(T, (uint64_t) x_star);
-      const int64_t nA = std::max<int64_t>(0, P.bA1 - P.bA0);
-      const int64_t nC1 = std::max<int64_t>(0, P.bC11 - P.bC10);
-      const int64_t nC2 = std::max<int64_t>(0, P.bC21 - P.bC20);
-      // C1 products: count q per b, then expand
-      int64_t nQ = 0;
-      DevBuf& qlo = c.tmp[T_AC_QLO];
-      DevBuf& qcnt = c.tmp[T_AC_QCNT];
-      DevBuf& qoff = c.tmp[T_AC_QOFF];
-      std::vector<int64_t> hq;
-      if (nC1 > 0) {
-        qlo.alloc((size_t) nC1 * 8);
-        qcnt.alloc((size_t) nC1 * 8);
-        qoff.alloc((size_t) nC1 * 8);
-        k_c1_qcount<<<(unsigned) ((nC1 + 127) / 128), 128, 0, s>>>(P, qlo.as<int64_t>(), qcnt.as<int64_t>());
-        PCG_CUDA(cudaGetLastError());
-        (*nl)++;
-        hq.resize((size_t) nC1);
-        PCG_CUDA(cudaMemcpyAsync(hq.data(), qcnt.p, (size_t) nC1 * 8, cudaMemcpyDeviceToHost, s));
-        PCG_CUDA(cudaStreamSynchronize(s));
-        std::vector<int64_t> off((size_t) nC1);
-        for (int64_t j = 0; j < nC1; j++) { off[(size_t) j] = nQ; nQ += hq[(size_t) j]; }
-        PCG_CUDA(cudaMemcpyAsync(qoff.p, off.data(), (size_t) nC1 * 8, cudaMemcpyHostToDevice, s));
-      }
-      const int64_t nout = nA + nC1 + nQ + nC2;
-      i128 sum = 0;
-      if (nout > 0) {
-        DevBuf& outs = c.tmp[T_AC_OUTS];
-        outs.alloc((size_t) nout * sizeof(PairOuter));
-        PairOuter* o = outs.as<PairOuter>();
-        if (nA) k_outer_A<<<(unsigned) ((nA + 127) / 128), 128, 0, s>>>(P, o);
-        if (nC1) k_outer_C1<<<(unsigned) ((nC1 + 127) / 128), 128, 0, s>>>(P, o + nA);
-        if (nQ) k_c1_expand<<<(unsigned) ((nC1 + 127) / 128), 128, 0, s>>>(P, qlo.as<int64_t>(), qcnt.as<int64_t>(),
-                                                                            qoff.as<int64_t>(), o + nA + nC1);
-        if (nC2) k_outer_C2<<<(unsigned) ((nC2 + 127) / 128), 128, 0, s>>>(P, o + nA + nC1 + nQ);
-        PCG_CUDA(cudaGetLastError());
-        *nl += 4;
-        sum = run_pairs(c, o, nout, s, nl);
-      }
-      R.ac = sum;
-      R.ms_ac = fnow_ms() - t1;
-    }
-
+    const double t1 = fnow_ms();
+    const u128 xy = x / (u128) y, xz = x / (u128) z;
+    const int64_t sqrt_xy = isqrt(xy);
+    auto partials = [&](DevBuf& b, int n) {
+      std::vector<i128> h((size_t) n);
+      if (n) PCG_CUDA(cudaMemcpyAsync(h.data(), b.p, (size_t) n * 16, cudaMemcpyDeviceToHost, s));
+      return h;
+    };
     // ---- B = sum over primes y < p <= sqrt(x) of pi(x / p)
-    {
-      double t1 = fnow_ms();
-      R.b = sum_pi_x_over_p(c, x, y, sqrtx, s, nl);
-      R.ms_b = fnow_ms() - t1;
-    }
+    const int64_t n0 = (int64_t) (x / (u128) sqrtx), n1 = (int64_t) (x / (u128) (y + 1)) + 1;
+    PsOut ps;
+    if (sqrtx > y && n1 > n0) ps = launch_psieve(c, x, n0, n1, true, y, sqrtx, s, nl);
 
     // ---- Phi0
-    {
-      double t1 = fnow_ms();
-      const int64_t size = wheel2310().to_index((uint64_t) z) + 1;
-      const int grid = c.num_sms * 8;
-      DevBuf& part = c.tmp[T_PHI0_PART];
-      part.alloc((size_t) grid * 16);
-      PCG_CUDA(cudaMemsetAsync(part.p, 0, (size_t) grid * 16, s));
-      PhiTab PT = phi_tab(c);
-      if (T.fd_bytes == 2)
-        k_phi0<uint16_t><<<grid, 256, 0, s>>>((uint64_t) x, (uint64_t) (x >> 64), T.factor_d.as<uint16_t>(), size,
-                                              (uint32_t) (2 * k + 1), (uint64_t) T.h_primes[(size_t) k], PT, T.coprime.as<uint16_t>(), part.as<i128>());
-      else
-        k_phi0<uint32_t><<<grid, 256, 0, s>>>((uint64_t) x, (uint64_t) (x >> 64), T.factor_d.as<uint32_t>(), size,
-                                              (uint32_t) (2 * k + 1), (uint64_t) T.h_primes[(size_t) k], PT, T.coprime.as<uint16_t>(), part.as<i128>());
-      PCG_CUDA(cudaGetLastError());
-      (*nl)++;
-      R.phi0 = sum_partials(part, grid, s);
-      R.ms_phi0 = fnow_ms() - t1;
+    const int64_t size = wheel2310().to_index((uint64_t) z) + 1;
+    const int grid0 = (int) std::min<int64_t>((int64_t) c.num_sms * 8, (size + 255) / 256);
+    DevBuf& part0 = c.tmp[T_PHI0_PART];
+    part0.alloc((size_t) grid0 * 16);
+    const PhiTab PT = phi_tab(c);
+    const uint64_t pk = T.h_primes[(size_t) k];
+    if (T.fd_bytes == 2)
+      k_phi0<uint16_t><<<grid0, 256, 0, s>>>((uint64_t) x, (uint64_t) (x >> 64), T.factor_d.as<uint16_t>(), size,
+                                             (uint32_t) (2 * k + 1), pk, PT, T.coprime.as<uint16_t>(), part0.as<i128>());
+    else
+      k_phi0<uint32_t><<<grid0, 256, 0, s>>>((uint64_t) x, (uint64_t) (x >> 64), T.factor_d.as<uint32_t>(), size,
+                                             (uint32_t) (2 * k + 1), pk, PT, T.coprime.as<uint16_t>(), part0.as<i128>());
+    PCG_CUDA(cudaGetLastError());
+    (*nl)++;
+
+    // ---- Sigma's sums, and the values of pi that it and B need
+    SigmaArgs sg;
+    memset(&sg, 0, sizeof(sg));
+    sg.x_lo = (uint64_t) x;
+    sg.x_hi = (uint64_t) (x >> 64);
+    sg.y = y;
+    sg.sqrt_xy = sqrt_xy;
+    sg.i0 = host_pi(T, (uint64_t) x_star);
+    sg.i1 = host_pi(T, (uint64_t) x13);
+    sg.look[0] = (uint64_t) sqrtx;
+    sg.look[1] = (uint64_t) sqrt_xy;
+    sg.look[2] = ps.lo0 > 0 ? (uint64_t) (ps.lo0 - 1) : 0;
+    sg.nlook = 3;
+    // the largest argument is the first prime's: the others' are smaller
+    u128 most = std::max<u128>((u128) sqrtx, std::max<u128>((u128) sqrt_xy, (u128) sg.look[2]));
+    if (sg.i0 < sg.i1) {
+      const u128 p = T.h_primes[(size_t) sg.i0 + 1];
+      most = std::max(most, (int64_t) p <= sqrt_xy ? x / p / (u128) y : x / p / p);
     }
+    if (most > (u128) c.tab.pibig_limit) fail(PCG_EINTERNAL, "pi lookup beyond the PiTable");
+    DevBuf& sbuf = c.tmp[T_SIGMA];
+    const int sblocks = (int) std::max<int64_t>(1, std::min<int64_t>(SIGMA_BLOCKS, (sg.i1 - sg.i0 + 255) / 256));
+    sbuf.alloc((size_t) (3 * sblocks + 2) * 16);
+    k_sigma<<<sblocks, 256, 0, s>>>(sg, T.primes.as<uint32_t>(), T.pibig.as<uint64_t>(), sbuf.as<i128>(),
+                                    (int64_t*) (sbuf.as<i128>() + 3 * sblocks));
+    PCG_CUDA(cudaGetLastError());
+    (*nl)++;
+
+    // ---- A + C
+    AcParams P;
+    memset(&P, 0, sizeof(P));
+    P.x_lo = (uint64_t) x;
+    P.x_hi = (uint64_t) (x >> 64);
+    P.y = y;
+    P.z = z;
+    P.k = k;
+    P.x_star = x_star;
+    P.x13 = x13;
+    P.sqrtx = sqrtx;
+    P.primes = T.primes.as<uint32_t>();
+    P.pismall = T.pitab.as<uint64_t>();
+    P.pibig = T.pibig.as<uint64_t>();
+    const int64_t pi_sqrtz = host_pi(T, (uint64_t) isqrt((u128) z));
+    P.bA0 = sg.i0;
+    P.bA1 = sg.i1;
+    P.bC10 = std::max<int64_t>(k, host_pi(T, (uint64_t) iroot(xz, 3)));
+    P.bC11 = pi_sqrtz;
+    P.bC20 = std::max<int64_t>({k, host_pi(T, (uint64_t) iroot(xy, 3)), pi_sqrtz});
+    P.bC21 = sg.i0;
+    const int64_t nA = std::max<int64_t>(0, P.bA1 - P.bA0);
+    const int64_t nC1 = std::max<int64_t>(0, P.bC11 - P.bC10);
+    const int64_t nC2 = std::max<int64_t>(0, P.bC21 - P.bC20);
+    // C1 products: the range of q per b, then one outer each
+    int64_t nQ = 0;
+    std::vector<int64_t> q((size_t) (2 * nC1));            // qlo, then the outers before
+    for (int64_t j = 0; j < nC1; j++) {
+      q[(size_t) (nC1 + j)] = nQ;
+      nQ += c1_q_range(T, P, P.bC10 + 1 + j, &q[(size_t) j]);
+    }
+    const int64_t nout = nA + nC1 + nQ + nC2;
+    int gridp = 0;
+    if (nout > 0) {
+      DevBuf& outs = c.tmp[T_AC_OUTS];
+      outs.alloc((size_t) nout * sizeof(PairOuter));
+      PairOuter* o = outs.as<PairOuter>();
+      if (nA) k_outer_A<<<(unsigned) ((nA + 127) / 128), 128, 0, s>>>(P, o);
+      if (nC1) k_outer_C1<<<(unsigned) ((nC1 + 127) / 128), 128, 0, s>>>(P, o + nA);
+      if (nQ) {
+        DevBuf& qb = c.tmp[T_AC_Q];
+        qb.alloc(q.size() * 8);
+        PCG_CUDA(cudaMemcpyAsync(qb.p, q.data(), q.size() * 8, cudaMemcpyHostToDevice, s));
+        k_c1_expand<<<(unsigned) ((nQ + 127) / 128), 128, 0, s>>>(P, qb.as<int64_t>(), qb.as<int64_t>() + nC1, nC1, nQ,
+                                                                  o + nA + nC1);
+      }
+      if (nC2) k_outer_C2<<<(unsigned) ((nC2 + 127) / 128), 128, 0, s>>>(P, o + nA + nC1 + nQ);
+      PCG_CUDA(cudaGetLastError());
+      *nl += 4;
+      gridp = launch_pairs(c, o, nout, s, nl);
+    }
+
+    // ---- the results
+    const double t2 = fnow_ms();
+    std::vector<i128> hac = partials(c.tmp[T_PR_PART], gridp);
+    PCG_CUDA(cudaStreamSynchronize(s));
+    const double t3 = fnow_ms();
+    ps.r.resize((size_t) (3 * ps.nseg));
+    if (ps.nseg > 0)
+      PCG_CUDA(cudaMemcpyAsync(ps.r.data(), c.tmp[T_PS_C].p, ps.r.size() * 8, cudaMemcpyDeviceToHost, s));
+    std::vector<i128> h0 = partials(part0, grid0), hs = partials(sbuf, 3 * sblocks + 2);
+    PCG_CUDA(cudaStreamSynchronize(s));
+    for (const i128& v : hac) R.ac += v;
+    for (const i128& v : h0) R.phi0 += v;
+    int64_t found[3];
+    memcpy(found, &hs[(size_t) (3 * sblocks)], sizeof(found));
+    R.b = b_sum(ps.r.data(), ps.nseg, found[2]);
 
     // ---- Sigma (Sigma.cpp:25-140)
     {
-      double t1 = fnow_ms();
       const i128 a = host_pi(T, (uint64_t) y);
-      const i128 b = host_pi(T, (uint64_t) x13);
-      const int64_t sqrt_xy = isqrt(x / (u128) y);
-      std::vector<uint64_t> q;
-      q.push_back((uint64_t) sqrtx);
-      q.push_back((uint64_t) sqrt_xy);
-      // primes in (x_star, x^(1/3)]: arguments of Sigma4..6
-      const int64_t i0 = host_pi(T, (uint64_t) x_star) + 1, i1 = host_pi(T, (uint64_t) x13);
-      for (int64_t i = i0; i <= i1; i++) {
-        const u128 p = T.h_primes[(size_t) i];
-        if ((int64_t) p <= sqrt_xy) q.push_back((uint64_t) (x / (p * (u128) y)));
-        else q.push_back((uint64_t) (x / (p * p)));
-        q.push_back((uint64_t) isqrt(x / p));
-      }
-      std::vector<int64_t> r = pi_lookup(c, q, s);
-      const i128 pi_sqrtx = r[0];
-      const i128 cc = r[1];
-      const i128 d = host_pi(T, (uint64_t) x_star);
+      const i128 b = sg.i1;
+      const i128 pi_sqrtx = found[0];
+      const i128 cc = found[1];
+      const i128 d = sg.i0;
       i128 s0 = a - 1 + (pi_sqrtx * (pi_sqrtx - 1)) / 2 - (a * (a - 1)) / 2;
       i128 s1 = (a - b) * (a - b - 1) / 2;
       i128 s2 = a * (b - cc - (cc * (cc - 3)) / 2 + (d * (d - 3)) / 2);
       i128 s3 = (b * (b - 1) * (2 * b - 1)) / 6 - b - (d * (d - 1) * (2 * d - 1)) / 6 + d;
       i128 s4 = 0, s5 = 0, s6 = 0;
-      size_t j = 2;
-      for (int64_t i = i0; i <= i1; i++) {
-        const int64_t p = T.h_primes[(size_t) i];
-        if (p <= sqrt_xy) s4 += r[j]; else s5 += r[j];
-        j++;
-        s6 += (i128) r[j] * r[j];
-        j++;
+      for (int i = 0; i < sblocks; i++) {
+        s4 += hs[(size_t) (3 * i)];
+        s5 += hs[(size_t) (3 * i + 1)];
+        s6 += hs[(size_t) (3 * i + 2)];
       }
       R.sigma = s0 + s1 + s2 + s3 + s4 * a + s5 - s6;
-      R.ms_sigma = fnow_ms() - t1;
     }
+    // wall times: B, Phi0 and Sigma run ahead of the pair sums on one stream
+    R.ms_b = t2 - t1;
+    R.ms_ac = t3 - t2;
+    R.ms_sigma = fnow_ms() - t3;
   };
   uint64_t launches2 = 0;
   if (!with_d) {
@@ -1251,7 +1328,6 @@ void pi_dr_terms(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, i128 out[7]
     const int grid = c.num_sms * 8;
     DevBuf& part = c.tmp[T_PHI0_PART];
     part.alloc((size_t) grid * 16);
-    PCG_CUDA(cudaMemsetAsync(part.p, 0, (size_t) grid * 16, s));
     PhiTab PT = phi_tab(c);
     if (T.fr_bytes == 2)
       k_phi0<uint16_t><<<grid, 256, 0, s>>>((uint64_t) x, (uint64_t) (x >> 64), T.factor_dr.as<uint16_t>(), size,
@@ -1323,8 +1399,19 @@ void pi_dr_terms(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, i128 out[7]
   out[6] = (i128) pi_y + s1 + s2_trivial + s2_easy + s2_hard - 1 - p2;
 }
 
-// x <= 1e10 is counted by the sieve directly
+// x <= 1e10 is counted by the sieve directly, from GOURDON_MIN on only by a
+// context without the tables of Gourdon's formula: with them (a context made
+// for such x) the formula takes 0.3 ms where the sieve takes 0.3 ms at 1.2e9
+// and 2.4 ms at 1e10; building them takes 2 ms.
 static const int64_t PI_SIEVE_LIMIT = 10000000000ll;
+static const int64_t GOURDON_MIN = 1200000000ll;
+
+static bool gourdon_resident(const Ctx& c, u128 x, const Tuning& tune)
+{
+  const GourdonParams g = gourdon_params(x, tune.alpha_y, tune.alpha_z);
+  const Tables& T = c.tab;
+  return T.prime_limit >= g.y && T.fd_z >= g.z && (T.fd_y == g.y || (g.y >= g.z && T.fd_y >= g.z));
+}
 
 i128 pi_any(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, pcg_stats* st)
 {
@@ -1332,7 +1419,7 @@ i128 pi_any(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, pcg_stats* st)
   i128 r;
   pcg_stats z{};
   if (x < 2) r = 0;
-  else if (x <= (u128) PI_SIEVE_LIMIT) {
+  else if (x <= (u128) PI_SIEVE_LIMIT && (x < (u128) GOURDON_MIN || !gourdon_resident(c, x, tune))) {
     uint64_t l = 0;
     r = pi_sieve_count(c, (int64_t) x, s, &l);
     z.kernel_launches = l;
@@ -1452,10 +1539,7 @@ int64_t phi_any(Ctx& c, int64_t x, int64_t a, const Tuning& tune, cudaStream_t s
       // plus 2, 3, 5 when the sieve starts at 0 (lo0 is a multiple of 240)
       i128 run = 3;
       if (o.lo0 > 0) run = pi_lookup(c, std::vector<uint64_t>{(uint64_t) (o.lo0 - 1)}, s)[0];
-      for (int64_t i = 0; i < o.nseg; i++) {
-        B += (i128) o.l[(size_t) i] + (i128) o.m[(size_t) i] * run;
-        run += o.c[(size_t) i];
-      }
+      B = b_sum(o.r.data(), o.nseg, run);
     }
     const i128 n2 = pi_sq;
     const i128 P2 = B - (n2 * (n2 - 1) - (i128) a * (a - 1)) / 2;
@@ -1487,7 +1571,6 @@ int64_t phi_any(Ctx& c, int64_t x, int64_t a, const Tuning& tune, cudaStream_t s
     const int grid = c.num_sms * 8;
     DevBuf& part = c.tmp[T_PHI0_PART];
     part.alloc((size_t) grid * 16);
-    PCG_CUDA(cudaMemsetAsync(part.p, 0, (size_t) grid * 16, s));
     PhiTab PT = phi_tab(c);
     if (T.fd_bytes == 2)
       k_phi0<uint16_t><<<grid, 256, 0, s>>>((uint64_t) x, 0, T.factor_d.as<uint16_t>(), size, (uint32_t) (2 * cc + 1),

@@ -2178,6 +2178,23 @@ static void write_checkpoint(const std::string& path, const CkptHeader& h, const
   if (!ok || rename(tmp.c_str(), path.c_str()) != 0) fail(PCG_EINVAL, "cannot write the checkpoint " + path);
 }
 
+// x / p_b (low, high word) and min(x / p_b^3, 2^63 - 1) per level
+__global__ void k_sweep_xp(uint64_t x_lo, uint64_t x_hi, const uint32_t* __restrict__ primes, int cols,
+                           uint64_t* __restrict__ xp)
+{
+  const int b = (int) (blockIdx.x * blockDim.x + threadIdx.x);
+  if (b >= cols) return;
+  u128 q = 0, q3 = 0;
+  if (b > 0) {
+    const uint64_t p = primes[b];
+    q = div128(((u128) x_hi << 64) | x_lo, p);
+    q3 = div128(div128(q, p), p);
+  }
+  xp[3 * b] = (uint64_t) q;
+  xp[3 * b + 1] = (uint64_t) (q >> 64);
+  xp[3 * b + 2] = q3 > (u128) INT64_MAX ? (uint64_t) INT64_MAX : (uint64_t) q3;
+}
+
 SweepResult run_sweep(Ctx& c, const SweepProblem& pb, const Tuning& tune_in, cudaStream_t s)
 {
   SweepResult res;
@@ -2222,17 +2239,6 @@ SweepResult run_sweep(Ctx& c, const SweepProblem& pb, const Tuning& tune_in, cud
   }
   const int cols = (int) bglob + 1;
 
-  // x / p_b and x / p_b^3 per level
-  std::vector<uint64_t> xp((size_t) cols * 3, 0);
-  for (int64_t b = 1; b <= bglob; b++) {
-    u128 p = c.tab.h_primes[(size_t) b];
-    u128 q = x / p;
-    u128 q3 = q / (p * p);
-    xp[3 * b] = (uint64_t) q;
-    xp[3 * b + 1] = (uint64_t) (q >> 64);
-    xp[3 * b + 2] = q3 > (u128) INT64_MAX ? (uint64_t) INT64_MAX : (uint64_t) q3;
-  }
-
   // tuning: threads per CTA, bitmap words per CTA, leaf-record capacity,
   // resident CTAs per SM; a configuration chosen by pcg_autotune for this
   // decade of x replaces the defaults the caller left at 0
@@ -2275,10 +2281,6 @@ SweepResult run_sweep(Ctx& c, const SweepProblem& pb, const Tuning& tune_in, cud
   }
   const std::vector<int64_t>& seglo = c.plan;
   int64_t nseg = (int64_t) seglo.size() - 1;
-  DevBuf& segbuf = c.tmp[T_SW_SEG];
-  segbuf.alloc(seglo.size() * 8);
-  PCG_CUDA(cudaMemcpyAsync(segbuf.p, seglo.data(), seglo.size() * 8, cudaMemcpyHostToDevice, s));
-
   // this call's segments: shard pb.shard of pb.nshards (all of them by default)
   if (pb.nshards < 1 || pb.shard < 0 || pb.shard >= pb.nshards) fail(PCG_EINVAL, "invalid shard");
   const int64_t seg_begin = nseg * pb.shard / pb.nshards;
@@ -2292,71 +2294,17 @@ SweepResult run_sweep(Ctx& c, const SweepProblem& pb, const Tuning& tune_in, cud
   int64_t max_rows = std::max<int64_t>(1, (int64_t) (1ull << 30) / ((int64_t) cols * 8));
   int64_t wave_len = std::max<int64_t>(1, std::min<int64_t>({nmine, wave_cap, max_rows}));
 
-  c.cnt.alloc((size_t) wave_len * cols * 4);
-  c.smu.alloc((size_t) wave_len * cols * 4);
+  // count rows, then sign rows
+  c.cnt.alloc((size_t) wave_len * cols * 8);
   c.segsum.alloc((size_t) wave_len * 8);
-  c.run.alloc((size_t) cols * 8);
-  c.acc.alloc((size_t) cols * 16);
-  c.msum.alloc((size_t) cols * 8);
-  c.misc.alloc(4096);
-  uint64_t* d_xp = nullptr;
-  DevBuf& xpbuf = c.tmp[T_SW_XP];
-  xpbuf.alloc(xp.size() * 8);
-  d_xp = xpbuf.as<uint64_t>();
-  PCG_CUDA(cudaMemcpyAsync(d_xp, xp.data(), xp.size() * 8, cudaMemcpyHostToDevice, s));
-  PCG_CUDA(cudaMemsetAsync(c.run.p, 0, (size_t) cols * 8, s));
-  PCG_CUDA(cudaMemsetAsync(c.acc.p, 0, (size_t) cols * 16, s));
-  PCG_CUDA(cudaMemsetAsync(c.msum.p, 0, (size_t) cols * 8, s));
-  PCG_CUDA(cudaMemsetAsync(c.misc.p, 0, 4096, s));
-  unsigned long long* d_counters = (unsigned long long*) c.misc.p;
-  int* d_queue = (int*) ((char*) c.misc.p + 256);   // after the 32 counters
-
-  // the problem, the row offsets of a wave's items and the combine jobs of a
-  // full wave and of the last (shorter) one
-  SweepQ q0;
-  memset(&q0, 0, sizeof(q0));
-  q0.x_lo = (uint64_t) x;
-  q0.x_hi = (uint64_t) (x >> 64);
-  q0.y = pb.y;
-  q0.z = pb.z;
-  q0.k = pb.k;
-  q0.L = L;
-  q0.x_star = x_star;
-  q0.item0 = 0;
-  q0.seglo = segbuf.as<int64_t>();
-  q0.xp_tab = d_xp;
-  q0.gourdon = pb.gourdon;
-  q0.pi_sqrt = (int) pi_sqrt;
-  q0.bglob = (int) bglob;
-  std::vector<int64_t> rowoff((size_t) wave_len);
-  for (int64_t i = 0; i < wave_len; i++) rowoff[(size_t) i] = i * cols;
-  DevBuf& qbuf = c.tmp[T_SW_Q];
-  DevBuf& rowbuf = c.tmp[T_SW_ROW];
-  DevBuf& jobbuf = c.tmp[T_SW_JOB];
-  qbuf.alloc(sizeof(SweepQ));
-  rowbuf.alloc(rowoff.size() * 8);
-  PCG_CUDA(cudaMemcpyAsync(qbuf.p, &q0, sizeof(SweepQ), cudaMemcpyHostToDevice, s));
-  PCG_CUDA(cudaMemcpyAsync(rowbuf.p, rowoff.data(), rowoff.size() * 8, cudaMemcpyHostToDevice, s));
-
-  SweepArgs a;
-  memset(&a, 0, sizeof(a));
-  a.qs = qbuf.as<SweepQ>();
-  a.nq = 1;
-  a.rowoff = rowbuf.as<int64_t>();
-  a.words = words;
-  a.primes = c.tab.primes.as<uint32_t>();
-  a.nprimes = c.tab.nprimes;
-  a.pitab = c.tab.pitab.as<uint64_t>();
-  a.pi_max = c.tab.prime_limit;
-  a.factor = pb.gourdon ? c.tab.factor_d.p : c.tab.factor_dr.p;
-  a.coprime = c.tab.coprime.as<uint16_t>();
-  a.group_max = tune.group >= 0 ? std::min(tune.group, GROUP_MAX) : sweep_group_max();
-  a.cindex = c.tab.cindex.as<int16_t>();
-  a.pmagic = c.tab.pmagic.as<uint64_t>();
-  a.cnt = c.cnt.as<uint32_t>();
-  a.smu = c.smu.as<int32_t>();
-  a.segsum = c.segsum.as<int64_t>();
-  a.counters = d_counters;
+  // what starts at zero, cleared at once: acc, counters and queue, run, msum
+  const size_t n_acc = (size_t) cols * 16, n_zero = n_acc + 4096 + n_acc;
+  c.acc.alloc(n_zero);
+  unsigned long long* d_counters = (unsigned long long*) ((char*) c.acc.p + n_acc);
+  int* d_queue = (int*) ((char*) d_counters + 256);   // after the 32 counters
+  int64_t* d_run = (int64_t*) ((char*) c.acc.p + n_acc + 4096);
+  int64_t* d_msum = d_run + cols;
+  PCG_CUDA(cudaMemsetAsync(c.acc.p, 0, n_zero, s));
 
   // resume from a checkpoint of the same problem and plan
   CkptHeader ck;
@@ -2375,8 +2323,8 @@ SweepResult run_sweep(Ctx& c, const SweepProblem& pb, const Tuning& tune_in, cud
   ck.nt = NT;
   ck.nseg = nseg;
   ck.cols = cols;
-  ck.plan_hash = plan_hash(seglo);
   const bool use_ckpt = !tune.checkpoint.empty();
+  if (use_ckpt) ck.plan_hash = plan_hash(seglo);
   int64_t start_first = seg_begin;
   if (use_ckpt) {
     CkptHeader got;
@@ -2384,9 +2332,9 @@ SweepResult run_sweep(Ctx& c, const SweepProblem& pb, const Tuning& tune_in, cud
     std::vector<i128> a0;
     if (read_checkpoint(tune.checkpoint, ck, got, r0, a0, m0) && got.next_first >= seg_begin &&
         got.next_first <= seg_end) {
-      PCG_CUDA(cudaMemcpyAsync(c.run.p, r0.data(), (size_t) cols * 8, cudaMemcpyHostToDevice, s));
+      PCG_CUDA(cudaMemcpyAsync(d_run, r0.data(), (size_t) cols * 8, cudaMemcpyHostToDevice, s));
       PCG_CUDA(cudaMemcpyAsync(c.acc.p, a0.data(), (size_t) cols * 16, cudaMemcpyHostToDevice, s));
-      PCG_CUDA(cudaMemcpyAsync(c.msum.p, m0.data(), (size_t) cols * 8, cudaMemcpyHostToDevice, s));
+      PCG_CUDA(cudaMemcpyAsync(d_msum, m0.data(), (size_t) cols * 8, cudaMemcpyHostToDevice, s));
       PCG_CUDA(cudaMemcpyAsync(d_counters, got.counters, sizeof(got.counters), cudaMemcpyHostToDevice, s));
       PCG_CUDA(cudaStreamSynchronize(s));
       start_first = got.next_first;
@@ -2397,9 +2345,9 @@ SweepResult run_sweep(Ctx& c, const SweepProblem& pb, const Tuning& tune_in, cud
   auto save = [&](int64_t next_first) {
     std::vector<int64_t> r0((size_t) cols), m0((size_t) cols);
     std::vector<i128> a0((size_t) cols);
-    PCG_CUDA(cudaMemcpyAsync(r0.data(), c.run.p, (size_t) cols * 8, cudaMemcpyDeviceToHost, s));
+    PCG_CUDA(cudaMemcpyAsync(r0.data(), d_run, (size_t) cols * 8, cudaMemcpyDeviceToHost, s));
     PCG_CUDA(cudaMemcpyAsync(a0.data(), c.acc.p, (size_t) cols * 16, cudaMemcpyDeviceToHost, s));
-    PCG_CUDA(cudaMemcpyAsync(m0.data(), c.msum.p, (size_t) cols * 8, cudaMemcpyDeviceToHost, s));
+    PCG_CUDA(cudaMemcpyAsync(m0.data(), d_msum, (size_t) cols * 8, cudaMemcpyDeviceToHost, s));
     PCG_CUDA(cudaMemcpyAsync(ck.counters, d_counters, sizeof(ck.counters), cudaMemcpyDeviceToHost, s));
     PCG_CUDA(cudaStreamSynchronize(s));
     ck.next_first = next_first;
@@ -2407,14 +2355,65 @@ SweepResult run_sweep(Ctx& c, const SweepProblem& pb, const Tuning& tune_in, cud
     last_write = now_ms();
   };
 
-  // combine jobs of a full wave and of the last one (from start_first on)
+  // the inputs in one copy: the problem, the segment bounds, the row offsets
+  // of a wave's items, and the combine jobs of a full wave and of the last
+  // (shorter) one from start_first on; x / p per level is made on the device
   const int64_t last_len = seg_end > start_first ? (seg_end - start_first - 1) % wave_len + 1 : wave_len;
   std::vector<CombineJob> jobs;
   add_combine_jobs(jobs, 0, 0, (int) wave_len, cols);
   const int njobs = (int) jobs.size();
-  add_combine_jobs(jobs, 0, 0, (int) last_len, cols);
-  jobbuf.alloc(jobs.size() * sizeof(CombineJob));
-  PCG_CUDA(cudaMemcpyAsync(jobbuf.p, jobs.data(), jobs.size() * sizeof(CombineJob), cudaMemcpyHostToDevice, s));
+  if (last_len != wave_len) add_combine_jobs(jobs, 0, 0, (int) last_len, cols);
+  const size_t at_seg = (sizeof(SweepQ) + 15) / 16 * 16, at_row = at_seg + seglo.size() * 8,
+               at_job = at_row + (size_t) wave_len * 8, n_in = at_job + jobs.size() * sizeof(CombineJob);
+  DevBuf& inbuf = c.tmp[T_SW_SEG];
+  DevBuf& xpbuf = c.tmp[T_SW_XP];
+  inbuf.alloc(n_in);
+  xpbuf.alloc((size_t) cols * 24);
+  char* const d_in = inbuf.as<char>();
+  SweepQ q0;
+  memset(&q0, 0, sizeof(q0));
+  q0.x_lo = (uint64_t) x;
+  q0.x_hi = (uint64_t) (x >> 64);
+  q0.y = pb.y;
+  q0.z = pb.z;
+  q0.k = pb.k;
+  q0.L = L;
+  q0.x_star = x_star;
+  q0.item0 = 0;
+  q0.seglo = (const int64_t*) (d_in + at_seg);
+  q0.xp_tab = xpbuf.as<uint64_t>();
+  q0.gourdon = pb.gourdon;
+  q0.pi_sqrt = (int) pi_sqrt;
+  q0.bglob = (int) bglob;
+  std::vector<char> in(n_in, 0);
+  memcpy(in.data(), &q0, sizeof(q0));
+  memcpy(in.data() + at_seg, seglo.data(), seglo.size() * 8);
+  for (int64_t i = 0; i < wave_len; i++) ((int64_t*) (in.data() + at_row))[i] = i * cols;
+  memcpy(in.data() + at_job, jobs.data(), jobs.size() * sizeof(CombineJob));
+  PCG_CUDA(cudaMemcpyAsync(d_in, in.data(), n_in, cudaMemcpyHostToDevice, s));
+  k_sweep_xp<<<(unsigned) ((cols + 127) / 128), 128, 0, s>>>((uint64_t) x, (uint64_t) (x >> 64),
+                                                             c.tab.primes.as<uint32_t>(), cols, xpbuf.as<uint64_t>());
+  PCG_CUDA(cudaGetLastError());
+  const CombineJob* d_jobs = (const CombineJob*) (d_in + at_job);
+
+  SweepArgs a;
+  memset(&a, 0, sizeof(a));
+  a.qs = (const SweepQ*) d_in;
+  a.nq = 1;
+  a.rowoff = (const int64_t*) (d_in + at_row);
+  a.words = words;
+  a.primes = c.tab.primes.as<uint32_t>();
+  a.nprimes = c.tab.nprimes;
+  a.pitab = c.tab.pitab.as<uint64_t>();
+  a.pi_max = c.tab.prime_limit;
+  a.factor = pb.gourdon ? c.tab.factor_d.p : c.tab.factor_dr.p;
+  a.coprime = c.tab.coprime.as<uint16_t>();
+  a.group_max = tune.group >= 0 ? std::min(tune.group, GROUP_MAX) : sweep_group_max();
+  a.cindex = c.tab.cindex.as<int16_t>();
+  a.pmagic = c.tab.pmagic.as<uint64_t>();
+  a.cnt = c.cnt.as<uint32_t>();
+  a.segsum = c.segsum.as<int64_t>();
+  a.counters = d_counters;
 
   PCG_CUDA(cudaEventRecord(c.ev[0], s));
   uint64_t launches = 0;
@@ -2425,8 +2424,8 @@ SweepResult run_sweep(Ctx& c, const SweepProblem& pb, const Tuning& tune_in, cud
     a.wave_first = first;
     a.wave_len = wl;
     a.queue = d_queue + (waves % 16);
-    PCG_CUDA(cudaMemsetAsync(c.cnt.p, 0, (size_t) wl * cols * 4, s));
-    PCG_CUDA(cudaMemsetAsync(c.smu.p, 0, (size_t) wl * cols * 4, s));
+    a.smu = c.cnt.as<int32_t>() + (size_t) wl * cols;
+    PCG_CUDA(cudaMemsetAsync(c.cnt.p, 0, (size_t) wl * cols * 8, s));
     if (waves % 16 == 0 && waves > 0) PCG_CUDA(cudaMemsetAsync(d_queue, 0, 64, s));
     int g = (int) std::min<int64_t>(grid, wl);
     if ((size_t) (2 * waves + 2) > c.kev.size()) {
@@ -2440,9 +2439,8 @@ SweepResult run_sweep(Ctx& c, const SweepProblem& pb, const Tuning& tune_in, cud
     else { if (fbytes == 2) launch_sweep<uint16_t, 128>(a, g, smem, s); else launch_sweep<uint32_t, 128>(a, g, smem, s); }
     PCG_CUDA(cudaGetLastError());
     PCG_CUDA(cudaEventRecord(c.kev[2 * waves + 1], s));
-    const CombineJob* wj = jobbuf.as<CombineJob>() + (wl == wave_len ? 0 : njobs);
-    k_combine<<<njobs, 32 * COMBINE_WARPS, 0, s>>>(a.cnt, a.smu, a.rowoff, a.segsum, wj, c.run.as<int64_t>(),
-                                                  c.acc.as<i128>(), c.msum.as<int64_t>());
+    const CombineJob* wj = d_jobs + (wl == wave_len ? 0 : njobs);
+    k_combine<<<njobs, 32 * COMBINE_WARPS, 0, s>>>(a.cnt, a.smu, a.rowoff, a.segsum, wj, d_run, c.acc.as<i128>(), d_msum);
     PCG_CUDA(cudaGetLastError());
     launches += 2;
     waves++;
@@ -2457,17 +2455,18 @@ SweepResult run_sweep(Ctx& c, const SweepProblem& pb, const Tuning& tune_in, cud
     }
   }
   PCG_CUDA(cudaEventRecord(c.ev[1], s));
-  std::vector<i128> acc((size_t) cols);
-  unsigned long long ctr[5];
-  PCG_CUDA(cudaMemcpyAsync(acc.data(), c.acc.p, (size_t) cols * 16, cudaMemcpyDeviceToHost, s));
-  PCG_CUDA(cudaMemcpyAsync(ctr, d_counters, sizeof(ctr), cudaMemcpyDeviceToHost, s));
+  unsigned long long ctr[6];                              // 48 bytes: the sums and the counters in one copy
+  std::vector<i128> acc((size_t) cols + sizeof(ctr) / 16);
+  PCG_CUDA(cudaMemcpyAsync(acc.data(), c.acc.p, n_acc + sizeof(ctr), cudaMemcpyDeviceToHost, s));
   if (pb.parts) {
     res.msum.resize((size_t) cols);
     res.csum.resize((size_t) cols);
-    PCG_CUDA(cudaMemcpyAsync(res.msum.data(), c.msum.p, (size_t) cols * 8, cudaMemcpyDeviceToHost, s));
-    PCG_CUDA(cudaMemcpyAsync(res.csum.data(), c.run.p, (size_t) cols * 8, cudaMemcpyDeviceToHost, s));
+    PCG_CUDA(cudaMemcpyAsync(res.msum.data(), d_msum, (size_t) cols * 8, cudaMemcpyDeviceToHost, s));
+    PCG_CUDA(cudaMemcpyAsync(res.csum.data(), d_run, (size_t) cols * 8, cudaMemcpyDeviceToHost, s));
   }
   PCG_CUDA(cudaStreamSynchronize(s));
+  memcpy(ctr, &acc[(size_t) cols], sizeof(ctr));
+  acc.resize((size_t) cols);
   if (pb.parts) res.acc = acc;
   PCG_CUDA(cudaEventElapsedTime(&ms_sweep, c.ev[0], c.ev[1]));
   double kms = 0;
@@ -2478,9 +2477,8 @@ SweepResult run_sweep(Ctx& c, const SweepProblem& pb, const Tuning& tune_in, cud
   }
   st.sweep_kernel_ms = kms;
   st.sweep_launches = (uint64_t) waves;
-  st.h2d_bytes = xp.size() * 8 + seglo.size() * 8 + sizeof(SweepQ) + rowoff.size() * 8 +
-                 jobs.size() * sizeof(CombineJob);
-  st.d2h_bytes = (uint64_t) cols * 16 + sizeof(ctr);
+  st.h2d_bytes = n_in;
+  st.d2h_bytes = n_acc + sizeof(ctr);
   i128 sum = 0;
   for (int b = 0; b < cols; b++) sum += acc[(size_t) b];
   res.sum = sum;
