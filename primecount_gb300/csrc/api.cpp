@@ -515,9 +515,11 @@ pcg_status pcg_autotune(pcg_i128 xi, const pcg_opts* opts, pcg_tuning* best)
     double bms = 1e300;
     i128 ref = 0;
     bool have = false;
+    const bool is_long = long_interval(1, (int64_t) (x / (u128) g.z));
     for (const auto& k : cand) {
       Tuning t;
-      t.segment_words = k[0];
+      // of a long interval its own default shape in the place of 16384 words
+      t.segment_words = is_long && k[0] == 16384 ? 20480 : k[0];
       t.ctas_per_sm = k[1];
       t.cta_threads = k[2];
       t.group = k[3];

@@ -168,6 +168,8 @@ SweepResult run_sweep(Ctx& c, const SweepProblem& p, const Tuning& t, cudaStream
 // as one CUDA graph; sums[i] = D of pbs[i]
 void run_sweep_batch(Ctx& c, const std::vector<SweepProblem>& pbs, const Tuning& t, cudaStream_t s,
                      std::vector<i128>& sums, pcg_stats* st);
+// whether a sweep of [0, L) takes the launch shape of long intervals
+bool long_interval(int gourdon, int64_t L);
 // device working memory of one sweep over [0, L) with cols columns
 uint64_t sweep_device_bytes(int num_sms, int64_t L, int64_t cols, int words);
 // frees a context's per-call working memory (the tables stay); bytes freed

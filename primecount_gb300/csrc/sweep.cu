@@ -390,18 +390,19 @@ __device__ __forceinline__ uint64_t div_xp(uint64_t xlo, uint64_t xhi, uint64_t 
 }
 
 // Exclusive prefix of the chunk counts, one value per 4 chunks (32 words), n4
-// of them, by the first SCAN_WARPS warps (ccount 16-byte aligned).  scan_part
-// leaves each warp's part relative to its start and the parts' sums in wtmp;
+// of them, by the first SW warps (ccount 16-byte aligned).  scan_part leaves
+// each warp's part relative to its start and the parts' sums in wtmp;
 // scan_chunks, called by the whole block, the whole prefix.
-#define SCAN_WARPS 4
 // values per warp
-__device__ __forceinline__ int scan_per(int n4) { return 32 * ((n4 + 32 * SCAN_WARPS - 1) / (32 * SCAN_WARPS)); }
+template <int SW>
+__device__ __forceinline__ int scan_per(int n4) { return 32 * ((n4 + 32 * SW - 1) / (32 * SW)); }
 
+template <int SW>
 __device__ __forceinline__ void scan_part(const uint32_t* __restrict__ ccount, uint32_t* __restrict__ pref, int n4,
                                           uint32_t* wtmp)
 {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int ql = scan_per(n4) / 32;                    // values per lane
+  const int ql = scan_per<SW>(n4) / 32;                // values per lane
   const int i0 = min(n4, (warp * 32 + lane) * ql), i1 = min(n4, i0 + ql);
   uint32_t sum = 0;
   for (int i = i0; i < i1; i++) {
@@ -418,14 +419,15 @@ __device__ __forceinline__ void scan_part(const uint32_t* __restrict__ ccount, u
   for (int i = i0; i < i1; i++) pref[i] += incl - sum;
 }
 
+template <int SW>
 __device__ __forceinline__ void scan_chunks(const uint32_t* __restrict__ ccount, uint32_t* __restrict__ pref, int n4,
                                             uint32_t* wtmp)
 {
   const int warp = threadIdx.x >> 5;
-  if (warp < SCAN_WARPS) scan_part(ccount, pref, n4, wtmp);
+  if (warp < SW) scan_part<SW>(ccount, pref, n4, wtmp);
   __syncthreads();
-  if (warp < SCAN_WARPS && warp > 0) {
-    const int per = scan_per(n4);
+  if (warp < SW && warp > 0) {
+    const int per = scan_per<SW>(n4);
     uint32_t base = 0;
     for (int w = 0; w < warp; w++) base += wtmp[w];
     for (int i = warp * per + (threadIdx.x & 31); i < min(n4, (warp + 1) * per); i += 32) pref[i] += base;
@@ -481,7 +483,8 @@ static __device__ __forceinline__ uint32_t leaf_quotient(uint64_t r, uint32_t m)
   return __float2uint_rz(rf * inv);
 }
 
-// m < 2^30: the remainder fits 32 signed bits
+// m < 2^30 in a segment of at most LEAF_SPAN numbers: the remainder fits 32
+// signed bits
 static __device__ __forceinline__ uint32_t leaf_narrow(uint64_t xlo, uint64_t low, uint32_t m)
 {
   const uint64_t r = xlo - low * m;
@@ -632,7 +635,7 @@ constexpr int sweep_batch(int nt) { return nt < 256 ? nt : 256; }
 // 2 words / 67 + 1 of the longest level, p = 67, up to 21 000 words);
 // collisions of a group kept for the end of its clears
 #define REC_CAP 3584
-#define MASK_WORDS 640
+constexpr int sweep_mask_words(int nt) { return nt >= 512 ? 1280 : 640; }
 #define COLLISIONS 512
 
 // dynamic shared memory of k_sweep: byte offsets; then the chunk counts
@@ -649,9 +652,9 @@ constexpr SweepLayout sweep_layout(int nt)
   y.wofs = y.lp + lb * (int) sizeof(LevelP);
   y.rec = y.wofs + (lb + 1) * 4;
   y.masks = y.rec + REC_CAP * 4;
-  y.clist = y.masks + 2 * (MASK_WORDS + 1) * 4;
+  y.clist = y.masks + 2 * (sweep_mask_words(nt) + 1) * 4;
   y.mpre = y.clist + COLLISIONS * 4;
-  y.cop = y.mpre + (MASK_WORDS + 2) * 2;
+  y.cop = y.mpre + (sweep_mask_words(nt) + 2) * 2;
   y.bits = (y.cop + 480 * 2 + 15) / 16 * 16;
   return y;
 }
@@ -663,6 +666,8 @@ template <typename FT, int NT>
 __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k_sweep(const SweepArgs A)
 {
   constexpr int NW = NT / 32;
+  constexpr int MASK_WORDS = sweep_mask_words(NT);
+  constexpr int SW = NT >= 512 ? 8 : 4;                // warps that scan the chunk counts
   constexpr int LB = sweep_batch(NT);                  // levels per batch
   constexpr int OB = 23;                               // offset bits of a record
   constexpr uint32_t OM = (1u << OB) - 1u;
@@ -1192,6 +1197,10 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
                 first = false;
               }
             };
+            // a lane's first collision waits for the end, so that the lanes list
+            // theirs together
+            uint32_t pend = NO_FIRST;
+            auto note = [&](uint32_t o) { if (pend == NO_FIRST) pend = o; else collide(o); };
             if (shortl) {
               for (int l = li + warp; l < lj; l += 4 * NW) {
                 uint32_t h[4], m[4], nw[4], p[4], w[4];
@@ -1225,7 +1234,7 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
                   while (lost) {
                     const LevelM Q = lm[l + (__ffs((int) lost) - 1) * NW];
                     lost &= lost - 1;
-                    collide(Q.first + Q.prime * (s_delta[(Q.jn8 & 7) * 32 + lane] + 120 * j));
+                    note(Q.first + Q.prime * (s_delta[(Q.jn8 & 7) * 32 + lane] + 120 * j));
                   }
                 }
               }
@@ -1256,11 +1265,12 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
                 while (lost) {
                   const uint32_t d = (uint32_t) __ffs((int) lost) - 1;
                   lost &= lost - 1;
-                  collide(120 * (h + d * p) + res);
+                  note(120 * (h + d * p) + res);
                 }
               }
               wi = e;
             }
+            if (pend != NO_FIRST) collide(pend);
             __syncthreads();
             if (s_ncoll) {
               const int nc = min(s_ncoll, COLLISIONS);
@@ -1269,7 +1279,7 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
               if (tid == 0) s_ncoll = 0;                 // next used after two more barriers
             }
             // 3. the prefix of the masks' counts (the last warp) and of the
-            // chunk counts (the first SCAN_WARPS warps, each its part)
+            // chunk counts (the first SW warps, each its part)
             if (warp == NW - 1) {
               const int per = ((W + 31) / 32) | 1;      // odd: no bank conflicts
               const int i0 = min(W, lane * per), i1 = min(W, i0 + per);
@@ -1287,7 +1297,7 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
               }
               if (lane == 31) { mpre[W] = (uint16_t) run; mk[W] = 0; }
             }
-            if (rb > ra && warp < SCAN_WARPS) scan_part(ccount, pref, n4, wtmp);
+            if (rb > ra && warp < SW) scan_part<SW>(ccount, pref, n4, wtmp);
             __syncthreads();
             // the levels' counts C(s, b)
             for (int t = tid; t < G; t += NT)
@@ -1295,15 +1305,24 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
             total -= mpre[W];
             // 4. the records
             if (rb > ra) {
-              const uint32_t t0 = wtmp[0], t1 = t0 + wtmp[1], t2 = t1 + wtmp[2];
-              const uint32_t per = 4 * (uint32_t) scan_per(n4);   // chunks per scan warp
-              auto part_base = [&](uint32_t ch) { return ch < per ? 0u : (ch < 2 * per ? t0 : (ch < 3 * per ? t1 : t2)); };
+              // the scan warps' parts start at these counts
+              uint32_t pbase[SW];
+              pbase[0] = 0;
+#pragma unroll
+              for (int i = 1; i < SW; i++) pbase[i] = pbase[i - 1] + wtmp[i - 1];
+              const uint32_t per = 4 * (uint32_t) scan_per<SW>(n4);   // chunks per scan warp
+              auto part_base = [&](uint32_t ch) {
+                uint32_t v = 0;
+#pragma unroll
+                for (int i = 1; i < SW; i++) v = ch >= i * per ? pbase[i] : v;
+                return v;
+              };
               if (rb - ra <= LANE_RECORDS || G > LANE_LEVELS) {
                 // A warp takes a run of records, drops the rejected ones and
                 // answers four at a time: eight lanes each for the words of the
                 // record's chunk, then all lanes over the group's levels, each
                 // level's parameters loaded once for the four.
-                const int run = rb - ra <= 8 * NW ? 8 : (rb - ra <= 16 * NW ? 16 : 32);
+                const int run = rb - ra <= 24 * NW ? 8 : (rb - ra <= 64 * NW ? 16 : 32);
                 const int sub = lane & 7, own = lane >> 3;
                 for (int k0 = ra + run * warp; k0 < rb; k0 += run * NW) {
                   const uint32_t rv = lane < run && k0 + lane < rb ? rec[k0 + lane] : REC_NONE;
@@ -1406,7 +1425,7 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
         if (tid == NT - 1) A.cnt[rowbase + l] = total;   // the last thread: rarely a multiple to cross off
         const int64_t E2 = loff[li + 1] - loff[li];
         if (E2 > 0) {
-          if (dirty) { scan_chunks(ccount, pref, n4, wtmp); dirty = false; wp_ok = false; }
+          if (dirty) { scan_chunks<SW>(ccount, pref, n4, wtmp); dirty = false; wp_ok = false; }
           const bool by_word = wp_fits && E2 > WORD_RECORDS;
           if (by_word && !wp_ok) {
             for (int c = tid; c < nchu; c += NT) {
@@ -2178,6 +2197,16 @@ static void write_checkpoint(const std::string& path, const CkptHeader& h, const
   if (!ok || rename(tmp.c_str(), path.c_str()) != 0) fail(PCG_EINVAL, "cannot write the checkpoint " + path);
 }
 
+// The launch shape of a long interval [0, L): one CTA of 512 threads per SM
+// with the longest segment that fits, so that the chain of levels is walked
+// for 2.5 times the numbers.  Two CTAs of 256 threads with 8192 words overlap
+// each other's waits and cut the short ones better: D(10^16.5) (L = 4.3e9)
+// 5.57 against 5.80 ms, D(1e17) (8.4e9) 11.3 against 11.0, D(1e18) 44.2 / 43.3,
+// D(1e20) 753 / 704; 640 or 768 threads instead of 512: 760, 876.
+#define LONG_WORDS 20480
+#define LONG_THREADS 512
+bool long_interval(int gourdon, int64_t L) { return gourdon == 1 && L >= 6000000000ll; }
+
 // x / p_b (low, high word) and min(x / p_b^3, 2^63 - 1) per level
 __global__ void k_sweep_xp(uint64_t x_lo, uint64_t x_hi, const uint32_t* __restrict__ primes, int cols,
                            uint64_t* __restrict__ xp)
@@ -2252,6 +2281,10 @@ SweepResult run_sweep(Ctx& c, const SweepProblem& pb, const Tuning& tune_in, cud
       tune.ctas_per_sm = c.tuned_cfg[e].ctas_per_sm;
       tune.group = c.tuned_cfg[e].group;
     }
+  }
+  if (!tune.segment_words && !tune.cta_threads && long_interval(pb.gourdon, L)) {
+    tune.segment_words = LONG_WORDS;
+    tune.cta_threads = LONG_THREADS;
   }
   const int NT = (tune.cta_threads == 512 || tune.cta_threads == 128) ? tune.cta_threads : 256;
   int words = tune.segment_words > 0 ? tune.segment_words : 8192;
