@@ -675,6 +675,9 @@ static uint64_t pi_query_bytes(const Ctx& c, u128 x)
   uint64_t b = sweep_device_bytes(c.num_sms, (int64_t) (x / (u128) g.z), cols, 8192);
   b += psieve_bytes(sqrtx, (int64_t) (x / (u128) g.y) + 1);
   b += (uint64_t) pi_estimate(c, iroot(x, 3)) * 4 * 64;      // A + C outer terms
+  // their pieces, 12 bytes each, 131072 outers at a time: 5.6e4 at 1e15, 4.6e6
+  // at 1e18, 3.2e7 at 1e20, 1.1e8 at 1e21
+  b += (uint64_t) (12 * 8e7 * std::pow((double) x / 1e20, 0.58));
   b += table_bytes_beyond(c, g.y, g.z, sqrtx);
   return b + 65536;
 }

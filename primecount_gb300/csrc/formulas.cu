@@ -287,35 +287,253 @@ __device__ __forceinline__ long long outer_terms(const PairOuter& O, const uint3
   return pair_terms<MODE, 1, LOWN>(O, primes, magic, pt, s_mask);
 }
 
-// outers of more than PAIR_SPLIT terms are cut into pieces of PAIR_SPLIT so
-// that the pieces spread evenly over the blocks
+// ---- pieces of the outers
+// A gather of the PiTable from global memory is one 32-byte sector per term:
+// 1 per clock and SM from the L2, 0.26 from HBM once the table is longer than
+// the L2.  The terms' n = xp / q lie almost all near their lower end (their
+// number falls as 1 / n), so the range n < PSEG_COUNT * PSEG_NUMBERS is cut
+// into segments whose part of the table fits shared memory (14 gathers per
+// clock), {count since the segment's start, bits} per 120 numbers, and the
+// outers into pieces of at most PSEG_PIECE terms of one segment, a list per
+// segment (k_pairs_seg).  n - start is the single-precision quotient of
+// xp - start q by q with one correction, as in the sweep's leaves: primes
+// below 2^30, segments below 2^21 numbers.  The terms of larger n, few per
+// outer and segment, are the last list, in pieces of PAIR_SPLIT terms for
+// k_pairs.  Bound by integer issue (about 30 instructions a term).  Measured
+// on a GB300, all terms by k_pairs -> this: A + C of 1e16 1.28 -> 0.77 ms, 1e18
+// 21.0 -> 13.6 ms, 1e20 496 -> 271 ms; 256 threads a block 360 ms, 64 segments
+// 308 ms, 512 segments 273 ms.
+#define PSEG_ENTRIES 13312
+#define PSEG_NUMBERS (PSEG_ENTRIES * 120)
+#define PSEG_COUNT 256
+#define PSEG_THREADS 512
+#define PSEG_PIECE 4096
 #define PAIR_SPLIT 16384
-__global__ void k_pair_pieces(const PairOuter* __restrict__ outs, int64_t n, uint32_t* __restrict__ pieces)
+struct PairPiece { uint32_t o, lo, hi; };    // the prime indices (lo, hi] of outer o
+
+struct PieceArgs {
+  const PairOuter* outs;
+  int64_t n_outer;
+  int32_t nseg;                  // segments; list nseg holds the rest
+  int64_t prime_limit, nprimes;
+  const uint64_t* pismall;
+  uint32_t* count;               // [nseg + 1] pieces per list
+  uint32_t* cursor;              // [nseg + 1] pieces placed
+  const uint32_t* first;         // [nseg + 1] first piece of each list
+  PairPiece* pieces;
+};
+
+// floor(xp / n) capped, v = floor((2^64 - 1) / n): the largest q with xp / q >= n
+static __device__ __forceinline__ int64_t pseg_q(const PairOuter& O, uint64_t n, uint64_t v, int64_t cap)
 {
-  const int64_t j = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
-  if (j > n) return;
-  const int64_t c = j < n ? dmax(0, outs[j].i_hi - outs[j].i_lo) : 0;
-  pieces[j] = (uint32_t) ((c + PAIR_SPLIT - 1) / PAIR_SPLIT);
+  if (n == 0) return cap;
+  if (O.xp_hi == 0) {
+    const uint64_t q = div_magic(O.xp_lo, n, v);
+    return q < (uint64_t) cap ? (int64_t) q : cap;
+  }
+  return divcap(((u128) O.xp_hi << 64) | O.xp_lo, n, cap);
 }
 
-__global__ void k_pair_split(const PairOuter* __restrict__ outs, int64_t n, const uint64_t* __restrict__ first,
-                             PairOuter* __restrict__ split)
+// count of primes in (start, start + d], less the table's start, for the
+// thread's primes i = first, first + step, ... <= hi
+template <bool LOW>
+__device__ __forceinline__ long long pseg_terms(const uint2* __restrict__ tab, const uint8_t* s_sh,
+                                                const uint32_t* __restrict__ primes, uint64_t xp, uint64_t start,
+                                                uint32_t first, uint32_t hi, uint32_t step, uint32_t base)
 {
-  const int64_t j = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  const PairOuter O = outs[j];
-  const int64_t np = (int64_t) (first[j + 1] - first[j]);
-  for (int64_t t = 0; t < np; t++) {
-    PairOuter P = O;
-    P.i_lo = O.i_lo + t * PAIR_SPLIT;
-    P.i_hi = dmin(O.i_hi, P.i_lo + PAIR_SPLIT);
-    split[first[j] + t] = P;
+  auto term = [&](uint32_t q) -> uint32_t {
+    const uint64_t r = xp - start * q;
+    float inv;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(__uint2float_rn(q)));
+    const float rf = __fmaf_rn(__uint2float_rn((uint32_t) (r >> 32)), 4294967296.0f, __uint2float_rn((uint32_t) r));
+    uint32_t d = __float2uint_rz(rf * inv);
+    const int32_t t = (int32_t) ((uint32_t) r - d * q);
+    if (t < 0) d--;
+    if (t >= (int32_t) q) d++;
+    const uint32_t h = d / 120;
+    const uint2 e = tab[h];
+    uint32_t m;
+    asm("shr.u32 %0, %1, %2;" : "=r"(m) : "r"(0xFFFFFFFFu), "r"((uint32_t) s_sh[d - 120 * h]));
+    uint32_t c = e.x + __popc(e.y & m);
+    // the first word's count holds 2, 3 and 5 (base is 0 there)
+    if (LOW && d < 6) c = (0x322100u >> (4 * d)) & 15u;
+    return c;
+  };
+  long long sum = 0;
+  uint32_t i = first;
+  while (i <= hi) {
+    // at most 4096 terms of less than 2^20 before the sum is widened
+    uint32_t acc = 0, n = 0;
+    for (; n < 4096 && (uint64_t) i + 7ull * step <= hi; n += 8, i += 8 * step) {
+      uint32_t q[8];
+#pragma unroll
+      for (int u = 0; u < 8; u++) q[u] = __ldg(&primes[i + u * step]);
+#pragma unroll
+      for (int u = 0; u < 8; u++) acc += term(q[u]);
+    }
+    if (n < 4096)
+      for (; i <= hi; i += step, n++) acc += term(__ldg(&primes[i]));
+    sum += (long long) acc + (long long) n * base;
   }
+  return sum;
+}
+
+// the value of the thread's part of the terms (lo, hi] of outer O: indices
+// lo + 1 + at + step t
+template <bool LOW>
+__device__ __forceinline__ long long pseg_outer(const PairOuter& O, uint32_t lo, uint32_t hi, uint32_t at, uint32_t step,
+                                                const uint2* tab, const uint8_t* s_sh, const uint32_t* primes,
+                                                uint64_t start, uint32_t base)
+{
+  if (O.mode == 0) {
+    const uint32_t ic = (uint32_t) min((uint64_t) hi, max((uint64_t) lo, O.cap));
+    long long v = 0;
+    if (ic > lo) v = pseg_terms<false>(tab, s_sh, primes, O.xp_lo, start, lo + 1 + at, ic, step, base);
+    if (hi > ic) v += 2 * pseg_terms<false>(tab, s_sh, primes, O.xp_lo, start, ic + 1 + at, hi, step, base);
+    return v;
+  }
+  const uint32_t first = lo + 1 + at;
+  const long long v = pseg_terms<LOW>(tab, s_sh, primes, O.xp_lo, start, first, hi, step, base);
+  const long long c = first <= hi ? (long long) ((hi - first) / step + 1) : 0;
+  if (O.mode == 3) return v - c * ((long long) first - 1) - (long long) step * (c * (c - 1) / 2);
+  const long long t = v - c * ((long long) O.b - 2);
+  return O.mode == 1 || O.mode == 5 ? t : -t;
+}
+
+// calls f(list, lo, hi) for the parts of outer O, from the smallest n up
+template <class F>
+__device__ __forceinline__ void outer_parts(const PairOuter& O, const PieceArgs& A, F f)
+{
+  int64_t hi = O.i_hi;
+  if (hi <= O.i_lo) return;
+  for (int s = 0; s < A.nseg && hi > O.i_lo; s++) {
+    // the primes with n >= the segment's end
+    const uint64_t n1 = (uint64_t) (s + 1) * PSEG_NUMBERS;
+    const int64_t q = pseg_q(O, n1, UINT64_MAX / n1, A.prime_limit);
+    const int64_t l = q >= A.prime_limit ? A.nprimes : dpi(A.pismall, (uint64_t) q);
+    const int64_t lo = dmax(O.i_lo, dmin(hi, l));
+    if (hi > lo) f(s, (uint32_t) lo, (uint32_t) hi);
+    hi = lo;
+  }
+  if (hi > O.i_lo) f(A.nseg, (uint32_t) O.i_lo, (uint32_t) hi);
+}
+
+static __device__ __forceinline__ uint32_t piece_terms(const PieceArgs& A, int s) { return s < A.nseg ? PSEG_PIECE : PAIR_SPLIT; }
+
+__global__ void __launch_bounds__(128) k_piece_count(const PieceArgs A)
+{
+  __shared__ uint32_t cnt[PSEG_COUNT + 1];
+  for (int s = threadIdx.x; s <= A.nseg; s += blockDim.x) cnt[s] = 0;
+  __syncthreads();
+  const int64_t j = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
+  if (j < A.n_outer)
+    outer_parts(A.outs[j], A, [&](int s, uint32_t lo, uint32_t hi) {
+      const uint32_t m = piece_terms(A, s);
+      atomicAdd(&cnt[s], (hi - lo + m - 1) / m);
+    });
+  __syncthreads();
+  for (int s = threadIdx.x; s <= A.nseg; s += blockDim.x)
+    if (cnt[s]) atomicAdd(&A.count[s], cnt[s]);
+}
+
+// the same parts counted per block, a run of each list taken, then placed
+__global__ void __launch_bounds__(128) k_piece_fill(const PieceArgs A)
+{
+  __shared__ uint32_t cnt[PSEG_COUNT + 1];
+  for (int s = threadIdx.x; s <= A.nseg; s += blockDim.x) cnt[s] = 0;
+  __syncthreads();
+  const int64_t j = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
+  PairOuter O;
+  O.i_lo = O.i_hi = 0;
+  if (j < A.n_outer) O = A.outs[j];
+  outer_parts(O, A, [&](int s, uint32_t lo, uint32_t hi) {
+    const uint32_t m = piece_terms(A, s);
+    atomicAdd(&cnt[s], (hi - lo + m - 1) / m);
+  });
+  __syncthreads();
+  for (int s = threadIdx.x; s <= A.nseg; s += blockDim.x)
+    if (cnt[s]) cnt[s] = A.first[s] + atomicAdd(&A.cursor[s], cnt[s]);
+  __syncthreads();
+  outer_parts(O, A, [&](int s, uint32_t lo, uint32_t hi) {
+    const uint32_t m = piece_terms(A, s), n = (hi - lo + m - 1) / m;
+    const uint32_t at = atomicAdd(&cnt[s], n);
+    for (uint32_t t = 0; t < n; t++) A.pieces[at + t] = PairPiece{(uint32_t) j, lo + t * m, min(hi, lo + (t + 1) * m)};
+  });
+}
+
+// The pieces of the segments.  A work item is up to PSEG_ITEM pieces of one
+// segment's list (items of segment s: [item0[s], item0[s + 1])); a warp takes
+// a piece at a time.
+#define PSEG_ITEM 128
+struct PsegArgs {
+  const PairOuter* outs;
+  const PairPiece* pieces;
+  int32_t nseg;
+  const uint32_t* first;         // [nseg + 1] first piece of each list
+  const uint32_t* item0;         // [nseg + 1] first item of each segment
+  const uint32_t* primes;
+  const ulonglong2* pibig;
+  int64_t big_words;             // words of pibig
+  int* queue;
+  i128* partial;
+};
+
+__global__ void __launch_bounds__(PSEG_THREADS, 2) k_pairs_seg(const PsegArgs A)
+{
+  extern __shared__ __align__(16) unsigned char psm[];
+  uint2* const tab = (uint2*) psm;
+  __shared__ uint8_t s_sh[120];                          // 32 - # wheel residues <= r
+  __shared__ uint32_t s_item0[PSEG_COUNT + 1];
+  __shared__ int s_item, s_next;
+  const int tid = threadIdx.x, lane = tid & 31;
+  for (int r = tid; r < 120; r += PSEG_THREADS) s_sh[r] = (uint8_t) (32 - ((r / 30) * 8 + cnt8((uint32_t) (r % 30))));
+  for (int s = tid; s <= A.nseg; s += PSEG_THREADS) s_item0[s] = A.item0[s];
+  i128 acc = 0;
+  int cur = -1;                                          // segment in tab
+  uint32_t base = 0;
+  for (;;) {
+    __syncthreads();
+    if (tid == 0) { s_item = atomicAdd(A.queue, 1); s_next = 0; }
+    __syncthreads();
+    const uint32_t item = (uint32_t) s_item;
+    if (item >= s_item0[A.nseg]) break;
+    int seg = max(cur, 0);                               // items come in order
+    while (item >= s_item0[seg + 1]) seg++;
+    const uint64_t n0 = (uint64_t) seg * PSEG_NUMBERS;
+    if (seg != cur) {
+      const int64_t w0 = (int64_t) (n0 / 240);
+      base = seg == 0 ? 0u : (uint32_t) A.pibig[w0].x;
+      for (int w = tid; w < PSEG_ENTRIES / 2; w += PSEG_THREADS) {
+        ulonglong2 e = make_ulonglong2(base, 0);
+        if (w0 + w < A.big_words) e = __ldg(&A.pibig[w0 + w]);
+        const uint32_t c = (uint32_t) e.x - base, b0 = (uint32_t) e.y;
+        tab[2 * w] = make_uint2(c, b0);
+        tab[2 * w + 1] = make_uint2(c + __popc(b0), (uint32_t) (e.y >> 32));
+      }
+      cur = seg;
+      __syncthreads();
+    }
+    const uint32_t p0 = A.first[seg] + (item - s_item0[seg]) * PSEG_ITEM;
+    const int np = (int) min((uint32_t) PSEG_ITEM, A.first[seg + 1] - p0);
+    for (;;) {
+      int o = 0;
+      if (lane == 0) o = atomicAdd(&s_next, 1);
+      o = __shfl_sync(0xffffffffu, o, 0);
+      if (o >= np) break;
+      const PairPiece P = A.pieces[p0 + o];
+      const PairOuter O = A.outs[P.o];
+      acc += seg == 0 ? pseg_outer<true>(O, P.lo, P.hi, lane, 32, tab, s_sh, A.primes, n0, base)
+                      : pseg_outer<false>(O, P.lo, P.hi, lane, 32, tab, s_sh, A.primes, n0, base);
+    }
+  }
+  block_sum_i128<PSEG_THREADS>(acc, &A.partial[blockIdx.x]);
 }
 
 // SMALL: every prime of the table is below 2^31 and the PiTable ends below 2^36
+// pieces: the parts of the outers to sum, or nullptr for the outers whole
 template <bool SMALL>
 __global__ void __launch_bounds__(256) k_pairs(const PairOuter* __restrict__ outs, int64_t n_outer,
+                                               const PairPiece* __restrict__ pieces,
                                                const uint32_t* __restrict__ primes,
                                                const uint64_t* __restrict__ magic,
                                                const uint64_t* __restrict__ pibig, i128* __restrict__ partial)
@@ -326,7 +544,15 @@ __global__ void __launch_bounds__(256) k_pairs(const PairOuter* __restrict__ out
   const ulonglong2* __restrict__ pt = (const ulonglong2*) pibig;
   i128 acc = 0;
   for (int64_t o = blockIdx.x; o < n_outer; o += gridDim.x) {
-    const PairOuter O = outs[o];
+    PairOuter O;
+    if (pieces) {
+      const PairPiece P = pieces[o];
+      O = outs[P.o];
+      O.i_lo = P.lo;
+      O.i_hi = P.hi;
+    } else {
+      O = outs[o];
+    }
     long long s;
     if (O.mode == 0) s = outer_terms<0, SMALL, false>(O, primes, magic, pt, s_mask);
     else if (O.mode == 1) s = outer_terms<1, SMALL, false>(O, primes, magic, pt, s_mask);
@@ -340,47 +566,103 @@ __global__ void __launch_bounds__(256) k_pairs(const PairOuter* __restrict__ out
 }
 
 // Launches the sum of the terms of nout outers, its blocks' partial sums in
-// T_PR_PART; returns their number.  Outers are cut into pieces of PAIR_SPLIT
-// terms, one block per piece, when the prime table is long enough for an
-// outer to hold several (at most DIRECT_TERMS terms each: as they are, without
-// the scan and the wait for the number of pieces: 60 us of a small pi(x)).
+// T_PR_PART; returns their number.  While an outer has at most DIRECT_TERMS
+// terms (the whole prime table: x up to about 1e14) the outers go to k_pairs
+// as they are: listing pieces waits for their number, 60 us of a small pi(x).
+// Else PIECE_OUTERS outers at a time, which bounds the lists (about 100 pieces
+// an outer at 1e20).
 #define DIRECT_TERMS 65536
+#define PIECE_OUTERS 131072
 static int launch_pairs(Ctx& c, const PairOuter* outs, int64_t nout, cudaStream_t s, uint64_t* launches)
 {
   if (nout <= 0) return 0;
-  uint64_t np = (uint64_t) nout;
-  if (c.tab.nprimes > DIRECT_TERMS) {
-    DevBuf& pieces = c.tmp[T_PR_PIECES];
-    DevBuf& first = c.tmp[T_PR_FIRST];
-    pieces.alloc((size_t) (nout + 1) * 4);
-    first.alloc((size_t) (nout + 1) * 8);
-    k_pair_pieces<<<(unsigned) ((nout + 256) / 256), 256, 0, s>>>(outs, nout, pieces.as<uint32_t>());
-    PCG_CUDA(cudaGetLastError());
-    exclusive_scan_u32(pieces.as<uint32_t>(), nout + 1, first.as<uint64_t>(), s, &c.tmp[T_PR_SUMS]);
-    PCG_CUDA(cudaMemcpyAsync(&np, first.as<uint64_t>() + nout, 8, cudaMemcpyDeviceToHost, s));
-    PCG_CUDA(cudaStreamSynchronize(s));
-    if (np == 0) return 0;
-    DevBuf& split = c.tmp[T_PR_SPLIT];
-    split.alloc((size_t) np * sizeof(PairOuter));
-    k_pair_split<<<(unsigned) ((nout + 127) / 128), 128, 0, s>>>(outs, nout, first.as<uint64_t>(),
-                                                                 split.as<PairOuter>());
-    PCG_CUDA(cudaGetLastError());
-    outs = split.as<PairOuter>();
-    if (launches) *launches += 5;
-  }
-  const int grid = (int) std::min<uint64_t>(np, (uint64_t) c.num_sms * 8);
+  const Tables& T = c.tab;
+  const int seg_blocks = 2 * c.num_sms, pair_blocks = 8 * c.num_sms;
+  const int64_t nbatch = (nout + PIECE_OUTERS - 1) / PIECE_OUTERS;
   DevBuf& part = c.tmp[T_PR_PART];
-  part.alloc((size_t) grid * 16);
-  const bool small = c.tab.prime_limit < (1ll << 31) && c.tab.pibig_limit + 240 < (1ll << 36);
-  if (small)
-    k_pairs<true><<<grid, 256, 0, s>>>(outs, (int64_t) np, c.tab.primes.as<uint32_t>(), c.tab.pmagic.as<uint64_t>(),
-                                       c.tab.pibig.as<uint64_t>(), part.as<i128>());
-  else
-    k_pairs<false><<<grid, 256, 0, s>>>(outs, (int64_t) np, c.tab.primes.as<uint32_t>(), c.tab.pmagic.as<uint64_t>(),
-                                        c.tab.pibig.as<uint64_t>(), part.as<i128>());
-  PCG_CUDA(cudaGetLastError());
-  if (launches) *launches += 1;
-  return grid;
+  int nparts = 0;
+  auto pairs = [&](const PairOuter* o, int64_t n, const PairPiece* pieces) {
+    const int grid = (int) std::min<int64_t>(n, pair_blocks);
+    if (T.prime_limit < (1ll << 31) && T.pibig_limit + 240 < (1ll << 36))
+      k_pairs<true><<<grid, 256, 0, s>>>(o, n, pieces, T.primes.as<uint32_t>(), T.pmagic.as<uint64_t>(),
+                                         T.pibig.as<uint64_t>(), part.as<i128>() + nparts);
+    else
+      k_pairs<false><<<grid, 256, 0, s>>>(o, n, pieces, T.primes.as<uint32_t>(), T.pmagic.as<uint64_t>(),
+                                          T.pibig.as<uint64_t>(), part.as<i128>() + nparts);
+    PCG_CUDA(cudaGetLastError());
+    if (launches) *launches += 1;
+    nparts += grid;
+  };
+  if (T.nprimes <= DIRECT_TERMS) {
+    part.alloc((size_t) pair_blocks * 16);
+    pairs(outs, nout, nullptr);
+    return nparts;
+  }
+  part.alloc((size_t) nbatch * (seg_blocks + pair_blocks) * 16);
+  const bool segs = T.prime_limit < (1ll << 30) && T.pibig_limit + 240 < (1ll << 36);
+  // counts, cursors, queue (cleared), then first pieces and items per list
+  const int nl = PSEG_COUNT + 2;
+  DevBuf& lists = c.tmp[T_PR_LISTS];
+  DevBuf& pieces = c.tmp[T_PR_PIECES];
+  lists.alloc((size_t) (4 * nl + 4) * 4);
+  uint32_t* const d = lists.as<uint32_t>();
+  for (int64_t o0 = 0; o0 < nout; o0 += PIECE_OUTERS) {
+    PieceArgs a;
+    memset(&a, 0, sizeof(a));
+    a.outs = outs + o0;
+    a.n_outer = std::min<int64_t>(nout - o0, PIECE_OUTERS);
+    a.nseg = segs ? (int) std::min<int64_t>(PSEG_COUNT, T.pibig_limit / PSEG_NUMBERS + 1) : 0;
+    a.prime_limit = T.prime_limit;
+    a.nprimes = T.nprimes;
+    a.pismall = T.pitab.as<uint64_t>();
+    a.count = d;
+    a.cursor = d + nl;
+    a.first = d + 2 * nl + 4;
+    PCG_CUDA(cudaMemsetAsync(d, 0, (size_t) (2 * nl + 4) * 4, s));
+    const unsigned blocks = (unsigned) ((a.n_outer + 127) / 128);
+    k_piece_count<<<blocks, 128, 0, s>>>(a);
+    PCG_CUDA(cudaGetLastError());
+    uint32_t count[PSEG_COUNT + 1], in[2 * nl] = {0};
+    PCG_CUDA(cudaMemcpyAsync(count, d, sizeof(uint32_t) * (size_t) (a.nseg + 1), cudaMemcpyDeviceToHost, s));
+    PCG_CUDA(cudaStreamSynchronize(s));
+    uint64_t total = 0;
+    for (int i = 0; i <= a.nseg; i++) {
+      in[i] = (uint32_t) total;
+      in[nl + i + 1] = in[nl + i] + (count[i] + PSEG_ITEM - 1) / PSEG_ITEM;
+      total += count[i];
+    }
+    if (total >= (1ull << 32)) fail(PCG_ERANGE, "pair sums: too many terms");
+    if (total == 0) continue;
+    const uint32_t nitems = in[nl + a.nseg];
+    PCG_CUDA(cudaMemcpyAsync(d + 2 * nl + 4, in, sizeof(in), cudaMemcpyHostToDevice, s));
+    pieces.alloc((size_t) total * sizeof(PairPiece));
+    a.pieces = pieces.as<PairPiece>();
+    k_piece_fill<<<blocks, 128, 0, s>>>(a);
+    PCG_CUDA(cudaGetLastError());
+    if (launches) *launches += 2;
+    if (nitems > 0) {
+      PsegArgs g;
+      memset(&g, 0, sizeof(g));
+      g.outs = a.outs;
+      g.pieces = a.pieces;
+      g.nseg = a.nseg;
+      g.first = a.first;
+      g.item0 = a.first + nl;
+      g.primes = T.primes.as<uint32_t>();
+      g.pibig = T.pibig.as<ulonglong2>();
+      g.big_words = std::max<int64_t>(T.pibig_limit, 240 * 4) / 240 + 1;
+      g.queue = (int*) (d + 2 * nl);
+      g.partial = part.as<i128>() + nparts;
+      PCG_CUDA(cudaFuncSetAttribute(k_pairs_seg, cudaFuncAttributeMaxDynamicSharedMemorySize, PSEG_ENTRIES * 8));
+      const int grid = (int) std::min<uint32_t>(nitems, (uint32_t) seg_blocks);
+      k_pairs_seg<<<grid, PSEG_THREADS, PSEG_ENTRIES * 8, s>>>(g);
+      PCG_CUDA(cudaGetLastError());
+      if (launches) *launches += 1;
+      nparts += grid;
+    }
+    if (count[a.nseg]) pairs(a.outs, count[a.nseg], a.pieces + in[a.nseg]);
+  }
+  return nparts;
 }
 
 // the sum itself

@@ -118,7 +118,7 @@ enum TmpSlot {
   T_PS_BASE, T_PS_C,                                          // prime sieve (B, small pi)
   T_LK_V, T_LK_R,                                             // PiTable lookups
   T_AC_Q, T_AC_OUTS, T_SIGMA,                                 // A + C outers, Sigma's sums
-  T_PR_PIECES, T_PR_FIRST, T_PR_SPLIT, T_PR_PART, T_PR_SUMS,  // pair sums
+  T_PR_PIECES, T_PR_LISTS, T_PR_PART,                         // pair sums
   T_PHI0_PART, T_PHI_ONE, T_PHI_OUTS,                         // Phi0, phi(x, a)
   T_SW_SEG, T_SW_XP, T_SW_Q, T_SW_ROW, T_SW_JOB,              // sweep: segments, x/p, problems, rows, jobs
   T_COUNT
