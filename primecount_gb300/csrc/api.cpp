@@ -659,21 +659,23 @@ static uint64_t table_bytes_beyond(const Ctx& c, int64_t y, int64_t z, int64_t s
 }
 
 // B's prime sieve over [lo, hi): per-segment sums and the sieving primes
-static uint64_t psieve_bytes(int64_t lo, int64_t hi)
+static uint64_t psieve_bytes(const Ctx& c, int64_t lo, int64_t hi)
 {
   if (hi <= lo) return 0;
   const int64_t seg = 12288ll * 240;                          // shorter ranges: up to 4 segments per SM
-  return (uint64_t) ((hi - lo) / seg + 1024) * 24 + (uint64_t) (isqrt((u128) hi) / 8 + 64) * 12;
+  const uint64_t primes = (uint64_t) (isqrt((u128) hi) / 8 + 64);
+  const uint64_t state = (hi - lo) / seg >= 64 * c.num_sms ? primes * 4 * 2 * (uint64_t) c.num_sms : 0;
+  return (uint64_t) ((hi - lo) / seg + 1024) * 24 + primes * 12 + state;
 }
 
 static uint64_t pi_query_bytes(const Ctx& c, u128 x)
 {
-  if (x <= (u128) 10000000000ull) return psieve_bytes(0, (int64_t) x + 1) + 4096;
+  if (x <= (u128) 10000000000ull) return psieve_bytes(c, 0, (int64_t) x + 1) + 4096;
   const GourdonParams g = gourdon_params(x);
   const int64_t sqrtx = isqrt(x);
   const int64_t cols = pi_estimate(c, g.x_star) + 1;
   uint64_t b = sweep_device_bytes(c.num_sms, (int64_t) (x / (u128) g.z), cols, 8192);
-  b += psieve_bytes(sqrtx, (int64_t) (x / (u128) g.y) + 1);
+  b += psieve_bytes(c, sqrtx, (int64_t) (x / (u128) g.y) + 1);
   b += (uint64_t) pi_estimate(c, iroot(x, 3)) * 4 * 64;      // A + C outer terms
   // their pieces, 12 bytes each, 131072 outers at a time: 5.6e4 at 1e15, 4.6e6
   // at 1e18, 3.2e7 at 1e20, 1.1e8 at 1e21
@@ -695,7 +697,7 @@ static uint64_t phi_query_bytes(const Ctx& c, int64_t x, int64_t a)
   const double la = std::log((double) std::max<int64_t>(a, 3));
   const int64_t pa = (int64_t) ((double) a * (la + std::log(std::max(la, 1.0))));   // above p_a for a >= 6
   if ((u128) pa * pa * pa * pa > (u128) x)                    // P2 + P3
-    return pi_query_bytes(c, (u128) x) + psieve_bytes(sq, x / std::max<int64_t>(pa / 2, 1) + 1) +
+    return pi_query_bytes(c, (u128) x) + psieve_bytes(c, sq, x / std::max<int64_t>(pa / 2, 1) + 1) +
            (uint64_t) pi_estimate(c, iroot((u128) x, 3)) * 64;
   const int64_t y = std::max<int64_t>(pa, std::min<int64_t>(sq - 1, 8 * iroot((u128) x, 3)));
   uint64_t b = sweep_device_bytes(c.num_sms, x / y, a + 1, 8192);

@@ -107,6 +107,18 @@ constexpr WheelPatterns wheel_patterns()
 }
 static __device__ const WheelPatterns g_patterns = wheel_patterns();
 
+// r / m in single precision, rounded down, m given as a float: relative error
+// 2^-24 for m, 2^-23 for its approximate reciprocal, 2^-23 for r, 2^-24 for the
+// product, so for quotients below 2^21 it is off by at most one, below 5e6 by
+// at most two, below 2^23 by at most three
+static __device__ __forceinline__ uint32_t quot_f32(uint64_t r, float m)
+{
+  float inv;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(m));
+  const float rf = __fmaf_rn(__uint2float_rn((uint32_t) (r >> 32)), 4294967296.0f, __uint2float_rn((uint32_t) r));
+  return __float2uint_rz(rf * inv);
+}
+
 // floor(n / q) from m = floor((2^64 - 1) / q), q >= 1: the high product is
 // floor(n / q) or one less
 static __device__ __forceinline__ uint64_t div_magic(uint64_t n, uint64_t q, uint64_t m)

@@ -343,10 +343,7 @@ __device__ __forceinline__ long long pseg_terms(const uint2* __restrict__ tab, c
 {
   auto term = [&](uint32_t q) -> uint32_t {
     const uint64_t r = xp - start * q;
-    float inv;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(__uint2float_rn(q)));
-    const float rf = __fmaf_rn(__uint2float_rn((uint32_t) (r >> 32)), 4294967296.0f, __uint2float_rn((uint32_t) r));
-    uint32_t d = __float2uint_rz(rf * inv);
+    uint32_t d = quot_f32(r, __uint2float_rn(q));
     const int32_t t = (int32_t) ((uint32_t) r - d * q);
     if (t < 0) d--;
     if (t >= (int32_t) q) d++;
@@ -877,7 +874,10 @@ __global__ void k_outer_S2e(uint64_t x_lo, uint64_t x_hi, int64_t y, int64_t z, 
 // one correction step.  Bound by integer issue (the primes' starts and the
 // multiples).  Measured on a GB300: the starts of 32 primes at once and medium
 // primes up to segment / 128 instead of a warp per start and segment / 256:
-// pi(5e9) 1.34 -> 1.20 ms, B of pi(2e19) beside D 84 -> 70 ms.
+// pi(5e9) 1.34 -> 1.20 ms, B of pi(2e19) beside D 84 -> 70 ms; then four medium
+// multiples per round, the next large multiples kept over 16 segments, and the
+// queries' quotients in single precision: pi(5e9) 1.21 -> 1.04 ms, B of pi(1e20)
+// 175 -> 143 ms, all its easy terms 445 -> 414 ms.
 #define PS_NT 512
 #define PS_SMALL PAT_PRIMES
 #define PS_GAPS 0x26424246u       // gaps between consecutive wheel offsets, a nibble each
@@ -892,6 +892,8 @@ struct PsArgs {
   int32_t words;         // 64-bit words per segment (a multiple of 64, at most 16384)
   int32_t nbase;         // primes >= 67 up to sqrt(end)
   int32_t nmid;          // base[0, nmid) crossed off a warp per prime
+  int32_t run;           // consecutive segments per work item
+  uint32_t* state;       // [block][nbase - nmid] next multiples of the large primes, or nullptr (run = 1)
   const uint32_t* base;
   const uint64_t* magic; // floor((2^64 - 1) / base[k])
   const uint64_t* pibig; // PiTable bits for the B queries
@@ -928,12 +930,25 @@ __global__ void __launch_bounds__(PS_NT, 2) k_psieve(const PsArgs A)
 #pragma unroll
   for (int i = 0; i < PS_SMALL; i++) small_mask |= 1ull << bit_of(SP[i]);
   const uint32_t lane_res = 30u * (uint32_t) (lane >> 3) + woff((uint32_t) lane & 7);
+  int64_t s = 0;                                         // segment
+  int left = 0;                                          // segments left in the run
+  bool fresh = true;                                     // first of its run
+  uint32_t* const state = A.state ? A.state + (int64_t) blockIdx.x * (A.nbase - A.nmid) : nullptr;
   for (;;) {
     __syncthreads();
-    if (tid == 0) s_s = atomicAdd(A.queue, 1);
-    __syncthreads();
-    const int64_t s = s_s;
-    if (s >= A.nseg) break;
+    // the next segment of the run, or a new run
+    if (left == 0) {
+      if (tid == 0) s_s = atomicAdd(A.queue, 1);
+      __syncthreads();
+      s = (int64_t) s_s * A.run;
+      if (s >= A.nseg) break;
+      left = (int) dmin(A.run, A.nseg - s);
+      fresh = true;
+    } else {
+      s++;
+      fresh = false;
+    }
+    left--;
     const uint64_t lo = (uint64_t) (A.lo0 + s * A.len);
     const uint64_t hi = (uint64_t) dmin((int64_t) lo + A.len, A.end);
     const uint32_t span = (uint32_t) (hi - lo);
@@ -993,27 +1008,42 @@ __global__ void __launch_bounds__(PS_NT, 2) k_psieve(const PsArgs A)
         uint32_t w = off / 120;
         const uint32_t msk = ~(1u << s_bit[off - 120 * w]);
         if (off >= span) w = nw32;
+        for (; w + 3 * pt < nw32; w += 4 * pt) {
+          atomicAnd(&bits32[w], msk);
+          atomicAnd(&bits32[w + pt], msk);
+          atomicAnd(&bits32[w + 2 * pt], msk);
+          atomicAnd(&bits32[w + 3 * pt], msk);
+        }
         for (; w < nw32; w += pt) atomicAnd(&bits32[w], msk);
       }
     }
-    // large primes: a lane per prime along the 30-wheel
+    // large primes: a lane per prime along the 30-wheel; the next multiple
+    // (offset, wheel index << 29) is kept from one segment of a run to the
+    // next, found anew in its first one and where the prime's square lies
     for (int k = A.nmid + tid; k < A.nbase; k += PS_NT) {
       const uint32_t p = A.base[k];
-      if ((uint64_t) p * p >= hi) break;
-      uint64_t qmin = ceil_div_magic(lo, p, A.magic[k]);
-      if (qmin < p) qmin = p;
-      const uint64_t j = cnt_le(qmin - 1);              // wheel index of the first q >= qmin
-      const uint64_t q = 30 * (j >> 3) + woff((uint32_t) (j & 7));
-      const uint64_t pq = (uint64_t) p * q;
-      if (pq >= hi) continue;
-      uint32_t off = (uint32_t) (pq - lo);
-      uint32_t jj = (uint32_t) (j & 7);
+      const uint64_t pp = (uint64_t) p * p;
+      if (pp >= hi) break;
+      uint32_t off, jj;
+      if (fresh || pp >= lo) {
+        uint64_t qmin = ceil_div_magic(lo, p, A.magic[k]);
+        if (qmin < p) qmin = p;
+        const uint64_t j = cnt_le(qmin - 1);            // wheel index of the first q >= qmin
+        const uint64_t q = 30 * (j >> 3) + woff((uint32_t) (j & 7));
+        off = (uint32_t) dmin((int64_t) ((uint64_t) p * q - lo), 0x1FFFFFFF);
+        jj = (uint32_t) (j & 7);
+      } else {
+        const uint32_t v = state[k - A.nmid];
+        off = v & 0x1FFFFFFFu;
+        jj = v >> 29;
+      }
       while (off < span) {
         const uint32_t w = off / 120;
         atomicAnd(&bits32[w], ~(1u << s_bit[off - 120 * w]));
         off += p * ((PS_GAPS >> (4 * jj)) & 15u);
         jj = (jj + 1) & 7;
       }
+      if (left) state[k - A.nmid] = (off - span) | (jj << 29);
     }
     __syncthreads();
     // chunk prefix (8 words per chunk; up to 4 chunks per thread)
@@ -1059,8 +1089,13 @@ __global__ void __launch_bounds__(PS_NT, 2) k_psieve(const PsArgs A)
             bw &= bw - 1;
             const int64_t p = 240 * w + 30 * (j >> 3) + woff(j & 7);
             if (p <= pa || p > pb) continue;
-            const uint64_t n = (uint64_t) div128(x, (uint64_t) p);
-            const uint32_t off = (uint32_t) (n - lo);
+            // x / p - lo = (x - lo p) / p < len < 2^22: the single-precision
+            // quotient is off by at most two
+            const uint64_t rem = A.x_lo - lo * (uint64_t) p;
+            uint32_t off = quot_f32(rem, __ull2float_rn((uint64_t) p));
+            int64_t t = (int64_t) (rem - (uint64_t) off * (uint64_t) p);
+            while (t < 0) { t += p; off--; }
+            while (t >= p) { t -= p; off++; }
             const uint32_t ww = off / 240, r = off - ww * 240;
             uint32_t v = pref[ww >> 3];
             for (uint32_t i = ww & ~7u; i < ww; i++) v += __popcll(bits[i]);
@@ -1199,6 +1234,16 @@ static PsOut launch_psieve(Ctx& c, u128 x, int64_t lo0, int64_t end, bool b_mode
   int occ = 0;
   PCG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_psieve, PS_NT, smem));
   const int grid = (int) std::min<int64_t>((int64_t) c.num_sms * std::max(occ, 1), o.nseg);
+  // runs of segments once a block has many: the next multiples of 16 in a row
+  // are kept (an offset and its step, below 7 p, fit 29 bits for p < 2^26)
+  const int64_t nlarge = nbase - nmid;
+  a.run = 1;
+  if (nlarge > 0 && o.nseg >= 64ll * grid && limit < (1ll << 26)) {
+    a.run = 16;
+    DevBuf& st = c.tmp[T_PS_STATE];
+    st.alloc((size_t) grid * nlarge * 4);
+    a.state = st.as<uint32_t>();
+  }
   k_psieve<<<grid, PS_NT, smem, s>>>(a);
   PCG_CUDA(cudaGetLastError());
   if (launches) *launches += 1;

@@ -115,7 +115,7 @@ void exclusive_scan_u32(const uint32_t* in, int64_t n, uint64_t* out, cudaStream
 
 // slots of Ctx::tmp
 enum TmpSlot {
-  T_PS_BASE, T_PS_C,                                          // prime sieve (B, small pi)
+  T_PS_BASE, T_PS_C, T_PS_STATE,                              // prime sieve (B, small pi)
   T_LK_V, T_LK_R,                                             // PiTable lookups
   T_AC_Q, T_AC_OUTS, T_SIGMA,                                 // A + C outers, Sigma's sums
   T_PR_PIECES, T_PR_LISTS, T_PR_PART,                         // pair sums

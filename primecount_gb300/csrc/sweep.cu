@@ -469,26 +469,17 @@ __device__ __forceinline__ uint32_t query(const uint64_t* __restrict__ bits, con
 // Offset of the leaf n = floor(xp / m) in the segment [low, ...), xp = x / p
 // given by its low word: r = xp - low m lies in [0, span m), so xp's high
 // word is not needed, and n - low = floor(r / m) < span comes from a
-// single-precision quotient.  Relative error: 2^-24 for m, 2^-23 for its
-// approximate reciprocal, 2^-23 for r, 2^-24 for the product, below 0.75 for
-// span <= 2^21 (LEAF_SPAN), so the quotient is off by at most one and the
-// remainder corrects it.  No reciprocal table: the gather of 8 bytes per leaf
-// was the longest wait of the dense segments.
+// single-precision quotient (quot_f32), off by at most one for span <= 2^21
+// (LEAF_SPAN), which the remainder corrects.  No reciprocal table: the gather
+// of 8 bytes per leaf was the longest wait of the dense segments.
 #define LEAF_SPAN (1u << 21)
-static __device__ __forceinline__ uint32_t leaf_quotient(uint64_t r, uint32_t m)
-{
-  float inv;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(__uint2float_rn(m)));
-  const float rf = __fmaf_rn(__uint2float_rn((uint32_t) (r >> 32)), 4294967296.0f, __uint2float_rn((uint32_t) r));
-  return __float2uint_rz(rf * inv);
-}
 
 // m < 2^30 in a segment of at most LEAF_SPAN numbers: the remainder fits 32
 // signed bits
 static __device__ __forceinline__ uint32_t leaf_narrow(uint64_t xlo, uint64_t low, uint32_t m)
 {
   const uint64_t r = xlo - low * m;
-  uint32_t d = leaf_quotient(r, m);
+  uint32_t d = quot_f32(r, __uint2float_rn(m));
   const int32_t t = (int32_t) ((uint32_t) r - d * m);
   if (t < 0) d--;
   if (t >= (int32_t) m) d++;
@@ -499,7 +490,7 @@ static __device__ __forceinline__ uint32_t leaf_narrow(uint64_t xlo, uint64_t lo
 static __device__ __forceinline__ uint32_t leaf_wide(uint64_t xlo, uint64_t low, uint32_t m)
 {
   const uint64_t r = xlo - low * m;
-  uint32_t d = leaf_quotient(r, m);
+  uint32_t d = quot_f32(r, __uint2float_rn(m));
   int64_t t = (int64_t) (r - (uint64_t) d * m);
   while (t < 0) { t += m; d--; }
   while (t >= (int64_t) m) { t -= m; d++; }

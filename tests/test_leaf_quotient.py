@@ -1,5 +1,5 @@
-"""The single-precision quotient of the leaf offsets (leaf_quotient, leaf_narrow
-and leaf_wide in csrc/sweep.cu), restated in numpy with the reciprocal one unit
+"""The single-precision quotient of the leaf offsets (quot_f32 in
+csrc/dev_common.cuh; leaf_narrow and leaf_wide in csrc/sweep.cu), restated in numpy with the reciprocal one unit
 in the last place off in either direction (its documented error): the quotient
 is off by at most the corrections that follow it, so the offset is exact."""
 import numpy as np
