@@ -1417,7 +1417,7 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
         const int64_t E2 = loff[li + 1] - loff[li];
         if (E2 > 0) {
           if (dirty) { scan_chunks<SW>(ccount, pref, n4, wtmp); dirty = false; wp_ok = false; }
-          const bool by_word = wp_fits && E2 > WORD_RECORDS;
+          const bool by_word = wp_fits && E2 > max(512, 2 * nchu);
           if (by_word && !wp_ok) {
             for (int c = tid; c < nchu; c += NT) {
               const ulonglong2* q = (const ulonglong2*) (bits + 8 * c);
@@ -1483,22 +1483,30 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
               int sum_t = 0;                               // at most 14 counts below 2^23
               if ((lflags & 32) && by_word) {
                 const uint32_t c0 = (uint32_t) (hi0 - f0);
-                for (int j0 = 0; j0 < tot; j0 += 32 * 4) {
+                auto leaf = [&](uint32_t e) -> uint32_t {
+                  const uint32_t mi = c0 - (e & 0x7FFFu);
+                  return leaf_narrow(xlo, (uint64_t) low, 2310u * (mi / 480u) + cop[mi % 480u]);
+                };
+                // four leaves a lane while there are 128, then one
+                int j0 = 0;
+                for (; j0 + 128 <= tot; j0 += 128) {
                   uint32_t e[4], off[4];
 #pragma unroll
-                  for (int d = 0; d < 4; d++) e[d] = wl[min(j0 + 32 * d + lane, tot - 1)];
+                  for (int d = 0; d < 4; d++) e[d] = wl[j0 + 32 * d + lane];
 #pragma unroll
-                  for (int d = 0; d < 4; d++) {
-                    const uint32_t mi = c0 - (e[d] & 0x7FFFu);
-                    off[d] = leaf_narrow(xlo, (uint64_t) low, 2310u * (mi / 480u) + cop[mi % 480u]);
-                  }
+                  for (int d = 0; d < 4; d++) off[d] = leaf(e[d]);
 #pragma unroll
                   for (int d = 0; d < 4; d++) {
                     const int c = count(off[d]);
-                    const bool on = j0 + 32 * d + lane < tot;
-                    sum_t += on ? (e[d] & 0x8000u ? -c : c) : 0;
-                    smu_t += on ? (e[d] & 0x8000u ? -1 : 1) : 0;
+                    sum_t += e[d] & 0x8000u ? -c : c;
+                    smu_t += e[d] & 0x8000u ? -1 : 1;
                   }
+                }
+                for (int j = j0 + lane; j < tot; j += 32) {
+                  const uint32_t e = wl[j];
+                  const int c = count(leaf(e));
+                  sum_t += e & 0x8000u ? -c : c;
+                  smu_t += e & 0x8000u ? -1 : 1;
                 }
               } else {
                 const uint64_t xhi = (lflags & 16) ? PQ.xp_tab[3 * (int64_t) l + 1] : 0ull;
