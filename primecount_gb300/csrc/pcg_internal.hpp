@@ -120,7 +120,7 @@ enum TmpSlot {
   T_AC_Q, T_AC_OUTS, T_SIGMA,                                 // A + C outers, Sigma's sums
   T_PR_PIECES, T_PR_LISTS, T_PR_PART,                         // pair sums
   T_PHI0_PART, T_PHI_ONE, T_PHI_OUTS,                         // Phi0, phi(x, a)
-  T_SW_SEG, T_SW_XP, T_SW_Q, T_SW_ROW, T_SW_JOB,              // sweep: segments, x/p, problems, rows, jobs
+  T_SW_SEG, T_SW_XP, T_SW_Q, T_SW_ROW, T_SW_JOB, T_SW_PLAN,   // sweep: segments, x/p, problems, rows, jobs, plan
   T_COUNT
 };
 // PiTable {count, bits} over [0, limit] without the primes array

@@ -1999,34 +1999,40 @@ static void launch_sweep(const SweepArgs& a, int grid, size_t smem, cudaStream_t
 
 // Segment planner (the role of LoadBalancerS2's growing segment sizes,
 // src/LoadBalancerS2.cpp:195-264, decided up front): an analytic estimate of
-// the leaves of every family per interval (m-range length times the density
-// of square-free numbers without prime factors <= p_b, or the prime density
-// for the p_b * p_l leaves) plus a per-level cost, integrated on a geometric
-// grid; segments are cut at equal estimated cost, never longer than smax.
-// dens[b] = 0.56 / log(p_b) for b in [1, bglob].  The grid cells are costed
-// on nth host threads (1: the calling thread only, no thread is created).
-// Each segment end is passed to push(end) in order, starting with 0; a push
-// returning false stops the plan (the return value is then false).  G grid
-// cells (at most PLAN_GRID).
+// the leaves of every family (m-range length times the density of square-free
+// numbers without prime factors <= p_b, or the prime density for the
+// p_b * p_l leaves) and of the levels, on a geometric grid of cells; segments
+// are cut at equal estimated cost, never longer than smax.
 #define PLAN_GRID 1200
-template <class Push>
-static bool plan_segments_core(const SweepProblem& pb, const Tables& t, int64_t L, int64_t x_star,
-                               int64_t pi_sqrt, int64_t bglob, int64_t smax, int grid, const double* dens,
-                               unsigned nth, Push push, int G = PLAN_GRID)
+struct PlanCells {
+  int G;
+  double g[PLAN_GRID + 1];       // cell i = [g[i], g[i + 1])
+  double leaves[PLAN_GRID];      // leaves in the cell
+  double lev[PLAN_GRID];         // levels of a segment that starts in it
+};
+
+static void plan_grid(PlanCells& P, int64_t L, int G)
+{
+  P.G = std::max(2, std::min(G, PLAN_GRID));
+  const double a0 = 240;
+  const double ratio = std::pow((double) L / a0, 1.0 / (P.G - 1));
+  P.g[0] = 0;
+  for (int i = 0; i < P.G; i++) P.g[i + 1] = std::min((double) L, a0 * std::pow(ratio, i));
+  P.g[P.G] = (double) L;
+}
+
+// The cells' leaves and levels on the calling thread; dens[b] = 0.56 /
+// log(p_b) for b in [1, bglob].
+static void plan_cells(PlanCells& P, const SweepProblem& pb, const Tables& t, int64_t x_star, int64_t pi_sqrt,
+                       int64_t bglob, const double* dens)
 {
   const double x = (double) pb.x;
   const double y = (double) pb.y, z = (double) pb.z;
-  G = std::max(2, std::min(G, PLAN_GRID));
-  double g[PLAN_GRID + 1], cost[PLAN_GRID], cum[PLAN_GRID + 1];
-  g[0] = 0;
-  const double a0 = 240;
-  const double ratio = std::pow((double) L / a0, 1.0 / (G - 1));
-  for (int i = 0; i < G; i++) g[i + 1] = std::min((double) L, a0 * std::pow(ratio, i));
-  g[G] = (double) L;
-  auto leaves = [&](double lo, double hi) {
+  for (int i = 0; i < P.G; i++) {
+    const double lo = P.g[i], hi = P.g[i + 1];
     double sum = 0;
-    double l1 = std::max(lo, 1.0);
-    for (int64_t b = pb.k + 1; b <= bglob; b++) {
+    const double l1 = std::max(lo, 1.0);
+    for (int64_t b = pb.k + 1; hi > lo && b <= bglob; b++) {
       const double p = (double) t.h_primes[(size_t) b], xp = x / p;
       double mlo, mhi;
       if (pb.gourdon == 2) { mlo = std::max({y / p, xp / hi, p}); mhi = std::min(xp / l1, y); }
@@ -2040,84 +2046,132 @@ static bool plan_segments_core(const SweepProblem& pb, const Tables& t, int64_t 
       if (mhi <= mlo) continue;
       sum += (b <= pi_sqrt) ? (mhi - mlo) * dens[b] : (mhi - mlo) / std::log(std::max(mhi, 3.0));
     }
-    return sum;
-  };
-  auto levels = [&](double a) {
-    double lim = pb.gourdon ? std::min((double) x_star, std::sqrt(x / std::max(a, 1.0)))
-                            : std::min(std::sqrt(z), std::sqrt(x / std::max(a, 1.0)));
-    return (double) host_pi(t, (uint64_t) std::min(lim, (double) t.prime_limit));
-  };
-  // a level of a segment costs about as much as this many leaves
-  const double c_level = 100.0;
-  auto cell = [&](unsigned k, unsigned step) {
-    for (int i = (int) k; i < G; i += (int) step) {
-      const double len = g[i + 1] - g[i];
-      cost[i] = len > 0 ? leaves(g[i], g[i + 1]) + c_level * levels(g[i]) * len / (double) smax : 0;
-    }
-  };
-  if (nth <= 1) cell(0, 1);
-  else {
-    std::vector<std::thread> th;
-    for (unsigned k = 0; k < nth; k++) th.emplace_back(cell, k, nth);
-    for (auto& h : th) h.join();
+    P.leaves[i] = sum;
+    const double lim = pb.gourdon ? std::min((double) x_star, std::sqrt(x / std::max(lo, 1.0)))
+                                  : std::min(std::sqrt(z), std::sqrt(x / std::max(lo, 1.0)));
+    P.lev[i] = (double) host_pi(t, (uint64_t) std::min(lim, (double) t.prime_limit));
   }
-  cum[0] = 0;
-  for (int i = 0; i < G; i++) cum[i + 1] = cum[i] + cost[i];
-  const double total = cum[G];
-  // One segment per CTA while that keeps a segment below 10^7 leaves, else as
-  // many per CTA as it takes, equally many for all: every cut repeats the
-  // chain of levels, which is most of the work of a small x.  Six per CTA
-  // instead: D(1e13) 0.84 -> 0.38 ms, D(1e15) 2.65 -> 1.15 ms, D(1e17) 15.1 ->
-  // 11.2 ms; at 1e18 (45.7 ms by two per CTA) one is 48.4 ms, six 48.4 ms; at
-  // 1e20 segments of 6e6, 1.2e7, 2.4e7: 780, 771, 775 ms.  Below 1000 leaves
-  // a segment is all overhead (D(1e11) 0.19 -> 0.15 ms).
+}
+
+// The same on the device, a block per cell, in single precision: a new x waits
+// 40 us for it instead of up to 6 ms on 16 host threads (1e20).
+struct PlanArgs {
+  float x, y, z;
+  int gourdon, k, pi_sqrt, bglob, G;
+  int64_t x_star, prime_limit;
+  const uint32_t* primes;
+  const uint64_t* pitab;
+  double* buf;                   // g[G + 1], then leaves[G], lev[G]
+};
+__global__ void __launch_bounds__(128) k_plan_cells(const PlanArgs A)
+{
+  const int i = (int) blockIdx.x;
+  const float lo = (float) A.buf[i], hi = (float) A.buf[i + 1], l1 = fmaxf(lo, 1.0f);
+  float sum = 0;
+  if (hi > lo)
+    for (int b = A.k + 1 + (int) threadIdx.x; b <= A.bglob; b += 128) {
+      const float p = (float) A.primes[b], xp = A.x / p;
+      const bool one = b <= A.pi_sqrt;
+      float mlo, mhi;
+      if (A.gourdon == 2) { mlo = fmaxf(fmaxf(A.y / p, xp / hi), p); mhi = fminf(xp / l1, A.y); }
+      else if (A.gourdon) {
+        mlo = fmaxf(one ? A.z / p : p, xp / hi);
+        mhi = fminf(fminf(xp / (p * p), one ? A.z : A.y), xp / l1);
+      } else {
+        mlo = fmaxf(one ? A.y / p : p, xp / hi);
+        mhi = fminf(fminf(xp / l1, A.y), one ? A.y : A.z / p);
+      }
+      if (mhi > mlo) sum += (mhi - mlo) * (one ? 0.56f / logf(fmaxf(p, 3.0f)) : 1.0f / logf(fmaxf(mhi, 3.0f)));
+    }
+  __shared__ double w[4];
+  double v = sum;
+  for (int d = 16; d > 0; d >>= 1) v += __shfl_down_sync(0xffffffffu, v, d);
+  if ((threadIdx.x & 31) == 0) w[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    A.buf[A.G + 1 + i] = w[0] + w[1] + w[2] + w[3];
+    const float r = sqrtf(A.x / l1);
+    const float lim = fminf(A.gourdon ? fminf((float) A.x_star, r) : fminf(sqrtf(A.z), r), (float) A.prime_limit);
+    A.buf[2 * A.G + 1 + i] = (double) dpi(A.pitab, (uint64_t) dmin((int64_t) lim, A.prime_limit));
+  }
+}
+
+static void plan_cells_device(Ctx& c, PlanCells& P, const SweepProblem& pb, int64_t x_star, int64_t pi_sqrt,
+                              int64_t bglob, cudaStream_t s)
+{
+  DevBuf& b = c.tmp[T_SW_PLAN];
+  b.alloc((size_t) (3 * P.G + 1) * 8);
+  PlanArgs a;
+  memset(&a, 0, sizeof(a));
+  a.x = (float) pb.x;
+  a.y = (float) pb.y;
+  a.z = (float) pb.z;
+  a.gourdon = pb.gourdon;
+  a.k = (int) pb.k;
+  a.pi_sqrt = (int) pi_sqrt;
+  a.bglob = (int) bglob;
+  a.G = P.G;
+  a.x_star = x_star;
+  a.prime_limit = c.tab.prime_limit;
+  a.primes = c.tab.primes.as<uint32_t>();
+  a.pitab = c.tab.pitab.as<uint64_t>();
+  a.buf = b.as<double>();
+  PCG_CUDA(cudaMemcpyAsync(b.p, P.g, (size_t) (P.G + 1) * 8, cudaMemcpyHostToDevice, s));
+  k_plan_cells<<<(unsigned) P.G, 128, 0, s>>>(a);
+  PCG_CUDA(cudaGetLastError());
+  double out[2 * PLAN_GRID];
+  PCG_CUDA(cudaMemcpyAsync(out, b.as<double>() + P.G + 1, (size_t) (2 * P.G) * 8, cudaMemcpyDeviceToHost, s));
+  PCG_CUDA(cudaStreamSynchronize(s));
+  memcpy(P.leaves, out, (size_t) P.G * 8);
+  memcpy(P.lev, out + P.G, (size_t) P.G * 8);
+}
+
+// Cuts [0, L) for grid CTAs: each segment end is passed to push(end) in order,
+// starting with 0; a push returning false stops the cut (the return value is
+// then false).
+//
+// One segment per CTA while that keeps a segment below 10^7 leaves, else as
+// many per CTA as it takes, equally many for all: every cut repeats the chain
+// of levels, which is most of the work of a small x.  Six per CTA always:
+// D(1e13) 0.84 -> 0.38 ms, D(1e15) 2.65 -> 1.15 ms, D(1e17) 15.1 -> 11.2 ms; at
+// 1e18 (45.7 ms by two per CTA) one is 48.4 ms, six 48.4 ms; at 1e20 segments
+// of 6e6, 1.2e7, 2.4e7: 780, 771, 775 ms.  Below 1000 leaves a segment is all
+// overhead (D(1e11) 0.19 -> 0.15 ms).  The levels of a full segment count as
+// 100 leaves each; in D with fewer full segments than CTAs, where the longest
+// chain of levels is the last to end, as 300 (D(1e13) 0.39 -> 0.28 ms, D(1e14)
+// 0.56 -> 0.52 ms; S2_hard(1e14) 0.81 -> 0.89 ms and D(1e16) 3.04 -> 3.56 ms
+// the other way).
+template <class Push>
+static bool cut_segments(const PlanCells& P, int gourdon, int64_t L, int64_t smax, int grid, Push push)
+{
+  const int G = P.G;
+  const double c_level = gourdon == 1 && L < smax * grid ? 300.0 : 100.0;
+  double rate[PLAN_GRID], total = 0;
+  for (int i = 0; i < G; i++) {
+    const double len = P.g[i + 1] - P.g[i];
+    rate[i] = len > 0 ? P.leaves[i] / len + c_level * P.lev[i] / (double) smax : 0;
+    total += rate[i] * std::max(len, 0.0);
+  }
   const double per_cta = std::max(1.0, std::ceil(total / (grid * 1e7)));
   const double target = std::max(total / (grid * per_cta), 1000.0);
-  // cumulative cost at n (linear inside a grid cell)
-  auto C = [&](double n) {
-    const int i = (int) (std::upper_bound(g, g + G + 1, n) - g);
-    if (i == 0) return 0.0;
-    if (i > G) return total;
-    const double f = (g[i] > g[i - 1]) ? (n - g[i - 1]) / (g[i] - g[i - 1]) : 0;
-    return cum[i - 1] + f * (cum[i] - cum[i - 1]);
-  };
-  // largest n with C(n) <= v (C is piecewise linear and non-decreasing)
-  auto Cinv = [&](double v) {
-    if (v >= total) return (double) L;
-    const int i = (int) (std::upper_bound(cum, cum + G + 1, v) - cum);   // cum[i - 1] <= v < cum[i]
-    const double d = cum[i] - cum[i - 1];
-    const double f = d > 0 ? (v - cum[i - 1]) / d : 0;
-    return g[i - 1] + f * (g[i] - g[i - 1]);
-  };
+  int i = 0;
   int64_t a = 0;
   if (!push(a)) return false;
   while (a < L) {
-    const int64_t lo = a + 240, hi = std::min(a + smax, L);
-    if (hi <= lo) {
-      a = std::min(a + smax, L);
-      if (!push(a)) return false;
-      continue;
+    while (i + 1 < G && P.g[i + 1] <= (double) a) i++;
+    const int64_t most = std::min(a + smax, L);
+    double need = target, pos = (double) a, end = (double) most;
+    for (int j = i; j < G && pos < (double) most; j++) {
+      const double have = rate[j] * (P.g[j + 1] - pos);
+      if (have >= need && rate[j] > 0) { end = pos + need / rate[j]; break; }
+      need -= have;
+      pos = P.g[j + 1];
     }
-    // the largest end (a multiple of 240, or hi) with cost <= target
-    const double n = Cinv(C((double) a) + target);
-    int64_t best = n >= (double) hi ? hi : (int64_t) (n / 240) * 240;
-    best = std::max(lo, std::min(best, hi));
-    a = std::min(best, L);
+    const int64_t e = end >= (double) most ? most : (int64_t) (end / 240) * 240;
+    a = std::min(std::max(e, a + 240), most);
     if (!push(a)) return false;
   }
   return true;
-}
-
-static std::vector<int64_t> plan_segments(const SweepProblem& pb, const Tables& t, int64_t L, int64_t x_star,
-                                          int64_t pi_sqrt, int64_t bglob, int64_t smax, int grid)
-{
-  std::vector<double> dens((size_t) bglob + 1, 0.0);
-  for (int64_t b = 1; b <= bglob; b++) dens[b] = 0.56 / std::log(std::max((double) t.h_primes[(size_t) b], 3.0));
-  std::vector<int64_t> seg;
-  const unsigned nth = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
-  plan_segments_core(pb, t, L, x_star, pi_sqrt, bglob, smax, grid, dens.data(), nth,
-                     [&](int64_t v) { seg.push_back(v); return true; });
-  return seg;
 }
 
 // levels answered together at most (PCG_SWEEP_GROUP overrides; 0: each by itself)
@@ -2308,7 +2362,11 @@ SweepResult run_sweep(Ctx& c, const SweepProblem& pb, const Tuning& tune_in, cud
   const std::vector<int64_t> key = {(int64_t) (uint64_t) x, (int64_t) (uint64_t) (x >> 64), pb.y, pb.z, pb.k,
                                     (int64_t) pb.gourdon, (int64_t) words, (int64_t) grid};
   if (c.plan_key != key) {
-    c.plan = plan_segments(pb, c.tab, L, x_star, pi_sqrt, bglob, (int64_t) words * 240, grid);
+    PlanCells P;
+    plan_grid(P, L, PLAN_GRID);
+    plan_cells_device(c, P, pb, x_star, pi_sqrt, bglob, s);
+    c.plan.clear();
+    cut_segments(P, pb.gourdon, L, (int64_t) words * 240, grid, [&](int64_t v) { c.plan.push_back(v); return true; });
     c.plan_key = key;
   }
   const std::vector<int64_t>& seglo = c.plan;
@@ -2672,8 +2730,10 @@ void run_sweep_batch(Ctx& c, const std::vector<SweepProblem>& pbs, const Tuning&
               : (int) std::max(1.0, std::min((double) grid, std::ceil(2.0 * grid * std::pow((double) x, 0.6) / work_all)));
           // small problems: one cost cell per segment is plenty
           const int G = (int) std::min<int64_t>(PLAN_GRID, std::max<int64_t>(16, 4 * (L / smax + 1)));
-          plan_segments_core(pb, T, L, x_star, pi_sqrt, bglob, smax, spread, dens.data(), 1,
-                             [&](int64_t v) { P.seg.push_back(v); return true; }, G);
+          PlanCells cells;
+          plan_grid(cells, L, G);
+          plan_cells(cells, pb, T, x_star, pi_sqrt, bglob, dens.data());
+          cut_segments(cells, pb.gourdon, L, smax, spread, [&](int64_t v) { P.seg.push_back(v); return true; });
           P.q.x_lo = (uint64_t) x;
           P.q.x_hi = (uint64_t) (x >> 64);
           P.q.y = pb.y;
@@ -3010,12 +3070,14 @@ SweepResult run_sweep_noalloc(Ctx& c, const SweepProblem& pb, cudaStream_t s)
     for (int64_t b = 1; b <= bglob; b++) h_dens[b] = 0.56 / std::log(std::max((double) T.h_primes[(size_t) b], 3.0));
     int64_t n = 0;
     h_nseg = -1;
-    const bool ok = plan_segments_core(pb, T, L, x_star, pi_sqrt, bglob, (int64_t) words * 240, grid, h_dens, 1,
-                                       [&](int64_t v) {
-                                         if (n > PCG_NOALLOC_MAX_SEGS) return false;
-                                         h_seg[n++] = v;
-                                         return true;
-                                       });
+    PlanCells cells;
+    plan_grid(cells, L, PLAN_GRID);
+    plan_cells(cells, pb, T, x_star, pi_sqrt, bglob, h_dens);
+    const bool ok = cut_segments(cells, pb.gourdon, L, (int64_t) words * 240, grid, [&](int64_t v) {
+      if (n > PCG_NOALLOC_MAX_SEGS) return false;
+      h_seg[n++] = v;
+      return true;
+    });
     if (!ok) fail(PCG_ERANGE, "pcg_D_noalloc: too many segments for the fixed segment table");
     h_nseg = n - 1;
     memcpy(h_plan_key, key, sizeof(key));
