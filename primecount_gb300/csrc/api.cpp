@@ -172,6 +172,10 @@ DrParams dr_params(u128 x)
 // ---------------------------------------------------------------- contexts
 Ctx::~Ctx()
 {
+  if (pin.p) {                             // no kernel may still write to it
+    if (stream) cudaStreamSynchronize(stream);
+    if (aux) cudaStreamSynchronize(aux);
+  }
   for (auto& e : ev) if (e) cudaEventDestroy(e);
   for (auto& e : kev) if (e) cudaEventDestroy(e);
   if (aux) cudaStreamDestroy(aux);
@@ -253,10 +257,14 @@ pcg_status guarded_call(const pcg_opts* opts, void (*fn)(Ctx&, cudaStream_t, voi
     cp = ctx_from(opts);
     std::lock_guard<std::recursive_mutex> lk(cp->call_mu);
     cp->last_error.clear();
+    const cudaStream_t s = stream_from(*cp, opts);
     try {
-      fn(*cp, stream_from(*cp, opts), arg);
+      fn(*cp, s, arg);
     } catch (const Failure& e) {
       cp->last_error = e.msg;
+      // what the failed call launched must not write into the next call's results
+      cudaStreamSynchronize(s);
+      if (cp->aux) cudaStreamSynchronize(cp->aux);
       throw;
     }
   });

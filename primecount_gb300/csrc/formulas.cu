@@ -894,12 +894,31 @@ struct PsArgs {
   int32_t nmid;          // base[0, nmid) crossed off a warp per prime
   int32_t run;           // consecutive segments per work item
   uint32_t* state;       // [block][nbase - nmid] next multiples of the large primes, or nullptr (run = 1)
-  const uint32_t* base;
+  const uint32_t* base;  // nullptr: g_ps_small
   const uint64_t* magic; // floor((2^64 - 1) / base[k])
   const uint64_t* pibig; // PiTable bits for the B queries
   int64_t* seg;          // [nseg][3]: primes of the segment, its B queries, the sum of their counts
-  int* queue;
+  int* queue;            // nullptr: a block per segment
 };
+
+// the sieving primes 67..3163 and their reciprocals, for ranges below 1e7 on a
+// context without tables
+#define PS_SMALL_PRIMES 429
+struct SmallPrimes { uint32_t p[PS_SMALL_PRIMES]; uint64_t m[PS_SMALL_PRIMES]; };
+constexpr SmallPrimes small_primes67()
+{
+  SmallPrimes t{};
+  int n = 0;
+  for (uint32_t v = 67; n < PS_SMALL_PRIMES; v += 2) {
+    bool prime = true;
+    for (uint32_t d = 3; d * d <= v; d += 2)
+      if (v % d == 0) { prime = false; break; }
+    if (prime) { t.p[n] = v; t.m[n] = UINT64_MAX / v; n++; }
+  }
+  return t;
+}
+static constexpr SmallPrimes h_ps_small = small_primes67();
+static __device__ const SmallPrimes g_ps_small = small_primes67();
 
 static __device__ __forceinline__ uint64_t ceil_div_magic(uint64_t n, uint32_t p, uint64_t m)
 {
@@ -930,7 +949,9 @@ __global__ void __launch_bounds__(PS_NT, 2) k_psieve(const PsArgs A)
 #pragma unroll
   for (int i = 0; i < PS_SMALL; i++) small_mask |= 1ull << bit_of(SP[i]);
   const uint32_t lane_res = 30u * (uint32_t) (lane >> 3) + woff((uint32_t) lane & 7);
-  int64_t s = 0;                                         // segment
+  int64_t s = -1;                                        // segment
+  const uint32_t* const pbase = A.base ? A.base : g_ps_small.p;
+  const uint64_t* const pmag = A.base ? A.magic : g_ps_small.m;
   int left = 0;                                          // segments left in the run
   bool fresh = true;                                     // first of its run
   uint32_t* const state = A.state ? A.state + (int64_t) blockIdx.x * (A.nbase - A.nmid) : nullptr;
@@ -938,9 +959,13 @@ __global__ void __launch_bounds__(PS_NT, 2) k_psieve(const PsArgs A)
     __syncthreads();
     // the next segment of the run, or a new run
     if (left == 0) {
-      if (tid == 0) s_s = atomicAdd(A.queue, 1);
-      __syncthreads();
-      s = (int64_t) s_s * A.run;
+      if (A.queue) {
+        if (tid == 0) s_s = atomicAdd(A.queue, 1);
+        __syncthreads();
+        s = (int64_t) s_s * A.run;
+      } else {
+        s = s < 0 ? (int64_t) blockIdx.x : A.nseg;
+      }
       if (s >= A.nseg) break;
       left = (int) dmin(A.run, A.nseg - s);
       fresh = true;
@@ -991,9 +1016,9 @@ __global__ void __launch_bounds__(PS_NT, 2) k_psieve(const PsArgs A)
       uint32_t p = 0, qm = 0;
       uint32_t o = 0xFFFFFFFFu;                          // offset of p qmin, or nothing to do
       if (lane < n) {
-        p = A.base[k];
+        p = pbase[k];
         if ((uint64_t) p * p < hi) {
-          uint64_t qmin = ceil_div_magic(lo, p, A.magic[k]);
+          uint64_t qmin = ceil_div_magic(lo, p, pmag[k]);
           if (qmin < p) qmin = p;
           qm = (uint32_t) (qmin % 120);
           const uint64_t pq = (uint64_t) p * qmin;
@@ -1021,12 +1046,12 @@ __global__ void __launch_bounds__(PS_NT, 2) k_psieve(const PsArgs A)
     // (offset, wheel index << 29) is kept from one segment of a run to the
     // next, found anew in its first one and where the prime's square lies
     for (int k = A.nmid + tid; k < A.nbase; k += PS_NT) {
-      const uint32_t p = A.base[k];
+      const uint32_t p = pbase[k];
       const uint64_t pp = (uint64_t) p * p;
       if (pp >= hi) break;
       uint32_t off, jj;
       if (fresh || pp >= lo) {
-        uint64_t qmin = ceil_div_magic(lo, p, A.magic[k]);
+        uint64_t qmin = ceil_div_magic(lo, p, pmag[k]);
         if (qmin < p) qmin = p;
         const uint64_t j = cnt_le(qmin - 1);            // wheel index of the first q >= qmin
         const uint64_t q = 30 * (j >> 3) + woff((uint32_t) (j & 7));
@@ -1139,6 +1164,9 @@ static std::vector<uint32_t> base_primes67(int64_t limit)
 struct PsOut {
   std::vector<int64_t> r;
   int64_t lo0 = 0, nseg = 0;
+  bool pinned = false;           // the kernel writes them to Ctx::pin, else to T_PS_C
+  // after the wait for the launch: the results into r
+  void take(const Ctx& c) { r.assign((const int64_t*) c.pin.p, (const int64_t*) c.pin.p + 3 * nseg); }
 };
 
 // segment words and the warp/lane split of the prime sieve (PCG_PS_WORDS,
@@ -1194,6 +1222,10 @@ static PsOut launch_psieve(Ctx& c, u128 x, int64_t lo0, int64_t end, bool b_mode
   if (resident) {
     nbase = std::max<int64_t>(0, host_pi(c.tab, (uint64_t) limit) - 18);
     nmid = (int) std::max<int64_t>(0, std::min<int64_t>(nbase, host_pi(c.tab, (uint64_t) std::min(limit, std::max<int64_t>(mid_limit, 1)) - 1) - 18));
+  } else if (limit <= (int64_t) h_ps_small.p[PS_SMALL_PRIMES - 1]) {
+    const uint32_t* const p = h_ps_small.p;
+    nbase = std::upper_bound(p, p + PS_SMALL_PRIMES, (uint32_t) limit) - p;
+    nmid = (int) std::min<int64_t>(nbase, std::lower_bound(p, p + PS_SMALL_PRIMES, (uint32_t) mid_limit) - p);
   } else {
     const std::vector<uint32_t> base = base_primes67(limit);
     nbase = (int64_t) base.size();
@@ -1206,8 +1238,23 @@ static PsOut launch_psieve(Ctx& c, u128 x, int64_t lo0, int64_t end, bool b_mode
     d_base.alloc(std::max<size_t>(made.size(), 1) * 8);
     if (nbase) PCG_CUDA(cudaMemcpyAsync(d_base.p, made.data(), made.size() * 8, cudaMemcpyHostToDevice, s));
   }
-  d_seg.alloc((size_t) (3 * o.nseg + 1) * 8);              // results, then the work queue
-  PCG_CUDA(cudaMemsetAsync(d_seg.p, 0, (size_t) (3 * o.nseg + 1) * 8, s));
+  // A block per segment while they fit the chip at once: no queue, and the
+  // results go straight to host memory (a clear and a copy less, 8 us of
+  // pi(1e6)).
+  const size_t smem = (size_t) words * 8 + (size_t) (words / 8) * 4 + PAT_WORDS * 8;
+  // the largest size whatever this call's: threads with other sizes set it too
+  PCG_CUDA(cudaFuncSetAttribute(k_psieve, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                16384 * 8 + 16384 / 8 * 4 + PAT_WORDS * 8));
+  int occ = 1;
+  if (o.nseg > c.num_sms) PCG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_psieve, PS_NT, smem));
+  const int grid = (int) std::min<int64_t>((int64_t) c.num_sms * std::max(occ, 1), o.nseg);
+  o.pinned = o.nseg <= grid && (size_t) (3 * o.nseg) * 8 <= PIN_BYTES;
+  if (o.pinned) {
+    c.pin.alloc();
+  } else {
+    d_seg.alloc((size_t) (3 * o.nseg + 1) * 8);            // results, then the work queue
+    PCG_CUDA(cudaMemsetAsync(d_seg.as<int64_t>() + 3 * o.nseg, 0, 8, s));
+  }
   PsArgs a;
   memset(&a, 0, sizeof(a));
   a.x_lo = (uint64_t) x;
@@ -1222,18 +1269,16 @@ static PsOut launch_psieve(Ctx& c, u128 x, int64_t lo0, int64_t end, bool b_mode
   a.words = words;
   a.nbase = (int) nbase;
   a.nmid = nmid;
-  a.base = resident ? c.tab.primes.as<uint32_t>() + 19 : (const uint32_t*) (d_base.as<uint64_t>() + nbase);
-  a.magic = resident ? c.tab.pmagic.as<uint64_t>() + 19 : d_base.as<uint64_t>();
+  if (resident) {
+    a.base = c.tab.primes.as<uint32_t>() + 19;
+    a.magic = c.tab.pmagic.as<uint64_t>() + 19;
+  } else if (!made.empty()) {
+    a.base = (const uint32_t*) (d_base.as<uint64_t>() + nbase);
+    a.magic = d_base.as<uint64_t>();
+  }
   a.pibig = c.tab.pibig.as<uint64_t>();
-  a.seg = d_seg.as<int64_t>();
-  a.queue = (int*) (d_seg.as<int64_t>() + 3 * o.nseg);
-  const size_t smem = (size_t) words * 8 + (size_t) (words / 8) * 4 + PAT_WORDS * 8;
-  // the largest size whatever this call's: threads with other sizes set it too
-  PCG_CUDA(cudaFuncSetAttribute(k_psieve, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                16384 * 8 + 16384 / 8 * 4 + PAT_WORDS * 8));
-  int occ = 0;
-  PCG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_psieve, PS_NT, smem));
-  const int grid = (int) std::min<int64_t>((int64_t) c.num_sms * std::max(occ, 1), o.nseg);
+  a.seg = o.pinned ? (int64_t*) c.pin.p : d_seg.as<int64_t>();
+  a.queue = o.pinned ? nullptr : (int*) (d_seg.as<int64_t>() + 3 * o.nseg);
   // runs of segments once a block has many: the next multiples of 16 in a row
   // are kept (an offset and its step, below 7 p, fit 29 bits for p < 2^26)
   const int64_t nlarge = nbase - nmid;
@@ -1254,8 +1299,11 @@ static PsOut run_psieve(Ctx& c, u128 x, int64_t lo0, int64_t end, bool b_mode, i
                         cudaStream_t s, uint64_t* launches)
 {
   PsOut o = launch_psieve(c, x, lo0, end, b_mode, qlo, qhi, s, launches);
-  o.r.resize((size_t) (3 * o.nseg));
-  if (o.nseg > 0) {
+  if (o.pinned) {
+    PCG_CUDA(cudaStreamSynchronize(s));
+    o.take(c);
+  } else if (o.nseg > 0) {
+    o.r.resize((size_t) (3 * o.nseg));
     PCG_CUDA(cudaMemcpyAsync(o.r.data(), c.tmp[T_PS_C].p, o.r.size() * 8, cudaMemcpyDeviceToHost, s));
     PCG_CUDA(cudaStreamSynchronize(s));
   }
@@ -1545,11 +1593,12 @@ static PiParts pi_gourdon(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, bo
     std::vector<i128> hac = partials(c.tmp[T_PR_PART], gridp);
     PCG_CUDA(cudaStreamSynchronize(s));
     const double t3 = fnow_ms();
-    ps.r.resize((size_t) (3 * ps.nseg));
-    if (ps.nseg > 0)
+    if (!ps.pinned) ps.r.resize((size_t) (3 * ps.nseg));
+    if (ps.nseg > 0 && !ps.pinned)
       PCG_CUDA(cudaMemcpyAsync(ps.r.data(), c.tmp[T_PS_C].p, ps.r.size() * 8, cudaMemcpyDeviceToHost, s));
     std::vector<i128> h0 = partials(part0, grid0), hs = partials(sbuf, 3 * sblocks + 2);
     PCG_CUDA(cudaStreamSynchronize(s));
+    if (ps.pinned) ps.take(c);
     for (const i128& v : hac) R.ac += v;
     for (const i128& v : h0) R.phi0 += v;
     int64_t found[3];

@@ -71,6 +71,16 @@ struct DevBuf {
   template <class T> T* as() const { return (T*) p; }
 };
 
+// Host memory that kernels write small results to, page-locked: making it takes
+// 0.2 ms, so up to PIN_KEPT of them outlive their contexts for the next ones.
+#define PIN_KEPT 32
+#define PIN_BYTES 32768
+struct PinBuf {
+  void* p = nullptr;
+  ~PinBuf();
+  void alloc();
+};
+
 // Device-resident tables of one context.
 struct Tables {
   // primes (uint32, 1-indexed, primes[0] = 0) and PiTable {count, bits} per 240
@@ -192,6 +202,7 @@ struct Ctx {
   // (no cudaMalloc / cudaFree per call: cudaFree synchronises the device and
   // would serialise the contexts of a worker pool)
   DevBuf tmp[32];
+  PinBuf pin;
   // sweep configurations chosen by pcg_autotune, by decimal exponent of x
   bool tuned[64] = {};
   Tuning tuned_cfg[64];

@@ -1749,6 +1749,41 @@ void DevBuf::free_()
 
 DevBuf::~DevBuf() { free_(); }
 
+static std::mutex g_pin_mu;
+static std::vector<void*>& pin_free()
+{
+  static std::vector<void*>* v = new std::vector<void*>;   // never destroyed: contexts may outlive statics
+  return *v;
+}
+
+void PinBuf::alloc()
+{
+  if (p) return;
+  {
+    std::lock_guard<std::mutex> g(g_pin_mu);
+    if (!pin_free().empty()) {
+      p = pin_free().back();
+      pin_free().pop_back();
+      return;
+    }
+  }
+  const cudaError_t e = cudaHostAlloc(&p, PIN_BYTES, cudaHostAllocMapped | cudaHostAllocPortable);
+  if (e != cudaSuccess) {
+    p = nullptr;
+    cudaGetLastError();
+    fail(PCG_ENOMEM, std::string("cudaHostAlloc failed: ") + cudaGetErrorString(e));
+  }
+}
+
+// the owner waits for its kernels before
+PinBuf::~PinBuf()
+{
+  if (!p) return;
+  std::lock_guard<std::mutex> g(g_pin_mu);
+  if (pin_free().size() < PIN_KEPT) pin_free().push_back(p);
+  else cudaFreeHost(p);
+}
+
 static std::vector<uint32_t> small_primes(int64_t limit)
 {
   std::vector<uint8_t> c((size_t) limit + 1, 0);
