@@ -390,9 +390,8 @@ __device__ __forceinline__ uint64_t div_xp(uint64_t xlo, uint64_t xhi, uint64_t 
 }
 
 // Exclusive prefix of the chunk counts, one value per 4 chunks (32 words), n4
-// of them, by the first SW warps (ccount 16-byte aligned).  scan_part leaves
-// each warp's part relative to its start and the parts' sums in wtmp;
-// scan_chunks, called by the whole block, the whole prefix.
+// of them, by the first SW warps (ccount 16-byte aligned): each warp's part
+// relative to its start, the parts' sums in wtmp, which the reader adds.
 // values per warp
 template <int SW>
 __device__ __forceinline__ int scan_per(int n4) { return 32 * ((n4 + 32 * SW - 1) / (32 * SW)); }
@@ -417,22 +416,6 @@ __device__ __forceinline__ void scan_part(const uint32_t* __restrict__ ccount, u
   }
   if (lane == 31) wtmp[warp] = incl;
   for (int i = i0; i < i1; i++) pref[i] += incl - sum;
-}
-
-template <int SW>
-__device__ __forceinline__ void scan_chunks(const uint32_t* __restrict__ ccount, uint32_t* __restrict__ pref, int n4,
-                                            uint32_t* wtmp)
-{
-  const int warp = threadIdx.x >> 5;
-  if (warp < SW) scan_part<SW>(ccount, pref, n4, wtmp);
-  __syncthreads();
-  if (warp < SW && warp > 0) {
-    const int per = scan_per<SW>(n4);
-    uint32_t base = 0;
-    for (int w = 0; w < warp; w++) base += wtmp[w];
-    for (int i = warp * per + (threadIdx.x & 31); i < min(n4, (warp + 1) * per); i += 32) pref[i] += base;
-  }
-  __syncthreads();
 }
 
 // the count before chunk c: the prefix of its 4 chunks and the chunks before it
@@ -688,7 +671,7 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
   __shared__ int s_ncoll;
   __shared__ int s_stop;
   __shared__ uint32_t s_rem[3];
-  __shared__ uint32_t s_total;
+  __shared__ uint32_t s_prem[18];                      // numbers removed by each of the first levels
   __shared__ uint64_t s_mlow, s_mhigh;                 // floor((2^64 - 1) / d) of low1 and high
   __shared__ long long wt2[32][2];
   __shared__ uint8_t s_gend[LB];                       // [l]: levels of a group that starts at level l, less 1
@@ -772,25 +755,20 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
       bits[w] = v;
     }
     if (tid == 0) {
-      s_total = 0; s_rem[0] = s_rem[1] = s_rem[2] = 0; s_smu = 0; s_stop = 0x7FFFFFFF;
+      s_rem[0] = s_rem[1] = s_rem[2] = 0; s_smu = 0; s_stop = 0x7FFFFFFF;
       s_mlow = UINT64_MAX / (uint64_t) low1;
       s_mhigh = UINT64_MAX / (uint64_t) high;
       s_ncoll = 0;
     }
-    __syncthreads();
-    {
-      uint32_t part = 0;
-      for (int c = tid; c < nch; c += NT) {
-        uint32_t t = 0;
-        for (int i = 0; i < 8; i++) t += __popcll(bits[8 * c + i]);
-        ccount[c] = t;
-        part += t;
-      }
-      part = __reduce_add_sync(0xffffffffu, part);
-      if (lane == 0) atomicAdd(&s_total, part);
+    if (tid < 18) s_prem[tid] = 0;
+    // 64 numbers a word but for the last one
+    const uint32_t cut = 64u - (uint32_t) __popcll(mask_le((span - 1) % 240));
+    for (int c = tid; c < nch; c += NT) {
+      const int full = min(8, wused - 8 * c);
+      ccount[c] = full > 0 ? 64u * full - (8 * c + full == wused ? cut : 0u) : 0u;
     }
+    uint32_t total = 64u * (uint32_t) wused - cut;
     __syncthreads();
-    uint32_t total = s_total;
     bool dirty = true;
     // prefix counts per word of the segment, in the bitmap's unused tail: a
     // query then takes one word instead of the 8 of its chunk
@@ -798,6 +776,20 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
     uint32_t* const wpre = (uint32_t*) (bits + 8 * nchu);
     const bool wp_fits = 12 * nchu <= nch_all * 8;
     bool wp_ok = false;
+    // the scan warps' parts of the prefix start at these counts
+    uint32_t pbase[SW];
+    auto load_pbase = [&] {
+      pbase[0] = 0;
+#pragma unroll
+      for (int i = 1; i < SW; i++) pbase[i] = pbase[i - 1] + wtmp[i - 1];
+    };
+    const uint32_t per = 4 * (uint32_t) scan_per<SW>(n4);   // chunks per scan warp
+    auto part_base = [&](uint32_t ch) {
+      uint32_t v = 0;
+#pragma unroll
+      for (int i = 1; i < SW; i++) v = ch >= i * per ? pbase[i] : v;
+      return v;
+    };
     long long lsum = 0;
     unsigned long long nleaves = 0, ntwo = 0, nentries = 0;
     unsigned alone_n = 0;  // levels answered alone so far (rotates s_rem)
@@ -940,6 +932,54 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
       if (tid < nb && !(lp[tid].flags & 2)) nentries += (unsigned long long) (loff[tid + 1] - loff[tid]);
 
       int li = 0;          // next batch level to finish
+      // ---- the first levels without leaves, up to p = 61: all their wheel
+      // patterns in one pass over the words, the removals counted level by
+      // level (one load and store of a word and one barrier for all of them)
+      if (b0 == 1) {
+        const bool in = lane < nb && lane < 18 && loff[lane + 1] == 0;
+        const int run = __ffs((int) ~__ballot_sync(0xffffffffu, in)) - 1;
+        if (run >= 5) {
+          for (int w = 4 * tid; w - 4 * lane < 8 * nch; w += 4 * NT) {
+            ulonglong2 v0 = make_ulonglong2(0, 0), v1 = v0;
+            const bool on = w < wused;
+            if (on) { v0 = *(const ulonglong2*) (bits + w); v1 = *(const ulonglong2*) (bits + w + 2); }
+            uint32_t all = 0;
+            int po = 0;
+            for (int t = 3; t < run; t++) {              // p = 7, 11, ...
+              const uint32_t p = lm[t].prime, r0 = lm[t].first + (uint32_t) w;
+              uint32_t d = 0;
+              if (on) {
+                // words past the segment's end are zero already
+                const uint32_t r = r0 - p * div_small(r0, p, lm[t].pinv);
+                const uint32_t r1 = r + 1 == p ? 0u : r + 1;
+                const uint32_t r2 = r1 + 1 == p ? 0u : r1 + 1;
+                const uint32_t r3 = r2 + 1 == p ? 0u : r2 + 1;
+                const uint64_t a0 = pat[po + r], a1 = pat[po + r1], a2 = pat[po + r2], a3 = pat[po + r3];
+                d = __popcll(v0.x & ~a0) + __popcll(v0.y & ~a1) + __popcll(v1.x & ~a2) + __popcll(v1.y & ~a3);
+                v0.x &= a0; v0.y &= a1; v1.x &= a2; v1.y &= a3;
+              }
+              all += d;
+              d = __reduce_add_sync(0xffffffffu, d);
+              if (lane == 0 && d) atomicAdd(&s_prem[t], d);
+              po += (int) p;
+            }
+            if (on) { *(ulonglong2*) (bits + w) = v0; *(ulonglong2*) (bits + w + 2) = v1; }
+            // 2 consecutive lanes own the 8 words of one chunk
+            all += __shfl_down_sync(0xffffffffu, all, 1, 2);
+            if ((lane & 1) == 0 && all) ccount[w >> 3] -= all;
+          }
+          __syncthreads();
+          uint32_t gone = lane < run ? s_prem[lane] : 0u, incl = gone;
+          for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d) incl += t;
+          }
+          if (warp == 0 && lane < run) A.cnt[rowbase + 1 + lane] = total - (incl - gone);
+          total -= __shfl_sync(0xffffffffu, incl, 31);
+          dirty = true;
+          li = run;
+        }
+      }
       while (li < nb) {
         // the next level answered alone, from li on
         int ns = nb;
@@ -1296,18 +1336,7 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
             total -= mpre[W];
             // 4. the records
             if (rb > ra) {
-              // the scan warps' parts start at these counts
-              uint32_t pbase[SW];
-              pbase[0] = 0;
-#pragma unroll
-              for (int i = 1; i < SW; i++) pbase[i] = pbase[i - 1] + wtmp[i - 1];
-              const uint32_t per = 4 * (uint32_t) scan_per<SW>(n4);   // chunks per scan warp
-              auto part_base = [&](uint32_t ch) {
-                uint32_t v = 0;
-#pragma unroll
-                for (int i = 1; i < SW; i++) v = ch >= i * per ? pbase[i] : v;
-                return v;
-              };
+              load_pbase();
               if (rb - ra <= LANE_RECORDS || G > LANE_LEVELS) {
                 // A warp takes a run of records, drops the rejected ones and
                 // answers four at a time: eight lanes each for the words of the
@@ -1416,12 +1445,18 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
         if (tid == NT - 1) A.cnt[rowbase + l] = total;   // the last thread: rarely a multiple to cross off
         const int64_t E2 = loff[li + 1] - loff[li];
         if (E2 > 0) {
-          if (dirty) { scan_chunks<SW>(ccount, pref, n4, wtmp); dirty = false; wp_ok = false; }
+          if (dirty) {
+            if (warp < SW) scan_part<SW>(ccount, pref, n4, wtmp);
+            __syncthreads();
+            dirty = false;
+            wp_ok = false;
+          }
+          load_pbase();
           const bool by_word = wp_fits && E2 > max(512, 2 * nchu);
           if (by_word && !wp_ok) {
             for (int c = tid; c < nchu; c += NT) {
               const ulonglong2* q = (const ulonglong2*) (bits + 8 * c);
-              uint32_t run = before_chunk(ccount, pref, (uint32_t) c);
+              uint32_t run = before_chunk(ccount, pref, (uint32_t) c) + part_base((uint32_t) c);
               uint4 o[2];
 #pragma unroll
               for (int i = 0; i < 2; i++) {
@@ -1442,7 +1477,7 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
           int smu_t = 0;
           // the numbers of [low, low + off] left
           auto count = [&](uint32_t off) -> int {
-            if (!by_word) return (int) query(bits, ccount, pref, s_nb, off);
+            if (!by_word) return (int) (query(bits, ccount, pref, s_nb, off) + part_base(off / 1920));
             const uint32_t w = off / 240;
             return (int) (wpre[w] + (uint32_t) __popcll(bits[w] & mask_le_t(s_nb, off - 240 * w)));
           };
