@@ -150,6 +150,16 @@ GourdonParams gourdon_params(u128 x, double user_alpha_y, double user_alpha_z)
   return p;
 }
 
+GourdonParams pi_params(u128 x, double alpha_y, double alpha_z)
+{
+  // z = y, the reference's choice for CPUs, sieves [0, x / z) for longer than
+  // the extra leaves of z = 2 y take: pi(1e17) 15.0 -> 13.5 ms, pi(1e18) 62.2 ->
+  // 56.4 ms, pi(2e19) 394 -> 358 ms; z = 1.5 y and 3 y: 57.1 and 55.8 ms at
+  // 1e18; pi(1e16) 3.99 -> 3.76 ms, but its tables take that much longer.
+  if (alpha_z <= 0 && x >= (u128) 30000000000000000ull) alpha_z = 2.0;
+  return gourdon_params(x, alpha_y, alpha_z);
+}
+
 DrParams dr_params(u128 x)
 {
   double x16 = (double) iroot(x, 6);
@@ -322,7 +332,11 @@ pcg_status pcg_ctx_create(pcg_i128 max_x, uint64_t mem_budget, pcg_ctx** out)
     if (x >= 10) {
       GourdonParams g = gourdon_params(x);
       ensure_prime_tables(*c, std::max<int64_t>(g.y, isqrt(x) / 1 > 0 ? g.y : g.y), c->stream);
-      ensure_factor_d(*c, g.z, g.z, c->stream);
+      // as far as pi(x) reads it where the budget allows
+      const GourdonParams p = pi_params(x, 0, 0);
+      const uint64_t table = 4 * ((uint64_t) wheel2310().to_index((uint64_t) p.z) + 2);   // at most 4 bytes each
+      const bool fits = pcg_ctx_device_bytes(c) + table <= c->mem_budget;
+      ensure_factor_d(*c, g.y, fits ? p.z : g.z, c->stream);
       if (pcg_ctx_device_bytes(c) > c->mem_budget)
         fail(PCG_ENOMEM, "resident tables exceed the memory budget");
     }
@@ -679,7 +693,7 @@ static uint64_t psieve_bytes(const Ctx& c, int64_t lo, int64_t hi)
 static uint64_t pi_query_bytes(const Ctx& c, u128 x)
 {
   if (x <= (u128) 10000000000ull) return psieve_bytes(c, 0, (int64_t) x + 1) + 4096;
-  const GourdonParams g = gourdon_params(x);
+  const GourdonParams g = pi_params(x, 0, 0);
   const int64_t sqrtx = isqrt(x);
   const int64_t cols = pi_estimate(c, g.x_star) + 1;
   uint64_t b = sweep_device_bytes(c.num_sms, (int64_t) (x / (u128) g.z), cols, 8192);

@@ -1442,12 +1442,15 @@ __global__ void __launch_bounds__(256) k_sigma(const SigmaArgs A, const uint32_t
   if (blockIdx.x == 0 && (int) threadIdx.x < A.nlook) found[threadIdx.x] = dpi(pibig, A.look[threadIdx.x]);
 }
 
+// own_params: y and z as pi_params picks them, else the reference's.
 // with_d = false leaves D out (R.d = 0, R.pi without it): the batch form
 // computes the D of all its queries in one batched sweep
-static PiParts pi_gourdon(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, bool with_d = true)
+static PiParts pi_gourdon(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, bool with_d = true,
+                          bool own_params = false)
 {
   PiParts R;
-  GourdonParams g = gourdon_params(x, tune.alpha_y, tune.alpha_z);
+  const GourdonParams g = own_params ? pi_params(x, tune.alpha_y, tune.alpha_z)
+                                     : gourdon_params(x, tune.alpha_y, tune.alpha_z);
   const int64_t y = g.y, z = g.z, k = g.k, x_star = g.x_star;
   if (x > ((u128) y << 62)) fail(PCG_ERANGE, "pi_gourdon(x): x is too large");
   const int64_t sqrtx = isqrt(x);
@@ -1800,7 +1803,7 @@ i128 pi_any(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, pcg_stats* st)
     r = pi_sieve_count(c, (int64_t) x, s, &l);
     z.kernel_launches = l;
   } else {
-    PiParts P = pi_gourdon(c, x, tune, s);
+    PiParts P = pi_gourdon(c, x, tune, s, true, true);
     r = P.pi;
     z = P.dstats;
     z.kernel_launches = P.launches;

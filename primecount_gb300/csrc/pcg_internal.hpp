@@ -57,6 +57,9 @@ GourdonParams gourdon_params(u128 x);    // src/gourdon/pi_gourdon.cpp:44-62
 // the same with alpha_y / alpha_z given (<= 0: default), clamped as the
 // reference clamps --alpha-y / --alpha-z (src/gourdon/pi_gourdon.cpp:44-62)
 GourdonParams gourdon_params(u128 x, double alpha_y, double alpha_z);
+// the parameters pi(x) is computed with: z = 2 y from 3e16 on unless alpha_z is
+// given (the result does not depend on them)
+GourdonParams pi_params(u128 x, double alpha_y, double alpha_z);
 DrParams dr_params(u128 x);              // src/app/main.cpp:435-461
 int64_t x_star_gourdon(u128 x, int64_t y);   // src/util.cpp:362-386
 int64_t get_c(int64_t y);                // src/PhiTiny.hpp:47-50
@@ -91,8 +94,9 @@ struct Tables {
   DevBuf pitab;              // uint64[2 * (prime_limit / 240 + 1)]
   std::vector<uint32_t> h_primes;   // host copy of the primes (small part)
   std::vector<uint64_t> h_pitab;    // host copy of the PiTable
-  // FactorTableD (Gourdon): entries for coprime-to-2310 n <= fd_z, mpf filter fd_y
-  int64_t fd_y = -1, fd_z = -1;
+  // FactorTableD (Gourdon): entries for coprime-to-2310 n <= fd_z, mpf filter
+  // fd_y; of the primes <= fd_y those above fd_cut are zero at the moment
+  int64_t fd_y = -1, fd_z = -1, fd_cut = -1;
   int fd_bytes = 2;          // 2 = uint16_t entries, 4 = uint32_t
   DevBuf factor_d;
   // FactorTable (Deleglise-Rivat): n <= fr_y
@@ -118,6 +122,8 @@ struct Ctx;
 void ensure_prime_tables(Ctx& c, int64_t limit, cudaStream_t s);
 // FactorTableD for (y, z); FactorTable (DR) for y.
 void ensure_factor_d(Ctx& c, int64_t y, int64_t z, cudaStream_t s);
+// whether the resident FactorTableD serves (y, z); if so it does on s from here
+bool factor_d_serves(Ctx& c, int64_t y, int64_t z, cudaStream_t s);
 void ensure_factor_dr(Ctx& c, int64_t y, cudaStream_t s);
 
 // device exclusive scan (uint32 -> uint64), synchronous on s

@@ -2000,11 +2000,57 @@ static void build_factor(Ctx& c, DevBuf& out, int64_t limit, int64_t y, int gour
   }
 }
 
+// entries of the primes primes[i], i in (i0, i1]: v
+template <typename T>
+__global__ void k_factor_primes(T* __restrict__ out, const uint32_t* __restrict__ primes, int64_t i0, int64_t i1, T v,
+                                const int16_t* __restrict__ cindex)
+{
+  const int64_t i = i0 + 1 + (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
+  if (i > i1) return;
+  const uint32_t p = primes[i];
+  out[480 * (int64_t) (p / 2310) + cindex[p % 2310]] = v;
+}
+
+// For z < 13 y the numbers n <= z with a prime factor above y are the primes in
+// (y, z] (every other prime factor is at least 13), so a table of a larger y
+// serves after its primes above y are made zero, and again once they are T_MAX:
+// the tables of all the x of a context differ by the primes between their y.
+bool factor_d_serves(Ctx& c, int64_t y, int64_t z, cudaStream_t s)
+{
+  Tables& t = c.tab;
+  if (t.fd_z < z) return false;
+  int64_t cut = t.fd_cut;
+  if (y >= z && t.fd_y >= z) {
+    if (cut < z) cut = t.fd_y;
+  } else if (t.fd_y == y || (y < t.fd_y && z / 13 < y)) {
+    cut = y;
+  } else {
+    return false;
+  }
+  if (cut == t.fd_cut) return true;
+  const int64_t lo = std::max<int64_t>(11, std::min(cut, t.fd_cut)), hi = std::min(t.fd_z, std::max(cut, t.fd_cut));
+  if (hi > t.prime_limit) return false;
+  const int64_t i0 = host_pi(t, (uint64_t) lo), i1 = host_pi(t, (uint64_t) std::max(lo, hi));
+  if (i1 > i0) {
+    const unsigned blocks = (unsigned) ((i1 - i0 + 255) / 256);
+    const bool on = cut > t.fd_cut;
+    if (t.fd_bytes == 2)
+      k_factor_primes<uint16_t><<<blocks, 256, 0, s>>>(t.factor_d.as<uint16_t>(), t.primes.as<uint32_t>(), i0, i1,
+                                                       (uint16_t) (on ? 0xFFFF : 0), t.cindex.as<int16_t>());
+    else
+      k_factor_primes<uint32_t><<<blocks, 256, 0, s>>>(t.factor_d.as<uint32_t>(), t.primes.as<uint32_t>(), i0, i1,
+                                                       on ? 0xFFFFFFFFu : 0u, t.cindex.as<int16_t>());
+    PCG_CUDA(cudaGetLastError());
+    PCG_CUDA(cudaStreamSynchronize(s));                    // the next call may come on another stream
+  }
+  t.fd_cut = cut;
+  return true;
+}
+
 void ensure_factor_d(Ctx& c, int64_t y, int64_t z, cudaStream_t s)
 {
   Tables& t = c.tab;
-  bool ok = t.fd_z >= z && (t.fd_y == y || (y >= z && t.fd_y >= z));
-  if (ok) return;
+  if (factor_d_serves(c, y, z, s)) return;
   double t0 = now_ms();
   ensure_prime_tables(c, std::max<int64_t>(y, isqrt((u128) z) + 1), s);
   // 16-bit entries whenever possible, as the reference's D() chooses
@@ -2016,7 +2062,7 @@ void ensure_factor_d(Ctx& c, int64_t y, int64_t z, cudaStream_t s)
   if (t.fd_bytes == 2) build_factor<uint16_t>(c, t.factor_d, z, y, 1, s);
   else build_factor<uint32_t>(c, t.factor_d, z, y, 1, s);
   PCG_CUDA(cudaStreamSynchronize(s));
-  t.fd_y = y;
+  t.fd_y = t.fd_cut = y;
   t.fd_z = z;
   t.build_ms += now_ms() - t0;
 }
@@ -3098,7 +3144,7 @@ SweepResult run_sweep_noalloc(Ctx& c, const SweepProblem& pb, cudaStream_t s)
   const Tables& T = c.tab;
   // the tables are inputs: they must already be resident (no building here)
   if (!pb.gourdon) fail(PCG_EINVAL, "pcg_D_noalloc computes D only");
-  if (T.prime_limit < pb.y || !(T.fd_z >= pb.z && (T.fd_y == pb.y || (pb.y >= pb.z && T.fd_y >= pb.z))))
+  if (T.prime_limit < pb.y || !factor_d_serves(c, pb.y, pb.z, s))
     fail(PCG_ERANGE, "pcg_D_noalloc: the context's resident tables do not cover y = " + std::to_string(pb.y) +
                          ", z = " + std::to_string(pb.z) + " (create the context with a larger max_x)");
   const int64_t L = (int64_t) (x / (u128) pb.z);
