@@ -718,14 +718,19 @@ static uint64_t phi_query_bytes(const Ctx& c, int64_t x, int64_t a)
   if (a > pis) return pi_query_bytes(c, (u128) x);
   const double la = std::log((double) std::max<int64_t>(a, 3));
   const int64_t pa = (int64_t) ((double) a * (la + std::log(std::max(la, 1.0))));   // above p_a for a >= 6
-  if ((u128) pa * pa * pa * pa > (u128) x)                    // P2 + P3
-    return pi_query_bytes(c, (u128) x) + psieve_bytes(c, sq, x / std::max<int64_t>(pa / 2, 1) + 1) +
-           (uint64_t) pi_estimate(c, iroot((u128) x, 3)) * 64;
-  const int64_t y = std::max<int64_t>(pa, std::min<int64_t>(sq - 1, 8 * iroot((u128) x, 3)));
-  uint64_t b = sweep_device_bytes(c.num_sms, x / y, a + 1, 8192);
-  b += (uint64_t) (wheel2310().to_index((uint64_t) y) + 1) * 2 + (uint64_t) (y / 240 + 1) * 36;
-  b += (uint64_t) c.num_sms * 8 * 16;                         // the ordinary leaves' partial sums
-  return b + 65536;
+  const int64_t pl = pa / 2;                                  // below p_a: both forms near their line
+  uint64_t b = 0;
+  if (!phi_by_leaves(x, pa, pa))                              // P2 + P3
+    b = pi_query_bytes(c, (u128) x) + psieve_bytes(c, sq, x / std::max<int64_t>(pl, 1) + 1) +
+        (uint64_t) pi_estimate(c, iroot((u128) x, 3)) * 64;
+  if (phi_by_leaves(x, pl, pl)) {
+    const int64_t y = phi_y(x, pl);
+    uint64_t l = sweep_device_bytes(c.num_sms, x / phi_y(x, pa), a + 1, 8192);
+    l += (uint64_t) (wheel2310().to_index((uint64_t) y) + 1) * 2 + (uint64_t) (y / 240 + 1) * 36;
+    l += (uint64_t) c.num_sms * 8 * 16;                       // the ordinary leaves' partial sums
+    b = std::max(b, l + 65536);
+  }
+  return b;
 }
 }  // namespace pcg
 

@@ -1850,11 +1850,36 @@ void pi_gourdon_terms(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, i128 o
 // (reference semantics and shortcuts: src/phi.cpp:341-430).
 //   a <= 8:               the primorial identity (phi_tiny)
 //   a > pi(sqrt(x)):      pi(x) - a + 1 (1 once a >= pi(x))       (phi_pix)
-//   p_{a+1}^4 > x:        1 + (pi(x) - a) + P2(x, a) + P3(x, a), the
-//                         counts of n <= x with 2 and 3 prime factors > p_a
-//   otherwise:            ordinary leaves n <= y plus the special leaves
-//                         x / (p_b m), m <= y < p_b m, of the Legendre
+//   phi_by_leaves(x, p_a, p_{a+1}):  ordinary leaves n <= y plus the special
+//                         leaves x / (p_b m), m <= y < p_b m, of the Legendre
 //                         recursion, the latter by the sweep (mode phi)
+//   otherwise (p_{a+1}^4 > x):  1 + (pi(x) - a) + P2(x, a) + P3(x, a), the
+//                         counts of n <= x with 2 and 3 prime factors > p_a
+bool phi_by_leaves(int64_t x, int64_t pa, int64_t pa1)
+{
+  if ((u128) pa1 * pa1 * pa1 * pa1 <= (u128) x) return true;
+  // P2 sieves as far as x / p_a, the leaves take a level per prime: 169 and 5.3 ms
+  // at x = 1e16, p_a = 2.1 x^(1/4); equal at p_a = 3e4 (1e14), 5.5e4 (1e15), 1.5e5
+  // (1e16); 0.88 and 0.43 ms at 1e13, 1e4.  A level's bound 2 b + 1 has to stay
+  // below the entries of primes in 16 bits: p_b < 386093.
+  return pa < 380000 && (double) pa <= 50000.0 * std::pow((double) x / 1e15, 0.35);
+}
+
+// y of the ordinary and special leaves: a larger y shortens the sieve of
+// [0, x / y) and adds leaves, the more of them the larger p_a.  Against
+// 8 x^(1/3) for every a: 10.7 -> 1.5 ms at x = 1e16, p_a = x^(1/4) / 8, 5.4 -> 3.7
+// at x^(1/4); 20.0 -> 12.6 at 1e17; within 10 % of the best of 1.5, 2.5, 4 and 6.5
+// in place of 4 for x of 1e9 .. 1e17.  From 1e17 on less: 117 ms with a factor
+// of 24 at 1e18, 164 with 64 (p_a = 4 x^(1/4)).
+int64_t phi_y(int64_t x, int64_t pa)
+{
+  const double xd = (double) x, cbrt = (double) iroot((u128) x, 3);
+  const double f = std::min(20.0, 4.0 * std::pow(xd / 1e14, 0.301)) *
+                   std::sqrt(std::pow(xd, 0.25) / (double) std::max<int64_t>(pa, 1));
+  const int64_t y = (int64_t) (cbrt * std::min(32.0, std::max(1.0, f)));
+  return std::max<int64_t>(pa, std::min<int64_t>(isqrt((u128) x) - 1, y));
+}
+
 __global__ void k_phi_one(uint64_t x, PhiTab T, i128* out) { *out = dphi_tiny((u128) x, T); }
 
 // P3 outers: i in (a, pi(x^(1/3))], j in [i, pi(sqrt(x / p_i))]
@@ -1905,7 +1930,7 @@ int64_t phi_any(Ctx& c, int64_t x, int64_t a, const Tuning& tune, cudaStream_t s
   if (a + 1 > c.tab.nprimes) fail(PCG_EINTERNAL, "phi: prime table too small");
   const int64_t pa = c.tab.h_primes[(size_t) a];
   const int64_t pa1 = c.tab.h_primes[(size_t) a + 1];
-  if ((u128) pa1 * pa1 * pa1 * pa1 > (u128) x) {
+  if (!phi_by_leaves(x, pa, pa1)) {
     // 1 + (pi(x) - a) + P2 + P3
     const int64_t pix = (int64_t) pi_any(c, (u128) x, tune, s, nullptr);
     ensure_pibig(c, sq + 240, s);
@@ -1938,8 +1963,7 @@ int64_t phi_any(Ctx& c, int64_t x, int64_t a, const Tuning& tune, cudaStream_t s
   }
   // ordinary + special leaves with m <= y
   const int64_t cc = 8;
-  int64_t y = std::max<int64_t>(pa, std::min<int64_t>(sq - 1, 8 * iroot((u128) x, 3)));
-  y = std::max<int64_t>(y, pa);
+  const int64_t y = phi_y(x, pa);
   ensure_prime_tables(c, y, s);
   ensure_factor_d(c, pa, y, s);
   ensure_phi_tiny(c, (int) cc, s);

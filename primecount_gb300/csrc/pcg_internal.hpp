@@ -62,6 +62,9 @@ GourdonParams gourdon_params(u128 x, double alpha_y, double alpha_z);
 GourdonParams pi_params(u128 x, double alpha_y, double alpha_z);
 DrParams dr_params(u128 x);              // src/app/main.cpp:435-461
 int64_t x_star_gourdon(u128 x, int64_t y);   // src/util.cpp:362-386
+// phi(x, a): whether by ordinary and special leaves, and their y
+bool phi_by_leaves(int64_t x, int64_t pa, int64_t pa1);
+int64_t phi_y(int64_t x, int64_t pa);
 int64_t get_c(int64_t y);                // src/PhiTiny.hpp:47-50
 
 // ---------------------------------------------------------------- device buffers
