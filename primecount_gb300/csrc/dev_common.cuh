@@ -14,6 +14,7 @@ namespace pcg {
 #define PCG_CNT8_HI 0x0087777776666554ull
 // wheel offsets packed as bytes
 #define PCG_WOFF 0x1D1713110D0B0701ull
+#define WHEEL_GAPS 0x26424246u    // gaps between consecutive wheel offsets, a nibble each
 
 static __device__ __forceinline__ uint32_t cnt8(uint32_t t)
 {

@@ -70,18 +70,37 @@ static i128 sum_partials(const DevBuf& buf, int n, cudaStream_t s)
 // phi(v, k) = (v / P) * phi(P) + phi(v mod P, k), P = p_1 ... p_k
 // (the identity of the reference's PhiTiny, src/PhiTiny.hpp:2-12); phi(r, k)
 // for r < P from a bitmap of the numbers coprime to p_1..p_k.
+// 64 remainders by 8 primes per word took 65 us; the words of a prime's multiples
+// repeat with the word's start mod p: 4 us.
+struct PhiMasks { uint64_t w[77]; };                     // 2 + 3 + 5 + ... + 19
+constexpr PhiMasks phi_masks()
+{
+  constexpr uint32_t pr[8] = {2, 3, 5, 7, 11, 13, 17, 19};
+  PhiMasks t{};
+  int at = 0;
+  for (int i = 0; i < 8; i++)
+    for (uint32_t r = 0; r < pr[i]; r++) {
+      uint64_t v = 0;
+      for (uint32_t j = 0; j < 64; j++)
+        if ((r + j) % pr[i]) v |= 1ull << j;
+      t.w[at++] = v;
+    }
+  return t;
+}
+static __device__ const PhiMasks g_phi_masks = phi_masks();
+
 __global__ void k_phi_bits(uint64_t* __restrict__ bits, uint32_t* __restrict__ pc, int64_t nwords, uint64_t P, int k)
 {
-  int64_t w = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
+  constexpr uint32_t pr[8] = {2, 3, 5, 7, 11, 13, 17, 19};
+  const int64_t w = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
   if (w >= nwords) return;
-  const uint32_t pr[8] = {2, 3, 5, 7, 11, 13, 17, 19};
-  uint64_t v = 0;
-  for (int j = 0; j < 64; j++) {
-    uint64_t t = 64 * (uint64_t) w + j;
-    if (t >= P) break;
-    bool ok = true;
-    for (int i = 0; i < k; i++) ok = ok && (t % pr[i] != 0);
-    if (ok) v |= 1ull << j;
+  const uint32_t t0 = 64 * (uint32_t) w;                 // < 9699690
+  uint64_t v = P - t0 >= 64 ? ~0ull : (1ull << (P - t0)) - 1;
+  uint32_t at = 0;
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    if (i < k) v &= g_phi_masks.w[at + t0 % pr[i]];
+    at += pr[i];
   }
   bits[w] = v;
   pc[w] = __popcll(v);
@@ -880,7 +899,6 @@ __global__ void k_outer_S2e(uint64_t x_lo, uint64_t x_hi, int64_t y, int64_t z, 
 // 175 -> 143 ms, all its easy terms 445 -> 414 ms.
 #define PS_NT 512
 #define PS_SMALL PAT_PRIMES
-#define PS_GAPS 0x26424246u       // gaps between consecutive wheel offsets, a nibble each
 struct PsArgs {
   uint64_t x_lo, x_hi;
   int64_t lo0;           // first segment start (multiple of 240)
@@ -1065,7 +1083,7 @@ __global__ void __launch_bounds__(PS_NT, 2) k_psieve(const PsArgs A)
       while (off < span) {
         const uint32_t w = off / 120;
         atomicAnd(&bits32[w], ~(1u << s_bit[off - 120 * w]));
-        off += p * ((PS_GAPS >> (4 * jj)) & 15u);
+        off += p * ((WHEEL_GAPS >> (4 * jj)) & 15u);
         jj = (jj + 1) & 7;
       }
       if (left) state[k - A.nmid] = (off - span) | (jj << 29);
@@ -1370,7 +1388,7 @@ struct PiParts {
 static void ensure_pibig(Ctx& c, int64_t limit, cudaStream_t s)
 {
   if (c.tab.pibig_limit >= limit) return;
-  build_pitab_only(c.tab.pibig, limit, s);
+  build_pitab_only(c, c.tab.pibig, limit, s);
   c.tab.pibig_limit = limit;
 }
 

@@ -143,7 +143,7 @@ enum TmpSlot {
   T_COUNT
 };
 // PiTable {count, bits} over [0, limit] without the primes array
-void build_pitab_only(DevBuf& out, int64_t limit, cudaStream_t s);
+void build_pitab_only(Ctx& c, DevBuf& out, int64_t limit, cudaStream_t s);
 
 // host PiTable lookup on the host copy
 int64_t host_pi(const Tables& t, uint64_t x);

@@ -46,46 +46,103 @@
 namespace pcg {
 
 // ================================================================ prime tables
-// PiTable bits: word w holds the primes >= 7 among 240w + {1,7,...}
-__global__ void k_prime_bits(uint64_t* __restrict__ out_bits, uint32_t* __restrict__ out_pc,
-                             int64_t nwords, int64_t limit,
-                             const uint32_t* __restrict__ base, int nbase)
+// PiTable bits: word w holds the primes >= 7 among 240w + {1,7,...}; base are
+// the primes from 7 on.  Bound by shared atomics and, in tables of few blocks, by
+// the latency of one: words by range so that each SM has a block, patterns of
+// 7..61 in the fill, then a warp per prime below the number of words (a residue
+// class of the co-factor mod 120 per lane: one addition a multiple) and a lane per
+// larger prime.  Blocks of 2048 words whatever the range and a 64-bit
+// multiplication per multiple took 162 us for [0, 240000], 371 us for [0, 3e7];
+// now 8 and 15 us, 42 us for [0, 1e8], 187 us for [0, 1e9].
+#define PB_NT 256
+__global__ void __launch_bounds__(PB_NT) k_prime_bits(uint64_t* __restrict__ out_bits, uint32_t* __restrict__ out_pc,
+                                                      int64_t nwords, int64_t limit, int words,
+                                                      const uint32_t* __restrict__ base, int nbase)
 {
+  constexpr uint32_t SP[PAT_PRIMES] = {7, 11, 13, 17, 19, 23, 29, 31, 37, 41, 43, 47, 53, 59, 61};
   extern __shared__ uint64_t sb[];
-  const int WB = 2048;
-  int64_t w0 = (int64_t) blockIdx.x * WB;
-  int64_t wn = dmin(WB, nwords - w0);
-  uint64_t lo = (uint64_t) w0 * 240;
-  uint64_t hi = lo + (uint64_t) wn * 240;   // [lo, hi)
-  for (int i = threadIdx.x; i < wn; i += blockDim.x) {
-    uint64_t v = ~0ull;
-    uint64_t wl = lo + (uint64_t) i * 240;
-    if (wl + 239 > (uint64_t) limit) v = ((uint64_t) limit >= wl) ? mask_le((uint32_t) (limit - wl)) : 0;
-    if (w0 + i == 0) v &= ~1ull;            // 1 is not prime
+  uint32_t* const sb32 = (uint32_t*) sb;                 // 120 numbers each
+  __shared__ uint64_t pat[PAT_WORDS];
+  __shared__ uint8_t s_bit[120];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int i = tid; i < PAT_WORDS; i += PB_NT) pat[i] = g_patterns.w[i];
+  for (int i = tid; i < 120; i += PB_NT) s_bit[i] = (uint8_t) bit_of((uint32_t) i);
+  const int64_t w0 = (int64_t) blockIdx.x * words;
+  const int wn = (int) dmin(words, nwords - w0);
+  const uint64_t lo = (uint64_t) w0 * 240, hi = lo + (uint64_t) wn * 240;   // [lo, hi)
+  const uint32_t span = 240u * (uint32_t) wn, nw32 = 2u * (uint32_t) wn;
+  uint32_t ph[PAT_PRIMES];                               // pattern phases of the first word
+#pragma unroll
+  for (int k = 0; k < PAT_PRIMES; k++) ph[k] = (uint32_t) ((uint64_t) w0 % SP[k]);
+  __syncthreads();
+  for (int i = tid; i < wn; i += PB_NT) {
+    const uint64_t wl = lo + (uint64_t) i * 240;
+    uint64_t v = ~0ull, small = 0;
+    uint32_t po = 0;
+#pragma unroll
+    for (int k = 0; k < PAT_PRIMES; k++) {
+      v &= pat[po + (ph[k] + (uint32_t) i) % SP[k]];
+      po += SP[k];
+      small |= 1ull << bit_of(SP[k]);
+    }
+    if (wl == 0) v = (v | small) & ~1ull;                // 7..61 are prime, 1 is not
+    if (wl + 239 > (uint64_t) limit) v &= ((uint64_t) limit >= wl) ? mask_le((uint32_t) (limit - wl)) : 0;
     sb[i] = v;
   }
   __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int k = warp; k < nbase; k += nw) {
-    uint64_t p = base[k];
-    if (p * p >= hi) break;
-    uint64_t qlo = (lo + p - 1) / p;
-    if (qlo < p) qlo = p;
-    uint64_t qhi = (hi - 1) / p;
-    if (qlo > qhi) continue;
-    uint64_t jlo = cnt_le(qlo - 1), jhi = cnt_le(qhi);
-    for (uint64_t j = jlo + lane; j < jhi; j += 32) {
-      uint64_t q = 30 * (j >> 3) + woff((uint32_t) (j & 7));
-      uint32_t off = (uint32_t) (p * q - lo);
-      uint32_t w = off / 240, r = off - w * 240;
-      atomicAnd((unsigned long long*) &sb[w], ~(1ull << bit_of(r)));
+  const uint32_t bound = (uint32_t) words;
+  const uint32_t lane_res = 30u * (uint32_t) (lane >> 3) + woff((uint32_t) lane & 7);
+  // primes below bound: lane l finds the first co-factor of the l-th
+  for (int k0 = PAT_PRIMES + warp; k0 < nbase && base[k0] < bound; k0 += PB_NT) {
+    const int k = k0 + lane * (PB_NT / 32);
+    const uint32_t p = k < nbase ? base[k] : bound;
+    uint32_t qm = 0, o = 0xFFFFFFFFu;                    // offset of p qmin, or nothing to do
+    if (p < bound && p * p < hi) {
+      const uint64_t qmin = (uint64_t) dmax(p, (int64_t) ((lo + p - 1) / p));
+      qm = (uint32_t) (qmin % 120);
+      if (p * qmin < hi) o = (uint32_t) (p * qmin - lo);
+    }
+    for (int t = 0; t < 32; t++) {
+      const uint32_t ot = __shfl_sync(0xffffffffu, o, t);
+      if (ot == 0xFFFFFFFFu) continue;
+      const uint32_t pt = __shfl_sync(0xffffffffu, p, t), qt = __shfl_sync(0xffffffffu, qm, t);
+      const uint32_t off = ot + pt * (lane_res >= qt ? lane_res - qt : lane_res + 120 - qt);
+      const uint32_t w = off / 120;
+      const uint32_t msk = ~(1u << s_bit[off - 120 * w]);
+      for (uint32_t v = w; v < nw32; v += pt) atomicAnd(&sb32[v], msk);
+    }
+  }
+  // the others along the wheel
+  for (int k = PAT_PRIMES + tid; k < nbase; k += PB_NT) {
+    const uint32_t p = base[k];
+    if (p < bound) continue;
+    if ((uint64_t) p * p >= hi) break;
+    const uint64_t qmin = (uint64_t) dmax(p, (int64_t) ((lo + p - 1) / p));
+    const uint64_t j = cnt_le(qmin - 1);                 // wheel index of the first q >= qmin
+    const uint64_t first = p * (30 * (j >> 3) + woff((uint32_t) (j & 7)));
+    uint32_t jj = (uint32_t) (j & 7);
+    for (uint64_t off = first - lo; off < span;) {
+      const uint32_t w = (uint32_t) off / 120;
+      atomicAnd(&sb32[w], ~(1u << s_bit[(uint32_t) off - 120 * w]));
+      off += p * ((WHEEL_GAPS >> (4 * jj)) & 15u);
+      jj = (jj + 1) & 7;
     }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < wn; i += blockDim.x) {
+  for (int i = tid; i < wn; i += PB_NT) {
     out_bits[w0 + i] = sb[i];
     out_pc[w0 + i] = __popcll(sb[i]);
   }
+}
+
+// the bits and their counts over [0, limit] from the primes of base
+static void prime_bits(DevBuf& bits, DevBuf& pc, int64_t nwords, int64_t limit, const DevBuf& base, size_t nbase,
+                       int num_sms, cudaStream_t s)
+{
+  const int words = (int) std::min<int64_t>(2048, std::max<int64_t>(128, (nwords + num_sms - 1) / num_sms));
+  k_prime_bits<<<(unsigned) ((nwords + words - 1) / words), PB_NT, (size_t) words * 8, s>>>(
+      bits.as<uint64_t>(), pc.as<uint32_t>(), nwords, limit, words, base.as<uint32_t>(), (int) nbase);
+  PCG_CUDA(cudaGetLastError());
 }
 
 // ---- exclusive scan uint32 -> uint64 (three phases)
@@ -206,59 +263,90 @@ __global__ void k_pitab_primes(const uint64_t* __restrict__ bits, const uint64_t
 // multiples p*q (q coprime to 2310) with shared-memory atomics: minimum
 // prime index, product of distinct small primes, factor count and a square
 // flag; the cofactor n / product is then the one prime factor > sqrt(limit).
-#define FT_E 4096
+// A block is 8 turns of the 2310 wheel, so that offsets fit 32 bits; a warp per
+// prime with more than 32 multiples in it, a lane per larger prime (a warp for
+// each of those, with 64-bit remainders per multiple: 41 ms for z = 4.9e8, most
+// of it finding starts).  Now 2.3 ms; 6.4e7: 2.43 -> 0.23 ms.
+#define FT_TURNS 8
+#define FT_E (FT_TURNS * 480)
+#define FT_WARP 120                    // a warp per prime below this
 template <typename T>
-__global__ void k_factor(T* __restrict__ out, int64_t size, int64_t limit, int64_t y, int gourdon,
-                         const uint32_t* __restrict__ primes, int64_t nsmall,
-                         const uint16_t* __restrict__ g_coprime, const int16_t* __restrict__ g_cindex)
+__global__ void __launch_bounds__(512) k_factor(T* __restrict__ out, int64_t size, int64_t limit, int64_t y, int gourdon,
+                                                const uint32_t* __restrict__ primes, int64_t nsmall,
+                                                const uint16_t* __restrict__ g_coprime,
+                                                const int16_t* __restrict__ g_cindex)
 {
   extern __shared__ __align__(16) unsigned char fsm[];
   unsigned long long* prod = (unsigned long long*) fsm;
   uint32_t* lpfi = (uint32_t*) (prod + FT_E);
-  uint32_t* nf = lpfi + FT_E;          // bits 0..7 count, bit 30 square, bits 8..29 max prime index
+  uint32_t* nf = lpfi + FT_E;          // bits 0..7 count, bit 30 square
   uint16_t* cop = (uint16_t*) (nf + FT_E);
   int16_t* cid = (int16_t*) (cop + 480);
   for (int i = threadIdx.x; i < 480; i += blockDim.x) cop[i] = g_coprime[i];
   for (int i = threadIdx.x; i < 2310; i += blockDim.x) cid[i] = g_cindex[i];
-  int64_t i0 = (int64_t) blockIdx.x * FT_E;
-  int64_t en = dmin(FT_E, size - i0);
+  const int64_t i0 = (int64_t) blockIdx.x * FT_E;
+  const int en = (int) dmin(FT_E, size - i0);
   for (int i = threadIdx.x; i < FT_E; i += blockDim.x) { prod[i] = 1; lpfi[i] = 0xFFFFFFFFu; nf[i] = 0; }
   __syncthreads();
-  auto to_number = [&](uint64_t i) -> uint64_t { return 2310 * (i / 480) + cop[i % 480]; };
-  auto to_index = [&](uint64_t n) -> int64_t { return 480 * (int64_t) (n / 2310) + cid[n % 2310]; };
-  uint64_t nlo = to_number((uint64_t) i0), nhi = to_number((uint64_t) (i0 + en - 1));
+  const uint64_t nlo = 2310ull * FT_TURNS * blockIdx.x;
+  auto offset = [&](uint32_t i) -> uint32_t { return 2310 * (i / 480) + cop[i % 480]; };
+  const int64_t last = (int64_t) offset((uint32_t) en - 1);
+  // the first multiple of p in the block: q = qb + offset(r), p qb = nlo + at; qm = qb % p
+  auto start = [&](uint32_t p, uint64_t& qb, uint32_t& r, uint32_t& qm, int64_t& at) {
+    const uint64_t qlo = nlo >> 32 ? (nlo + p - 1) / p : ((uint32_t) nlo ? ((uint32_t) nlo - 1) / p + 1 : 0);
+    const uint64_t v = qlo ? qlo - 1 : 0;                // the co-factors above v
+    qb = v >> 32 ? v / 2310 : (uint32_t) v / 2310;
+    r = (uint32_t) (cid[v - 2310 * qb] + 1);             // 480: the next turn's first
+    qb *= 2310;
+    qm = qb >> 32 ? (uint32_t) (qb % p) : (uint32_t) qb % p;
+    at = (int64_t) (p * qb) - (int64_t) nlo;
+  };
+  auto mark = [&](uint32_t k, uint32_t p, uint32_t off, bool sq) {
+    const uint32_t li = 480 * (off / 2310) + (uint32_t) cid[off % 2310];
+    atomicMin(&lpfi[li], k);
+    atomicAdd(&nf[li], 1u);
+    if (sq) atomicOr(&nf[li], 1u << 30);
+    unsigned long long old = prod[li], assumed;
+    do {
+      assumed = old;
+      old = atomicCAS(&prod[li], assumed, assumed * p);
+    } while (old != assumed);
+  };
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   // small primes: index 6 (p = 13) .. nsmall
-  for (int64_t k = 6 + warp; k <= nsmall; k += nw) {
-    uint64_t p = primes[k];
-    uint64_t qlo = (nlo + p - 1) / p;
-    uint64_t qhi = nhi / p;
-    if (qlo > qhi) continue;
-    int64_t jlo = (qlo <= 1) ? 0 : to_index(qlo - 1) + 1;
-    int64_t jhi = to_index(qhi);
-    for (int64_t j = jlo + lane; j <= jhi; j += 32) {
-      uint64_t q = to_number((uint64_t) j);
-      uint64_t n = p * q;
-      int64_t li = to_index(n) - i0;
-      atomicMin(&lpfi[li], (uint32_t) k);
-      atomicAdd(&nf[li], 1u);
-      if (q % p == 0) atomicOr(&nf[li], 1u << 30);
-      unsigned long long old = prod[li], assumed;
-      do {
-        assumed = old;
-        old = atomicCAS(&prod[li], assumed, assumed * p);
-      } while (old != assumed);
+  uint64_t qb;
+  uint32_t r, qm;
+  int64_t at;
+  for (int k = 6 + warp; k <= nsmall && primes[k] < FT_WARP; k += nw) {
+    const uint32_t p = primes[k];
+    start(p, qb, r, qm, at);
+    for (uint32_t j = r + lane;; j += 32) {
+      const uint32_t q = offset(j);
+      const int64_t off = at + (int64_t) p * q;
+      if (off > last) break;
+      mark(k, p, (uint32_t) off, (qm + q) % p == 0);
+    }
+  }
+  for (int k = 6 + threadIdx.x; k <= nsmall; k += blockDim.x) {
+    const uint32_t p = primes[k];
+    if (p < FT_WARP) continue;
+    start(p, qb, r, qm, at);
+    for (uint32_t j = r;; j++) {
+      const uint32_t q = offset(j);
+      const int64_t off = at + (int64_t) ((uint64_t) p * q);
+      if (off > last) break;
+      mark(k, p, (uint32_t) off, (qm + q) % p == 0);
     }
   }
   __syncthreads();
   const uint64_t TMAX = sizeof(T) == 2 ? 0xFFFFull : 0xFFFFFFFFull;
   for (int i = threadIdx.x; i < en; i += blockDim.x) {
-    uint64_t n = to_number((uint64_t) (i0 + i));
+    const uint64_t n = nlo + offset((uint32_t) i);
     uint64_t v;
     if (n == 1) v = TMAX ^ 1;
     else {
       uint64_t P = prod[i];
-      uint64_t large = n / P;
+      uint64_t large = n >> 32 ? n / P : (uint32_t) n / (uint32_t) P;
       uint32_t cnt = (nf[i] & 0xFFu) + (large > 1 ? 1u : 0u);
       bool sq = (nf[i] >> 30) & 1u;
       if (sq) v = 0;
@@ -1888,10 +1976,7 @@ void ensure_prime_tables(Ctx& c, int64_t limit, cudaStream_t s)
   d_sums.alloc((size_t) nblk * 8);
   if (!b7.empty())
     PCG_CUDA(cudaMemcpyAsync(d_base.p, b7.data(), b7.size() * 4, cudaMemcpyHostToDevice, s));
-  int64_t pblocks = (nwords + 2047) / 2048;
-  k_prime_bits<<<(unsigned) pblocks, 512, 2048 * 8, s>>>(d_bits.as<uint64_t>(), d_pc.as<uint32_t>(), nwords, limit,
-                                                         d_base.as<uint32_t>(), (int) b7.size());
-  PCG_CUDA(cudaGetLastError());
+  prime_bits(d_bits, d_pc, nwords, limit, d_base, b7.size(), c.num_sms, s);
   k_scan_sums<<<(unsigned) nblk, 512, 0, s>>>(d_pc.as<uint32_t>(), nwords, d_sums.as<uint64_t>());
   k_scan_serial<<<1, 1024, 0, s>>>(d_sums.as<uint64_t>(), nblk);
   k_scan_apply<<<(unsigned) nblk, 512, 0, s>>>(d_pc.as<uint32_t>(), nwords, d_sums.as<uint64_t>(), d_excl.as<uint64_t>());
@@ -1947,7 +2032,7 @@ __global__ void k_pitab_pack(const uint64_t* __restrict__ bits, const uint64_t* 
 
 // PiTable {count, bits} per 240 numbers over [0, limit] without the primes
 // array (for the lookups of pi(n), n <= sqrt(x), of the A, B, C formulas).
-void build_pitab_only(DevBuf& out, int64_t limit, cudaStream_t s)
+void build_pitab_only(Ctx& c, DevBuf& out, int64_t limit, cudaStream_t s)
 {
   limit = std::max<int64_t>(limit, 240 * 4);
   int64_t nwords = limit / 240 + 1;
@@ -1961,10 +2046,7 @@ void build_pitab_only(DevBuf& out, int64_t limit, cudaStream_t s)
   d_excl.alloc((size_t) nwords * 8);
   if (!b7.empty())
     PCG_CUDA(cudaMemcpyAsync(d_base.p, b7.data(), b7.size() * 4, cudaMemcpyHostToDevice, s));
-  int64_t pblocks = (nwords + 2047) / 2048;
-  k_prime_bits<<<(unsigned) pblocks, 512, 2048 * 8, s>>>(d_bits.as<uint64_t>(), d_pc.as<uint32_t>(), nwords, limit,
-                                                         d_base.as<uint32_t>(), (int) b7.size());
-  PCG_CUDA(cudaGetLastError());
+  prime_bits(d_bits, d_pc, nwords, limit, d_base, b7.size(), c.num_sms, s);
   exclusive_scan_u32(d_pc.as<uint32_t>(), nwords, d_excl.as<uint64_t>(), s);
   out.alloc((size_t) nwords * 16);
   k_pitab_pack<<<(unsigned) ((nwords + 255) / 256), 256, 0, s>>>(d_bits.as<uint64_t>(), d_excl.as<uint64_t>(), nwords,
