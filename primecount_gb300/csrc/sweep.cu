@@ -595,13 +595,13 @@ static __device__ __forceinline__ void dec_if(bool on, uint32_t* a, uint32_t i)
 // factor-table indices below these are numbers below 2^30 and 2^32
 #define NARROW_INDEX 223000000ll
 #define WIDE_INDEX 892000000ll
-// a level answered alone with more records than this uses prefix counts per
-// word where they fit (see k_sweep)
-#define WORD_RECORDS 1024
 // levels answered together at most (see k_sweep)
 #define GROUP_MAX 256
-// a level with more records than this is answered alone
-#define SOLO_RECORDS 256
+// a level with more records than this is answered alone: 8 warps take them in
+// one or two turns (S2_hard(1e17), 256 threads: 48, 80, 128, 160, 256, 512 records:
+// 16.8, 17.5, 16.7, 16.8, 17.4, 18.7 ms; D(1e13) 0.32, 0.30, 0.28, 0.27, 0.28,
+// 0.28 ms; D(1e20), 512 threads: 128, 256, 512: 691, 682, 683 ms)
+__host__ __device__ constexpr int solo_records(int nt) { return nt >= 512 ? 256 : 160; }
 // a group holds at most this many records, and levels times records; with
 // more than LANE_RECORDS in at most LANE_LEVELS levels, a thread per record
 #define GROUP_RECORDS 1024
@@ -663,7 +663,7 @@ static __device__ __forceinline__ uint32_t removed_le(const LevelM& Q, uint32_t 
 
 // k_sweep: one CTA per segment at a time, the levels in order.
 //
-// A level with p >= 64 and at most SOLO_RECORDS records is answered in a
+// A level with p >= 64 and at most solo_records() records is answered in a
 // group of up to GROUP_MAX consecutive levels, all records against one bitmap
 // state:
 //   1. every level's multiples still unsieved before the group, as 32-bit
@@ -683,7 +683,7 @@ static __device__ __forceinline__ uint32_t removed_le(const LevelM& Q, uint32_t 
 // with (levels / p)^2 times the segment's length and the corrections of step 4
 // with levels times records: GROUP_WORK and the p / 32 levels of a full
 // segment are where longer groups stop gaining (p / 24 and p / 48: 0.5-1 %
-// slower).  A level with more than SOLO_RECORDS records fills the block by
+// slower).  A level with more than solo_records() records fills the block by
 // itself and needs no corrections (128 and 384: up to 4 % slower).
 // Measured on a GB300, levels one at a time -> groups: D(1e20) 1323 -> 947 ms,
 // D(1e18) 89.2 -> 58.4 ms, D(1e15) 3.38 -> 2.89 ms, S2_hard(1e17) 42.0 -> 27.9 ms;
@@ -988,7 +988,7 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
       {
         // goto next_segment (D.cpp:131-132): no leaves from s_stop on
         if (b0 + tid >= s_stop) E = 0;
-        const bool alone = tid < nb && ((lp[tid].flags & 4) || E > SOLO_RECORDS);
+        const bool alone = tid < nb && ((lp[tid].flags & 4) || E > solo_records(NT));
         const unsigned bal = __ballot_sync(0xffffffffu, alone);
         if (lane == 0 && warp < LB / 32) s_solo[warp] = bal;
         // flat offsets of records and of mask words
