@@ -896,9 +896,18 @@ __global__ void k_outer_S2e(uint64_t x_lo, uint64_t x_hi, int64_t y, int64_t z, 
 // pi(5e9) 1.34 -> 1.20 ms, B of pi(2e19) beside D 84 -> 70 ms; then four medium
 // multiples per round, the next large multiples kept over 16 segments, and the
 // queries' quotients in single precision: pi(5e9) 1.21 -> 1.04 ms, B of pi(1e20)
-// 175 -> 143 ms, all its easy terms 445 -> 414 ms.
+// 175 -> 143 ms, all its easy terms 445 -> 414 ms; then lanes that stay together
+// (PS_TOGETHER): pi(5e9) 1.02 -> 0.94 ms.  The medium multiples by lanes p words
+// apart (no bank conflicts, two shuffles a class) took 1.7 times as long.
 #define PS_NT 512
 #define PS_SMALL PAT_PRIMES
+// In segments of this many words on the lanes of a warp take as many multiples of
+// their large primes as the one with the most, without a branch (clear_if), and
+// large primes start at segment / 256 instead of / 128: phi(1e16, 20000) 14.9 ->
+// 12.6 ms, the terms of pi(1e18) one after another 62.1 -> 60.9 ms, pi(5e9) 1.02 ->
+// 1.00 ms.  In shorter ones, where a prime has few, the vote costs more: pi(1e6)
+// 22 -> 24 us.
+#define PS_TOGETHER 2048
 struct PsArgs {
   uint64_t x_lo, x_hi;
   int64_t lo0;           // first segment start (multiple of 240)
@@ -943,6 +952,13 @@ static __device__ __forceinline__ uint64_t ceil_div_magic(uint64_t n, uint32_t p
   uint64_t q = __umul64hi(n, m);     // floor(n / p) or one less
   if (n - q * p >= p) q++;
   return q + (q * p != n);
+}
+
+// a[i] &= m of the lanes with on, without a branch: the others clear nothing of
+// word lane (lanes that leave a loop early serialise the others' atomics)
+static __device__ __forceinline__ void clear_if(bool on, uint32_t* a, uint32_t i, uint32_t m)
+{
+  atomicAnd(&a[on ? i : threadIdx.x & 31], on ? m : 0xFFFFFFFFu);
 }
 
 __global__ void __launch_bounds__(PS_NT, 2) k_psieve(const PsArgs A)
@@ -1050,14 +1066,15 @@ __global__ void __launch_bounds__(PS_NT, 2) k_psieve(const PsArgs A)
         const uint32_t off = ot + pt * (lane_res >= qt ? lane_res - qt : lane_res + 120 - qt);
         uint32_t w = off / 120;
         const uint32_t msk = ~(1u << s_bit[off - 120 * w]);
-        if (off >= span) w = nw32;
-        for (; w + 3 * pt < nw32; w += 4 * pt) {
+        // all lanes' words lie within pt of the first: full rounds, then the ends
+        uint32_t first = ot / 120;
+        for (; first + 4 * pt + 1 < nw32; first += 4 * pt, w += 4 * pt) {
           atomicAnd(&bits32[w], msk);
           atomicAnd(&bits32[w + pt], msk);
           atomicAnd(&bits32[w + 2 * pt], msk);
           atomicAnd(&bits32[w + 3 * pt], msk);
         }
-        for (; w < nw32; w += pt) atomicAnd(&bits32[w], msk);
+        for (; first < nw32; first += pt, w += pt) clear_if(w < nw32, bits32, w, msk);
       }
     }
     // large primes: a lane per prime along the 30-wheel; the next multiple
@@ -1080,16 +1097,30 @@ __global__ void __launch_bounds__(PS_NT, 2) k_psieve(const PsArgs A)
         off = v & 0x1FFFFFFFu;
         jj = v >> 29;
       }
-      while (off < span) {
-        const uint32_t w = off / 120;
-        atomicAnd(&bits32[w], ~(1u << s_bit[off - 120 * w]));
-        off += p * ((WHEEL_GAPS >> (4 * jj)) & 15u);
-        jj = (jj + 1) & 7;
+      if (words >= PS_TOGETHER) {
+        const unsigned act = __activemask();
+        while (__any_sync(act, off < span)) {
+          const bool on = off < span;
+          const uint32_t w = off / 120;
+          clear_if(on, bits32, w, ~(1u << s_bit[off - 120 * w]));
+          if (on) {
+            off += p * ((WHEEL_GAPS >> (4 * jj)) & 15u);
+            jj = (jj + 1) & 7;
+          }
+        }
+      } else {
+        while (off < span) {
+          const uint32_t w = off / 120;
+          atomicAnd(&bits32[w], ~(1u << s_bit[off - 120 * w]));
+          off += p * ((WHEEL_GAPS >> (4 * jj)) & 15u);
+          jj = (jj + 1) & 7;
+        }
       }
       if (left) state[k - A.nmid] = (off - span) | (jj << 29);
     }
     __syncthreads();
-    // chunk prefix (8 words per chunk; up to 4 chunks per thread)
+    // chunk prefix (8 words per chunk, each lane from another one on, or a warp's
+    // reads meet in 4 banks; up to 4 chunks per thread)
     {
       const int cpt = (nch + PS_NT - 1) / PS_NT;
       const int base = tid * cpt;
@@ -1099,7 +1130,7 @@ __global__ void __launch_bounds__(PS_NT, 2) k_psieve(const PsArgs A)
       for (int c = 0; c < 4; c++) {
         uint32_t t = 0;
         if (c < cpt && base + c < nch)
-          for (int i = 0; i < 8; i++) t += __popcll(bits[8 * (base + c) + i]);
+          for (int i = 0; i < 8; i++) t += __popcll(bits[8 * (base + c) + ((i + lane) & 7)]);
         loc[c] = t;
         sum += t;
       }
@@ -1205,14 +1236,14 @@ static int ps_words(int64_t numbers, int num_sms)
   return (int) std::max<int64_t>(256, std::min<int64_t>(12288, (per + 63) / 64 * 64));
 }
 
-static int64_t ps_mid_div()
+static int64_t ps_mid_div(int words)
 {
   static const int64_t d = [] {
     const char* e = getenv("PCG_PS_MID");
-    const int64_t v = e ? atoll(e) : 128;
-    return v > 0 ? v : 128;
+    const int64_t v = e ? atoll(e) : 0;
+    return v > 0 ? v : 0;
   }();
-  return d;
+  return d ? d : words >= PS_TOGETHER ? 256 : 128;
 }
 
 // launches the sieve of [lo0, end) in segments, results in T_PS_C; B queries
@@ -1233,7 +1264,7 @@ static PsOut launch_psieve(Ctx& c, u128 x, int64_t lo0, int64_t end, bool b_mode
   const bool resident = c.tab.prime_limit >= limit;
   std::vector<uint64_t> made;                              // reciprocals, then the primes
   int64_t nbase;
-  const int64_t mid_limit = len / ps_mid_div();
+  const int64_t mid_limit = len / ps_mid_div(words);
   int nmid = 0;
   DevBuf& d_base = c.tmp[T_PS_BASE];
   DevBuf& d_seg = c.tmp[T_PS_C];
