@@ -186,11 +186,17 @@ pcg_status run_pool(size_t n, const pcg_opts* opts, const std::vector<size_t>& o
 extern "C" {
 
 // pi(x) of n queries.  The hard special leaves (Gourdon's D) of every query
-// with x > 1e10 run as the work items of one batched sweep on the caller's
+// with 1e10 < x < BATCH_D_MAX run as the work items of one batched sweep on the caller's
 // context (one persistent kernel per wave over all queries' segments, the
 // waves launched as one CUDA graph), while the worker pool computes the other
-// terms of those queries and the small queries whole; each answer is then
-// the pool's part plus its D.
+// terms of those queries and the small and large queries whole; each answer is
+// then the pool's part plus its D.
+//
+// A large query fills the GPU by itself, with segments cut for it and pi(x)'s own
+// z.  D batched / whole, GB300: 64 queries below 1e14 16 / 27 ms, 48 below 1e15
+// 59 / 44 ms, 32 below 1.8e16 202 / 138 ms, 16 below 1e17 305 / 167 ms.
+static const u128 BATCH_D_MAX = 300000000000000ull;
+
 pcg_status pcg_pi_batch(const pcg_i128* xs, size_t n, pcg_i128* out, const pcg_opts* opts)
 {
   if ((!xs || !out) && n) return PCG_EINVAL;
@@ -210,7 +216,7 @@ pcg_status pcg_pi_batch(const pcg_i128* xs, size_t n, pcg_i128* out, const pcg_o
     for (size_t i = 0; i < n; i++) {
       if (xs[i].hi < 0) continue;
       const u128 x = make_u128(xs[i]);
-      if (x <= (u128) 10000000000ull) continue;
+      if (x <= (u128) 10000000000ull || x >= BATCH_D_MAX) continue;
       const GourdonParams g = gourdon_params(x, tune.alpha_y, tune.alpha_z);
       if (g.y < g.z || x > ((u128) g.y << 62)) continue;
       SweepProblem p;
