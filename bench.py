@@ -15,8 +15,7 @@ roofline     the sieve/leaf kernel (k_sweep) against the measured HBM copy
              peak, with the algorithmic bytes of the hot-path table: 2 B per
              FactorTable entry read, 4 B per two-prime leaf (its prime),
              16 B per (segment, b) step (PiTable word of the level bounds),
-             over its CUDA-event launch time; the 8 B reciprocal per leaf is
-             implementation traffic, reported apart.  traffic = DRAM bytes
+             over its CUDA-event launch time.  traffic = DRAM bytes
              per launch, scaled from the committed ncu capture of a smaller
              D by the algorithmic bytes.  int_ops: algorithmic integer and
              shared-memory operations (per leaf one division and one prefix
@@ -522,10 +521,10 @@ def main():
     peak, peak_kind = measured_peaks()
     # algorithmic bytes of the hot-path table: 2 B per FactorTableD entry
     # read, 4 B per two-prime leaf (its prime), 16 B per (segment, level)
-    # step (PiTable word of the level bounds); the 8 B reciprocal of m (or of
-    # the prime) per leaf is this implementation's own traffic
+    # step (PiTable word of the level bounds); this implementation reads
+    # nothing else per leaf
     alg_bytes = 2 * st["factor_entries"] + 4 * st["two_prime_leaves"] + 16 * st["levels"]
-    impl_bytes = 8 * st["leaves"]
+    impl_bytes = 0
     k_ms_call = kernel_ms / args.steps
     launches_call = launches / args.steps
     launch_s = k_ms_call / launches_call / 1000.0

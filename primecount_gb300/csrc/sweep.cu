@@ -677,19 +677,20 @@ static __device__ __forceinline__ uint32_t removed_le(const LevelM& Q, uint32_t 
 //   4. a record n of level l: the numbers <= n left after the group plus
 //      those that the group's levels from l on removed at or below n.
 // Three barriers per group instead of two to four per level: what bounds the
-// sparse segments is the latency of the chain of levels (2 CTAs of 8 warps
-// per SM, issue active 44 %), so levels are taken together as long as the
+// sparse segments is the latency of the chain of levels (16 warps per SM, issue
+// active 53 %; 1.4 to 1.7 barrier stalls per issue), so levels are taken together as long as the
 // work that grows with the group stays small.  The collisions of step 2 grow
 // with (levels / p)^2 times the segment's length and the corrections of step 4
 // with levels times records: GROUP_WORK and the p / 32 levels of a full
 // segment are where longer groups stop gaining (p / 24 and p / 48: 0.5-1 %
 // slower).  A level with more than solo_records() records fills the block by
-// itself and needs no corrections (128 and 384: up to 4 % slower).
+// itself and needs no corrections.
 // Measured on a GB300, levels one at a time -> groups: D(1e20) 1323 -> 947 ms,
 // D(1e18) 89.2 -> 58.4 ms, D(1e15) 3.38 -> 2.89 ms, S2_hard(1e17) 42.0 -> 27.9 ms;
 // then leaf offsets without the reciprocal table and a level alone streamed
 // by independent warps: 797, 50.1, 2.70, 25.8 ms; then branch-free shared
-// atomics: 775, 48.4, 2.65, 25.2 ms.
+// atomics: 775, 48.4, 2.65, 25.2 ms; with the segment plan, the 512-thread shape and
+// the first pattern levels in one pass: 682, 41.6, 1.08, 16.8 ms.
 // levels per batch (a thread each)
 constexpr int sweep_batch(int nt) { return nt < 256 ? nt : 256; }
 
