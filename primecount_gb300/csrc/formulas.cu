@@ -318,7 +318,8 @@ __device__ __forceinline__ long long outer_terms(const PairOuter& O, const uint3
 // xp - start q by q with one correction, as in the sweep's leaves: primes
 // below 2^30, segments below 2^21 numbers.  The terms of larger n, few per
 // outer and segment, are the last list, in pieces of PAIR_SPLIT terms for
-// k_pairs.  Bound by integer issue (about 30 instructions a term).  Measured
+// k_pairs.  Bound by integer issue (20 warp instructions per 32 terms, 75 % of the
+// issue slots at 1e18).  Measured
 // on a GB300, all terms by k_pairs -> this: A + C of 1e16 1.28 -> 0.77 ms, 1e18
 // 21.0 -> 13.6 ms, 1e20 496 -> 271 ms; 256 threads a block 360 ms, 64 segments
 // 308 ms, 512 segments 273 ms.
