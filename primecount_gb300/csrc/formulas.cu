@@ -319,10 +319,10 @@ __device__ __forceinline__ long long outer_terms(const PairOuter& O, const uint3
 // below 2^30, segments below 2^21 numbers.  The terms of larger n, few per
 // outer and segment, are the last list, in pieces of PAIR_SPLIT terms for
 // k_pairs.  Bound by integer issue (20 warp instructions per 32 terms, 75 % of the
-// issue slots at 1e18).  Measured
-// on a GB300, all terms by k_pairs -> this: A + C of 1e16 1.28 -> 0.77 ms, 1e18
-// 21.0 -> 13.6 ms, 1e20 496 -> 271 ms; 256 threads a block 360 ms, 64 segments
-// 308 ms, 512 segments 273 ms.
+// issue slots at 1e18).  Measured on a GB300, all terms by k_pairs -> this: A + C
+// of 1e16 1.28 -> 0.77 ms, 1e18 21.0 -> 13.6 ms, 1e20 496 -> 271 ms; 256 threads a
+// block 360 ms, 64 segments 308 ms, 512 segments 273 ms.  Then 32-bit starts and
+// d / 120 by one product: A + C and B of 1e19 85.0 -> 83.3 ms.
 #define PSEG_ENTRIES 13312
 #define PSEG_NUMBERS (PSEG_ENTRIES * 120)
 #define PSEG_COUNT 256
@@ -358,16 +358,16 @@ static __device__ __forceinline__ int64_t pseg_q(const PairOuter& O, uint64_t n,
 // thread's primes i = first, first + step, ... <= hi
 template <bool LOW>
 __device__ __forceinline__ long long pseg_terms(const uint2* __restrict__ tab, const uint8_t* s_sh,
-                                                const uint32_t* __restrict__ primes, uint64_t xp, uint64_t start,
+                                                const uint32_t* __restrict__ primes, uint64_t xp, uint32_t start,
                                                 uint32_t first, uint32_t hi, uint32_t step, uint32_t base)
 {
   auto term = [&](uint32_t q) -> uint32_t {
-    const uint64_t r = xp - start * q;
+    const uint64_t r = xp - (uint64_t) start * q;
     uint32_t d = quot_f32(r, __uint2float_rn(q));
     const int32_t t = (int32_t) ((uint32_t) r - d * q);
     if (t < 0) d--;
     if (t >= (int32_t) q) d++;
-    const uint32_t h = d / 120;
+    const uint32_t h = __umulhi(d, 35791395u);           // d / 120: 120 * 35791395 = 2^32 + 104, d < 2^25
     const uint2 e = tab[h];
     uint32_t m;
     asm("shr.u32 %0, %1, %2;" : "=r"(m) : "r"(0xFFFFFFFFu), "r"((uint32_t) s_sh[d - 120 * h]));
@@ -400,7 +400,7 @@ __device__ __forceinline__ long long pseg_terms(const uint2* __restrict__ tab, c
 template <bool LOW>
 __device__ __forceinline__ long long pseg_outer(const PairOuter& O, uint32_t lo, uint32_t hi, uint32_t at, uint32_t step,
                                                 const uint2* tab, const uint8_t* s_sh, const uint32_t* primes,
-                                                uint64_t start, uint32_t base)
+                                                uint32_t start, uint32_t base)
 {
   if (O.mode == 0) {
     const uint32_t ic = (uint32_t) min((uint64_t) hi, max((uint64_t) lo, O.cap));
@@ -516,7 +516,7 @@ __global__ void __launch_bounds__(PSEG_THREADS, 2) k_pairs_seg(const PsegArgs A)
     if (item >= s_item0[A.nseg]) break;
     int seg = max(cur, 0);                               // items come in order
     while (item >= s_item0[seg + 1]) seg++;
-    const uint64_t n0 = (uint64_t) seg * PSEG_NUMBERS;
+    const uint32_t n0 = (uint32_t) seg * PSEG_NUMBERS;     // below PSEG_COUNT * PSEG_NUMBERS < 2^32
     if (seg != cur) {
       const int64_t w0 = (int64_t) (n0 / 240);
       base = seg == 0 ? 0u : (uint32_t) A.pibig[w0].x;
