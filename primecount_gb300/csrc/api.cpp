@@ -762,6 +762,9 @@ pcg_status pcg_ctx_trim(pcg_ctx* ctx, uint64_t* freed)
   });
 }
 
+// not part of the interface: refuse_alloc for the tests
+void pcg_test_refuse_alloc(int64_t n) { refuse_alloc(n); }
+
 pcg_status pcg_device_memory(uint64_t* free_bytes, uint64_t* total_bytes)
 {
   return guard(nullptr, [&] {

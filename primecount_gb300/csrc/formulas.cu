@@ -131,6 +131,7 @@ static void ensure_phi_tiny(Ctx& c, int k, cudaStream_t s)
   uint64_t P = 1, tot = 1;
   for (int i = 0; i < k; i++) { P *= pr[i]; tot *= pr[i] - 1; }
   int64_t nwords = (int64_t) ((P + 63) / 64);
+  t.phik = -1;
   t.phi_bits.alloc((size_t) nwords * 8);
   t.phi_pref.alloc((size_t) nwords * 8);
   DevBuf pc;
@@ -1420,6 +1421,7 @@ struct PiParts {
 static void ensure_pibig(Ctx& c, int64_t limit, cudaStream_t s)
 {
   if (c.tab.pibig_limit >= limit) return;
+  c.tab.pibig_limit = -1;
   build_pitab_only(c, c.tab.pibig, limit, s);
   c.tab.pibig_limit = limit;
 }

@@ -87,6 +87,9 @@ struct PinBuf {
   void alloc();
 };
 
+// For tests: the n-th allocation from now on fails as out of memory (0: none).
+void refuse_alloc(int64_t n);
+
 // Device-resident tables of one context.
 struct Tables {
   // primes (uint32, 1-indexed, primes[0] = 0) and PiTable {count, bits} per 240

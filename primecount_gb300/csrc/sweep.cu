@@ -1849,12 +1849,16 @@ static double now_ms()
   return duration<double, std::milli>(steady_clock::now().time_since_epoch()).count();
 }
 
+static std::atomic<int64_t> g_refuse{0};
+void refuse_alloc(int64_t n) { g_refuse = n; }
+static bool refused() { return g_refuse.load(std::memory_order_relaxed) > 0 && g_refuse.fetch_sub(1) == 1; }
+
 void DevBuf::alloc(size_t n)
 {
   if (n <= bytes && p) return;
   free_();
   if (n == 0) n = 16;
-  cudaError_t e = cudaMalloc(&p, n);
+  cudaError_t e = refused() ? cudaErrorMemoryAllocation : cudaMalloc(&p, n);
   if (e != cudaSuccess) {
     p = nullptr;
     bytes = 0;
@@ -1891,7 +1895,8 @@ void PinBuf::alloc()
       return;
     }
   }
-  const cudaError_t e = cudaHostAlloc(&p, PIN_BYTES, cudaHostAllocMapped | cudaHostAllocPortable);
+  const cudaError_t e = refused() ? cudaErrorMemoryAllocation
+                                  : cudaHostAlloc(&p, PIN_BYTES, cudaHostAllocMapped | cudaHostAllocPortable);
   if (e != cudaSuccess) {
     p = nullptr;
     cudaGetLastError();
@@ -1920,10 +1925,13 @@ static std::vector<uint32_t> small_primes(int64_t limit)
   return p;
 }
 
+// A table counts as resident by its limit (prime_limit, fd_z, ...), set when it is
+// complete.  Before its buffers are replaced the limit is taken back: a build that
+// fails leaves no table, and the next call that needs one builds it.
 static void ensure_wheel(Ctx& c, cudaStream_t s)
 {
   Tables& t = c.tab;
-  if (t.coprime.p) return;
+  if (t.coprime.p && t.cindex.p) return;
   const Wheel2310& w = wheel2310();
   t.coprime.alloc(sizeof(w.coprime));
   t.cindex.alloc(sizeof(w.index));
@@ -1989,6 +1997,8 @@ void ensure_prime_tables(Ctx& c, int64_t limit, cudaStream_t s)
   PCG_CUDA(cudaMemcpyAsync(&last_pc, d_pc.as<uint32_t>() + nwords - 1, 4, cudaMemcpyDeviceToHost, s));
   PCG_CUDA(cudaStreamSynchronize(s));
   int64_t np = 3 + (int64_t) last_excl + last_pc;
+  t.prime_limit = -1;
+  t.nprimes = 0;
   t.primes.alloc((size_t) (np + 2) * 4);
   t.pitab.alloc((size_t) nwords * 16);
   uint32_t head[4] = {0, 2, 3, 5};
@@ -2141,6 +2151,7 @@ void ensure_factor_d(Ctx& c, int64_t y, int64_t z, cudaStream_t s)
   // whose size limit no practical z reaches, so that it can be tested
   const char* f32 = getenv("PCG_FACTOR_D_U32");
   const bool force32 = f32 && atoi(f32) == 1;
+  t.fd_y = t.fd_z = t.fd_cut = -1;
   t.fd_bytes = (z <= 386083ll * 386083 - 1 && !force32) ? 2 : 4;
   if (t.fd_bytes == 2) build_factor<uint16_t>(c, t.factor_d, z, y, 1, s);
   else build_factor<uint32_t>(c, t.factor_d, z, y, 1, s);
@@ -2156,6 +2167,7 @@ void ensure_factor_dr(Ctx& c, int64_t y, cudaStream_t s)
   if (t.fr_y >= y) return;
   double t0 = now_ms();
   ensure_prime_tables(c, std::max<int64_t>(y, isqrt((u128) y) + 1), s);
+  t.fr_y = -1;
   t.fr_bytes = (y <= 65534ll * 65534 - 1) ? 2 : 4;
   if (t.fr_bytes == 2) build_factor<uint16_t>(c, t.factor_dr, y, y, 0, s);
   else build_factor<uint32_t>(c, t.factor_dr, y, y, 0, s);
@@ -2564,6 +2576,7 @@ SweepResult run_sweep(Ctx& c, const SweepProblem& pb, const Tuning& tune_in, cud
     PlanCells P;
     plan_grid(P, L, PLAN_GRID);
     plan_cells_device(c, P, pb, x_star, pi_sqrt, bglob, s);
+    c.plan_key.clear();
     c.plan.clear();
     cut_segments(P, pb.gourdon, L, (int64_t) words * 240, grid, [&](int64_t v) { c.plan.push_back(v); return true; });
     c.plan_key = key;
