@@ -111,7 +111,10 @@ typedef struct {
 
 /* Create a context on the current CUDA device whose tables cover every
  * query with x <= max_x (Gourdon default parameters).  mem_budget bounds
- * the device memory the context may hold (0 = 90% of free memory). */
+ * the device memory the tables may hold (0 = 90% of free memory): PCG_ENOMEM
+ * if the primes, the PiTable and a FactorTable to z do not fit.  pi(x) from
+ * x = 3e16 on is computed with z = 2 y; where the budget has no room for that
+ * table the context holds the one to y and pi(x) is computed with z = y. */
 pcg_status pcg_ctx_create(pcg_i128 max_x, uint64_t mem_budget, pcg_ctx** out);
 void pcg_ctx_destroy(pcg_ctx* ctx);
 /* Message of the last failure on ctx (NULL: of the calling thread). */

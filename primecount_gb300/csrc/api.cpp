@@ -150,14 +150,19 @@ GourdonParams gourdon_params(u128 x, double user_alpha_y, double user_alpha_z)
   return p;
 }
 
-GourdonParams pi_params(u128 x, double alpha_y, double alpha_z)
+GourdonParams pi_params(const Ctx& c, u128 x, double alpha_y, double alpha_z)
 {
+  const GourdonParams g = gourdon_params(x, alpha_y, alpha_z);
   // z = y, the reference's choice for CPUs, sieves [0, x / z) for longer than
   // the extra leaves of z = 2 y take: pi(1e17) 15.0 -> 13.5 ms, pi(1e18) 62.2 ->
   // 56.4 ms, pi(2e19) 394 -> 358 ms; z = 1.5 y and 3 y: 57.1 and 55.8 ms at
   // 1e18; pi(1e16) 3.99 -> 3.76 ms, but its tables take that much longer.
-  if (alpha_z <= 0 && x >= (u128) 30000000000000000ull) alpha_z = 2.0;
-  return gourdon_params(x, alpha_y, alpha_z);
+  if (alpha_z > 0 || x < (u128) 30000000000000000ull) return g;
+  const GourdonParams w = gourdon_params(x, alpha_y, 2.0);
+  if (c.mem_budget == 0 || factor_d_covers(c.tab, w.y, w.z)) return w;
+  // its table has to be built: z = y where the budget has no room for it
+  const uint64_t now = c.tab.factor_d.bytes, then = std::max<uint64_t>(now, factor_d_bytes(w.z));
+  return device_bytes(c) - now + then <= c.mem_budget ? w : g;
 }
 
 DrParams dr_params(u128 x)
@@ -180,6 +185,16 @@ DrParams dr_params(u128 x)
 }
 
 // ---------------------------------------------------------------- contexts
+uint64_t device_bytes(const Ctx& c)
+{
+  const Tables& t = c.tab;
+  uint64_t b = t.primes.bytes + t.pitab.bytes + t.factor_d.bytes + t.factor_dr.bytes + t.coprime.bytes +
+               t.cindex.bytes + t.pibig.bytes + t.pmagic.bytes + t.phi_bits.bytes + t.phi_pref.bytes + c.cnt.bytes +
+               c.smu.bytes + c.segsum.bytes + c.run.bytes + c.acc.bytes + c.misc.bytes + c.msum.bytes;
+  for (const DevBuf& d : c.tmp) b += d.bytes;
+  return b;
+}
+
 Ctx::~Ctx()
 {
   if (pin.p) {                             // no kernel may still write to it
@@ -333,11 +348,8 @@ pcg_status pcg_ctx_create(pcg_i128 max_x, uint64_t mem_budget, pcg_ctx** out)
       GourdonParams g = gourdon_params(x);
       ensure_prime_tables(*c, std::max<int64_t>(g.y, isqrt(x) / 1 > 0 ? g.y : g.y), c->stream);
       // as far as pi(x) reads it where the budget allows
-      const GourdonParams p = pi_params(x, 0, 0);
-      const uint64_t table = 4 * ((uint64_t) wheel2310().to_index((uint64_t) p.z) + 2);   // at most 4 bytes each
-      const bool fits = pcg_ctx_device_bytes(c) + table <= c->mem_budget;
-      ensure_factor_d(*c, g.y, fits ? p.z : g.z, c->stream);
-      if (pcg_ctx_device_bytes(c) > c->mem_budget)
+      ensure_factor_d(*c, g.y, pi_params(*c, x, 0, 0).z, c->stream);
+      if (device_bytes(*c) > c->mem_budget)
         fail(PCG_ENOMEM, "resident tables exceed the memory budget");
     }
   });
@@ -357,21 +369,7 @@ const char* pcg_last_error(const pcg_ctx* c)
   return tl_error.c_str();
 }
 
-static uint64_t tmp_bytes(const Ctx& c)
-{
-  uint64_t t = 0;
-  for (const DevBuf& b : c.tmp) t += b.bytes;
-  return t;
-}
-
-uint64_t pcg_ctx_device_bytes(const pcg_ctx* c)
-{
-  if (!c) return 0;
-  const Tables& t = c->tab;
-  return t.primes.bytes + t.pitab.bytes + t.factor_d.bytes + t.factor_dr.bytes + t.coprime.bytes + t.cindex.bytes +
-         t.pibig.bytes + t.pmagic.bytes + t.phi_bits.bytes + t.phi_pref.bytes + c->cnt.bytes + c->smu.bytes +
-         c->segsum.bytes + c->run.bytes + c->acc.bytes + c->misc.bytes + c->msum.bytes + tmp_bytes(*c);
-}
+uint64_t pcg_ctx_device_bytes(const pcg_ctx* c) { return c ? device_bytes(*c) : 0; }
 
 pcg_status pcg_last_stats(const pcg_ctx* c, pcg_stats* out)
 {
@@ -693,7 +691,7 @@ static uint64_t psieve_bytes(const Ctx& c, int64_t lo, int64_t hi)
 static uint64_t pi_query_bytes(const Ctx& c, u128 x)
 {
   if (x <= (u128) 10000000000ull) return psieve_bytes(c, 0, (int64_t) x + 1) + 4096;
-  const GourdonParams g = pi_params(x, 0, 0);
+  const GourdonParams g = pi_params(c, x, 0, 0);
   const int64_t sqrtx = isqrt(x);
   const int64_t cols = pi_estimate(c, g.x_star) + 1;
   uint64_t b = sweep_device_bytes(c.num_sms, (int64_t) (x / (u128) g.z), cols, 8192);

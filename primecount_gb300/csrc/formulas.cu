@@ -1501,7 +1501,7 @@ static PiParts pi_gourdon(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, bo
                           bool own_params = false)
 {
   PiParts R;
-  const GourdonParams g = own_params ? pi_params(x, tune.alpha_y, tune.alpha_z)
+  const GourdonParams g = own_params ? pi_params(c, x, tune.alpha_y, tune.alpha_z)
                                      : gourdon_params(x, tune.alpha_y, tune.alpha_z);
   const int64_t y = g.y, z = g.z, k = g.k, x_star = g.x_star;
   if (x > ((u128) y << 62)) fail(PCG_ERANGE, "pi_gourdon(x): x is too large");

@@ -57,9 +57,10 @@ GourdonParams gourdon_params(u128 x);    // src/gourdon/pi_gourdon.cpp:44-62
 // the same with alpha_y / alpha_z given (<= 0: default), clamped as the
 // reference clamps --alpha-y / --alpha-z (src/gourdon/pi_gourdon.cpp:44-62)
 GourdonParams gourdon_params(u128 x, double alpha_y, double alpha_z);
-// the parameters pi(x) is computed with: z = 2 y from 3e16 on unless alpha_z is
-// given (the result does not depend on them)
-GourdonParams pi_params(u128 x, double alpha_y, double alpha_z);
+struct Ctx;
+// the parameters pi(x) is computed with on c: z = 2 y from 3e16 on unless alpha_z is
+// given or c's memory budget has no room for its table (the result does not depend on them)
+GourdonParams pi_params(const Ctx& c, u128 x, double alpha_y, double alpha_z);
 DrParams dr_params(u128 x);              // src/app/main.cpp:435-461
 int64_t x_star_gourdon(u128 x, int64_t y);   // src/util.cpp:362-386
 // phi(x, a): whether by ordinary and special leaves, and their y
@@ -130,6 +131,9 @@ void ensure_prime_tables(Ctx& c, int64_t limit, cudaStream_t s);
 void ensure_factor_d(Ctx& c, int64_t y, int64_t z, cudaStream_t s);
 // whether the resident FactorTableD serves (y, z); if so it does on s from here
 bool factor_d_serves(Ctx& c, int64_t y, int64_t z, cudaStream_t s);
+// the same without switching it, and the bytes of the table for n <= z
+bool factor_d_covers(const Tables& t, int64_t y, int64_t z);
+uint64_t factor_d_bytes(int64_t z);
 void ensure_factor_dr(Ctx& c, int64_t y, cudaStream_t s);
 
 // device exclusive scan (uint32 -> uint64), synchronous on s
@@ -233,6 +237,8 @@ struct Ctx {
   ~Ctx();
 };
 
+// device memory that c holds: tables and the working memory kept between calls
+uint64_t device_bytes(const Ctx& c);
 Ctx& default_ctx();
 Ctx* ctx_from(const pcg_opts* o);
 cudaStream_t stream_from(Ctx& c, const pcg_opts* o);

@@ -2108,21 +2108,36 @@ __global__ void k_factor_primes(T* __restrict__ out, const uint32_t* __restrict_
 // (y, z] (every other prime factor is at least 13), so a table of a larger y
 // serves after its primes above y are made zero, and again once they are T_MAX:
 // the tables of all the x of a context differ by the primes between their y.
-bool factor_d_serves(Ctx& c, int64_t y, int64_t z, cudaStream_t s)
+// The cut that serves (y, z), -1: none; the primes that change lie in (lo, hi].
+static int64_t factor_d_cut(const Tables& t, int64_t y, int64_t z, int64_t& lo, int64_t& hi)
 {
-  Tables& t = c.tab;
-  if (t.fd_z < z) return false;
+  if (t.fd_z < z) return -1;
   int64_t cut = t.fd_cut;
   if (y >= z && t.fd_y >= z) {
     if (cut < z) cut = t.fd_y;
   } else if (t.fd_y == y || (y < t.fd_y && z / 13 < y)) {
     cut = y;
   } else {
-    return false;
+    return -1;
   }
+  lo = std::max<int64_t>(11, std::min(cut, t.fd_cut));
+  hi = std::min(t.fd_z, std::max(cut, t.fd_cut));
+  return cut == t.fd_cut || hi <= t.prime_limit ? cut : -1;
+}
+
+bool factor_d_covers(const Tables& t, int64_t y, int64_t z)
+{
+  int64_t lo, hi;
+  return factor_d_cut(t, y, z, lo, hi) >= 0;
+}
+
+bool factor_d_serves(Ctx& c, int64_t y, int64_t z, cudaStream_t s)
+{
+  Tables& t = c.tab;
+  int64_t lo, hi;
+  const int64_t cut = factor_d_cut(t, y, z, lo, hi);
+  if (cut < 0) return false;
   if (cut == t.fd_cut) return true;
-  const int64_t lo = std::max<int64_t>(11, std::min(cut, t.fd_cut)), hi = std::min(t.fd_z, std::max(cut, t.fd_cut));
-  if (hi > t.prime_limit) return false;
   const int64_t i0 = host_pi(t, (uint64_t) lo), i1 = host_pi(t, (uint64_t) std::max(lo, hi));
   if (i1 > i0) {
     const unsigned blocks = (unsigned) ((i1 - i0 + 255) / 256);
@@ -2140,19 +2155,28 @@ bool factor_d_serves(Ctx& c, int64_t y, int64_t z, cudaStream_t s)
   return true;
 }
 
+// 16-bit entries whenever possible, as the reference's D() chooses
+// (src/gourdon/D.cpp:477-499); PCG_FACTOR_D_U32=1 forces the 32-bit table,
+// whose size limit no practical z reaches, so that it can be tested
+static int factor_d_entry(int64_t z)
+{
+  const char* f32 = getenv("PCG_FACTOR_D_U32");
+  return z <= 386083ll * 386083 - 1 && !(f32 && atoi(f32) == 1) ? 2 : 4;
+}
+
+uint64_t factor_d_bytes(int64_t z)
+{
+  return (uint64_t) (wheel2310().to_index((uint64_t) std::max<int64_t>(z, 1)) + 1) * (uint64_t) factor_d_entry(z);
+}
+
 void ensure_factor_d(Ctx& c, int64_t y, int64_t z, cudaStream_t s)
 {
   Tables& t = c.tab;
   if (factor_d_serves(c, y, z, s)) return;
   double t0 = now_ms();
   ensure_prime_tables(c, std::max<int64_t>(y, isqrt((u128) z) + 1), s);
-  // 16-bit entries whenever possible, as the reference's D() chooses
-  // (src/gourdon/D.cpp:477-499); PCG_FACTOR_D_U32=1 forces the 32-bit table,
-  // whose size limit no practical z reaches, so that it can be tested
-  const char* f32 = getenv("PCG_FACTOR_D_U32");
-  const bool force32 = f32 && atoi(f32) == 1;
   t.fd_y = t.fd_z = t.fd_cut = -1;
-  t.fd_bytes = (z <= 386083ll * 386083 - 1 && !force32) ? 2 : 4;
+  t.fd_bytes = factor_d_entry(z);
   if (t.fd_bytes == 2) build_factor<uint16_t>(c, t.factor_d, z, y, 1, s);
   else build_factor<uint32_t>(c, t.factor_d, z, y, 1, s);
   PCG_CUDA(cudaStreamSynchronize(s));
