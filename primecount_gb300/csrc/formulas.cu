@@ -1532,9 +1532,15 @@ static PiParts pi_gourdon(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, bo
     R.launches += r.stats.kernel_launches;
     R.ms_d = fnow_ms() - t1;
   };
-  // All of them are launched before the one wait for their results.
+  // All of them are launched before the one wait for their results, but for pair
+  // sums in pieces, which wait for their number first.
   auto other_terms = [&](cudaStream_t s, uint64_t* nl) {
-    const double t1 = fnow_ms();
+    // events before B, Phi0, Sigma, A + C and behind them
+    auto mark = [&](int i) {
+      if (!c.tev[i]) PCG_CUDA(cudaEventCreate(&c.tev[i]));
+      PCG_CUDA(cudaEventRecord(c.tev[i], s));
+    };
+    mark(0);
     const u128 xy = x / (u128) y, xz = x / (u128) z;
     const int64_t sqrt_xy = isqrt(xy);
     auto partials = [&](DevBuf& b, int n) {
@@ -1546,6 +1552,7 @@ static PiParts pi_gourdon(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, bo
     const int64_t n0 = (int64_t) (x / (u128) sqrtx), n1 = (int64_t) (x / (u128) (y + 1)) + 1;
     PsOut ps;
     if (sqrtx > y && n1 > n0) ps = launch_psieve(c, x, n0, n1, true, y, sqrtx, s, nl);
+    mark(1);
 
     // ---- Phi0
     const int64_t size = wheel2310().to_index((uint64_t) z) + 1;
@@ -1562,6 +1569,7 @@ static PiParts pi_gourdon(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, bo
                                              (uint32_t) (2 * k + 1), pk, PT, T.coprime.as<uint16_t>(), part0.as<i128>());
     PCG_CUDA(cudaGetLastError());
     (*nl)++;
+    mark(2);
 
     // ---- Sigma's sums, and the values of pi that it and B need
     SigmaArgs sg;
@@ -1590,6 +1598,7 @@ static PiParts pi_gourdon(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, bo
                                     (int64_t*) (sbuf.as<i128>() + 3 * sblocks));
     PCG_CUDA(cudaGetLastError());
     (*nl)++;
+    mark(3);
 
     // ---- A + C
     AcParams P;
@@ -1639,15 +1648,14 @@ static PiParts pi_gourdon(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, bo
       }
       if (nC2) k_outer_C2<<<(unsigned) ((nC2 + 127) / 128), 128, 0, s>>>(P, o + nA + nC1 + nQ);
       PCG_CUDA(cudaGetLastError());
-      *nl += 4;
+      *nl += (nA > 0) + (nC1 > 0) + (nQ > 0) + (nC2 > 0);
       gridp = launch_pairs(c, o, nout, s, nl);
     }
+    mark(4);
 
     // ---- the results
-    const double t2 = fnow_ms();
     std::vector<i128> hac = partials(c.tmp[T_PR_PART], gridp);
     PCG_CUDA(cudaStreamSynchronize(s));
-    const double t3 = fnow_ms();
     if (!ps.pinned) ps.r.resize((size_t) (3 * ps.nseg));
     if (ps.nseg > 0 && !ps.pinned)
       PCG_CUDA(cudaMemcpyAsync(ps.r.data(), c.tmp[T_PS_C].p, ps.r.size() * 8, cudaMemcpyDeviceToHost, s));
@@ -1679,10 +1687,12 @@ static PiParts pi_gourdon(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, bo
       }
       R.sigma = s0 + s1 + s2 + s3 + s4 * a + s5 - s6;
     }
-    // wall times: B, Phi0 and Sigma run ahead of the pair sums on one stream
-    R.ms_b = t2 - t1;
-    R.ms_ac = t3 - t2;
-    R.ms_sigma = fnow_ms() - t3;
+    double* const ms[4] = {&R.ms_b, &R.ms_phi0, &R.ms_sigma, &R.ms_ac};
+    for (int i = 0; i < 4; i++) {
+      float t = 0;
+      PCG_CUDA(cudaEventElapsedTime(&t, c.tev[i], c.tev[i + 1]));
+      *ms[i] = t;
+    }
   };
   uint64_t launches2 = 0;
   if (!with_d) {
