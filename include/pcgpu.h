@@ -103,8 +103,8 @@ typedef struct {
   int ctas_per_sm;
   int threads_per_cta;
   /* pi(x) by Gourdon's formula: time of each term.  ac, b, phi0, sigma by
-   * CUDA events (they follow one another on one stream, beside D's kernels),
-   * d by the host clock. */
+   * the GPU's clock (they follow one another on one stream, beside D's
+   * kernels), d by the host's. */
   double ac_ms, b_ms, phi0_ms, sigma_ms, d_ms;
   uint64_t crossoff_multiples; /* multiples of the sieving primes crossed off in the
                                   segments (the sieve's shared-memory updates)      */

@@ -202,7 +202,6 @@ Ctx::~Ctx()
     if (aux) cudaStreamSynchronize(aux);
   }
   for (auto& e : ev) if (e) cudaEventDestroy(e);
-  for (auto& e : tev) if (e) cudaEventDestroy(e);
   for (auto& e : kev) if (e) cudaEventDestroy(e);
   if (aux) cudaStreamDestroy(aux);
   if (own_stream && stream) cudaStreamDestroy(stream);

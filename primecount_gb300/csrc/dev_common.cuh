@@ -120,6 +120,23 @@ static __device__ __forceinline__ uint32_t quot_f32(uint64_t r, float m)
   return __float2uint_rz(rf * inv);
 }
 
+// the GPU's clock in nanoseconds: *t = now by the grid's first thread, *t =
+// max(*t, now) by a thread per block (t may be nullptr)
+static __device__ __forceinline__ unsigned long long now_ns()
+{
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
+}
+static __device__ __forceinline__ void stamp_start(unsigned long long* t)
+{
+  if (t && blockIdx.x == 0 && threadIdx.x == 0) *t = now_ns();
+}
+static __device__ __forceinline__ void stamp_end(unsigned long long* t)
+{
+  if (t && threadIdx.x == 0) atomicMax(t, now_ns());
+}
+
 // floor(n / q) from m = floor((2^64 - 1) / q), q >= 1: the high product is
 // floor(n / q) or one less
 static __device__ __forceinline__ uint64_t div_magic(uint64_t n, uint64_t q, uint64_t m)

@@ -155,6 +155,12 @@ static PhiTab phi_tab(const Ctx& c)
   return T;
 }
 
+// The terms of pi(x) follow one another on their stream; their times come from
+// stamps that the kernels write beside Sigma's results: the starts of B, Phi0
+// and Sigma and the ends of Sigma and A + C, the last two cleared by Phi0's
+// kernel.  (Five events on the stream: pi(5e9) 172 -> 192 us.)
+struct TermStamps { unsigned long long b, phi0, sigma, sigma_end, ac_end, pad; };
+
 // ---------------------------------------------------------------- Phi0
 // Phi0 = sum over n = 1 and the square-free n <= z whose prime factors lie
 // in (p_k, y] of mu(n) phi(x / n, k) (Phi0.cpp:38-96).  Those n are the
@@ -164,8 +170,13 @@ static PhiTab phi_tab(const Ctx& c)
 template <typename FT>
 __global__ void __launch_bounds__(256) k_phi0(uint64_t x_lo, uint64_t x_hi, const FT* __restrict__ factor,
                                               int64_t size, uint32_t thr, uint64_t pk, PhiTab T,
-                                              const uint16_t* __restrict__ coprime, i128* __restrict__ partial)
+                                              const uint16_t* __restrict__ coprime, i128* __restrict__ partial,
+                                              TermStamps* stamps)
 {
+  if (stamps) {
+    stamp_start(&stamps->phi0);
+    if (blockIdx.x == 0 && threadIdx.x == 0) stamps->sigma_end = stamps->ac_end = 0;
+  }
   const u128 x = ((u128) x_hi << 64) | x_lo;
   i128 acc = 0;
   for (int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; i < size; i += (int64_t) gridDim.x * blockDim.x) {
@@ -494,6 +505,7 @@ struct PsegArgs {
   int64_t big_words;             // words of pibig
   int* queue;
   i128* partial;
+  unsigned long long* end;       // stamp, or nullptr
 };
 
 __global__ void __launch_bounds__(PSEG_THREADS, 2) k_pairs_seg(const PsegArgs A)
@@ -545,6 +557,7 @@ __global__ void __launch_bounds__(PSEG_THREADS, 2) k_pairs_seg(const PsegArgs A)
     }
   }
   block_sum_i128<PSEG_THREADS>(acc, &A.partial[blockIdx.x]);
+  stamp_end(A.end);
 }
 
 // SMALL: every prime of the table is below 2^31 and the PiTable ends below 2^36
@@ -554,7 +567,8 @@ __global__ void __launch_bounds__(256) k_pairs(const PairOuter* __restrict__ out
                                                const PairPiece* __restrict__ pieces,
                                                const uint32_t* __restrict__ primes,
                                                const uint64_t* __restrict__ magic,
-                                               const uint64_t* __restrict__ pibig, i128* __restrict__ partial)
+                                               const uint64_t* __restrict__ pibig, i128* __restrict__ partial,
+                                               unsigned long long* end)
 {
   __shared__ uint8_t s_mask[240];       // # wheel residues <= r
   for (int r = threadIdx.x; r < 240; r += blockDim.x) s_mask[r] = (uint8_t) ((r / 30) * 8 + cnt8((uint32_t) (r % 30)));
@@ -581,6 +595,7 @@ __global__ void __launch_bounds__(256) k_pairs(const PairOuter* __restrict__ out
     acc += s;
   }
   block_sum_i128<256>(acc, &partial[blockIdx.x]);
+  stamp_end(end);
 }
 
 // Launches the sum of the terms of nout outers, its blocks' partial sums in
@@ -591,7 +606,8 @@ __global__ void __launch_bounds__(256) k_pairs(const PairOuter* __restrict__ out
 // an outer at 1e20).
 #define DIRECT_TERMS 65536
 #define PIECE_OUTERS 131072
-static int launch_pairs(Ctx& c, const PairOuter* outs, int64_t nout, cudaStream_t s, uint64_t* launches)
+static int launch_pairs(Ctx& c, const PairOuter* outs, int64_t nout, cudaStream_t s, uint64_t* launches,
+                        unsigned long long* end = nullptr)
 {
   if (nout <= 0) return 0;
   const Tables& T = c.tab;
@@ -603,10 +619,10 @@ static int launch_pairs(Ctx& c, const PairOuter* outs, int64_t nout, cudaStream_
     const int grid = (int) std::min<int64_t>(n, pair_blocks);
     if (T.prime_limit < (1ll << 31) && T.pibig_limit + 240 < (1ll << 36))
       k_pairs<true><<<grid, 256, 0, s>>>(o, n, pieces, T.primes.as<uint32_t>(), T.pmagic.as<uint64_t>(),
-                                         T.pibig.as<uint64_t>(), part.as<i128>() + nparts);
+                                         T.pibig.as<uint64_t>(), part.as<i128>() + nparts, end);
     else
       k_pairs<false><<<grid, 256, 0, s>>>(o, n, pieces, T.primes.as<uint32_t>(), T.pmagic.as<uint64_t>(),
-                                          T.pibig.as<uint64_t>(), part.as<i128>() + nparts);
+                                          T.pibig.as<uint64_t>(), part.as<i128>() + nparts, end);
     PCG_CUDA(cudaGetLastError());
     if (launches) *launches += 1;
     nparts += grid;
@@ -671,6 +687,7 @@ static int launch_pairs(Ctx& c, const PairOuter* outs, int64_t nout, cudaStream_
       g.big_words = std::max<int64_t>(T.pibig_limit, 240 * 4) / 240 + 1;
       g.queue = (int*) (d + 2 * nl);
       g.partial = part.as<i128>() + nparts;
+      g.end = end;
       PCG_CUDA(cudaFuncSetAttribute(k_pairs_seg, cudaFuncAttributeMaxDynamicSharedMemorySize, PSEG_ENTRIES * 8));
       const int grid = (int) std::min<uint32_t>(nitems, (uint32_t) seg_blocks);
       k_pairs_seg<<<grid, PSEG_THREADS, PSEG_ENTRIES * 8, s>>>(g);
@@ -928,6 +945,7 @@ struct PsArgs {
   const uint64_t* pibig; // PiTable bits for the B queries
   int64_t* seg;          // [nseg][3]: primes of the segment, its B queries, the sum of their counts
   int* queue;            // nullptr: a block per segment
+  unsigned long long* start;   // stamp, or nullptr
 };
 
 // the sieving primes 67..3163 and their reciprocals, for ranges below 1e7 on a
@@ -979,6 +997,7 @@ __global__ void __launch_bounds__(PS_NT, 2) k_psieve(const PsArgs A)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nch = words / 8;
   const u128 x = ((u128) A.x_hi << 64) | A.x_lo;
+  stamp_start(A.start);
   for (int i = tid; i < 120; i += PS_NT) s_bit[i] = (uint8_t) bit_of((uint32_t) i);
   for (int i = tid; i < PAT_WORDS; i += PS_NT) pat[i] = g_patterns.w[i];
   uint64_t small_mask = 0;                               // 7..61 in word 0
@@ -1251,7 +1270,7 @@ static int64_t ps_mid_div(int words)
 // launches the sieve of [lo0, end) in segments, results in T_PS_C; B queries
 // for primes in (qlo, qhi]
 static PsOut launch_psieve(Ctx& c, u128 x, int64_t lo0, int64_t end, bool b_mode, int64_t qlo, int64_t qhi,
-                        cudaStream_t s, uint64_t* launches)
+                        cudaStream_t s, uint64_t* launches, unsigned long long* start = nullptr)
 {
   PsOut o;
   lo0 -= lo0 % 240;
@@ -1328,6 +1347,7 @@ static PsOut launch_psieve(Ctx& c, u128 x, int64_t lo0, int64_t end, bool b_mode
     a.magic = d_base.as<uint64_t>();
   }
   a.pibig = c.tab.pibig.as<uint64_t>();
+  a.start = start;
   a.seg = o.pinned ? (int64_t*) c.pin.p : d_seg.as<int64_t>();
   a.queue = o.pinned ? nullptr : (int*) (d_seg.as<int64_t>() + 3 * o.nseg);
   // runs of segments once a block has many: the next multiples of 16 in a row
@@ -1474,11 +1494,13 @@ struct SigmaArgs {
   int64_t y, sqrt_xy, i0, i1;
   uint64_t look[3];
   int nlook;
+  TermStamps* stamps;
 };
 __global__ void __launch_bounds__(256) k_sigma(const SigmaArgs A, const uint32_t* __restrict__ primes,
                                                const uint64_t* __restrict__ pibig, i128* __restrict__ part,
                                                int64_t* __restrict__ found)
 {
+  stamp_start(&A.stamps->sigma);
   const u128 x = ((u128) A.x_hi << 64) | A.x_lo;
   i128 s4 = 0, s5 = 0, s6 = 0;
   for (int64_t i = A.i0 + 1 + (int64_t) blockIdx.x * 256 + threadIdx.x; i <= A.i1; i += 256ll * gridDim.x) {
@@ -1492,6 +1514,7 @@ __global__ void __launch_bounds__(256) k_sigma(const SigmaArgs A, const uint32_t
   block_sum_i128<256>(s5, &part[3 * blockIdx.x + 1]);
   block_sum_i128<256>(s6, &part[3 * blockIdx.x + 2]);
   if (blockIdx.x == 0 && (int) threadIdx.x < A.nlook) found[threadIdx.x] = dpi(pibig, A.look[threadIdx.x]);
+  stamp_end(&A.stamps->sigma_end);
 }
 
 // own_params: y and z as pi_params picks them, else the reference's.
@@ -1535,12 +1558,13 @@ static PiParts pi_gourdon(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, bo
   // All of them are launched before the one wait for their results, but for pair
   // sums in pieces, which wait for their number first.
   auto other_terms = [&](cudaStream_t s, uint64_t* nl) {
-    // events before B, Phi0, Sigma, A + C and behind them
-    auto mark = [&](int i) {
-      if (!c.tev[i]) PCG_CUDA(cudaEventCreate(&c.tev[i]));
-      PCG_CUDA(cudaEventRecord(c.tev[i], s));
-    };
-    mark(0);
+    // Sigma's primes (i0, i1]; its blocks' sums, pi of three values, the stamps
+    const int64_t i0 = host_pi(T, (uint64_t) x_star), i1 = host_pi(T, (uint64_t) x13);
+    const int sblocks = (int) std::max<int64_t>(1, std::min<int64_t>(SIGMA_BLOCKS, (i1 - i0 + 255) / 256));
+    const int at_found = 3 * sblocks, at_stamps = at_found + 2, nsig = at_stamps + (int) sizeof(TermStamps) / 16;
+    DevBuf& sbuf = c.tmp[T_SIGMA];
+    sbuf.alloc((size_t) nsig * 16);
+    TermStamps* const stamps = (TermStamps*) (sbuf.as<i128>() + at_stamps);
     const u128 xy = x / (u128) y, xz = x / (u128) z;
     const int64_t sqrt_xy = isqrt(xy);
     auto partials = [&](DevBuf& b, int n) {
@@ -1551,8 +1575,7 @@ static PiParts pi_gourdon(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, bo
     // ---- B = sum over primes y < p <= sqrt(x) of pi(x / p)
     const int64_t n0 = (int64_t) (x / (u128) sqrtx), n1 = (int64_t) (x / (u128) (y + 1)) + 1;
     PsOut ps;
-    if (sqrtx > y && n1 > n0) ps = launch_psieve(c, x, n0, n1, true, y, sqrtx, s, nl);
-    mark(1);
+    if (sqrtx > y && n1 > n0) ps = launch_psieve(c, x, n0, n1, true, y, sqrtx, s, nl, &stamps->b);
 
     // ---- Phi0
     const int64_t size = wheel2310().to_index((uint64_t) z) + 1;
@@ -1563,13 +1586,14 @@ static PiParts pi_gourdon(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, bo
     const uint64_t pk = T.h_primes[(size_t) k];
     if (T.fd_bytes == 2)
       k_phi0<uint16_t><<<grid0, 256, 0, s>>>((uint64_t) x, (uint64_t) (x >> 64), T.factor_d.as<uint16_t>(), size,
-                                             (uint32_t) (2 * k + 1), pk, PT, T.coprime.as<uint16_t>(), part0.as<i128>());
+                                             (uint32_t) (2 * k + 1), pk, PT, T.coprime.as<uint16_t>(), part0.as<i128>(),
+                                             stamps);
     else
       k_phi0<uint32_t><<<grid0, 256, 0, s>>>((uint64_t) x, (uint64_t) (x >> 64), T.factor_d.as<uint32_t>(), size,
-                                             (uint32_t) (2 * k + 1), pk, PT, T.coprime.as<uint16_t>(), part0.as<i128>());
+                                             (uint32_t) (2 * k + 1), pk, PT, T.coprime.as<uint16_t>(), part0.as<i128>(),
+                                             stamps);
     PCG_CUDA(cudaGetLastError());
     (*nl)++;
-    mark(2);
 
     // ---- Sigma's sums, and the values of pi that it and B need
     SigmaArgs sg;
@@ -1578,8 +1602,9 @@ static PiParts pi_gourdon(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, bo
     sg.x_hi = (uint64_t) (x >> 64);
     sg.y = y;
     sg.sqrt_xy = sqrt_xy;
-    sg.i0 = host_pi(T, (uint64_t) x_star);
-    sg.i1 = host_pi(T, (uint64_t) x13);
+    sg.i0 = i0;
+    sg.i1 = i1;
+    sg.stamps = stamps;
     sg.look[0] = (uint64_t) sqrtx;
     sg.look[1] = (uint64_t) sqrt_xy;
     sg.look[2] = ps.lo0 > 0 ? (uint64_t) (ps.lo0 - 1) : 0;
@@ -1591,14 +1616,10 @@ static PiParts pi_gourdon(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, bo
       most = std::max(most, (int64_t) p <= sqrt_xy ? x / p / (u128) y : x / p / p);
     }
     if (most > (u128) c.tab.pibig_limit) fail(PCG_EINTERNAL, "pi lookup beyond the PiTable");
-    DevBuf& sbuf = c.tmp[T_SIGMA];
-    const int sblocks = (int) std::max<int64_t>(1, std::min<int64_t>(SIGMA_BLOCKS, (sg.i1 - sg.i0 + 255) / 256));
-    sbuf.alloc((size_t) (3 * sblocks + 2) * 16);
     k_sigma<<<sblocks, 256, 0, s>>>(sg, T.primes.as<uint32_t>(), T.pibig.as<uint64_t>(), sbuf.as<i128>(),
-                                    (int64_t*) (sbuf.as<i128>() + 3 * sblocks));
+                                    (int64_t*) (sbuf.as<i128>() + at_found));
     PCG_CUDA(cudaGetLastError());
     (*nl)++;
-    mark(3);
 
     // ---- A + C
     AcParams P;
@@ -1649,9 +1670,8 @@ static PiParts pi_gourdon(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, bo
       if (nC2) k_outer_C2<<<(unsigned) ((nC2 + 127) / 128), 128, 0, s>>>(P, o + nA + nC1 + nQ);
       PCG_CUDA(cudaGetLastError());
       *nl += (nA > 0) + (nC1 > 0) + (nQ > 0) + (nC2 > 0);
-      gridp = launch_pairs(c, o, nout, s, nl);
+      gridp = launch_pairs(c, o, nout, s, nl, &stamps->ac_end);
     }
-    mark(4);
 
     // ---- the results
     std::vector<i128> hac = partials(c.tmp[T_PR_PART], gridp);
@@ -1659,13 +1679,15 @@ static PiParts pi_gourdon(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, bo
     if (!ps.pinned) ps.r.resize((size_t) (3 * ps.nseg));
     if (ps.nseg > 0 && !ps.pinned)
       PCG_CUDA(cudaMemcpyAsync(ps.r.data(), c.tmp[T_PS_C].p, ps.r.size() * 8, cudaMemcpyDeviceToHost, s));
-    std::vector<i128> h0 = partials(part0, grid0), hs = partials(sbuf, 3 * sblocks + 2);
+    std::vector<i128> h0 = partials(part0, grid0), hs = partials(sbuf, nsig);
     PCG_CUDA(cudaStreamSynchronize(s));
     if (ps.pinned) ps.take(c);
     for (const i128& v : hac) R.ac += v;
     for (const i128& v : h0) R.phi0 += v;
     int64_t found[3];
-    memcpy(found, &hs[(size_t) (3 * sblocks)], sizeof(found));
+    memcpy(found, &hs[(size_t) at_found], sizeof(found));
+    TermStamps ts;
+    memcpy(&ts, &hs[(size_t) at_stamps], sizeof(ts));
     R.b = b_sum(ps.r.data(), ps.nseg, found[2]);
 
     // ---- Sigma (Sigma.cpp:25-140)
@@ -1687,12 +1709,10 @@ static PiParts pi_gourdon(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, bo
       }
       R.sigma = s0 + s1 + s2 + s3 + s4 * a + s5 - s6;
     }
-    double* const ms[4] = {&R.ms_b, &R.ms_phi0, &R.ms_sigma, &R.ms_ac};
-    for (int i = 0; i < 4; i++) {
-      float t = 0;
-      PCG_CUDA(cudaEventElapsedTime(&t, c.tev[i], c.tev[i + 1]));
-      *ms[i] = t;
-    }
+    if (ps.nseg > 0) R.ms_b = 1e-6 * (double) (ts.phi0 - ts.b);
+    R.ms_phi0 = 1e-6 * (double) (ts.sigma - ts.phi0);
+    R.ms_sigma = 1e-6 * (double) (ts.sigma_end - ts.sigma);
+    if (ts.ac_end > ts.sigma_end) R.ms_ac = 1e-6 * (double) (ts.ac_end - ts.sigma_end);
   };
   uint64_t launches2 = 0;
   if (!with_d) {
@@ -1773,11 +1793,11 @@ void pi_dr_terms(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, i128 out[7]
     if (T.fr_bytes == 2)
       k_phi0<uint16_t><<<grid, 256, 0, s>>>((uint64_t) x, (uint64_t) (x >> 64), T.factor_dr.as<uint16_t>(), size,
                                             (uint32_t) prime_c, (uint64_t) prime_c, PT, T.coprime.as<uint16_t>(),
-                                            part.as<i128>());
+                                            part.as<i128>(), nullptr);
     else
       k_phi0<uint32_t><<<grid, 256, 0, s>>>((uint64_t) x, (uint64_t) (x >> 64), T.factor_dr.as<uint32_t>(), size,
                                             (uint32_t) prime_c, (uint64_t) prime_c, PT, T.coprime.as<uint16_t>(),
-                                            part.as<i128>());
+                                            part.as<i128>(), nullptr);
     PCG_CUDA(cudaGetLastError());
     s1 = sum_partials(part, grid, s);
   }
@@ -2039,10 +2059,10 @@ int64_t phi_any(Ctx& c, int64_t x, int64_t a, const Tuning& tune, cudaStream_t s
     PhiTab PT = phi_tab(c);
     if (T.fd_bytes == 2)
       k_phi0<uint16_t><<<grid, 256, 0, s>>>((uint64_t) x, 0, T.factor_d.as<uint16_t>(), size, (uint32_t) (2 * cc + 1),
-                                            (uint64_t) T.h_primes[(size_t) cc], PT, T.coprime.as<uint16_t>(), part.as<i128>());
+                                            (uint64_t) T.h_primes[(size_t) cc], PT, T.coprime.as<uint16_t>(), part.as<i128>(), nullptr);
     else
       k_phi0<uint32_t><<<grid, 256, 0, s>>>((uint64_t) x, 0, T.factor_d.as<uint32_t>(), size, (uint32_t) (2 * cc + 1),
-                                            (uint64_t) T.h_primes[(size_t) cc], PT, T.coprime.as<uint16_t>(), part.as<i128>());
+                                            (uint64_t) T.h_primes[(size_t) cc], PT, T.coprime.as<uint16_t>(), part.as<i128>(), nullptr);
     PCG_CUDA(cudaGetLastError());
     s1 = sum_partials(part, grid, s);
   }

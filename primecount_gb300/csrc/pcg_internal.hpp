@@ -225,7 +225,6 @@ struct Ctx {
   pcg_stats last{};
   std::string last_error;
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
-  cudaEvent_t tev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};   // between pi(x)'s terms, made on first use
   std::vector<cudaEvent_t> kev;   // per-launch timing events of the sweep
   // the last segment plan of the sweep and the problem and launch shape it was made for
   std::vector<int64_t> plan, plan_key;
