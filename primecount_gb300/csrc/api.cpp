@@ -690,7 +690,7 @@ static uint64_t psieve_bytes(const Ctx& c, int64_t lo, int64_t hi)
 
 static uint64_t pi_query_bytes(const Ctx& c, u128 x)
 {
-  if (x <= (u128) 10000000000ull) return psieve_bytes(c, 0, (int64_t) x + 1) + 4096;
+  if (!pi_by_formula(c, x, Tuning())) return psieve_bytes(c, 0, (int64_t) x + 1) + 4096;
   const GourdonParams g = pi_params(c, x, 0, 0);
   const int64_t sqrtx = isqrt(x);
   const int64_t cols = pi_estimate(c, g.x_star) + 1;
@@ -701,7 +701,8 @@ static uint64_t pi_query_bytes(const Ctx& c, u128 x)
   // at 1e18, 3.2e7 at 1e20, 1.1e8 at 1e21
   b += (uint64_t) (12 * 8e7 * std::pow((double) x / 1e20, 0.58));
   b += table_bytes_beyond(c, g.y, g.z, sqrtx);
-  return b + 65536;
+  b += phi_tiny_bytes(c, (int) g.k);
+  return b + 131072;                                          // partial sums, lists, the plan's cells
 }
 
 }  // extern "C"
@@ -710,10 +711,13 @@ namespace pcg {
 // device bytes of one phi(x, a) query beyond the context's resident tables
 static uint64_t phi_query_bytes(const Ctx& c, int64_t x, int64_t a)
 {
-  if (x < 1 || a <= 8 || a > x / 2) return 4096;
+  if (x < 1 || a < 1 || a > x / 2) return 4096;
+  if (a <= 8) return phi_tiny_bytes(c, (int) a) + 4096;
   const int64_t sq = isqrt((u128) x);
   const int64_t pis = pi_estimate(c, sq);
-  if (a > pis) return pi_query_bytes(c, (u128) x);
+  const uint64_t both = pi_query_bytes(c, (u128) sq) +        // pi(sqrt(x)) and the primes to 2 sqrt(x)
+                        table_bytes_beyond(c, std::max<int64_t>(2 * sq + 10, 1000), 0, -240);
+  if (a > pis) return both + pi_query_bytes(c, (u128) x);
   const double la = std::log((double) std::max<int64_t>(a, 3));
   const int64_t pa = (int64_t) ((double) a * (la + std::log(std::max(la, 1.0))));   // above p_a for a >= 6
   const int64_t pl = pa / 2;                                  // below p_a: both forms near their line
@@ -725,10 +729,10 @@ static uint64_t phi_query_bytes(const Ctx& c, int64_t x, int64_t a)
     const int64_t y = phi_y(x, pl);
     uint64_t l = sweep_device_bytes(c.num_sms, x / phi_y(x, pa), a + 1, 8192);
     l += (uint64_t) (wheel2310().to_index((uint64_t) y) + 1) * 2 + (uint64_t) (y / 240 + 1) * 36;
-    l += (uint64_t) c.num_sms * 8 * 16;                       // the ordinary leaves' partial sums
-    b = std::max(b, l + 65536);
+    l += phi_tiny_bytes(c, 8);
+    b = std::max(b, l + 131072);                              // the ordinary leaves' partial sums, the plan's cells
   }
-  return b;
+  return b + both;
 }
 }  // namespace pcg
 

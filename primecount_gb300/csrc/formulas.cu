@@ -123,13 +123,27 @@ __device__ __forceinline__ i128 dphi_tiny(u128 v, const PhiTab& T)
   return (i128) q * (i128) T.tot + (i128) c;
 }
 
+static uint64_t primorial(int k, uint64_t* tot)
+{
+  static const uint64_t pr[8] = {2, 3, 5, 7, 11, 13, 17, 19};
+  uint64_t P = 1;
+  *tot = 1;
+  for (int i = 0; i < k; i++) { P *= pr[i]; *tot *= pr[i] - 1; }
+  return P;
+}
+
+uint64_t phi_tiny_bytes(const Ctx& c, int k)
+{
+  uint64_t tot;
+  return c.tab.phik == k ? 0 : (primorial(k, &tot) / 64 + 1) * (16 + 4) + 4096;
+}
+
 static void ensure_phi_tiny(Ctx& c, int k, cudaStream_t s)
 {
   Tables& t = c.tab;
   if (t.phik == k) return;
-  static const uint64_t pr[8] = {2, 3, 5, 7, 11, 13, 17, 19};
-  uint64_t P = 1, tot = 1;
-  for (int i = 0; i < k; i++) { P *= pr[i]; tot *= pr[i] - 1; }
+  uint64_t tot;
+  const uint64_t P = primorial(k, &tot);
   int64_t nwords = (int64_t) ((P + 63) / 64);
   t.phik = -1;
   t.phi_bits.alloc((size_t) nwords * 8);
@@ -1867,8 +1881,10 @@ void pi_dr_terms(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, i128 out[7]
 static const int64_t PI_SIEVE_LIMIT = 10000000000ll;
 static const int64_t GOURDON_MIN = 1200000000ll;
 
-static bool gourdon_resident(const Ctx& c, u128 x, const Tuning& tune)
+bool pi_by_formula(const Ctx& c, u128 x, const Tuning& tune)
 {
+  if (x > (u128) PI_SIEVE_LIMIT) return true;
+  if (x < (u128) GOURDON_MIN) return false;
   const GourdonParams g = gourdon_params(x, tune.alpha_y, tune.alpha_z);
   const Tables& T = c.tab;
   return T.prime_limit >= g.y && T.fd_z >= g.z && (T.fd_y == g.y || (g.y >= g.z && T.fd_y >= g.z));
@@ -1880,7 +1896,7 @@ i128 pi_any(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, pcg_stats* st)
   i128 r;
   pcg_stats z{};
   if (x < 2) r = 0;
-  else if (x <= (u128) PI_SIEVE_LIMIT && (x < (u128) GOURDON_MIN || !gourdon_resident(c, x, tune))) {
+  else if (!pi_by_formula(c, x, tune)) {
     uint64_t l = 0;
     r = pi_sieve_count(c, (int64_t) x, s, &l);
     z.kernel_launches = l;

@@ -63,6 +63,11 @@ struct Ctx;
 GourdonParams pi_params(const Ctx& c, u128 x, double alpha_y, double alpha_z);
 DrParams dr_params(u128 x);              // src/app/main.cpp:435-461
 int64_t x_star_gourdon(u128 x, int64_t y);   // src/util.cpp:362-386
+// pi(x) on c: whether by Gourdon's formula (else counted by the sieve)
+struct Tuning;
+bool pi_by_formula(const Ctx& c, u128 x, const Tuning& tune);
+// bytes of phi(n, k)'s bitmap and its build, 0 if resident
+uint64_t phi_tiny_bytes(const Ctx& c, int k);
 // phi(x, a): whether by ordinary and special leaves, and their y
 bool phi_by_leaves(int64_t x, int64_t pa, int64_t pa1);
 int64_t phi_y(int64_t x, int64_t pa);
