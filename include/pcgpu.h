@@ -136,7 +136,11 @@ uint64_t pcg_ctx_device_bytes(const pcg_ctx* ctx);
  *                        (PiTable::get_primes, src/PiTable.hpp)
  *   PCG_TABLE_PI         uint64 pairs {count, bits} per 240 numbers (src/PiTable.cpp)
  *   PCG_TABLE_FACTOR_D   FactorTableD entries, 2 or 4 bytes (src/gourdon/FactorTableD.hpp)
- *   PCG_TABLE_FACTOR_DR  FactorTable entries, 2 or 4 bytes (src/FactorTable.hpp) */
+ *   PCG_TABLE_FACTOR_DR  FactorTable entries, 2 or 4 bytes (src/FactorTable.hpp)
+ * PCG_TABLE_FACTOR_D is the FactorTableD(y, z) that was built last, whatever y
+ * the calls that it has served since then had: pcg_ctx_create builds the one
+ * of max_x's y and z, with z = 2 y in the place of y from max_x = 3e16 on
+ * where mem_budget has room for it. */
 enum {
   PCG_TABLE_PRIMES = 0,
   PCG_TABLE_PI = 1,

@@ -654,6 +654,8 @@ pcg_status pcg_ctx_read_table(const pcg_ctx* ctx, int table, uint64_t first, uin
     if (!buf || !out) fail(PCG_EINVAL, "the table is not resident or out is NULL");
     if (first > n || count > n - first) fail(PCG_ERANGE, "entries beyond the table");
     PCG_CUDA(cudaSetDevice(cp->device));
+    // a call with a smaller y has made the primes above it zero
+    if (table == PCG_TABLE_FACTOR_D) ensure_factor_d(*cp, t.fd_y, t.fd_z, cp->stream);
     PCG_CUDA(cudaStreamSynchronize(cp->stream));
     PCG_CUDA(cudaMemcpy(out, (const char*) buf->p + first * (uint64_t) eb, count * (uint64_t) eb,
                         cudaMemcpyDeviceToHost));
