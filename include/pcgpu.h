@@ -260,7 +260,9 @@ pcg_status pcg_dr_params(pcg_i128 x, int64_t* y, int64_t* z, int64_t* c);
 
 /* ---- prime counting on top of the engine ---- */
 
-/* pi(x), x < 2^127; -1 semantics are left to the primecount_* wrappers. */
+/* pi(x), x < 2^127; -1 semantics are left to the primecount_* wrappers.
+ * By Gourdon's formula above 1e10, and from 1.2e9 on by a context whose tables
+ * cover x; smaller x are counted by a sieve. */
 pcg_status pcg_pi(pcg_i128 x, const pcg_opts* opts, pcg_i128* out);
 /* The terms of Gourdon's formula for x > 1e10: out6 = {A + C, B, D, Phi0,
  * Sigma, pi(x)} with pi = (A + C) - B + D + Phi0 + Sigma (the reference's
@@ -269,7 +271,7 @@ pcg_status pcg_pi_terms(pcg_i128 x, const pcg_opts* opts, pcg_i128* out6);
 /* pi(x) by the Deleglise-Rivat formula (pi_deleglise_rivat_64/128,
  * src/deleglise-rivat/pi_deleglise_rivat.cpp:61-136; the reference's -d
  * option): pi(y) + S1 + S2_trivial + S2_easy + S2_hard - 1 - P2, S2_hard by
- * the engine.  x <= 1e10 is counted by a sieve. */
+ * the engine.  x <= 1e10 is counted by a sieve, never by Gourdon's formula. */
 pcg_status pcg_pi_deleglise_rivat(pcg_i128 x, const pcg_opts* opts, pcg_i128* out);
 /* Its terms for x > 1e10: out7 = {S1, S2_trivial, S2_easy, S2_hard, P2,
  * pi(y), pi(x)} (the reference's --S1, --S2-trivial, --S2-easy, --S2-hard,

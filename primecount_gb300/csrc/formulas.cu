@@ -1407,7 +1407,7 @@ static i128 b_sum(const int64_t* r, int64_t nseg, i128 run)
 }
 
 // pi(x) for small x: a direct sieve count (2, 3, 5 are not in the bitmap)
-static i128 pi_sieve_count(Ctx& c, int64_t x, cudaStream_t s, uint64_t* launches)
+i128 pi_sieve_count(Ctx& c, int64_t x, cudaStream_t s, uint64_t* launches)
 {
   if (x < 2) return 0;
   if (x < 7) return x >= 5 ? 3 : (x >= 3 ? 2 : 1);

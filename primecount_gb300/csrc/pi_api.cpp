@@ -12,6 +12,7 @@
 
 namespace pcg {
 i128 pi_any(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, pcg_stats* st);
+i128 pi_sieve_count(Ctx& c, int64_t x, cudaStream_t s, uint64_t* launches);
 i128 pi_without_d(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, bool* needs_d);
 void pi_gourdon_terms(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, i128 out[6]);
 void pi_dr_terms(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, i128 out[7]);
@@ -63,8 +64,8 @@ pcg_status pcg_pi_deleglise_rivat(pcg_i128 xi, const pcg_opts* opts, pcg_i128* o
   return pcg_guarded(opts, [&](Ctx& c, cudaStream_t s) {
     if (xi.hi < 0) { *out = to_pcg(0); return; }       // pi(x) = 0 for x < 2
     const u128 x = make_u128(xi);
-    if (x <= (u128) 10000000000ull) {                  // small x: counted by the sieve, as pcg_pi does
-      *out = to_pcg(pi_any(c, x, tune_of(opts), s, nullptr));
+    if (x <= (u128) 10000000000ull) {                  // small x: counted by the sieve
+      *out = to_pcg(pi_sieve_count(c, (int64_t) x, s, nullptr));
       return;
     }
     i128 t[7];
