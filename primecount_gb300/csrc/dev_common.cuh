@@ -120,6 +120,37 @@ static __device__ __forceinline__ uint32_t quot_f32(uint64_t r, float m)
   return __float2uint_rz(rf * inv);
 }
 
+// Offset of the leaf n = floor(xp / m) in the segment [low, ...), xp = x / p
+// given by its low word: r = xp - low m lies in [0, span m), so xp's high
+// word is not needed, and n - low = floor(r / m) < span comes from a
+// single-precision quotient (quot_f32), off by at most one for span <= 2^21
+// (LEAF_SPAN), which the remainder corrects.  No reciprocal table: the gather
+// of 8 bytes per leaf was the longest wait of the dense segments.
+#define LEAF_SPAN (1u << 21)
+
+// m < 2^30 in a segment of at most LEAF_SPAN numbers: the remainder fits 32
+// signed bits
+static __device__ __forceinline__ uint32_t leaf_narrow(uint64_t xlo, uint64_t low, uint32_t m)
+{
+  const uint64_t r = xlo - low * m;
+  uint32_t d = quot_f32(r, __uint2float_rn(m));
+  const int32_t t = (int32_t) ((uint32_t) r - d * m);
+  if (t < 0) d--;
+  if (t >= (int32_t) m) d++;
+  return d;
+}
+
+// m < 2^32, any segment (below 2^23 numbers: the quotient is off by at most 3)
+static __device__ __forceinline__ uint32_t leaf_wide(uint64_t xlo, uint64_t low, uint32_t m)
+{
+  const uint64_t r = xlo - low * m;
+  uint32_t d = quot_f32(r, __uint2float_rn(m));
+  int64_t t = (int64_t) (r - (uint64_t) d * m);
+  while (t < 0) { t += m; d--; }
+  while (t >= (int64_t) m) { t -= m; d++; }
+  return d;
+}
+
 // the GPU's clock in nanoseconds: *t = now by the grid's first thread, *t =
 // max(*t, now) by a thread per block (t may be nullptr)
 static __device__ __forceinline__ unsigned long long now_ns()

@@ -537,37 +537,6 @@ __device__ __forceinline__ uint32_t query(const uint64_t* __restrict__ bits, con
          part(5, w45.y) + part(6, w67.x) + part(7, w67.y);
 }
 
-// Offset of the leaf n = floor(xp / m) in the segment [low, ...), xp = x / p
-// given by its low word: r = xp - low m lies in [0, span m), so xp's high
-// word is not needed, and n - low = floor(r / m) < span comes from a
-// single-precision quotient (quot_f32), off by at most one for span <= 2^21
-// (LEAF_SPAN), which the remainder corrects.  No reciprocal table: the gather
-// of 8 bytes per leaf was the longest wait of the dense segments.
-#define LEAF_SPAN (1u << 21)
-
-// m < 2^30 in a segment of at most LEAF_SPAN numbers: the remainder fits 32
-// signed bits
-static __device__ __forceinline__ uint32_t leaf_narrow(uint64_t xlo, uint64_t low, uint32_t m)
-{
-  const uint64_t r = xlo - low * m;
-  uint32_t d = quot_f32(r, __uint2float_rn(m));
-  const int32_t t = (int32_t) ((uint32_t) r - d * m);
-  if (t < 0) d--;
-  if (t >= (int32_t) m) d++;
-  return d;
-}
-
-// m < 2^32, any segment (below 2^23 numbers: the quotient is off by at most 3)
-static __device__ __forceinline__ uint32_t leaf_wide(uint64_t xlo, uint64_t low, uint32_t m)
-{
-  const uint64_t r = xlo - low * m;
-  uint32_t d = quot_f32(r, __uint2float_rn(m));
-  int64_t t = (int64_t) (r - (uint64_t) d * m);
-  while (t < 0) { t += m; d--; }
-  while (t >= (int64_t) m) { t -= m; d++; }
-  return d;
-}
-
 // Shared-memory atomics of the lanes with on, without a branch: the others
 // update word lane of the array by nothing.  (A predicated atomic is compiled
 // to a branch around it: 55 cycles a warp each, one after another; these
@@ -595,6 +564,8 @@ static __device__ __forceinline__ void dec_if(bool on, uint32_t* a, uint32_t i)
 // factor-table indices below these are numbers below 2^30 and 2^32
 #define NARROW_INDEX 223000000ll
 #define WIDE_INDEX 892000000ll
+static_assert(2310ull * (NARROW_INDEX / 480 + 1) < 1ull << 30 && 2310ull * (WIDE_INDEX / 480 + 1) < 1ull << 32,
+              "leaf_narrow and leaf_wide");
 // levels answered together at most (see k_sweep)
 #define GROUP_MAX 256
 // a level with more records than this is answered alone: 8 warps take them in
