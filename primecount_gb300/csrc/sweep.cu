@@ -443,6 +443,7 @@ struct SweepArgs {
                                  // [4] multiples crossed off
   int* queue;
   int group_max;            // levels answered together (<= GROUP_MAX; < 2: off)
+  int collisions;           // entries of the collision list in use (<= COLLISIONS)
 };
 
 // primes 7..61 sieved with wheel patterns (their multiples repeat every p words)
@@ -667,7 +668,10 @@ constexpr int sweep_batch(int nt) { return nt < 256 ? nt : 256; }
 
 // leaf records per window; removal mask words of a group (at least the
 // 2 words / 67 + 1 of the longest level, p = 67, up to 21 000 words);
-// collisions of a group kept for the end of its clears
+// collisions of a group kept for the end of its clears: by the group rule
+// some 968 times the density of numbers without a prime factor below p, 130
+// at p = 67 and fewer beyond, but nothing bounds them, so a lane resolves by
+// itself what the list does not hold
 #define REC_CAP 3584
 constexpr int sweep_mask_words(int nt) { return nt >= 512 ? 1280 : 640; }
 #define COLLISIONS 512
@@ -1273,7 +1277,7 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
             // beyond the list's end this lane does the same by itself
             auto collide = [&](uint32_t o) {
               const int at = atomicAdd(&s_ncoll, 1);
-              if (at < COLLISIONS) { clist[at] = o; return; }
+              if (at < A.collisions) { clist[at] = o; return; }
               bool first = true;
               for (int t = 0; t < G; t++) {
                 const LevelM R = lm[li + t];
@@ -1364,7 +1368,7 @@ __global__ void __launch_bounds__(NT, (NT >= 512) ? 1 : ((NT >= 256) ? 2 : 4)) k
             if (pend != NO_FIRST) collide(pend);
             __syncthreads();
             if (s_ncoll) {
-              const int nc = min(s_ncoll, COLLISIONS);
+              const int nc = min(s_ncoll, A.collisions);
               for (int i = 4 * warp; i < nc; i += 4 * NW) resolve(clist + i, min(4, nc - i));
               __syncthreads();
               if (tid == 0) s_ncoll = 0;                 // next used after two more barriers
@@ -2391,6 +2395,17 @@ static int sweep_group_max()
   return g;
 }
 
+// entries of the collision list in use (PCG_SWEEP_COLLISIONS overrides, for tests)
+static int sweep_collisions()
+{
+  static const int n = [] {
+    const char* e = getenv("PCG_SWEEP_COLLISIONS");
+    const int v = e ? atoi(e) : COLLISIONS;
+    return v < 0 ? 0 : (v > COLLISIONS ? COLLISIONS : v);
+  }();
+  return n;
+}
+
 // ---- checkpoint / resume of a sweep: the phi-offset totals run[b], the leaf
 // sums acc[b] and msum[b] after the last finished wave, with the problem and
 // a hash of the segment plan they belong to
@@ -2706,6 +2721,7 @@ SweepResult run_sweep(Ctx& c, const SweepProblem& pb, const Tuning& tune_in, cud
   a.factor = pb.gourdon ? c.tab.factor_d.p : c.tab.factor_dr.p;
   a.coprime = c.tab.coprime.as<uint16_t>();
   a.group_max = tune.group >= 0 ? std::min(tune.group, GROUP_MAX) : sweep_group_max();
+  a.collisions = sweep_collisions();
   a.cindex = c.tab.cindex.as<int16_t>();
   a.pmagic = c.tab.pmagic.as<uint64_t>();
   a.cnt = c.cnt.as<uint32_t>();
@@ -3084,6 +3100,7 @@ void run_sweep_batch(Ctx& c, const std::vector<SweepProblem>& pbs, const Tuning&
   a.factor = T.factor_d.p;
   a.coprime = T.coprime.as<uint16_t>();
   a.group_max = tune.group >= 0 ? std::min(tune.group, GROUP_MAX) : sweep_group_max();
+  a.collisions = sweep_collisions();
   a.cindex = T.cindex.as<int16_t>();
   a.pmagic = T.pmagic.as<uint64_t>();
   a.cnt = c.cnt.as<uint32_t>();
@@ -3367,6 +3384,7 @@ SweepResult run_sweep_noalloc(Ctx& c, const SweepProblem& pb, cudaStream_t s)
   a.factor = T.factor_d.p;
   a.coprime = T.coprime.as<uint16_t>();
   a.group_max = sweep_group_max();
+  a.collisions = sweep_collisions();
   a.cindex = T.cindex.as<int16_t>();
   a.pmagic = T.pmagic.as<uint64_t>();
   a.cnt = d_cnt;
