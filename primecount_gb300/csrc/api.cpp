@@ -190,7 +190,7 @@ uint64_t device_bytes(const Ctx& c)
   const Tables& t = c.tab;
   uint64_t b = t.primes.bytes + t.pitab.bytes + t.factor_d.bytes + t.factor_dr.bytes + t.coprime.bytes +
                t.cindex.bytes + t.pibig.bytes + t.pmagic.bytes + t.phi_bits.bytes + t.phi_pref.bytes + c.cnt.bytes +
-               c.smu.bytes + c.segsum.bytes + c.run.bytes + c.acc.bytes + c.misc.bytes + c.msum.bytes;
+               c.smu.bytes + c.segsum.bytes + c.run.bytes + c.acc.bytes + c.misc.bytes;
   for (const DevBuf& d : c.tmp) b += d.bytes;
   return b;
 }

@@ -218,7 +218,7 @@ struct Ctx {
   uint64_t mem_budget = 0;
   Tables tab;
   // scratch of the sweep (grown on demand)
-  DevBuf cnt, smu, segsum, run, acc, misc, msum;
+  DevBuf cnt, smu, segsum, run, acc, misc;
   // per-call temporaries, one slot per use site, kept and grown across calls
   // (no cudaMalloc / cudaFree per call: cudaFree synchronises the device and
   // would serialise the contexts of a worker pool)

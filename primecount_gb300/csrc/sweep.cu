@@ -429,7 +429,6 @@ struct SweepArgs {
   int64_t wave_first;    // first work item of the wave
   const int64_t* rowoff; // [wave_len]: first cell of the item's row in cnt / smu
   const uint32_t* primes;
-  int64_t nprimes;
   const uint64_t* pitab;
   int64_t pi_max;
   const void* factor;
@@ -2715,7 +2714,6 @@ SweepResult run_sweep(Ctx& c, const SweepProblem& pb, const Tuning& tune_in, cud
   a.rowoff = (const int64_t*) (d_in + at_row);
   a.words = words;
   a.primes = c.tab.primes.as<uint32_t>();
-  a.nprimes = c.tab.nprimes;
   a.pitab = c.tab.pitab.as<uint64_t>();
   a.pi_max = c.tab.prime_limit;
   a.factor = pb.gourdon ? c.tab.factor_d.p : c.tab.factor_dr.p;
@@ -2833,13 +2831,12 @@ uint64_t sweep_device_bytes(int num_sms, int64_t L, int64_t cols, int words)
 // rows, per-call temporaries), freed; the resident tables stay.
 uint64_t ctx_trim(Ctx& c)
 {
-  uint64_t freed = c.cnt.bytes + c.smu.bytes + c.segsum.bytes + c.run.bytes + c.acc.bytes + c.msum.bytes;
+  uint64_t freed = c.cnt.bytes + c.smu.bytes + c.segsum.bytes + c.run.bytes + c.acc.bytes;
   c.cnt.free_();
   c.smu.free_();
   c.segsum.free_();
   c.run.free_();
   c.acc.free_();
-  c.msum.free_();
   for (DevBuf& b : c.tmp) {
     freed += b.bytes;
     b.free_();
@@ -3094,7 +3091,6 @@ void run_sweep_batch(Ctx& c, const std::vector<SweepProblem>& pbs, const Tuning&
   a.nq = (int) qs.size();
   a.words = words;
   a.primes = T.primes.as<uint32_t>();
-  a.nprimes = T.nprimes;
   a.pitab = T.pitab.as<uint64_t>();
   a.pi_max = T.prime_limit;
   a.factor = T.factor_d.p;
@@ -3378,7 +3374,6 @@ SweepResult run_sweep_noalloc(Ctx& c, const SweepProblem& pb, cudaStream_t s)
   a.rowoff = d_row;
   a.words = words;
   a.primes = T.primes.as<uint32_t>();
-  a.nprimes = T.nprimes;
   a.pitab = T.pitab.as<uint64_t>();
   a.pi_max = T.prime_limit;
   a.factor = T.factor_d.p;
