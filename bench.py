@@ -16,8 +16,8 @@ roofline     the sieve/leaf kernel (k_sweep) against the measured HBM copy
              FactorTable entry read, 4 B per two-prime leaf (its prime),
              16 B per (segment, b) step (PiTable word of the level bounds),
              over its CUDA-event launch time.  traffic = DRAM bytes
-             per launch, scaled from the committed ncu capture of a smaller
-             D by the algorithmic bytes.  int_ops: algorithmic integer and
+             per launch, the mean over the committed one-pass ncu capture of
+             every k_sweep launch of one D(1e20).  int_ops: algorithmic integer and
              shared-memory operations (per leaf one division and one prefix
              query of a counter load and up to 8 popcounts; per cross-off
              one shared-memory read-modify-write) against the SMs' lane
@@ -490,8 +490,8 @@ def main():
                    "seconds_all": ts,
                    "terms_ms": {"D": s3["d_ms"], "AC": s3["ac_ms"], "B": s3["b_ms"], "Phi0": s3["phi0_ms"],
                                 "Sigma": s3["sigma_ms"], "tables": s3["table_ms"]},
-                   "terms_note": "a new context per call (tables built inside it); D runs beside A+C, B, Phi0 "
-                                 "and Sigma, so the term times are wall times of the two host threads"}
+                   "terms_note": "a new context per call (tables built inside it); D (host clock) runs beside "
+                                 "A+C, B, Phi0 and Sigma, which follow one another (the GPU's clock)"}
 
     batch = run_batch(args, pcg) if args.batch > 0 and rank == 0 else None
     serve = None
@@ -524,7 +524,6 @@ def main():
     # step (PiTable word of the level bounds); this implementation reads
     # nothing else per leaf
     alg_bytes = 2 * st["factor_entries"] + 4 * st["two_prime_leaves"] + 16 * st["levels"]
-    impl_bytes = 0
     k_ms_call = kernel_ms / args.steps
     launches_call = launches / args.steps
     launch_s = k_ms_call / launches_call / 1000.0
@@ -544,8 +543,6 @@ def main():
     roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
             "frac": achieved / peak, "traffic": traffic, "peak_kind": peak_kind,
             "kernel": "k_sweep", "alg_bytes_per_launch": alg_bytes / launches_call,
-            "impl_bytes_per_launch": impl_bytes / launches_call,
-            "impl_achieved_gbs": (alg_bytes + impl_bytes) / launches_call / launch_s / 1e9,
             "traffic_source": tr["source"] if tr else None,
             "launch_ms": k_ms_call / launches_call, "launches_per_step": launches_call,
             "int_ops": {"ops_per_launch": ops / launches_call, "ops_per_leaf": ops / max(st["leaves"], 1),

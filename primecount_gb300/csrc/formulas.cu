@@ -6,15 +6,18 @@
 // over the whole interval instead of the reference's segments:
 //   A, C1, C2   src/gourdon/AC.cpp:40-300 (sums of pi(x / (p q)) and
 //               pi(x / (p q r)) over primes; the PiTable up to sqrt(x) lives
-//               in HBM and every (p, q) pair is one thread)
+//               in HBM, the parts that most terms read in shared memory, a
+//               segment of n = x / (p q) at a time)
 //   B           src/gourdon/B.cpp:38-131 (sum of pi(x / p), y < p <= sqrt(x):
 //               a segmented prime sieve of [sqrt(x), x / y) whose segments
 //               are joined by the same offset scan as the hard leaves)
 //   Phi0        src/gourdon/Phi0.cpp:38-96 (mu(n) phi(x / n, k) over the
 //               FactorTableD entries)
-//   Sigma       src/gourdon/Sigma.cpp:25-140 (closed forms, on the host)
-// pi(x) for x <= 1e10 is a direct sieve count (the reference routes small x
-// to other algorithms, src/api.cpp:75-91).
+//   Sigma       src/gourdon/Sigma.cpp:25-140 (its sums on the device, the closed
+//               forms on the host)
+// pi(x) for x <= 1e10 is a direct sieve count, from 1.2e9 on only on a context
+// without the formula's tables (the reference routes small x to other
+// algorithms, src/api.cpp:75-91).
 #include <cstdio>
 #include <cstring>
 #include <chrono>
@@ -613,9 +616,12 @@ __global__ void __launch_bounds__(256) k_pairs(const PairOuter* __restrict__ out
 }
 
 // Launches the sum of the terms of nout outers, its blocks' partial sums in
-// T_PR_PART; returns their number.  While an outer has at most DIRECT_TERMS
-// terms (the whole prime table: x up to about 1e14) the outers go to k_pairs
-// as they are: listing pieces waits for their number, 60 us of a small pi(x).
+// T_PR_PART; returns their number.  While the context's prime table has at most
+// DIRECT_TERMS primes, which bounds the terms of an outer (a context made for x
+// up to about 1e14), the outers go to k_pairs as they are: listing pieces waits
+// for their number, 60 us of a small pi(x).  On a context made for a larger x a
+// small one lists pieces as well: pi(1e12) 0.26 ms on its own, 0.33 ms on one made
+// for 1e20, pi(1e13) 0.34 and 0.40, pi(1e14) 0.61 and 0.59, pi(1e15) the same.
 // Else PIECE_OUTERS outers at a time, which bounds the lists (about 100 pieces
 // an outer at 1e20).
 #define DIRECT_TERMS 65536
@@ -1875,9 +1881,11 @@ void pi_dr_terms(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, i128 out[7]
 }
 
 // x <= 1e10 is counted by the sieve directly, from GOURDON_MIN on only by a
-// context without the tables of Gourdon's formula: with them (a context made
-// for such x) the formula takes 0.3 ms where the sieve takes 0.3 ms at 1.2e9
-// and 2.4 ms at 1e10; building them takes 2 ms.
+// context without the tables of Gourdon's formula (building them takes 0.5 ms).
+// With them the formula takes 0.21, 0.15, 0.15 and 0.17 ms at 1.2e9, 2e9, 5e9 and
+// 1e10, the sieve 0.29, 0.43, 0.95 and 1.80 ms; the formula against the sieve was
+// checked from 1.2e9 on only, where the two took the same when the line was laid.
+// Below it the sieve takes 0.27 ms at 1e9, 0.11 ms at 3e8.
 static const int64_t PI_SIEVE_LIMIT = 10000000000ll;
 static const int64_t GOURDON_MIN = 1200000000ll;
 
@@ -1917,8 +1925,8 @@ i128 pi_any(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, pcg_stats* st)
   return r;
 }
 
-// pi(x) without Gourdon's D term (x > 1e10), or pi(x) itself (x <= 1e10,
-// counted by the sieve): *needs_d tells whether D must still be added
+// pi(x) without Gourdon's D term (x > 1e10), or pi(x) itself (x <= 1e10):
+// *needs_d tells whether D must still be added
 i128 pi_without_d(Ctx& c, u128 x, const Tuning& tune, cudaStream_t s, bool* needs_d)
 {
   if (x <= (u128) PI_SIEVE_LIMIT) {
